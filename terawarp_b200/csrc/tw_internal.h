@@ -130,8 +130,9 @@ tw_status solve_status(tw_ctx *ctx, const int *d_status, cudaStream_t st);
 tw_status fit_affine_device(tw_ctx *ctx, const double *h_tar, const double *h_sub, int n, double M[16],
                             cudaStream_t st);
 // The affine fit kernel alone on caller-provided device buffers (d_status
-// must hold 0 when it starts; the kernel only sets failure bits).
-cudaError_t launch_affine_fit(const double *d_tar, const double *d_sub, int n, double *d_out, int *d_status,
+// must hold 0 when it starts; the kernel only sets failure bits; d_tar and
+// d_sub are normalised in place).
+cudaError_t launch_affine_fit(double *d_tar, double *d_sub, int n, double *d_out, int *d_status,
                               cudaStream_t st);
 
 // --------------------------------------------------------------- helpers

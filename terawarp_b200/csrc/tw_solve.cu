@@ -818,110 +818,343 @@ __global__ void k_eval_arrays(int n, const double *ctr, const double *C, double 
 }
 
 // ----------------------------------------------------------- affine DLT
+//
+// One CTA.  The fit is a serial chain -- the cyclic Jacobi iteration's angles,
+// each two square roots and three divisions after the one before -- so its
+// time is latency.  One thread doing every rotation, with the 39 element
+// pairs of each in a loop, took 580 of the kernel's 622 us at 16 pairs of
+// landmarks (8 sweeps).  Here the operations on every matrix element are the
+// same and in the same order, but spread over a wavefront:
+//  - the angle of rotation (p, q) needs only the elements of rows and columns
+//    p and q against each other, so (p, q) runs at step 2p + q of the sweep, 34
+//    steps instead of 78, up to four rotations a step, one warp each;
+//  - a rotation is applied at once to the indices p < k <= q + 1, to a later
+//    index k just before (p, k) needs it (by a second warp, while the angles of
+//    that step are computed), and to the indices k < p at the end of the sweep:
+//    no angle of the same sweep reads those;
+//  - the eigenvector matrix follows one sweep behind, on a warp of its own.
+// Every element so meets its rotations in the sequential order, and the matrix
+// is the same to the last bit.  Four warps compute angles, four catch up, one
+// keeps the vectors (one angle warp per SM sub-partition; 16 warps made every
+// barrier dearer and left too few registers for the rows).  169 us at 16 pairs:
+// 110 of them are the 34 x 7 angles' own square roots and divisions.
 
-__global__ void k_affine_fit(const double *tar, const double *sub, int n, double *out, int *status)
+constexpr int kFitRed = 256;                        // threads that hold landmarks in the sums
+constexpr int kFitAgents = 4;                       // warps computing angles: p and p + 4 are never active together
+constexpr int kFitThreads = 32 * (2 * kFitAgents + 1);  // + as many catch-up warps + the eigenvector warp
+constexpr int kFitDim = 13;
+constexpr int kFitUpper = kFitDim * (kFitDim + 1) / 2;  // entries of the normal matrix
+
+struct FitSmem {
+    double sh[6][kFitRed / 32];
+    double part[kFitRed / 32][kFitUpper];
+    double A[kFitDim][kFitDim], V[kFitDim][kFitDim];
+    double2 R[2][kFitDim - 1][kFitDim];             // (cos, sin) of rotation (p, q), this sweep's and the last one's
+    double one;                                     // 1.0, the homogeneous coordinate of every point
+    int go;
+};
+
+// N sums over the first kFitRed threads' values (the others pass zeros): a
+// tree inside each warp, then the warps in order.
+template <int N>
+__device__ __forceinline__ void fit_sums(double (&v)[N], FitSmem &S)
 {
-    __shared__ double sh[32];
-    __shared__ double ata[13][13];
-    __shared__ double nrm[2][4];  // scale, cx, cy, cz for A (tar) and B (sub)
-    for (int s = 0; s < 2; ++s) {
-        const double *p = s == 0 ? tar : sub;
-        double cx = 0, cy = 0, cz = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) { cx += p[3 * i]; cy += p[3 * i + 1]; cz += p[3 * i + 2]; }
-        cx = block_sum(cx, sh) / n;
-        cy = block_sum(cy, sh) / n;
-        cz = block_sum(cz, sh) / n;
-        double dsum = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            double dx = p[3 * i] - cx, dy = p[3 * i + 1] - cy, dz = p[3 * i + 2] - cz;
-            dsum += sqrt(dx * dx + dy * dy + dz * dz);
-        }
-        dsum = block_sum(dsum, sh) / n;
-        if (threadIdx.x == 0) { nrm[s][0] = 1.0 / dsum; nrm[s][1] = cx; nrm[s][2] = cy; nrm[s][3] = cz; }
-        __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+    if (lane == 0 && warp < kFitRed / 32)
+#pragma unroll
+        for (int i = 0; i < N; ++i) S.sh[i][warp] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kFitRed / 32; ++w) t += S.sh[i][w];
+        v[i] = t;
     }
-    // normal matrix of the 3n x 13 DLT system, row block per point:
-    // [a 1 0 0 -bx], [0 a 1 0 -by], [0 0 a 1 -bz] with a = (ax, ay, az)
-    for (int e = 0; e < 169; ++e) {
-        const int r = e / 13, c = e % 13;
-        if (c < r) continue;
-        double acc = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            double a[3], b[3];
-            for (int q = 0; q < 3; ++q) {
-                a[q] = (tar[3 * i + q] - nrm[0][1 + q]) * nrm[0][0];
-                b[q] = (sub[3 * i + q] - nrm[1][1 + q]) * nrm[1][0];
+}
+
+// The angle of the rotation that zeroes apq; kFitSkip when it is zero already.
+constexpr double kFitSkip = 2.0;  // in place of a cosine: the rotation is left out
+__device__ __forceinline__ double2 fit_angle(double app, double aqq, double apq)
+{
+    if (fabs(apq) < 1e-300) return make_double2(kFitSkip, 0.0);
+    const double theta = (aqq - app) / (2.0 * apq);
+    const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(fma(theta, theta, 1.0)));
+    const double cs = 1.0 / sqrt(fma(t, t, 1.0));
+    return make_double2(cs, t * cs);
+}
+
+__device__ __forceinline__ bool fit_used(double2 r) { return __double2hiint(r.x) != 0x40000000; }
+
+__device__ __forceinline__ void fit_rot(double &x, double &y, double2 r)
+{
+    const double a = x, b = y;
+    x = fma(r.x, a, -__dmul_rn(r.y, b));
+    y = fma(r.y, a, __dmul_rn(r.x, b));
+}
+
+// The same where `on`, without a branch: a chain of these stays a chain of
+// multiply-adds.
+__device__ __forceinline__ void fit_rot_if(double &x, double &y, double2 r, bool on)
+{
+    double a = x, b = y;
+    fit_rot(a, b, r);
+    x = on ? a : x;
+    y = on ? b : y;
+}
+
+// Rotations (p, q), p < q < qe, in order, on the pairs (row[p], row[q]) of a
+// row or column with element stride `st`; the loads come first, so that only
+// the chain through row[p] is serial.
+__device__ __forceinline__ void fit_catch_up(double *row, int st, int p, int qe, const double2 *R)
+{
+    constexpr int kMost = kFitDim - 3;
+    double x = row[p * st], y[kMost];
+    double2 r[kMost];
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+        const int q = min(p + 1 + j, kFitDim - 1);
+        y[j] = row[q * st];
+        r[j] = R[q];
+    }
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) fit_rot_if(x, y[j], r[j], p + 1 + j < qe && fit_used(r[j]));
+#pragma unroll
+    for (int j = 0; j < kMost; ++j)
+        if (p + 1 + j < qe) row[(p + 1 + j) * st] = y[j];
+    row[p * st] = x;
+}
+
+// All rotations of a sweep with p >= p0 (p0 uniform or not), in order, on one
+// row or column with element stride `st`, held in registers.
+__device__ __forceinline__ void fit_replay(double *row, int st, int p0, const double2 (*R)[kFitDim])
+{
+    double v[kFitDim];
+#pragma unroll
+    for (int k = 0; k < kFitDim; ++k) v[k] = row[k * st];
+#pragma unroll
+    for (int p = 0; p < kFitDim - 1; ++p)
+#pragma unroll
+        for (int q = p + 1; q < kFitDim; ++q) {
+            const double2 r = R[p][q];
+            fit_rot_if(v[p], v[q], r, p >= p0 && fit_used(r));
+        }
+#pragma unroll
+    for (int k = 0; k < kFitDim; ++k) row[k * st] = v[k];
+}
+
+// One sweep on A (warps 0 .. 2 kFitAgents - 1); R / skip get its rotations.
+__device__ __forceinline__ void fit_sweep(FitSmem &S, double2 (*R)[kFitDim])
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int agent = warp % kFitAgents;
+    const bool angles = warp < kFitAgents;
+    for (int s = 1; s <= 2 * (kFitDim - 2) + kFitDim - 1; ++s) {
+        // the agent's rotation of this step: (p, s - 2p) with p < s - 2p < kFitDim
+        int p = agent;
+        while (s - 2 * p >= kFitDim) p += kFitAgents;
+        const int q = s - 2 * p;
+        const bool on = p < kFitDim - 1 && q > p && q < kFitDim;
+        double2 r = make_double2(kFitSkip, 0.0);
+        double app = 0, aqq = 0, apq = 0, aqp = 0;
+        if (on && angles) {
+            app = S.A[p][p];
+            aqq = S.A[q][q];
+            apq = S.A[p][q];
+            aqp = S.A[q][p];
+            r = fit_angle(app, aqq, apq);
+            if (lane == 0) R[p][q] = r;
+        } else if (on && q + 1 < kFitDim && q > p + 1 && (lane & 15) == 0) {
+            const int k = q + 1;
+            fit_catch_up(lane == 0 ? &S.A[k][0] : &S.A[0][k], lane == 0 ? 1 : kFitDim, p, q, R[p]);
+        }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(64 * kFitAgents) : "memory");
+        if (on && angles && fit_used(r)) {
+            const int k = lane & 15;
+            const bool mine = k > p && k <= q + 1 && k < kFitDim && k != q;
+            const int kk = mine ? k : p;
+            double *x = lane < 16 ? &S.A[kk][p] : &S.A[p][kk];
+            double *y = lane < 16 ? &S.A[kk][q] : &S.A[q][kk];
+            double u = *x, v = *y;
+            fit_rot(u, v, r);
+            // the rotation's own 2 x 2 block: columns, then rows
+            fit_rot(app, apq, r);
+            fit_rot(aqp, aqq, r);
+            fit_rot(app, aqp, r);
+            fit_rot(apq, aqq, r);
+            __syncwarp();
+            if (mine) {
+                *x = u;
+                *y = v;
             }
-            for (int rb = 0; rb < 3; ++rb) {
-                double row[13] = {0};
-                row[rb * 4 + 0] = a[0]; row[rb * 4 + 1] = a[1]; row[rb * 4 + 2] = a[2]; row[rb * 4 + 3] = 1.0;
-                row[12] = -b[rb];
-                acc += row[r] * row[c];
+            if (lane == 0) {
+                S.A[p][p] = app;
+                S.A[p][q] = apq;
+                S.A[q][p] = aqp;
+                S.A[q][q] = aqq;
             }
         }
-        acc = block_sum(acc, sh);
-        if (threadIdx.x == 0) { ata[r][c] = acc; ata[c][r] = acc; }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(64 * kFitAgents) : "memory");
+    }
+    // the indices below each rotation's p
+    if (warp == 0) {
+        const int k = lane & 15;
+        if (k < kFitDim - 2) fit_replay(lane < 16 ? &S.A[k][0] : &S.A[0][k], lane < 16 ? 1 : kFitDim, k + 1, R);
+    }
+}
+
+__device__ __forceinline__ void fit_vectors(FitSmem &S, int buf)
+{
+    const int k = threadIdx.x & 31;
+    if (k < kFitDim) fit_replay(&S.V[k][0], 1, 0, S.R[buf]);
+}
+
+// tar and sub are the call's own copies and are normalised in place.
+__global__ void __launch_bounds__(kFitThreads) k_affine_fit(double *tar, double *sub, int n, double *out, int *status)
+{
+    __shared__ FitSmem S;
+    const int tid = threadIdx.x;
+    const int i0 = tid < kFitRed ? tid : n;  // threads past kFitRed hold no landmark
+    // Hartley normalisation of both sets (0: tar, 1: sub): centroid, 1 / mean distance
+    double c[6] = {0, 0, 0, 0, 0, 0}, scale[2] = {0, 0};
+    for (int i = i0; i < n; i += kFitRed)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            c[q] += tar[3 * i + q];
+            c[3 + q] += sub[3 * i + q];
+        }
+    if (tid == 0) S.one = 1.0;
+    fit_sums(c, S);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) c[q] /= n;
+    for (int i = i0; i < n; i += kFitRed)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const double *p = s == 0 ? tar : sub;
+            const double dx = p[3 * i] - c[3 * s], dy = p[3 * i + 1] - c[3 * s + 1], dz = p[3 * i + 2] - c[3 * s + 2];
+            scale[s] += sqrt(fma(dz, dz, fma(dx, dx, __dmul_rn(dy, dy))));
+        }
+    fit_sums(scale, S);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) scale[s] = 1.0 / (scale[s] / n);
+    for (int i = i0; i < n; i += kFitRed)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            tar[3 * i + q] = (tar[3 * i + q] - c[q]) * scale[0];
+            sub[3 * i + q] = (sub[3 * i + q] - c[3 + q]) * scale[1];
+        }
+    __syncthreads();
+    // normal matrix of the 3n x 13 DLT system, three rows per point,
+    // [a 1 0 0 -bx], [0 a 1 0 -by], [0 0 a 1 -bz] with a = (ax, ay, az): one
+    // thread per entry (r, c) and warp's share of the points, summed as the
+    // lanes of that warp would (products with a zero add nothing)
+    const int nw = min(kFitRed / 32, (n + 31) / 32);
+    for (int t = tid; t < kFitUpper * nw; t += kFitThreads) {
+        const int e = t % kFitUpper, w = t / kFitUpper;
+        int r = 0, f = e;
+        while (f >= kFitDim - r) {
+            f -= kFitDim - r;
+            ++r;
+        }
+        const int cc = r + f;
+        double v[32];
+#pragma unroll
+        for (int l = 0; l < 32; ++l) v[l] = 0.0;
+        if (cc == 12 || r / 4 == cc / 4) {
+            // the entry's factors: element k of a (1 for k = 3), or -b[k]
+            const bool bu = r == 12, bv = cc == 12;
+            const int kv = r / 4 % 3;  // of -b, for r < 12
+            const double *pu = bu ? sub : (r % 4 == 3 ? &S.one : tar + r % 4);
+            const double *pv = bv ? sub + (bu ? 0 : kv) : (cc % 4 == 3 ? &S.one : tar + cc % 4);
+            const int su = !bu && r % 4 == 3 ? 0 : 3, sv = !bv && cc % 4 == 3 ? 0 : 3;
+            const double sg = bv && !bu ? -1.0 : 1.0;
+            for (int b = 32 * w; b < n; b += kFitRed) {
+#pragma unroll
+                for (int l = 0; l < 32; ++l) {
+                    const int i = min(b + l, n - 1);
+                    const double x = pu[i * su], y = sg * pv[i * sv];
+                    double t = fma(x, y, v[l]);
+                    if (bu) {
+                        t = fma(pu[i * 3 + 1], pv[i * 3 + 1], t);
+                        t = fma(pu[i * 3 + 2], pv[i * 3 + 2], t);
+                    }
+                    if (b + l < n) v[l] = t;
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int l = 0; l < o; ++l) v[l] += v[l + o];
+        S.part[w][e] = v[0];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double Vm[13][13];
-        for (int i = 0; i < 13; ++i)
-            for (int j = 0; j < 13; ++j) Vm[i][j] = i == j ? 1.0 : 0.0;
-        for (int sweep = 0; sweep < 100; ++sweep) {
-            double off = 0, diag = 0;
-            for (int p = 0; p < 13; ++p) {
-                diag += ata[p][p] * ata[p][p];
-                for (int q = p + 1; q < 13; ++q) off += ata[p][q] * ata[p][q];
-            }
-            if (off <= 1e-30 * diag) break;
-            for (int p = 0; p < 12; ++p)
-                for (int q = p + 1; q < 13; ++q) {
-                    double apq = ata[p][q];
-                    if (fabs(apq) < 1e-300) continue;
-                    double theta = (ata[q][q] - ata[p][p]) / (2.0 * apq);
-                    double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-                    double cs = 1.0 / sqrt(t * t + 1.0), sn = t * cs;
-                    for (int k = 0; k < 13; ++k) {
-                        double akp = ata[k][p], akq = ata[k][q];
-                        ata[k][p] = cs * akp - sn * akq;
-                        ata[k][q] = sn * akp + cs * akq;
-                    }
-                    for (int k = 0; k < 13; ++k) {
-                        double apk = ata[p][k], aqk = ata[q][k];
-                        ata[p][k] = cs * apk - sn * aqk;
-                        ata[q][k] = sn * apk + cs * aqk;
-                    }
-                    for (int k = 0; k < 13; ++k) {
-                        double vkp = Vm[k][p], vkq = Vm[k][q];
-                        Vm[k][p] = cs * vkp - sn * vkq;
-                        Vm[k][q] = sn * vkp + cs * vkq;
-                    }
-                }
+    if (tid < kFitUpper) {
+        int r = 0, f = tid;
+        while (f >= kFitDim - r) {
+            f -= kFitDim - r;
+            ++r;
         }
+        double acc = 0.0;
+        for (int w = 0; w < nw; ++w) acc += S.part[w][tid];
+        S.A[r][r + f] = acc;
+        S.A[r + f][r] = acc;
+    }
+    for (int e = tid; e < kFitDim * kFitDim; e += kFitThreads) S.V[e / kFitDim][e % kFitDim] = e % (kFitDim + 1) == 0 ? 1.0 : 0.0;
+    __syncthreads();
+    const int warp = tid >> 5;
+    int sweep = 0;
+    for (; sweep < 100; ++sweep) {
+        if (tid == 0) {
+            double off = 0, diag = 0;
+#pragma unroll
+            for (int p = 0; p < kFitDim; ++p) {
+                diag += S.A[p][p] * S.A[p][p];
+#pragma unroll
+                for (int q = p + 1; q < kFitDim; ++q) off += S.A[p][q] * S.A[p][q];
+            }
+            S.go = !(off <= 1e-30 * diag);
+        }
+        __syncthreads();
+        if (!S.go) break;
+        if (warp < 2 * kFitAgents) fit_sweep(S, S.R[sweep & 1]);
+        else if (sweep > 0) fit_vectors(S, (sweep - 1) & 1);
+        __syncthreads();
+    }
+    if (warp == 2 * kFitAgents && sweep > 0) fit_vectors(S, (sweep - 1) & 1);
+    __syncthreads();
+    if (tid == 0) {
         int best = 0;
-        for (int p = 1; p < 13; ++p)
-            if (ata[p][p] < ata[best][best]) best = p;
-        double h[13];
-        for (int i = 0; i < 13; ++i) h[i] = Vm[i][best];
+        for (int p = 1; p < kFitDim; ++p)
+            if (S.A[p][p] < S.A[best][best]) best = p;
+        double h[kFitDim];
+        for (int i = 0; i < kFitDim; ++i) h[i] = S.V[i][best];
         if (h[12] == 0.0) {
             atomicOr(status, kStSingularX);
             return;
         }
-        for (int i = 0; i < 13; ++i) h[i] /= h[12];
+        for (int i = 0; i < kFitDim; ++i) h[i] /= h[12];
         // T = NB^-1 H NA with N = [s I, -s c; 0 1]:  NB^-1 = [I/sB, cB; 0 1]
-        const double sA = nrm[0][0], sB = nrm[1][0];
+        const double sA = scale[0], sB = scale[1];
         double H[3][4];
         for (int r = 0; r < 3; ++r)
-            for (int c = 0; c < 4; ++c) H[r][c] = h[r * 4 + c];
+            for (int k = 0; k < 4; ++k) H[r][k] = h[r * 4 + k];
         for (int r = 0; r < 3; ++r) {
             // (H NA)(r,:) = [sA H(r,0:3), H(r,3) - sA H(r,0:3).cA]
             double lin[3], tr = H[r][3];
-            for (int c = 0; c < 3; ++c) {
-                lin[c] = sA * H[r][c];
-                tr -= sA * H[r][c] * nrm[0][1 + c];
+            for (int k = 0; k < 3; ++k) {
+                lin[k] = sA * H[r][k];
+                tr = fma(-lin[k], c[k], tr);
             }
-            for (int c = 0; c < 3; ++c) out[r * 4 + c] = lin[c] / sB;
-            out[r * 4 + 3] = tr / sB + nrm[1][1 + r];
+            for (int k = 0; k < 3; ++k) out[r * 4 + k] = lin[k] / sB;
+            out[r * 4 + 3] = tr / sB + c[3 + r];
         }
         out[12] = 0; out[13] = 0; out[14] = 0; out[15] = 1;
     }
@@ -1065,7 +1298,7 @@ tw_status fit_affine_device(tw_ctx *ctx, const double *h_tar, const double *h_su
     TW_CUDA_TRY(cudaMemcpyAsync(d_tar, h_tar, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
     TW_CUDA_TRY(cudaMemcpyAsync(d_sub, h_sub, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
     TW_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));
-    k_affine_fit<<<1, 256, 0, st>>>(d_tar, d_sub, n, d_out, d_status);
+    k_affine_fit<<<1, kFitThreads, 0, st>>>(d_tar, d_sub, n, d_out, d_status);
     TW_CUDA_TRY(cudaGetLastError());
     count_launch(ctx, 1);
     int status = 0;
@@ -1076,10 +1309,10 @@ tw_status fit_affine_device(tw_ctx *ctx, const double *h_tar, const double *h_su
     return TW_OK;
 }
 
-cudaError_t launch_affine_fit(const double *d_tar, const double *d_sub, int n, double *d_out, int *d_status,
+cudaError_t launch_affine_fit(double *d_tar, double *d_sub, int n, double *d_out, int *d_status,
                               cudaStream_t st)
 {
-    k_affine_fit<<<1, 256, 0, st>>>(d_tar, d_sub, n, d_out, d_status);
+    k_affine_fit<<<1, kFitThreads, 0, st>>>(d_tar, d_sub, n, d_out, d_status);
     return cudaGetLastError();
 }
 
