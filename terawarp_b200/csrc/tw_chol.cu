@@ -1,0 +1,1086 @@
+// tw_chol.cu -- the FP64 Cholesky factorisation and the two triangular solves
+// of the projected TPS system, one cooperative kernel.
+//
+// A (m x m, symmetric positive definite) is held as 64 x 64 tiles of its lower
+// triangle, each stored with a row pitch of 66 doubles: a tile is one
+// contiguous 33,792-byte block that a single bulk copy moves between global
+// and shared memory, already in the layout whose 16-byte row loads are free of
+// bank conflicts.  Column 64 of a factored diagonal tile holds the reciprocals
+// of its diagonal and its upper triangle the transpose of the lower, so the
+// panel solves read both along rows.  The four right-hand sides are an extra
+// row block of 4 x 66 tiles, so the forward substitution is part of the
+// factorisation; the back substitution overwrites the same tiles.
+//
+// Roles.  CTA 0 runs the critical chain POTRF(k-1) -> TRSM(k, k-1) ->
+// SYRK(k, k, k-1) -> POTRF(k) with its tiles in shared memory and registers.
+// The other CTAs take tiles in column order from a counter; a tile's owner
+// holds it in registers, subtracts L(i,k) L(j,k)' for k = 0, 1, ... as the
+// panels become available (each product summed over its 64 columns first,
+// then subtracted), solves it against the factored diagonal tile and
+// publishes it.  The tiles (j, j) and (j+1, j) go to the chain instead, one
+// update and the solve short.  A task waits only for the chain and for tasks
+// before it in the order, and every CTA is resident (cooperative launch), so
+// the lowest unfinished task can always run.
+//
+// In each CTA 8 warps compute, one warp fetches tiles ahead of them (bulk
+// copies into a ring of shared-memory buffers, after the flag that publishes
+// each tile) and one warp stores results and publishes them, so neither a
+// flag's round trip nor a store's completion stands on the compute warps'
+// path.  What bounds it: the chain's latency up to about 3000 landmarks (per
+// 64 columns 16 dependent pivots x 4: reciprocal square root, multiply,
+// multiply-add, shuffle), the FP64 pipe beyond.
+//
+// Every element sees the operations of the plain right-looking tiled
+// factorisation in the same order, whatever the schedule.
+//
+// Every wait is bounded: a wait that gives up sets the error flag, and from
+// then on no wait of any CTA blocks, so every CTA runs to its end (indices do
+// not depend on data) and the host reports the time-out.
+
+#include "tw_internal.h"
+#include "tw_kdist.h"
+
+namespace tw {
+
+namespace {
+
+constexpr int kNB = 64;                        // tile
+constexpr int kTP = 66;                        // tile row pitch, doubles
+constexpr int kTileD = kNB * kTP;              // doubles of a tile
+constexpr uint32_t kTileB = kTileD * 8;        // bytes
+constexpr int kRhsD = 4 * kTP;                 // a right-hand-side tile
+constexpr uint32_t kRhsB = kRhsD * 8;
+constexpr int kCompute = 256;                  // compute threads
+constexpr int kThreads = kCompute + 64;        // + the fetching warp + the publishing warp
+constexpr int kFetchWarp = kCompute / 32, kPublishWarp = kFetchWarp + 1;
+constexpr int kBufs = 6;                       // tile buffers in shared memory
+
+// status word bits
+constexpr int kStNotSPD = 2;
+constexpr int kStTimeout = 4;
+
+static_assert(kTileB % 16 == 0 && kRhsB % 16 == 0, "bulk copies move multiples of 16 bytes");
+
+// Flags (zeroed before the launch).  tdone[i]: panel tiles of row block i that
+// are final (row block nblk: the right-hand sides); pre_d[j], pre_s[j]: tile
+// (j, j) / (j+1, j) has been handed to the chain; bcnt[i]: block i of the right-hand sides has
+// been handed to the chain's back substitution.
+struct Flags {
+    int err;    // a wait gave up
+    int pdone;  // diagonal tiles factored
+    int ddone;  // back-substitution blocks solved, from the last one down
+    int next;   // tasks claimed
+};
+
+struct Ctl {
+    double *tiles;  // lower-triangle tiles, column after column
+    double *rhs;    // nblk tiles of 4 x 66
+    double *x;      // the solution, 4 per row (rows 0 .. m-1)
+    int m, nblk;
+    int *status;
+    Flags *F;
+    int *tdone, *pre_d, *pre_s, *bcnt;
+    unsigned long long limit_ns;
+};
+
+__device__ __forceinline__ size_t tile_index(int i, int j, int nblk)
+{
+    return (size_t)j * nblk - (size_t)j * (j - 1) / 2 + (i - j);
+}
+__device__ __forceinline__ double *tile_ptr(const Ctl &C, int i, int j)
+{
+    return C.tiles + tile_index(i, j, C.nblk) * kTileD;
+}
+
+struct Smem {
+    double buf[kBufs][kTileD];
+    double z[4][kRhsD];        // back substitution: right-hand sides of the blocks in flight (block & 3)
+    double xs[4][kRhsD];       // and their solutions
+    double small[kRhsD];       // helpers: right-hand-side tile of a panel / x of a block
+    unsigned long long full[kBufs], empty[kBufs];
+    unsigned long long zfull[4];
+    unsigned long long post[2], freed[2];  // results handed to the publishing warp / their buffers read
+    unsigned long long xdone;
+    // a result to publish: shared source, global destination, bytes, flag and its value
+    struct Mail {
+        const double *src;
+        double *dst;
+        uint32_t bytes;
+        int *flag;
+        int value;
+    } mail[2];
+    uint32_t issued[kBufs], zissued[4];  // copies begun into each buffer (fetching warp)
+    int task;
+    int abort;
+};
+
+// ------------------------------------------------------------ small helpers
+
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ int ld_acquire(const int *p)
+{
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(int *p, int v)
+{
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+__device__ __forceinline__ void bar_init(unsigned long long *b, uint32_t n)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(b)), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned long long *b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned long long *b, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_try(unsigned long long *b, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(saddr(b)), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void bulk_copy(double *dst, const double *src, uint32_t bytes, unsigned long long *b)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(saddr(dst)),
+                 "l"(src), "r"(bytes), "r"(saddr(b))
+                 : "memory");
+}
+// One tile into buffer b, counted on its "full" barrier.
+__device__ __forceinline__ void load_buf(Smem &S, int b, const double *src, uint32_t bytes)
+{
+    ++S.issued[b];
+    bar_expect(&S.full[b], bytes);
+    bulk_copy(S.buf[b], src, bytes, &S.full[b]);
+}
+// barrier of the compute warps
+__device__ __forceinline__ void sync_compute()
+{
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(kCompute) : "memory");
+}
+
+__device__ __noinline__ void give_up(const Ctl &C, Smem &S)
+{
+    atomicOr(&C.F->err, 1);
+    atomicOr(C.status, kStTimeout);
+    *reinterpret_cast<volatile int *>(&S.abort) = 1;
+}
+
+__device__ __noinline__ void bar_wait_slow(const Ctl &C, Smem &S, unsigned long long *b, uint32_t parity)
+{
+    const unsigned long long t0 = now_ns();
+    for (unsigned i = 1;; ++i) {
+        if (bar_try(b, parity) || *reinterpret_cast<volatile int *>(&S.abort)) return;
+        if ((i & 15u) == 0 && now_ns() - t0 > C.limit_ns) {
+            give_up(C, S);
+            return;
+        }
+    }
+}
+// The n-th completion of the mbarrier (n counts from 0).  Returns at once
+// when the CTA has given up.
+__device__ __forceinline__ void bar_wait(const Ctl &C, Smem &S, unsigned long long *b, uint32_t n)
+{
+    if (!bar_try(b, n & 1u)) bar_wait_slow(C, S, b, n & 1u);
+}
+// A buffer's n-th reuse: the (n-1)-th release has happened (n = 0: it is free).
+__device__ __forceinline__ void bar_wait_free(const Ctl &C, Smem &S, unsigned long long *b, uint32_t n)
+{
+    if (n > 0) bar_wait(C, S, b, n - 1);
+}
+
+// Waits (one thread) until *flag >= want; false once anyone has given up.
+__device__ bool flag_wait(const Ctl &C, Smem &S, const int *flag, int want)
+{
+    if (ld_acquire(flag) >= want) return *reinterpret_cast<volatile int *>(&S.abort) == 0;
+    const unsigned long long t0 = now_ns();
+    for (;;) {
+        if (ld_acquire(flag) >= want) return *reinterpret_cast<volatile int *>(&S.abort) == 0;
+        if (*reinterpret_cast<volatile int *>(&S.abort)) return false;
+        if (*reinterpret_cast<volatile int *>(&C.F->err) || now_ns() - t0 > C.limit_ns) {
+            give_up(C, S);
+            return false;
+        }
+    }
+}
+
+// Hands a result in shared memory to the publishing warp (every compute
+// thread calls it after its last write; thread 0 describes the result).
+__device__ __forceinline__ void post(Smem &S, int b, const double *src, double *dst, uint32_t bytes, int *flag, int value)
+{
+    fence_async();
+    if (threadIdx.x == 0) S.mail[b] = {src, dst, bytes, flag, value};
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) bar_arrive(&S.post[b]);
+}
+
+// The publishing warp's lane 0: stores the n-th result of mailbox b and
+// raises its flag; false at the end.
+__device__ bool publish(const Ctl &C, Smem &S, int b, uint32_t n)
+{
+    bar_wait(C, S, &S.post[b], n);
+    if (*reinterpret_cast<volatile int *>(&S.abort)) return false;
+    const Smem::Mail M = S.mail[b];
+    if (!M.flag) return false;
+    if (M.bytes) {
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(M.dst), "r"(saddr(M.src)), "r"(M.bytes)
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+    bar_arrive(&S.freed[b]);
+    if (M.bytes) {
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        fence_async();
+    }
+    __threadfence();
+    st_release(M.flag, M.value);
+    return true;
+}
+
+// ------------------------------------------------------------- tile kernels
+//
+// Compute thread t owns the elements (tr + 16u, tc + 16v) of a tile, tr = t / 16,
+// tc = t % 16: two rows of a warp's operand loads are broadcast, the other
+// operand's 16 rows are conflict-free 16-byte loads.
+
+// acc[u][v] = sum over the 64 columns, in order, of Li(tr + 16u, .) Lj(tc + 16v, .);
+// DIAG: only v <= u.
+template <bool DIAG>
+__device__ __forceinline__ void tile_product(const double *__restrict__ Li, const double *__restrict__ Lj, double (&acc)[4][4])
+{
+    const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
+#pragma unroll 4
+    for (int p = 0; p < kNB; p += 2) {
+        double2 a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            a[u] = *reinterpret_cast<const double2 *>(Li + (tr + 16 * u) * kTP + p);
+            b[u] = *reinterpret_cast<const double2 *>(Lj + (tc + 16 * u) * kTP + p);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if (!DIAG || v <= u) acc[u][v] = fma(a[u].x, b[v].x, acc[u][v]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                if (!DIAG || v <= u) acc[u][v] = fma(a[u].y, b[v].y, acc[u][v]);
+    }
+}
+
+// Solves one row's 16 columns x (shared memory) against the 16 x 16 diagonal
+// block at D (its transpose in the upper triangle, reciprocals at rd, pitch
+// kTP): one thread per row, everything in registers, so a column costs a
+// multiply and a multiply-add of latency instead of a shuffle between lanes.
+__device__ __forceinline__ void solve_row16(double *x, const double *D, const double *rd)
+{
+    double v[16], r[16];
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) {
+        const double2 t = *reinterpret_cast<const double2 *>(x + k);
+        v[k] = t.x;
+        v[k + 1] = t.y;
+    }
+#pragma unroll
+    for (int c = 0; c < 16; ++c) r[c] = rd[c * kTP];
+    double2 l[8], ln[8];  // row c of the transpose, and the next one on its way
+#pragma unroll
+    for (int k = 0; k < 8; ++k) l[k] = *reinterpret_cast<const double2 *>(D + 2 * k);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+#pragma unroll
+        for (int k = (c + 2) >> 1; k < 8; ++k) ln[k] = *reinterpret_cast<const double2 *>(D + (c + 1) * kTP + 2 * k);
+        v[c] = v[c] * r[c];
+#pragma unroll
+        for (int k = (c + 1) >> 1; k < 8; ++k) {
+            if (2 * k > c) v[2 * k] = fma(-v[c], l[k].x, v[2 * k]);
+            v[2 * k + 1] = fma(-v[c], l[k].y, v[2 * k + 1]);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) l[k] = ln[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) *reinterpret_cast<double2 *>(x + k) = make_double2(v[k], v[k + 1]);
+}
+
+// X = X L^-T for the tile held in registers (a), L a factored diagonal tile;
+// the result goes to Xs.  With SYRK also acc = X X' (lower part), summed over
+// the columns in order.  In four 16-column panels: the panel is solved row by
+// row, then subtracted from the later columns.
+template <bool SYRK>
+__device__ __forceinline__ void tile_solve(double (&a)[4][4], const double *__restrict__ L, double *__restrict__ Xs,
+                                           double (&acc)[4][4])
+{
+    const int t = threadIdx.x, tr = t >> 4, tc = t & 15;
+    if (SYRK) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const int c0 = 16 * v;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) Xs[(tr + 16 * u) * kTP + c0 + tc] = a[u][v];
+        sync_compute();
+        if (t < kNB) solve_row16(Xs + t * kTP + c0, L + c0 * kTP + c0, L + c0 * kTP + kNB);
+        sync_compute();
+        if (v < 3 || SYRK) {
+#pragma unroll 4
+            for (int p = c0; p < c0 + 16; p += 2) {
+                double2 x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const double2 *>(Xs + (tr + 16 * u) * kTP + p);
+#pragma unroll
+                for (int w = v + 1; w < 4; ++w) {
+                    const double2 l = *reinterpret_cast<const double2 *>(L + (tc + 16 * w) * kTP + p);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) a[u][w] = fma(-x[u].y, l.y, fma(-x[u].x, l.x, a[u][w]));
+                }
+                if (SYRK) {
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        const double2 y = *reinterpret_cast<const double2 *>(Xs + (tc + 16 * w) * kTP + p);
+#pragma unroll
+                        for (int u = w; u < 4; ++u) acc[u][w] = fma(x[u].y, y.y, fma(x[u].x, y.x, acc[u][w]));
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Column J onwards of the Cholesky of a 16 x 16 block held by the lanes of
+// one warp, lane l (l = lane % 16) owning row l (v[k] = element (l, k)); d is
+// column J's pivot, in every lane.  The next pivot's own update needs no
+// other lane's value, so the chain per column is the reciprocal square root,
+// two products and one shuffle; the other columns' shuffles overlap it.  No
+// branches (they cost 235 of 343 cycles a column): every lane updates its whole
+// row, and what lands above the diagonal is never read; `bad` collects pivots
+// that are not positive (each replaced by 1).
+template <int J>
+__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, bool &bad)
+{
+    if constexpr (J < 16) {
+        const unsigned full = 0xffffffffu;
+        const bool ok = d > 0.0;
+        bad = bad || !ok;
+        d = ok ? d : 1.0;
+        const double inv = rsqrt(d);
+        const double col = v[J] * inv, piv = d * inv;
+        v[J] = l == J ? piv : col;
+        double dn = 1.0;
+        if constexpr (J + 1 < 16) dn = __shfl_sync(full, fma(-col, col, v[J + 1]), J + 1);  // lane J + 1: its pivot
+#pragma unroll
+        for (int k = J + 1; k < 16; ++k) {
+            const double lkj = __shfl_sync(full, col, k);  // L(k, J), from row k's lane
+            v[k] = fma(-v[J], lkj, v[k]);
+        }
+        factor16<J + 1>(v, dn, l, bad);
+    }
+}
+
+// Cholesky of the diagonal tile W (shared memory, lower triangle in; out: the
+// factor, its transpose above, the reciprocals in column 64).  Four 16-column
+// panels: warp 0 factors the panel's diagonal block while the other warps
+// finish the previous panel's trailing update; then one thread per row solves
+// the rows below, and all warps update the next diagonal block.
+__device__ void tile_potrf(double *__restrict__ W, int *status)
+{
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+#pragma unroll 1
+    for (int c0 = 0; c0 < kNB; c0 += 16) {
+        if (warp == 0) {
+            const int l = lane & 15;
+            double *row = W + (c0 + l) * kTP + c0;
+            double v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = k <= l ? row[k] : 0.0;
+            __syncwarp();
+            bool bad = false;
+            factor16<0>(v, __shfl_sync(0xffffffffu, v[0], 0), l, bad);
+            if (bad && lane == 0) atomicOr(status, kStNotSPD);
+            double dl = 1.0;
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (k == l) dl = v[k];
+            if (lane < 16) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    if (k <= l) {
+                        row[k] = v[k];
+                        W[(c0 + k) * kTP + c0 + l] = v[k];
+                    }
+                row[kNB - c0] = 1.0 / dl;
+            }
+        } else if (c0 > 0) {
+            // trailing update by panel c0 - 16 of the 16 x 16 blocks (bi, bj),
+            // c0 / 16 <= bj <= bi < 4, but for the diagonal block at c0 (done):
+            // half a block per warp and turn, four columns of one row per lane
+            const int b0 = c0 >> 4, nb = 4 - b0, units = nb * (nb + 1) - 2;
+            for (int e = warp - 1; e < units; e += kCompute / 32 - 1) {
+                int f = (e >> 1) + 1, bj = b0;  // f: block in column order
+                while (f >= 4 - bj) {
+                    f -= 4 - bj;
+                    ++bj;
+                }
+                const int bi = bj + f;
+                const int i = 16 * bi + (lane & 15), j0 = 16 * bj + 8 * (e & 1) + 4 * (lane >> 4);
+                const double *ri = W + i * kTP + c0 - 16;
+                double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+                for (int p = 0; p < 16; p += 2) {
+                    const double2 x = *reinterpret_cast<const double2 *>(ri + p);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const double2 y = *reinterpret_cast<const double2 *>(W + (j0 + k) * kTP + c0 - 16 + p);
+                        s[k] = fma(x.y, y.y, fma(x.x, y.x, s[k]));
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (j0 + k <= i) W[i * kTP + j0 + k] -= s[k];
+            }
+        }
+        sync_compute();
+        if (c0 + 16 >= kNB) break;
+        if (t < kNB - 16 - c0) {
+            double *x = W + (c0 + 16 + t) * kTP + c0;
+            solve_row16(x, W + c0 * kTP + c0, W + c0 * kTP + kNB);
+        }
+        sync_compute();
+        {
+            // the next diagonal block, one element per thread
+            const int r = t >> 4, c = t & 15, c1 = c0 + 16;
+            if (c <= r) {
+                const double *ri = W + (c1 + r) * kTP + c0, *rj = W + (c1 + c) * kTP + c0;
+                double s = 0.0;
+#pragma unroll
+                for (int p = 0; p < 16; p += 2) {
+                    const double2 x = *reinterpret_cast<const double2 *>(ri + p), y = *reinterpret_cast<const double2 *>(rj + p);
+                    s = fma(x.y, y.y, fma(x.x, y.x, s));
+                }
+                W[(c1 + r) * kTP + c1 + c] -= s;
+            }
+        }
+        sync_compute();
+    }
+    // the transpose of the panels below the diagonal blocks is not read
+}
+
+// ------------------------------------------------------------------ chain
+
+// The chain's buffers: 0, 1 the next step's tiles (k, k-1) and (k, k), 2 the
+// diagonal tile being factored, 5 the solved panel tile.  The back
+// substitution then uses all six as one ring.
+constexpr int kBufX = 0, kBufD = 1, kBufW = 2, kBufOut = 5;
+
+// The ring of the back substitution: per block kb, in order, the tiles
+// (kb+1, kb) and (kb, kb) of the chain warps and (kb+2, kb-1), (kb+1, kb-1)
+// of the look-ahead warps, as far as they exist.
+__device__ __forceinline__ bool back_tile(const Ctl &C, int kb, int which, const double *&p)
+{
+    int i, j;
+    if (which == 0) { i = kb + 1; j = kb; }
+    else if (which == 1) { i = kb; j = kb; }
+    else if (which == 2) { i = kb + 2; j = kb - 1; }
+    else { i = kb + 1; j = kb - 1; }
+    if (i >= C.nblk || j < 0) return false;
+    p = tile_ptr(C, i, j);
+    return true;
+}
+
+__device__ void chain_fetch(const Ctl &C, Smem &S)
+{
+    const int nblk = C.nblk;
+    for (int k = 1; k < nblk; ++k) {
+        const uint32_t n = (uint32_t)(k - 1);
+        if (k >= 2 && !flag_wait(C, S, &C.pre_s[k - 1], 1)) return;
+        bar_wait_free(C, S, &S.empty[kBufX], n);
+        fence_async();
+        load_buf(S, kBufX, tile_ptr(C, k, k - 1), kTileB);
+        if (k >= 2 && !flag_wait(C, S, &C.pre_d[k], 1)) return;
+        bar_wait_free(C, S, &S.empty[kBufD], n);
+        fence_async();
+        load_buf(S, kBufD, tile_ptr(C, k, k), kTileB);
+    }
+    // back substitution: every panel tile of a row of right-hand sides that
+    // is final has been published, and so have the tiles it was solved with;
+    // the ring starts once the chain's own last tiles have left the buffers
+    if (!flag_wait(C, S, &C.F->pdone, nblk) || !flag_wait(C, S, &C.tdone[nblk], nblk)) return;
+    bar_wait(C, S, &S.xdone, 0);
+    if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+    fence_async();
+    uint32_t q = 0;  // position in the ring
+    uint32_t used[kBufs];
+#pragma unroll
+    for (int b = 0; b < kBufs; ++b) used[b] = (b == kBufX || b == kBufD) && nblk > 1 ? (uint32_t)(nblk - 1) : 0u;
+    int zb = nblk - 1;  // next block whose right-hand sides are fetched
+    for (int kb = nblk - 1; kb >= 0; --kb) {
+        // the right-hand sides of block kb - 1 (and, at the start, kb) join;
+        // their slot's last user, block kb + 3, is done: the tiles fetched so
+        // far are all of blocks > kb, so two blocks' worth of the ring's six
+        // buffers, those of block kb + 2 at least, have been released
+        for (; zb >= 0 && zb >= kb - 1; --zb) {
+            if (zb + 4 < nblk && !flag_wait(C, S, &C.bcnt[zb], 1)) return;
+            fence_async();
+            bar_expect(&S.zfull[zb & 3], kRhsB);
+            bulk_copy(S.z[zb & 3], C.rhs + (size_t)zb * kRhsD, kRhsB, &S.zfull[zb & 3]);
+            ++S.zissued[zb & 3];
+        }
+        for (int w = 0; w < 4; ++w) {
+            const double *src;
+            if (!back_tile(C, kb, w, src)) continue;
+            const int b = (int)(q % kBufs);
+            // (constant indices keep `used` in registers)
+            uint32_t u = 0;
+#pragma unroll
+            for (int k = 0; k < kBufs; ++k)
+                if (k == b) u = used[k]++;
+            bar_wait_free(C, S, &S.empty[b], u);
+            if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+            load_buf(S, b, src, kTileB);
+            ++q;
+        }
+    }
+}
+
+// Back substitution of one 64-row block for one right-hand side by one warp:
+// D' x = b, lane l holding rows l and l + 32.  A row's update is a product
+// with 0 in the lanes it does not concern, so that the chain per row is one
+// shuffle, one product and one multiply-add without a select.
+__device__ __forceinline__ void back_diag(const double *__restrict__ D, double &b0, double &b1)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned full = 0xffffffffu;
+    double x0 = 0.0, x1 = 0.0;
+#pragma unroll 16
+    for (int j = kNB - 1; j >= 32; --j) {
+        const double rd = D[j * kTP + kNB], d0 = -D[j * kTP + lane], d1 = lane + 32 < j ? -D[j * kTP + lane + 32] : 0.0;
+        const double xj = __shfl_sync(full, b1, j & 31) * rd;
+        x1 = lane == (j & 31) ? xj : x1;
+        b1 = fma(d1, xj, b1);
+        b0 = fma(d0, xj, b0);
+    }
+#pragma unroll 16
+    for (int j = 31; j >= 0; --j) {
+        const double rd = D[j * kTP + kNB], d0 = lane < j ? -D[j * kTP + lane] : 0.0;
+        const double xj = __shfl_sync(full, b0, j) * rd;
+        x0 = lane == j ? xj : x0;
+        b0 = fma(d0, xj, b0);
+    }
+    b0 = x0;
+    b1 = x1;
+}
+
+// s0, s1: rows `lane` and `lane + 32` of L' x for a tile L and 64 values x in
+// shared memory, summed over L's rows in order.
+__device__ __forceinline__ void back_product(const double *__restrict__ L, const double *__restrict__ x, double &s0, double &s1)
+{
+    const int lane = threadIdx.x & 31;
+    s0 = s1 = 0.0;
+#pragma unroll 8
+    for (int p = 0; p < kNB; p += 2) {
+        const double2 xp = *reinterpret_cast<const double2 *>(x + p);
+        s0 = fma(L[p * kTP + lane], xp.x, s0);
+        s1 = fma(L[p * kTP + lane + 32], xp.x, s1);
+        s0 = fma(L[(p + 1) * kTP + lane], xp.y, s0);
+        s1 = fma(L[(p + 1) * kTP + lane + 32], xp.y, s1);
+    }
+}
+
+__device__ void chain_compute(const Ctl &C, Smem &S)
+{
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, tr = t >> 4, tc = t & 15;
+    const int nblk = C.nblk;
+    double *W = S.buf[kBufW], *Xs = S.buf[kBufOut];
+    {
+        const double *src = tile_ptr(C, 0, 0);
+        for (int e = t; e < kTileD / 2; e += kCompute)
+            reinterpret_cast<double2 *>(W)[e] = reinterpret_cast<const double2 *>(src)[e];
+        sync_compute();
+        tile_potrf(W, C.status);
+        post(S, 1, W, tile_ptr(C, 0, 0), kTileB, &C.F->pdone, 1);
+    }
+    for (int k = 1; k < nblk; ++k) {
+        const uint32_t n = (uint32_t)(k - 1);
+        double a[4][4], ad[4][4], acc[4][4];
+        bar_wait(C, S, &S.full[kBufX], n);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) a[u][v] = S.buf[kBufX][(tr + 16 * u) * kTP + tc + 16 * v];
+        __syncwarp();
+        if (lane == 0) bar_arrive(&S.empty[kBufX]);
+        bar_wait_free(C, S, &S.freed[0], n);  // the previous panel tile has been stored
+        tile_solve<true>(a, W, Xs, acc);
+        post(S, 0, Xs, tile_ptr(C, k, k - 1), kTileB, &C.tdone[k], k);
+        bar_wait(C, S, &S.full[kBufD], n);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v <= u; ++v) ad[u][v] = S.buf[kBufD][(tr + 16 * u) * kTP + tc + 16 * v] - acc[u][v];
+        __syncwarp();
+        if (lane == 0) bar_arrive(&S.empty[kBufD]);
+        bar_wait(C, S, &S.freed[1], n);  // the previous diagonal tile has been stored
+        sync_compute();                  // and every warp has read it
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v <= u; ++v) W[(tr + 16 * u) * kTP + tc + 16 * v] = ad[u][v];
+        sync_compute();
+        tile_potrf(W, C.status);
+        post(S, 1, W, tile_ptr(C, k, k), kTileB, &C.F->pdone, k + 1);
+    }
+    // back substitution: the fetching warp may overwrite every buffer once
+    // the last two results have been stored
+    bar_wait(C, S, &S.freed[1], (uint32_t)(nblk - 1));
+    if (nblk > 1) bar_wait(C, S, &S.freed[0], (uint32_t)(nblk - 2));
+    sync_compute();
+    if (t == 0) bar_arrive(&S.xdone);
+    const int c = warp & 3;         // right-hand side
+    const bool head = warp < 4;     // the chain itself; the others look ahead
+    uint32_t q = 0;
+    uint32_t used[kBufs];
+#pragma unroll
+    for (int b = 0; b < kBufs; ++b) used[b] = (b == kBufX || b == kBufD) && nblk > 1 ? (uint32_t)(nblk - 1) : 0u;
+    for (int kb = nblk - 1; kb >= 0; --kb) {
+        double s0, s1, b0 = 0, b1 = 0;
+        if (head) {
+            bar_wait(C, S, &S.zfull[kb & 3], (uint32_t)((nblk - 1 - kb) >> 2));
+            b0 = S.z[kb & 3][c * kTP + lane];
+            b1 = S.z[kb & 3][c * kTP + lane + 32];
+        } else if (kb >= 1) {
+            bar_wait(C, S, &S.zfull[(kb - 1) & 3], (uint32_t)((nblk - kb) >> 2));
+            b0 = S.z[(kb - 1) & 3][c * kTP + lane];
+            b1 = S.z[(kb - 1) & 3][c * kTP + lane + 32];
+        }
+#pragma unroll 1
+        for (int w = 0; w < 4; ++w) {
+            const double *src;
+            if (!back_tile(C, kb, w, src)) continue;
+            const int b = (int)(q % kBufs);
+            uint32_t u = 0;
+#pragma unroll
+            for (int k = 0; k < kBufs; ++k)
+                if (k == b) u = used[k]++;
+            ++q;
+            if (head == (w < 2)) {
+                bar_wait(C, S, &S.full[b], u);
+                if (w == 1) {
+                    back_diag(S.buf[b], b0, b1);
+                } else {
+                    back_product(S.buf[b], S.xs[(w == 2 ? kb + 2 : kb + 1) & 3] + c * kTP, s0, s1);
+                    b0 -= s0;
+                    b1 -= s1;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) bar_arrive(&S.empty[b]);
+        }
+        if (head) {
+            S.xs[kb & 3][c * kTP + lane] = b0;
+            S.xs[kb & 3][c * kTP + lane + 32] = b1;
+            const int r = kb * kNB + lane;
+            if (r < C.m) C.x[(size_t)r * 4 + c] = b0;
+            if (r + 32 < C.m) C.x[(size_t)(r + 32) * 4 + c] = b1;
+        } else if (kb >= 1) {
+            S.z[(kb - 1) & 3][c * kTP + lane] = b0;
+            S.z[(kb - 1) & 3][c * kTP + lane + 32] = b1;
+        }
+        // the previous block's mail has been read (mailbox 0 carried nblk - 1 panel tiles before)
+        bar_wait_free(C, S, &S.freed[0], (uint32_t)(nblk - 1 + nblk - 1 - kb));
+        post(S, 0, nullptr, nullptr, 0, &C.F->ddone, nblk - kb);
+        sync_compute();
+    }
+}
+
+__device__ void chain_publish(const Ctl &C, Smem &S)
+{
+    uint32_t n0 = 0;
+    if (!publish(C, S, 1, 0)) return;
+    for (int k = 1; k < C.nblk; ++k) {
+        if (!publish(C, S, 0, n0++)) return;
+        if (!publish(C, S, 1, (uint32_t)k)) return;
+    }
+    for (int kb = C.nblk - 1; kb >= 0; --kb)
+        if (!publish(C, S, 0, n0++)) return;
+}
+
+// ---------------------------------------------------------------- helpers
+
+// Task t: tiles column by column, rows j .. nblk (nblk: the right-hand
+// sides), then the right-hand-side blocks nblk - 5 .. 0 of the back
+// substitution.  kind 0: none left.
+struct Task {
+    int kind;  // 1 tile, 2 right-hand sides of a column, 3 back substitution
+    int i, j;
+};
+
+__device__ Task task_of(int t, int nblk)
+{
+    for (int j = 0; j < nblk; ++j) {
+        const int n = nblk + 1 - j;
+        if (t < n) return {t == n - 1 ? 2 : 1, j + t, j};
+        t -= n;
+    }
+    if (t < nblk - 4) return {3, nblk - 5 - t, 0};
+    return {0, 0, 0};
+}
+
+// Ring of the helpers: two stages of two buffers (0, 1 and 2, 3); buffer 4 the
+// factored diagonal tile, 5 the result.
+constexpr int kBufL = 4;
+
+__device__ void helper_fetch(const Ctl &C, Smem &S, const Task &T, uint32_t &stage, uint32_t &diags)
+{
+    const int nblk = C.nblk;
+    if (T.kind == 3) {
+        // L(kb, i) needs no wait of its own: once x(kb) is asked for, the
+        // factorisation is over; the first wait covers them all
+        for (int kb = nblk - 1; kb >= T.i + 4; --kb) {
+            const int b = 2 * (int)(stage & 1u);
+            if (kb == nblk - 1 && (!flag_wait(C, S, &C.F->pdone, nblk) || !flag_wait(C, S, &C.tdone[nblk], nblk))) return;
+            bar_wait_free(C, S, &S.empty[b], stage >> 1);
+            fence_async();
+            load_buf(S, b, tile_ptr(C, kb, T.i), kTileB);
+            ++stage;
+        }
+        return;
+    }
+    const int kn = T.kind == 1 && T.i == T.j ? T.j - 1 : T.j;
+    int ready = 0;  // panels known to be final
+    for (int k = 0; k < kn; ++k, ++stage) {
+        const int b = 2 * (int)(stage & 1u);
+        if (ready <= k) {
+            if (!flag_wait(C, S, &C.tdone[T.j], k + 1) || !flag_wait(C, S, &C.tdone[T.kind == 2 ? nblk : T.i], k + 1)) return;
+            ready = min(ld_acquire(&C.tdone[T.j]), ld_acquire(&C.tdone[T.kind == 2 ? nblk : T.i]));
+        }
+        bar_wait_free(C, S, &S.empty[b], stage >> 1);
+        if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+        fence_async();
+        const bool two = T.kind == 2 || T.i != T.j;
+        // both operands count on the first buffer's barrier
+        ++S.issued[b];
+        bar_expect(&S.full[b], T.kind == 2 ? kTileB + kRhsB : two ? 2 * kTileB : kTileB);
+        bulk_copy(S.buf[b], tile_ptr(C, T.j, k), kTileB, &S.full[b]);
+        if (T.kind == 2) bulk_copy(S.buf[b + 1], C.rhs + (size_t)k * kRhsD, kRhsB, &S.full[b]);
+        else if (two) bulk_copy(S.buf[b + 1], tile_ptr(C, T.i, k), kTileB, &S.full[b]);
+    }
+    if (T.kind == 2 || T.i > T.j + 1) {
+        if (!flag_wait(C, S, &C.F->pdone, T.j + 1)) return;
+        bar_wait_free(C, S, &S.empty[kBufL], diags);
+        if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+        fence_async();
+        load_buf(S, kBufL, tile_ptr(C, T.j, T.j), kTileB);
+        ++diags;
+    }
+}
+
+__device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &stage, uint32_t &diags, uint32_t &posts)
+{
+    const int t = threadIdx.x, lane = t & 31, tr = t >> 4, tc = t & 15;
+    const int nblk = C.nblk;
+    double *Xs = S.buf[kBufOut];
+    if (T.kind == 1) {
+        const bool diag = T.i == T.j;
+        const int kn = diag ? T.j - 1 : T.j;
+        if (kn <= 0 && T.i <= T.j + 1) return;  // the chain reads the tile as it is
+        double *A = tile_ptr(C, T.i, T.j);
+        double a[4][4], acc[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) a[u][v] = A[(tr + 16 * u) * kTP + tc + 16 * v];
+        for (int k = 0; k < kn; ++k, ++stage) {
+            const int b = 2 * (int)(stage & 1u);
+            bar_wait(C, S, &S.full[b], stage >> 1);
+            if (diag) tile_product<true>(S.buf[b], S.buf[b], acc);
+            else tile_product<false>(S.buf[b + 1], S.buf[b], acc);
+            __syncwarp();
+            if (lane == 0) bar_arrive(&S.empty[b]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) a[u][v] -= acc[u][v];
+        }
+        bar_wait_free(C, S, &S.freed[0], posts);
+        if (T.i <= T.j + 1) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) Xs[(tr + 16 * u) * kTP + tc + 16 * v] = a[u][v];
+            post(S, 0, Xs, A, kTileB, diag ? &C.pre_d[T.j] : &C.pre_s[T.j], 1);
+        } else {
+            bar_wait(C, S, &S.full[kBufL], diags++);
+            tile_solve<false>(a, S.buf[kBufL], Xs, acc);
+            __syncwarp();
+            if (lane == 0) bar_arrive(&S.empty[kBufL]);
+            post(S, 0, Xs, A, kTileB, &C.tdone[T.i], T.j + 1);
+        }
+        ++posts;
+        return;
+    }
+    // four right-hand sides: thread (c, r), r = t / 64 the side, c = t % 64
+    const int r = t >> 6, c = t & 63;
+    if (T.kind == 2) {
+        double *A = C.rhs + (size_t)T.j * kRhsD;
+        double a = A[r * kTP + c];
+        for (int k = 0; k < T.j; ++k, ++stage) {
+            const int b = 2 * (int)(stage & 1u);
+            bar_wait(C, S, &S.full[b], stage >> 1);
+            const double *Li = S.buf[b + 1] + r * kTP, *Lj = S.buf[b] + c * kTP;
+            double s = 0.0;
+#pragma unroll 8
+            for (int p = 0; p < kNB; p += 2) {
+                const double2 x = *reinterpret_cast<const double2 *>(Li + p), y = *reinterpret_cast<const double2 *>(Lj + p);
+                s = fma(x.y, y.y, fma(x.x, y.x, s));
+            }
+            __syncwarp();
+            if (lane == 0) bar_arrive(&S.empty[b]);
+            a -= s;
+        }
+        bar_wait_free(C, S, &S.freed[0], posts);
+        bar_wait(C, S, &S.full[kBufL], diags++);
+        const double *L = S.buf[kBufL];
+        for (int c0 = 0; c0 < kNB; c0 += 16) {
+            if (c >= c0 && c < c0 + 16) Xs[r * kTP + c] = a;
+            sync_compute();
+            if (t < 4) solve_row16(Xs + t * kTP + c0, L + c0 * kTP + c0, L + c0 * kTP + kNB);
+            sync_compute();
+            if (c >= c0 + 16)
+#pragma unroll
+                for (int p = c0; p < c0 + 16; p += 2) {
+                    const double2 x = *reinterpret_cast<const double2 *>(Xs + r * kTP + p);
+                    const double2 l = *reinterpret_cast<const double2 *>(L + c * kTP + p);
+                    a = fma(-x.y, l.y, fma(-x.x, l.x, a));
+                }
+        }
+        if (t < 8) Xs[(t >> 1) * kTP + kNB + (t & 1)] = 0.0;  // the pitch's spare columns
+        __syncwarp();
+        if (lane == 0) bar_arrive(&S.empty[kBufL]);
+        post(S, 0, Xs, A, kRhsB, &C.tdone[nblk], T.j + 1);
+        ++posts;
+        return;
+    }
+    // back substitution of block i by the blocks nblk - 1 .. i + 4
+    double *A = C.rhs + (size_t)T.i * kRhsD;
+    bool first = true;
+    double a = 0.0;
+    for (int kb = nblk - 1; kb >= T.i + 4; --kb, ++stage) {
+        const int b = 2 * (int)(stage & 1u);
+        if (t == 0) flag_wait(C, S, &C.F->ddone, nblk - kb);
+        sync_compute();
+        if (first) a = __ldcg(&A[r * kTP + c]);
+        first = false;
+        S.small[r * kTP + c] = kb * kNB + c < C.m ? __ldcg(&C.x[(size_t)(kb * kNB + c) * 4 + r]) : 0.0;
+        sync_compute();
+        bar_wait(C, S, &S.full[b], stage >> 1);
+        const double *L = S.buf[b] + c, *x = S.small + r * kTP;
+        double s = 0.0;
+#pragma unroll 8
+        for (int p = 0; p < kNB; p += 2) {
+            const double2 xp = *reinterpret_cast<const double2 *>(x + p);
+            s = fma(L[p * kTP], xp.x, s);
+            s = fma(L[(p + 1) * kTP], xp.y, s);
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(&S.empty[b]);
+        a -= s;
+    }
+    bar_wait_free(C, S, &S.freed[0], posts);
+    Xs[r * kTP + c] = a;
+    if (t < 8) Xs[(t >> 1) * kTP + kNB + (t & 1)] = 0.0;
+    post(S, 0, Xs, A, kRhsB, &C.bcnt[T.i], 1);
+    ++posts;
+}
+
+// Waits (bounded) for the last of `n` copies counted on barrier b.
+__device__ void drain(unsigned long long *b, uint32_t n)
+{
+    if (n == 0) return;
+    const unsigned long long t0 = now_ns();
+    while (!bar_try(b, (n - 1) & 1u))
+        if (now_ns() - t0 > 2000000000ull) return;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_chol_solve(Ctl C)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    Smem &S = *reinterpret_cast<Smem *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < kBufs; ++b) {
+            bar_init(&S.full[b], 1);
+            bar_init(&S.empty[b], kCompute / 32);
+            S.issued[b] = 0;
+        }
+        for (int b = 0; b < 4; ++b) {
+            bar_init(&S.zfull[b], 1);
+            S.zissued[b] = 0;
+        }
+        for (int b = 0; b < 2; ++b) {
+            bar_init(&S.post[b], kCompute / 32);
+            bar_init(&S.freed[b], 1);
+        }
+        bar_init(&S.xdone, 1);
+        S.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {  // (the fetching and publishing warps' lanes meet again at the __syncwarp below)
+        if (warp < kFetchWarp) chain_compute(C, S);
+        else if (lane == 0) {
+            if (warp == kFetchWarp) chain_fetch(C, S);
+            else chain_publish(C, S);
+        }
+    } else {
+        uint32_t stage = 0, diags = 0, posts = 0;
+        bool live = true;  // the publishing warp: its mailbox is still in use
+        for (;;) {
+            if (threadIdx.x == 0)
+                S.task = *reinterpret_cast<volatile int *>(&S.abort) ? 0x7fffffff : atomicAdd(&C.F->next, 1);
+            __syncthreads();
+            const Task T = task_of(S.task, C.nblk);
+            __syncthreads();  // every thread has read the task
+            if (T.kind == 0) break;
+            if (warp < kFetchWarp) helper_compute(C, S, T, stage, diags, posts);
+            else if (lane == 0) {
+                if (warp == kFetchWarp) {
+                    helper_fetch(C, S, T, stage, diags);
+                } else {
+                    const int kn = T.kind == 1 ? (T.i == T.j ? T.j - 1 : T.j) : 1;
+                    const bool posted = !(T.kind == 1 && kn <= 0 && T.i <= T.j + 1);
+                    if (posted && live) live = publish(C, S, 0, posts++);
+                }
+            }
+            __syncwarp();
+        }
+    }
+    // no copy may still be writing this CTA's shared memory when it exits: on
+    // the normal path every copy has been waited for; after a time-out the
+    // thread that began them waits here (bounded)
+    if (warp == kFetchWarp && lane == 0) {
+        for (int b = 0; b < kBufs; ++b) drain(&S.full[b], S.issued[b]);
+        for (int b = 0; b < 4; ++b) drain(&S.zfull[b], S.zissued[b]);
+    }
+    __syncwarp();
+    __syncthreads();
+}
+
+// A, upper part included only inside the diagonal tiles' padding: tile (i, j)
+// of (Q'KQ)(4:,4:) + lambda I, i >= j, or the right-hand-side tile j, z(4:)'.
+// One CTA per tile, 256 threads; rows and columns past m are zero, with ones
+// on the diagonal.
+__global__ void __launch_bounds__(256) k_fill_tiles(const double *__restrict__ ctr, int n, const double *__restrict__ V,
+                                                    const double *__restrict__ W, const double *__restrict__ Z,
+                                                    double lambda, Ctl C)
+{
+    const int m = C.m, nblk = C.nblk;
+    const int ntri = nblk * (nblk + 1) / 2;
+    int t = (int)blockIdx.x;
+    if (t >= ntri) {
+        const int j = t - ntri;
+        double *R = C.rhs + (size_t)j * kRhsD;
+        for (int e = threadIdx.x; e < kRhsD; e += blockDim.x) {
+            const int r = e / kTP, c = j * kNB + e % kTP;
+            R[e] = e % kTP < kNB && c < m ? Z[(size_t)(c + 4) * 4 + r] : 0.0;
+        }
+        return;
+    }
+    int j = 0;
+    while (t >= nblk - j) {
+        t -= nblk - j;
+        ++j;
+    }
+    const int i = j + t;
+    double *T = tile_ptr(C, i, j);
+    for (int e = threadIdx.x; e < kTileD; e += blockDim.x) {
+        const int r = e / kTP, c = e % kTP;
+        const int ri = i * kNB + r, cj = j * kNB + c;
+        double v = 0.0;
+        if (c < kNB && ri < m && cj < m && ri >= cj) {
+            const int gi = ri + 4, gj = cj + 4;
+            v = kdist(ctr, gi, gj);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v -= V[gi * 4 + k] * W[gj * 4 + k] + W[gi * 4 + k] * V[gj * 4 + k];
+            if (ri == cj) v += lambda;
+        } else if (i == j && r == c) {
+            v = 1.0;
+        }
+        T[e] = v;
+    }
+}
+
+int blocks_of(int m) { return (m + kNB - 1) / kNB; }
+size_t flag_ints(int nblk) { return 4 + (size_t)(nblk + 1) + 3 * (size_t)nblk; }
+size_t tri_tiles(int nblk) { return (size_t)nblk * (nblk + 1) / 2; }
+
+}  // namespace
+
+size_t chol_work_bytes(int m)
+{
+    const int nblk = blocks_of(m);
+    return tri_tiles(nblk) * kTileB + (size_t)nblk * kRhsB + ((flag_ints(nblk) * sizeof(int) + 15) / 16) * 16;
+}
+
+cudaError_t launch_chol_solve(const double *ctr, int n, const double *V, const double *W, double *Z, double lambda,
+                              void *work, int *status, unsigned long long limit_ns, int sm_count, cudaStream_t st)
+{
+    Ctl C;
+    C.m = n - 4;
+    C.nblk = blocks_of(C.m);
+    C.tiles = static_cast<double *>(work);
+    C.rhs = C.tiles + tri_tiles(C.nblk) * kTileD;
+    int *flags = reinterpret_cast<int *>(C.rhs + (size_t)C.nblk * kRhsD);
+    C.F = reinterpret_cast<Flags *>(flags);
+    C.tdone = flags + 4;
+    C.pre_d = C.tdone + C.nblk + 1;
+    C.pre_s = C.pre_d + C.nblk;
+    C.bcnt = C.pre_s + C.nblk;
+    C.x = Z + 16;
+    C.status = status;
+    C.limit_ns = limit_ns;
+    cudaError_t e = cudaMemsetAsync(flags, 0, flag_ints(C.nblk) * sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    const size_t fill = tri_tiles(C.nblk) + (size_t)C.nblk;
+    k_fill_tiles<<<(unsigned)fill, 256, 0, st>>>(ctr, n, V, W, Z, lambda, C);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(k_chol_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+    if (e != cudaSuccess) return e;
+    // the chain and at most one helper per task: a small system leaves the
+    // other SMs to other work
+    const size_t want = 1 + fill;
+    const int grid = want < (size_t)sm_count ? (int)want : sm_count;
+    void *args[] = {(void *)&C};
+    return cudaLaunchCooperativeKernel((const void *)k_chol_solve, dim3(grid), dim3(kThreads), args, sizeof(Smem), st);
+}
+
+}  // namespace tw

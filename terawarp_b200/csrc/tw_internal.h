@@ -109,7 +109,14 @@ cudaError_t launch_tps_eval(const EvalParams &p, cudaStream_t st, int sm_count);
 
 // ------------------------------------------------------------------- solve
 
-struct SolveWork;   // device workspace of one solve
+// The projected system's Cholesky solve (tw_chol.cu): with m = n - 4 > 0,
+// A = (Q'KQ)(4:,4:) + lambda I from the reflectors V and update vectors W (n x
+// 4 each), right-hand sides Z(4:) (n x 4); the solution overwrites Z(4:).  Sets
+// bits 2 (not positive definite) and 4 (a wait longer than limit_ns) of
+// *status.  work: chol_work_bytes(m) of device memory, 16-byte aligned.
+size_t chol_work_bytes(int m);
+cudaError_t launch_chol_solve(const double *ctr, int n, const double *V, const double *W, double *Z, double lambda,
+                              void *work, int *status, unsigned long long limit_ns, int sm_count, cudaStream_t st);
 // Solves on `st`: c into d_c_out (n x 4), d into d_d_out (4 x 4) and the
 // status bits into d_status_out, all device memory that outlives the call.
 // With h_d_out it waits for `st` once, at the end, copies d to the host and

@@ -35,6 +35,7 @@
 // Jacobi, which is the right singular vector the reference uses.
 
 #include "tw_internal.h"
+#include "tw_kdist.h"
 
 #include <cmath>
 #include <cstring>
@@ -44,12 +45,12 @@ namespace tw {
 
 namespace {
 
-constexpr int kNB = 64;          // Cholesky block
 constexpr int kRedThreads = 1024;
 
 // status word bits
 constexpr int kStSingularX = 1;
-constexpr int kStNotSPD = 2;
+constexpr int kStNotSPD = 2;   // set by the Cholesky kernel (tw_chol.cu)
+constexpr int kStTimeout = 4;
 
 __device__ double block_sum(double v, double *sh)
 {
@@ -62,14 +63,6 @@ __device__ double block_sum(double v, double *sh)
     const int nw = (blockDim.x + 31) >> 5;
     for (int i = 0; i < nw; ++i) t += sh[i];
     return t;
-}
-
-__device__ __forceinline__ double kdist(const double *ctr, int i, int j)
-{
-    double dx = ctr[3 * i] - ctr[3 * j];
-    double dy = ctr[3 * i + 1] - ctr[3 * j + 1];
-    double dz = ctr[3 * i + 2] - ctr[3 * j + 2];
-    return -sqrt(dx * dx + dy * dy + dz * dz);
 }
 
 // 1. Householder QR of X = [1 s].  Xw (n x 4) is a work copy; V (n x 4) gets
@@ -195,571 +188,6 @@ __global__ void k_wvec(int n, const double *V, const double *tau, const double *
         }
     }
 }
-
-// The factorisation works on an (m + 4) x m row-major array: rows 0..m-1
-// hold A, rows m..m+3 hold the four right-hand sides z(4:) transposed.  Row
-// block ib < nblk covers rows 64 ib.., the extra row block nblk covers the
-// four right-hand-side rows.  The right-looking Cholesky treats that block like
-// any other row below the diagonal, so its panel solves and trailing updates
-// perform the forward substitution y = L^-1 z(4:) as part of the
-// factorisation, in parallel with it; rows m..m+3 end up holding y'.
-__device__ __forceinline__ int row_block_start(int ib, int nblk, int m) { return ib < nblk ? ib * kNB : m; }
-__device__ __forceinline__ int row_block_rows(int ib, int nblk, int m)
-{
-    return ib < nblk ? min(kNB, m - ib * kNB) : 4;
-}
-
-// 3a. A = (Q'KQ)(4:,4:) + lambda I, and the right-hand-side rows z(4:)'
-__global__ void k_fill_a(const double *__restrict__ ctr, int n, const double *__restrict__ V,
-                         const double *__restrict__ W, const double *__restrict__ Z, double lambda,
-                         double *__restrict__ A)
-{
-    const int m = n - 4;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= m + 4 || j >= m) return;
-    if (i >= m) {
-        A[(size_t)i * m + j] = Z[(j + 4) * 4 + (i - m)];
-        return;
-    }
-    const int gi = i + 4, gj = j + 4;
-    double v = kdist(ctr, gi, gj);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v -= V[gi * 4 + k] * W[gj * 4 + k] + W[gi * 4 + k] * V[gj * 4 + k];
-    if (i == j) v += lambda;
-    A[(size_t)i * m + j] = v;
-}
-
-// ---- 3b-4b: one cooperative kernel, one CTA of 256 threads per SM.
-//
-// The tiled right-looking Cholesky and both substitutions run as tasks on
-// 64 x 64 tiles, ordered by dependency counters in global memory instead of
-// grid-wide barriers: POTRF(k) factors diagonal tile k once every update of
-// it has landed; TRSM(i, k) solves row block i of panel k (the right-hand-side
-// block included) once POTRF(k) and the updates of tile (i, k) are done;
-// UPDATE(i, j, k) subtracts L(i,k) L(j,k)' from tile (i, j) once both panel
-// tiles exist and the tile's previous update is in.  The back substitution
-// is DIAG(kb) (the diagonal block's triangular solve) and BACK(ib, kb) (the
-// rows of block ib) in the same way.
-//
-// The critical path is the chain POTRF(k-1) -> TRSM(k, k-1) -> UPDATE(k, k,
-// k-1) -> POTRF(k): CTA 0 runs only that chain, one fused step per k with
-// its three tiles kept in shared memory, and then the back substitution's
-// chain.  The other CTAs take every other task in one order that respects
-// every dependency, CTA c taking every (G-1)-th; as all CTAs are resident
-// (cooperative launch) and every wait of a task is on tasks earlier in that
-// order, the lowest unfinished task can always run, so the schedule cannot
-// deadlock.  L1 is not coherent across SMs within a kernel, so every load of
-// data another CTA wrote (A, z) bypasses L1 (__ldcg).
-
-constexpr int kSolveThreads = 256;
-constexpr int kStTimeout = 4;
-// A CTA gives up on a dependency after limit_ns (the context's
-// solve_barrier_ns, 30 s unless a test shortened it).  The launch is
-// cooperative, so every CTA can be resident at once; while other work (the
-// previous job's resample, a caller's kernel on another stream) still holds
-// SMs, some CTAs start later than others and the early ones wait, so the
-// bound is generous, but it is a bound.
-
-// Dependency counters (zeroed before the launch); tdone[nblk + 1] (panel
-// tiles solved per row block), cnt[(nblk + 1) nblk] (updates applied per
-// tile) and bcnt[nblk] (back-substitution updates applied per row block)
-// follow in the same allocation.
-struct SolveFlags {
-    int err;    // set by a CTA that gave up waiting
-    int pdone;  // diagonal tiles factored
-    int ddone;  // back-substitution diagonal blocks solved, from the last block down
-    int pad;
-};
-
-__device__ __forceinline__ unsigned long long globaltimer_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ int ld_acquire(const int *p)
-{
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release(int *p, int v)
-{
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Thread 0 waits until *flag >= want; every thread returns true, or false
-// (on every thread) when this or another CTA gave up.
-__device__ bool wait_ge(const int *flag, int want, SolveFlags *F, int *status, unsigned long long limit_ns)
-{
-    __shared__ int ok_sh;
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        if (ld_acquire(flag) < want) {
-            const unsigned long long t0 = globaltimer_ns();
-            while (ld_acquire(flag) < want) {
-                if (*reinterpret_cast<volatile int *>(&F->err) || globaltimer_ns() - t0 > limit_ns) {
-                    atomicOr(&F->err, 1);
-                    atomicOr(status, kStTimeout);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        __threadfence();
-        ok_sh = ok;
-    }
-    __syncthreads();
-    return ok_sh != 0;
-}
-
-// Publishes a finished task: every thread's writes, then *flag = value.
-__device__ __forceinline__ void signal_done(int *flag, int value)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        st_release(flag, value);
-    }
-}
-
-// Column J onwards of the Cholesky of a 16 x 16 block held by the lanes of
-// one warp, lane l (l = lane % 16) owning row l (v[k] = element (l, k)): the
-// pivot comes from its row's lane, the scaled column goes to the other lanes
-// by shuffles.  Compile-time recursion over the columns keeps every index of
-// v constant, so v stays in registers.
-template <int J>
-__device__ __forceinline__ void panel_factor(double (&v)[16], int l, int lane, int *status)
-{
-    if constexpr (J < 16) {
-        const unsigned full = 0xffffffffu;
-        double d = __shfl_sync(full, v[J], J);  // the pivot, from its row's lane
-        if (!(d > 0.0)) {
-            if (lane == 0) atomicOr(status, kStNotSPD);
-            d = 1.0;
-        }
-        const double inv = rsqrt(d);
-        if (l > J) v[J] *= inv;
-        else if (l == J) v[J] = d * inv;
-#pragma unroll
-        for (int k = J + 1; k < 16; ++k) {
-            const double lkj = __shfl_sync(full, v[J], k);  // L(k, J), from row k's lane
-            if (l >= k) v[k] -= v[J] * lkj;
-        }
-        panel_factor<J + 1>(v, l, lane, status);
-    }
-}
-
-// Cholesky of a diagonal tile held in shared memory (lower triangle of
-// a[kNB][kNB + 1]; padding rows and columns hold the identity), in four
-// 16-column panels: warp 0 factors the panel's 16 x 16 diagonal block in
-// registers (lane l < 16 owns its row l; each finished column goes to the
-// other lanes by shuffles), then every thread solves the panel's rows below
-// it (four lanes per row) and applies the trailing update.  rdiag gets the
-// reciprocals of the diagonal.  Three CTA barriers per panel.
-__device__ void potrf_smem(double (*a)[kNB + 1], double *rdiag, int *status)
-{
-    const int t = threadIdx.x, lane = t & 31;
-    const unsigned full = 0xffffffffu;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kNB; c0 += 16) {
-        if (t < 32) {
-            const int l = lane & 15;
-            double v[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = k <= l ? a[c0 + l][c0 + k] : 0.0;
-            panel_factor<0>(v, l, lane, status);
-            if (lane < 16) {
-                double dl = 1.0;  // v[l], selected without a run-time index (v stays in registers)
-#pragma unroll
-                for (int k = 0; k < 16; ++k) {
-                    if (k <= l) a[c0 + l][c0 + k] = v[k];
-                    if (k == l) dl = v[k];
-                }
-                rdiag[c0 + l] = 1.0 / dl;
-            }
-        }
-        __syncthreads();
-        const int nr = kNB - c0 - 16;  // rows below the panel's diagonal block
-        {
-            // X(i, c0 + c) = (A(i, c0 + c) - sum_{k<c} X(i, c0 + k) L(c0 + c, c0 + k)) / L(c0 + c, c0 + c)
-            const int r = t >> 2, q = t & 3, base = lane & ~3;
-            const bool act = r < nr;
-            const int i = c0 + 16 + (act ? r : 0);
-            double x[4];
-#pragma unroll
-            for (int k4 = 0; k4 < 4; ++k4) x[k4] = act ? a[i][c0 + 4 * k4 + q] : 0.0;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                const double mine = x[c >> 2] * rdiag[c0 + c];  // meaningful in the owner lane only
-                const double xc = __shfl_sync(full, mine, base | (c & 3));
-                if (act && q == (c & 3)) a[i][c0 + c] = xc;
-#pragma unroll
-                for (int k4 = 0; k4 < 4; ++k4) {
-                    const int cp = 4 * k4 + q;
-                    if (cp > c) x[k4] -= xc * a[c0 + cp][c0 + c];
-                }
-            }
-        }
-        __syncthreads();
-        for (int e = t; e < nr * nr; e += blockDim.x) {
-            const int ii = e / nr, jj = e % nr;
-            if (jj <= ii) {
-                const int i = c0 + 16 + ii, j = c0 + 16 + jj;
-                double acc = 0.0;
-#pragma unroll
-                for (int k = 0; k < 16; ++k) acc += a[i][c0 + k] * a[j][c0 + k];
-                a[i][j] -= acc;
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// Loads tile (row block ib, column block jb) of A into t (rows x cols of it
-// valid; the rest: identity on the diagonal when `diag`, else zero).
-__device__ void load_tile(double (*t)[kNB + 1], const double *__restrict__ A, int m, int i0, int rows, int j0, int cols,
-                          bool diag)
-{
-#pragma unroll 4
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-        const int r = e / kNB, c = e % kNB;
-        t[r][c] = (r < rows && c < cols) ? __ldcg(&A[(size_t)(i0 + r) * m + j0 + c])
-                                         : ((diag && r == c) ? 1.0 : 0.0);
-    }
-}
-
-__device__ void store_tile(double *__restrict__ A, int m, const double (*t)[kNB + 1], int i0, int rows, int j0, int cols,
-                           bool lower)
-{
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-        const int r = e / kNB, c = e % kNB;
-        if (r < rows && c < cols) A[(size_t)(i0 + r) * m + j0 + c] = (!lower || c <= r) ? t[r][c] : 0.0;
-    }
-}
-
-// X = X L^-T for a tile X in shared memory against a factored diagonal tile
-// L (rdiag: reciprocals of its diagonal), nbk valid columns.  Rows are
-// independent: the four lanes (q = lane & 3) of one row keep its columns q,
-// q+4, .. in registers; column c is finished by its owner (x 1/L(c,c)),
-// handed to the other three by a warp shuffle, and subtracted from the later
-// columns: X(r,c') -= X(r,c) L(c',c).  No CTA barrier inside the column loop.
-__device__ void trsm_smem(const double (*L)[kNB + 1], double (*X)[kNB + 1], const double *rdiag, int nbk)
-{
-    const int lane = threadIdx.x & 31;
-    const int r = (threadIdx.x >> 5) * 8 + (lane >> 2);  // 8 rows per warp
-    const int q = lane & 3;
-    const int base = lane & ~3;
-    double x[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = X[r][4 * k + q];
-    // fully unrolled so that every index into x is a constant (x stays in
-    // registers); columns at or beyond nbk are skipped
-#pragma unroll
-    for (int c = 0; c < kNB; ++c) {
-        if (c >= nbk) break;
-        const double mine = x[c >> 2] * rdiag[c];  // meaningful in the owner lane only
-        const double xc = __shfl_sync(0xffffffffu, mine, base | (c & 3));
-        if (q == (c & 3)) X[r][c] = xc;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const int cp = 4 * k + q;
-            if (cp > c && cp < nbk) x[k] -= xc * L[cp][c];
-        }
-    }
-}
-
-// acc[u][v] = sum_p Li(tr + 16u, p) Lj(tc + 16v, p) over nbk columns, thread
-// (tr, tc) = (t / 16, t % 16): conflict-free reads of Lj with the 65-double pitch.
-__device__ __forceinline__ void syrk_acc(const double (*Li)[kNB + 1], const double (*Lj)[kNB + 1], int nbk,
-                                         double (&acc)[4][4])
-{
-    const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-    for (int p = 0; p < nbk; ++p) {
-        double a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            a[u] = Li[tr + 16 * u][p];
-            b[u] = Lj[tc + 16 * u][p];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) acc[u][v] += a[u] * b[v];
-    }
-}
-
-// trsm of row block ib against diagonal block kb: L(ib,kb) = A(ib,kb) L(kb,kb)^-T.
-__device__ void trsm_tile(double *__restrict__ A, int m, int kb, int ib, double *sm)
-{
-    double(*L)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm);
-    double(*X)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm + kNB * (kNB + 1));
-    double *rdiag = sm + 2 * kNB * (kNB + 1);
-    const int nblk = (m + kNB - 1) / kNB;
-    const int r0 = kb * kNB;
-    const int i0 = row_block_start(ib, nblk, m);
-    const int nbk = min(kNB, m - r0);
-    const int nbi = row_block_rows(ib, nblk, m);
-    __syncthreads();
-    load_tile(L, A, m, r0, nbk, r0, nbk, true);
-    load_tile(X, A, m, i0, nbi, r0, nbk, false);
-    __syncthreads();
-    if (threadIdx.x < kNB) rdiag[threadIdx.x] = 1.0 / L[threadIdx.x][threadIdx.x];
-    __syncthreads();
-    trsm_smem(L, X, rdiag, nbk);
-    __syncthreads();
-    store_tile(A, m, X, i0, nbi, r0, nbk, false);
-}
-
-// Trailing update of tile (ib, jb) at step kb: A(ib,jb) -= L(ib,kb) L(jb,kb)' for
-// kb < jb <= ib, jb a column block and ib a row block (the right-hand-side
-// block included); each thread owns a 4 x 4 patch.
-__device__ void syrk_tile(double *__restrict__ A, int m, int kb, int ib, int jb, double *sm)
-{
-    double(*Li)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm);
-    double(*Lj)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm + kNB * (kNB + 1));
-    const int nblk = (m + kNB - 1) / kNB;
-    const int r0 = kb * kNB, i0 = row_block_start(ib, nblk, m), j0 = jb * kNB;
-    const int nbk = min(kNB, m - r0), nbi = row_block_rows(ib, nblk, m), nbj = min(kNB, m - j0);
-    __syncthreads();
-    load_tile(Li, A, m, i0, nbi, r0, nbk, false);
-    load_tile(Lj, A, m, j0, nbj, r0, nbk, false);
-    __syncthreads();
-    double acc[4][4];
-    syrk_acc(Li, Lj, nbk, acc);
-    const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            int r = tr + 16 * u, c = tc + 16 * v;
-            if (r < nbi && c < nbj && (ib != jb || c <= r)) {
-                double *dst = &A[(size_t)(i0 + r) * m + j0 + c];
-                *dst = __ldcg(dst) - acc[u][v];
-            }
-        }
-}
-
-// Back substitution, diagonal block kb (CTA 0): solve D' x = z(block) for the
-// four right-hand sides; warp c takes right-hand side c, lane l rows l and
-// l + 32; row j of D is column j of D'.  x overwrites z(block).
-__device__ void bwd_diag(const double *__restrict__ A, int m, int kb, double *__restrict__ z, double *sm)
-{
-    double(*D)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm);
-    double *dinv = sm + kNB * (kNB + 1);
-    const int r0 = kb * kNB, nb = min(kNB, m - r0);
-    __syncthreads();
-#pragma unroll 4
-    for (int e = threadIdx.x; e < kNB * kNB; e += blockDim.x) {
-        const int r = e / kNB, c = e % kNB;
-        D[r][c] = (r < nb && c <= r) ? __ldcg(&A[(size_t)(r0 + r) * m + r0 + c]) : 0.0;
-    }
-    if (threadIdx.x < nb) dinv[threadIdx.x] = 1.0 / __ldcg(&A[(size_t)(r0 + threadIdx.x) * m + r0 + threadIdx.x]);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp < 4) {
-        double b0 = lane < nb ? __ldcg(&z[(r0 + lane) * 4 + warp]) : 0.0;
-        double b1 = lane + 32 < nb ? __ldcg(&z[(r0 + lane + 32) * 4 + warp]) : 0.0;
-        for (int j = nb - 1; j >= 0; --j) {
-            const double bj = __shfl_sync(0xffffffffu, j < 32 ? b0 : b1, j & 31);
-            const double xj = bj * dinv[j];
-            if (lane == (j & 31)) {
-                if (j < 32) b0 = xj;
-                else b1 = xj;
-            }
-            if (lane < j) b0 -= D[j][lane] * xj;
-            if (lane + 32 < j) b1 -= D[j][lane + 32] * xj;
-        }
-        if (lane < nb) z[(r0 + lane) * 4 + warp] = b0;
-        if (lane + 32 < nb) z[(r0 + lane + 32) * 4 + warp] = b1;
-    }
-}
-
-// Back substitution, rows of block ib: z(ib) -= L(kb, ib)' x(kb), x(kb)
-// already in z(kb); thread (row, rhs) accumulates over the 64 rows of L(kb, .)
-// in order.
-__device__ void bwd_update(const double *__restrict__ A, int m, int kb, int ib, double *__restrict__ z, double *sm)
-{
-    const int r0 = kb * kNB, nb = min(kNB, m - r0);
-    const int i0 = ib * kNB, nbi = min(kNB, m - i0);
-    double *x = sm;  // x(kb), 64 x 4
-    __syncthreads();
-    for (int e = threadIdx.x; e < 4 * nb; e += blockDim.x) x[e] = __ldcg(&z[r0 * 4 + e]);
-    __syncthreads();
-    const int il = threadIdx.x >> 2, r = threadIdx.x & 3;
-    if (il < nbi) {
-        double s = 0.0;
-#pragma unroll 16
-        for (int p = 0; p < nb; ++p) s += __ldcg(&A[(size_t)(r0 + p) * m + i0 + il]) * x[p * 4 + r];
-        double *zi = &z[(i0 + il) * 4 + r];
-        *zi = __ldcg(zi) - s;
-    }
-}
-
-// CTA 0: the critical chain.  Step k fuses TRSM(k, k-1), UPDATE(k, k, k-1)
-// and POTRF(k), keeping the factored diagonal tile, the new panel tile and
-// the next diagonal tile in shared memory; then the back substitution's
-// chain DIAG(kb), BACK(kb - 1, kb).
-__device__ void solve_chain(double *__restrict__ A, int m, double *__restrict__ z, int *status, SolveFlags *F,
-                            int *tdone, int *cnt, int *bcnt, unsigned long long limit_ns, double *sm)
-{
-    const int nblk = (m + kNB - 1) / kNB;
-    double(*Ld)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm);
-    double(*X)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm + kNB * (kNB + 1));
-    double(*Ad)[kNB + 1] = reinterpret_cast<double(*)[kNB + 1]>(sm + 2 * kNB * (kNB + 1));
-    double *rdiag = sm + 3 * kNB * (kNB + 1);
-    {
-        const int nb = min(kNB, m);
-        load_tile(Ld, A, m, 0, nb, 0, nb, true);
-        __syncthreads();
-        potrf_smem(Ld, rdiag, status);
-        store_tile(A, m, Ld, 0, nb, 0, nb, true);
-        signal_done(&F->pdone, 1);
-    }
-    for (int k = 1; k < nblk; ++k) {
-        const int r0 = (k - 1) * kNB, i0 = k * kNB, nbi = min(kNB, m - i0);
-        // TRSM(k, k-1): X = A(k, k-1) L(k-1, k-1)^-T
-        if (!wait_ge(&cnt[k * nblk + k - 1], k - 1, F, status, limit_ns)) return;
-        load_tile(X, A, m, i0, nbi, r0, kNB, false);
-        __syncthreads();
-        trsm_smem(Ld, X, rdiag, kNB);
-        __syncthreads();
-        store_tile(A, m, X, i0, nbi, r0, kNB, false);
-        signal_done(&tdone[k], k);
-        // UPDATE(k, k, k-1): A(k, k) -= X X'
-        if (!wait_ge(&cnt[k * nblk + k], k - 1, F, status, limit_ns)) return;
-        load_tile(Ad, A, m, i0, nbi, i0, nbi, true);
-        __syncthreads();
-        {
-            double acc[4][4];
-            syrk_acc(X, X, kNB, acc);
-            const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int r = tr + 16 * u, c = tc + 16 * v;
-                    if (r < nbi && c <= r) Ad[r][c] -= acc[u][v];
-                }
-        }
-        __syncthreads();
-        // POTRF(k)
-        potrf_smem(Ad, rdiag, status);
-        store_tile(A, m, Ad, i0, nbi, i0, nbi, true);
-        signal_done(&F->pdone, k + 1);
-        double(*t)[kNB + 1] = Ld;
-        Ld = Ad;
-        Ad = t;
-    }
-    for (int kb = nblk - 1; kb >= 0; --kb) {
-        if (!wait_ge(&tdone[nblk], kb + 1, F, status, limit_ns) ||
-            !wait_ge(&bcnt[kb], nblk - 1 - kb, F, status, limit_ns))
-            return;
-        bwd_diag(A, m, kb, z, sm);
-        signal_done(&F->ddone, nblk - kb);
-        if (kb >= 1) {
-            if (!wait_ge(&bcnt[kb - 1], nblk - 1 - kb, F, status, limit_ns)) return;
-            bwd_update(A, m, kb, kb - 1, z, sm);
-            signal_done(&bcnt[kb - 1], nblk - kb);
-        }
-    }
-}
-
-// CTAs 1 .. G-1: every other task, in one order that respects every
-// dependency, CTA c taking every (G-1)-th.  Step k: the panel tiles TRSM(i, k)
-// of rows i >= k + 2 (and the right-hand-side block), then the updates
-// UPDATE(i, j, k) column by column, without the chain's UPDATE(k+1, k+1, k).
-// Then the back substitution's BACK(ib, kb) for ib <= kb - 2.
-__device__ void solve_others(double *__restrict__ A, int m, double *__restrict__ z, int *status, SolveFlags *F,
-                             int *tdone, int *cnt, int *bcnt, unsigned long long limit_ns, double *sm)
-{
-    const int nblk = (m + kNB - 1) / kNB;
-    const long long G = gridDim.x - 1, bid = blockIdx.x - 1;
-    long long base = 0;  // number of the step's first task
-    for (int k = 0; k < nblk; ++k) {
-        const int lo_i = k + 1 < nblk ? k + 2 : k + 1;
-        const int nt = nblk - lo_i + 1;
-        const int first = k + 1 < nblk ? nblk - k - 1 : 0;  // updates of column block k+1, rows k+2 .. nblk
-        long long nu = first;
-        for (int j = k + 2; j < nblk; ++j) nu += nblk + 1 - j;
-        const long long count = nt + nu;
-        for (long long e = ((bid - base) % G + G) % G; e < count; e += G) {
-            if (e < nt) {
-                const int i = lo_i + (int)e;
-                if (!wait_ge(&F->pdone, k + 1, F, status, limit_ns) ||
-                    !wait_ge(&cnt[i * nblk + k], k, F, status, limit_ns))
-                    return;
-                trsm_tile(A, m, k, i, sm);
-                if (i == nblk) {
-                    // y' of block k is final: seed z(k) for the back substitution
-                    __syncthreads();
-                    const int r0 = k * kNB, nb = min(kNB, m - r0);
-                    for (int q = threadIdx.x; q < 4 * nb; q += blockDim.x)
-                        z[(r0 + (q >> 2)) * 4 + (q & 3)] = __ldcg(&A[(size_t)(m + (q & 3)) * m + r0 + (q >> 2)]);
-                }
-                signal_done(&tdone[i], k + 1);
-            } else {
-                long long f = e - nt;
-                int i, j;
-                if (f < first) {
-                    j = k + 1;
-                    i = k + 2 + (int)f;
-                } else {
-                    f -= first;
-                    j = k + 2;
-                    while (f >= nblk + 1 - j) {
-                        f -= nblk + 1 - j;
-                        ++j;
-                    }
-                    i = j + (int)f;
-                }
-                if (!wait_ge(&tdone[i], k + 1, F, status, limit_ns) ||
-                    !wait_ge(&tdone[j], k + 1, F, status, limit_ns) ||
-                    !wait_ge(&cnt[i * nblk + j], k, F, status, limit_ns))
-                    return;
-                syrk_tile(A, m, k, i, j, sm);
-                signal_done(&cnt[i * nblk + j], k + 1);
-            }
-        }
-        base += count;
-    }
-    for (int kb = nblk - 1; kb >= 0; --kb) {
-        const long long count = kb >= 2 ? kb - 1 : 0;  // BACK(ib, kb) for ib = kb-2 .. 0
-        for (long long e = ((bid - base) % G + G) % G; e < count; e += G) {
-            const int ib = kb - 2 - (int)e;
-            if (!wait_ge(&F->ddone, nblk - kb, F, status, limit_ns) ||
-                !wait_ge(&bcnt[ib], nblk - 1 - kb, F, status, limit_ns))
-                return;
-            bwd_update(A, m, kb, ib, z, sm);
-            signal_done(&bcnt[ib], nblk - kb);
-        }
-        base += count;
-    }
-}
-
-__global__ void __launch_bounds__(kSolveThreads) k_chol_solve(double *__restrict__ A, int m, double *__restrict__ Z,
-                                                              int *status, int *flags, unsigned long long limit_ns)
-{
-    extern __shared__ double sm[];
-    const int nblk = (m + kNB - 1) / kNB;
-    SolveFlags *F = reinterpret_cast<SolveFlags *>(flags);
-    int *tdone = flags + 4;
-    int *cnt = tdone + nblk + 1;
-    int *bcnt = cnt + (nblk + 1) * nblk;
-    double *z = Z + 16;  // z(4:), 4 per row; y' then x' overwrite it
-    if (blockIdx.x == 0) solve_chain(A, m, z, status, F, tdone, cnt, bcnt, limit_ns, sm);
-    else solve_others(A, m, z, status, F, tdone, cnt, bcnt, limit_ns, sm);
-}
-
-constexpr size_t kSolveSmem = sizeof(double) * (3 * kNB * (kNB + 1) + 3 * kNB);
 
 // 4c. c = H1 H2 H3 H4 [0; w]  (Z rows 0..3 are replaced by zeros)
 __global__ void k_apply_q(int n, const double *V, const double *tau, const double *Z, double *C)
@@ -1182,12 +610,8 @@ tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val
                            float4 *ctr32_out, float4 *coef32_out, cudaStream_t st, double *h_stage)
 {
     const int m = n - 4;
-    // workspace: ctr 3n, Y 4n, Xw 4n, V 4n, P 4n, W 4n, Z 4n, KC 4n, tau 4, R 16, d 16, status
-    // ctr 3n, Y/Xw/V/P/W/Z/KC 4n each, tau 4, R 16, then the solve kernel's
-    // dependency counters (ints)
-    const int nblk = m > 0 ? (m + kNB - 1) / kNB : 0;
-    const size_t nflags = 4 + (size_t)(nblk + 1) + (size_t)(nblk + 1) * nblk + (size_t)nblk;
-    const size_t small = 3 * (size_t)n + 7 * 4 * (size_t)n + 4 + 16 + (nflags + 1) / 2;
+    // workspace: ctr 3n, Y/Xw/V/P/W/Z/KC 4n each, tau 4, R 16
+    const size_t small = 3 * (size_t)n + 7 * 4 * (size_t)n + 4 + 16;
     // stream-ordered workspace on `st`, returned to the pool on `st` when this
     // function exits (after the final wait, or with the error)
     StreamBuf ws{ctx, st}, abuf{ctx, st};
@@ -1206,12 +630,10 @@ tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val
     double *d_R = d_tau + 4;
     double *d_d = d_d_out;
     int *d_status = d_status_out;
-    int *d_flags = reinterpret_cast<int *>(d_R + 16);
     if (m > 0) {
-        abuf.bytes = (size_t)(m + 4) * m * sizeof(double);
+        abuf.bytes = chol_work_bytes(m);
         TW_TRY(dmalloc_on(ctx, &abuf.p, abuf.bytes, st));
     }
-    double *d_A = static_cast<double *>(abuf.p);
 
     std::vector<double> hY(4 * (size_t)n);
     for (int i = 0; i < n; ++i) {
@@ -1241,20 +663,9 @@ tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val
     k_wvec<<<1, kRedThreads, 0, st>>>(n, d_V, d_tau, d_P, d_W, d_Y, d_Z);
     nl += 2;
     if (m > 0) {
-        dim3 b(32, 8), g((m + 31) / 32, (m + 4 + 7) / 8);
-        k_fill_a<<<g, b, 0, st>>>(d_ctr, n, d_V, d_W, d_Z, lambda, d_A);
-        ++nl;
-        TW_CUDA_TRY(cudaFuncSetAttribute(k_chol_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem));
-        int per_sm = 0;
-        TW_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chol_solve, kSolveThreads, kSolveSmem));
-        if (per_sm < 1) return fail(ctx, TW_ERR_CUDA, "solve kernel does not fit on an SM");
-        int grid = ctx->sm_count;
-        TW_CUDA_TRY(cudaMemsetAsync(d_flags, 0, sizeof(int) * nflags, st));
-        unsigned long long limit_ns = ctx->solve_barrier_ns.load();
-        void *args[] = {(void *)&d_A, (void *)&m, (void *)&d_Z, (void *)&d_status, (void *)&d_flags, (void *)&limit_ns};
-        TW_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_chol_solve, dim3(grid), dim3(kSolveThreads), args,
-                                                kSolveSmem, st));
-        ++nl;
+        TW_CUDA_TRY(launch_chol_solve(d_ctr, n, d_V, d_W, d_Z, lambda, abuf.p, d_status, ctx->solve_barrier_ns.load(),
+                                      ctx->sm_count, st));
+        nl += 2;
     }
     k_apply_q<<<1, kRedThreads, 0, st>>>(n, d_V, d_tau, d_Z, d_c_out);
     k_kmul<<<kgrid, 32 * warps_per_block, 0, st>>>(d_ctr, n, d_c_out, d_KC);
