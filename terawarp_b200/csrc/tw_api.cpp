@@ -135,8 +135,12 @@ bool is_pinned_ptr(const void *p)
     return a.type == cudaMemoryTypeHost;
 }
 
-// Device aux block of a TPS: d (16 doubles) then the status word.
-static constexpr size_t kTpsAuxBytes = sizeof(double) * 16 + 16;
+// Device block of a TPS: the FP32 centres and coefficients (float4 each), c (4
+// doubles each), d (16 doubles), the status word.
+static size_t tps_block_bytes(int n)
+{
+    return (2 * sizeof(float4) + 4 * sizeof(double)) * (size_t)n + sizeof(double) * 16 + 16;
+}
 
 // Device-resident TPS field of one job: coefficients + node grid.
 tw_status make_tps(tw_ctx *ctx, const tw_marker *centres, const tw_marker *values, int n, double lambda,
@@ -162,22 +166,17 @@ tw_status make_tps(tw_ctx *ctx, const tw_marker *centres, const tw_marker *value
     // coefficients and the FP32 evaluation arrays (centres relative to o,
     // negated coefficients) are all written on `st` by the solve, which waits
     // for `st` once at its end; after that every stream may use them
-    const size_t cbytes = sizeof(double) * 4 * (size_t)n;
-    const size_t fbytes = sizeof(float4) * (size_t)n;
-    tw_status s = dmalloc_on(ctx, (void **)&t->d_c, cbytes, st);
-    if (s == TW_OK) s = dmalloc_on(ctx, (void **)&t->d_ctr32, fbytes, st);
-    if (s == TW_OK) s = dmalloc_on(ctx, (void **)&t->d_coef32, fbytes, st);
-    if (s == TW_OK) s = dmalloc_on(ctx, (void **)&t->d_d, kTpsAuxBytes, st);
-    if (s == TW_OK) {
-        t->d_status = reinterpret_cast<int *>(t->d_d + 16);
-        s = solve_tps_device(ctx, hc.data(), hv.data(), n, lambda, t->d_c, t->d_d, t->d_status,
-                             wait ? t->h_d : nullptr, o, t->d_ctr32, t->d_coef32, st, h_stage);
-    }
+    void *block = nullptr;
+    TW_TRY(dmalloc_on(ctx, &block, tps_block_bytes(n), st));
+    t->d_ctr32 = static_cast<float4 *>(block);
+    t->d_coef32 = t->d_ctr32 + n;
+    t->d_c = reinterpret_cast<double *>(t->d_coef32 + n);
+    t->d_d = t->d_c + 4 * (size_t)n;
+    t->d_status = reinterpret_cast<int *>(t->d_d + 16);
+    const tw_status s = solve_tps_device(ctx, hc.data(), hv.data(), n, lambda, t->d_c, t->d_d, t->d_status,
+                                         wait ? t->h_d : nullptr, o, t->d_ctr32, t->d_coef32, st, h_stage);
     if (s != TW_OK) {
-        dfree_on(ctx, t->d_c, cbytes, st);
-        dfree_on(ctx, t->d_ctr32, fbytes, st);
-        dfree_on(ctx, t->d_coef32, fbytes, st);
-        dfree_on(ctx, t->d_d, kTpsAuxBytes, st);
+        dfree_on(ctx, block, tps_block_bytes(n), st);
         return s;
     }
     for (int a = 0; a < 3; ++a) t->o32[a] = o[a];
@@ -191,10 +190,7 @@ void destroy_tps(tw_tps *t)
 {
     if (!t) return;
     tw_ctx *ctx = t->ctx;
-    dfree(ctx, t->d_c, sizeof(double) * 4 * (size_t)t->n);
-    dfree(ctx, t->d_ctr32, sizeof(float4) * (size_t)t->n);
-    dfree(ctx, t->d_coef32, sizeof(float4) * (size_t)t->n);
-    dfree(ctx, t->d_d, kTpsAuxBytes);
+    dfree(ctx, t->d_ctr32, tps_block_bytes(t->n));
     delete[] t->h_ctr;
     delete t;
 }

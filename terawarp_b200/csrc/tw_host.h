@@ -48,7 +48,8 @@ tw_status make_param_affine(int warp_mode, int deformation_mode, const double pa
 // chunks and the output back in z slabs, overlapping H2D, compute and D2H on
 // three streams.  `need(z0, z1, &lo, &hi)` returns the inclusive source z
 // range output planes [z0, z1) read; `compute(z0, z1, d_src, d_dst, st)`
-// enqueues the resample of those planes.
+// enqueues the resample of those planes.  With source and output both on the
+// device there is one `compute` call over every plane, and no `need` call.
 struct SlabIO {
     const void *src;          // host or device, src_planes x src_plane_bytes
     void *dst;                // host or device, dst_planes x dst_plane_bytes

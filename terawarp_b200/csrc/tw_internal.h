@@ -118,7 +118,8 @@ size_t chol_work_bytes(int m);
 cudaError_t launch_chol_solve(const double *ctr, int n, const double *V, const double *W, double *Z, double lambda,
                               void *work, int *status, unsigned long long limit_ns, int sm_count, cudaStream_t st);
 // Solves on `st`: c into d_c_out (n x 4), d into d_d_out (4 x 4) and the
-// status bits into d_status_out, all device memory that outlives the call.
+// status bits into d_status_out (the word after d), all device memory that
+// outlives the call.
 // With h_d_out it waits for `st` once, at the end, copies d to the host and
 // turns the status into the return value; without it nothing waits and the
 // caller reads the status later (solve_status).  When ctr32_out and
@@ -196,6 +197,7 @@ struct tw_ctx {
 struct tw_tps {
     tw_ctx *ctx = nullptr;
     int n = 0;
+    // one device block, d_ctr32 first
     double *d_c = nullptr;     // device n x 4 (FP64)
     double h_d[16] = {0};      // host 4 x 4 (FP64), valid once the solve was waited for
     double *d_d = nullptr;     // device 4 x 4 (FP64)

@@ -74,6 +74,13 @@ struct StreamBlock {
     ~StreamBlock() { if (p) dfree_on(ctx, p, bytes, st); }
 };
 
+// A small block of the context's pool outside its budget.
+struct PoolBlock {
+    cudaStream_t st = nullptr;
+    void *p = nullptr;
+    ~PoolBlock() { if (p) cudaFreeAsync(p, st); }
+};
+
 }  // namespace
 
 tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
@@ -139,7 +146,7 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
         return TW_OK;
     }
     RJob *d_jobs = nullptr;
-    TW_CUDA_TRY(cudaMallocAsync((void **)&d_jobs, bytes, st));
+    TW_CUDA_TRY(cudaMallocFromPoolAsync((void **)&d_jobs, bytes, ctx->pool, st));
     TW_CUDA_TRY(cudaMemcpyAsync(d_jobs, jobs, bytes, cudaMemcpyHostToDevice, st));
     cudaError_t e = launch_resample(d_jobs, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
                                     ctx->sm_count, ctx->d_err, d_fb);
@@ -289,14 +296,17 @@ tw_status tps_layer_zhull(tw_ctx *ctx, const float4 *nodes, const int64_t gsz[3]
     zmin.assign(layers, 0.f);
     zmax.assign(layers, 0.f);
     if (layers <= 0) return TW_OK;
-    float *d = nullptr;
-    TW_CUDA_TRY(cudaMallocAsync((void **)&d, sizeof(float) * 2 * layers, st));
+    // from the context's pool, which keeps its blocks: the device's default
+    // pool gives its memory back at every synchronisation, so a block of it
+    // cost milliseconds of mapping per call
+    PoolBlock b{st};
+    TW_CUDA_TRY(cudaMallocFromPoolAsync(&b.p, sizeof(float) * 2 * (size_t)layers, ctx->pool, st));
+    float *d = static_cast<float *>(b.p);
     k_layer_zhull<<<(unsigned)layers, 256, 0, st>>>(nodes, gsz[0], gsz[1], g, d, d + layers);
     TW_CUDA_TRY(cudaGetLastError());
     count_launch(ctx);
     TW_CUDA_TRY(cudaMemcpyAsync(zmin.data(), d, sizeof(float) * layers, cudaMemcpyDeviceToHost, st));
     TW_CUDA_TRY(cudaMemcpyAsync(zmax.data(), d + layers, sizeof(float) * layers, cudaMemcpyDeviceToHost, st));
-    cudaFreeAsync(d, st);
     TW_CUDA_TRY(cudaStreamSynchronize(st));
     return TW_OK;
 }
@@ -315,18 +325,16 @@ tw_status tps_box_hull(tw_ctx *ctx, const float4 *nodes, const int64_t gsz[3], i
             hb[6 * i + a] = boxes[i].c0[a];
             hb[6 * i + 3 + a] = boxes[i].c1[a];
         }
-    int64_t *db = nullptr;
-    float *dh = nullptr;
-    TW_CUDA_TRY(cudaMallocAsync((void **)&db, sizeof(int64_t) * 6 * nb, st));
-    TW_CUDA_TRY(cudaMallocAsync((void **)&dh, sizeof(float) * 6 * nb, st));
+    PoolBlock b{st};
+    TW_CUDA_TRY(cudaMallocFromPoolAsync(&b.p, (sizeof(int64_t) + sizeof(float)) * 6 * nb, ctx->pool, st));
+    int64_t *db = static_cast<int64_t *>(b.p);
+    float *dh = reinterpret_cast<float *>(db + 6 * nb);
     TW_CUDA_TRY(cudaMemcpyAsync(db, hb.data(), sizeof(int64_t) * 6 * nb, cudaMemcpyHostToDevice, st));
     k_box_hull<<<(unsigned)nb, 256, 0, st>>>(nodes, gsz[0], gsz[1], gsz[2], g, db, dh, dh + 3 * nb);
     TW_CUDA_TRY(cudaGetLastError());
     count_launch(ctx);
     TW_CUDA_TRY(cudaMemcpyAsync(lo.data(), dh, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, st));
     TW_CUDA_TRY(cudaMemcpyAsync(hi.data(), dh + 3 * nb, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, st));
-    cudaFreeAsync(db, st);
-    cudaFreeAsync(dh, st);
     TW_CUDA_TRY(cudaStreamSynchronize(st));
     return TW_OK;
 }
@@ -431,6 +439,13 @@ tw_status stream_slabs(tw_ctx *ctx, const SlabIO &io,
                        const std::function<tw_status(int64_t, int64_t, const void *, void *, cudaStream_t)> &compute)
 {
     const bool src_dev = is_device_ptr(io.src), dst_dev = is_device_ptr(io.dst);
+    if (src_dev && dst_dev) {
+        // nothing to stream: the whole volume in one launch; in slabs only
+        // when its workspace does not fit the budget
+        const tw_status s = compute(0, io.dst_planes, io.src, io.dst, ctx->stream);
+        if (s == TW_OK) return check_kernel_errors(ctx);
+        if (s != TW_ERR_OOM) return s;
+    }
     const bool src_pin = !src_dev && is_pinned_ptr(io.src), dst_pin = !dst_dev && is_pinned_ptr(io.dst);
     const size_t src_bytes = io.src_plane_bytes * (size_t)io.src_planes;
     const size_t dst_bytes = io.dst_plane_bytes * (size_t)io.dst_planes;
@@ -448,8 +463,8 @@ tw_status stream_slabs(tw_ctx *ctx, const SlabIO &io,
         TW_TRY(dmalloc(ctx, &d_dst, dst_bytes));
         gd.p = d_dst; gd.b = dst_bytes;
     }
-    // source chunks of ~64 MiB (whole planes)
-    int64_t chunk = std::max<int64_t>(1, (int64_t)((64ull << 20) / std::max<size_t>(io.src_plane_bytes, 1)));
+    // source chunks of ~16 MiB (whole planes): 0.3 ms of the link each
+    int64_t chunk = std::max<int64_t>(1, (int64_t)((16ull << 20) / std::max<size_t>(io.src_plane_bytes, 1)));
     chunk = std::min(chunk, io.src_planes);
     const int64_t nchunks = (io.src_planes + chunk - 1) / chunk;
     const int64_t nslabs = (io.dst_planes + io.slab - 1) / io.slab;
@@ -514,7 +529,7 @@ tw_status stream_slabs(tw_ctx *ctx, const SlabIO &io,
     for (int64_t s = 0; s < nslabs; ++s) {
         const int64_t z0 = s * io.slab, z1 = std::min(io.dst_planes, z0 + io.slab);
         int64_t lo = 0, hi = io.src_planes - 1;
-        need(z0, z1, lo, hi);
+        if (!src_dev) need(z0, z1, lo, hi);
         hi = std::max<int64_t>(0, std::min(hi, io.src_planes - 1));
         TW_TRY(upload_until(hi));
         TW_TRY(compute(z0, z1, d_src, d_dst, ctx->stream));

@@ -13,11 +13,12 @@ using namespace tw;
 
 namespace {
 
+// A block used on the context's compute stream only (no host wait either way).
 struct DevGuard {
     tw_ctx *ctx;
     void *p = nullptr;
     size_t bytes = 0;
-    ~DevGuard() { if (p) dfree(ctx, p, bytes); }
+    ~DevGuard() { if (p) dfree_on(ctx, p, bytes, ctx->stream); }
 };
 
 struct TpsGuard {
@@ -27,10 +28,13 @@ struct TpsGuard {
 
 size_t elem_size(int dtype) { return dtype == TW_U8 ? 1 : 2; }
 
-// Output planes per slab: ~256 MiB of output, a multiple of `align`.
+// Output planes per slab: ~32 MiB of output, a multiple of `align`.  Copies in
+// both directions overlap only from the first finished slab on, and the last
+// slab's copy back overlaps nothing, so a slab is kept to about 0.6 ms of the
+// link; its launches take about 0.1 ms.
 int64_t pick_slab(size_t plane_bytes, int64_t planes, int64_t align)
 {
-    int64_t s = (int64_t)((256ull << 20) / std::max<size_t>(plane_bytes, 1));
+    int64_t s = (int64_t)((32ull << 20) / std::max<size_t>(plane_bytes, 1));
     s = std::max<int64_t>(align, (s / align) * align);
     return std::min<int64_t>(s, ((planes + align - 1) / align) * align);
 }
@@ -42,7 +46,7 @@ tw_status tps_warp_volume(tw_ctx *ctx, const float4 *nodes, int g, int dtype, in
 {
     const int64_t gsz[3] = {grid_size(dst_sz[0], g), grid_size(dst_sz[1], g), grid_size(dst_sz[2], g)};
     std::vector<float> zmin, zmax;
-    TW_TRY(tps_layer_zhull(ctx, nodes, gsz, g, ctx->stream, zmin, zmax));
+    if (!is_device_ptr(src)) TW_TRY(tps_layer_zhull(ctx, nodes, gsz, g, ctx->stream, zmin, zmax));
     const size_t es = elem_size(dtype);
     SlabIO io;
     io.src = src;
@@ -114,7 +118,7 @@ tw_status build_tps_field(tw_ctx *ctx, const tw_marker *centres, const tw_marker
     TW_TRY(make_tps(ctx, centres, values, n, lambda, scale, ctx->stream, &tg.t));
     const int64_t gsz[3] = {grid_size(dst_sz[0], g), grid_size(dst_sz[1], g), grid_size(dst_sz[2], g)};
     nodes.bytes = sizeof(float4) * (size_t)(gsz[0] * gsz[1] * gsz[2]);
-    TW_TRY(dmalloc(ctx, &nodes.p, nodes.bytes));
+    TW_TRY(dmalloc_on(ctx, &nodes.p, nodes.bytes, ctx->stream));
     const int64_t off[3] = {0, 0, 0};
     return eval_grid(ctx, tg.t, gsz, g, off, static_cast<float4 *>(nodes.p), ctx->stream);
 }

@@ -588,13 +588,6 @@ __global__ void __launch_bounds__(kFitThreads) k_affine_fit(double *tar, double 
     }
 }
 
-struct DevBuf {
-    tw_ctx *ctx = nullptr;
-    void *p = nullptr;
-    size_t bytes = 0;
-    ~DevBuf() { if (p) dfree(ctx, p, bytes); }
-};
-
 struct StreamBuf {
     tw_ctx *ctx = nullptr;
     cudaStream_t st = nullptr;
@@ -604,6 +597,18 @@ struct StreamBuf {
 };
 
 }  // namespace
+
+// The status word of a solve as a tw_status.
+static tw_status status_of(tw_ctx *ctx, int status)
+{
+    if (status & kStSingularX)
+        return fail(ctx, TW_ERR_SINGULAR, "TPS centres are degenerate: [1 s] is rank deficient (coplanar or < 4 distinct points)");
+    if (status & kStTimeout)
+        return fail(ctx, TW_ERR_TIMEOUT, "TPS solve: a wait on another block of the solve timed out");
+    if (status & kStNotSPD)
+        return fail(ctx, TW_ERR_SINGULAR, "projected TPS system is not positive definite");
+    return TW_OK;
+}
 
 tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val, int n, double lambda,
                            double *d_c_out, double *d_d_out, int *d_status_out, double *h_d_out, const double o[3],
@@ -645,14 +650,13 @@ tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val
     if (h_stage) {
         std::memcpy(h_stage, h_ctr, sizeof(double) * 3 * n);
         std::memcpy(h_stage + 3 * (size_t)n, hY.data(), sizeof(double) * 4 * n);
-        TW_CUDA_TRY(cudaMemcpyAsync(d_ctr, h_stage, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-        TW_CUDA_TRY(cudaMemcpyAsync(d_Y, h_stage + 3 * (size_t)n, sizeof(double) * 4 * n, cudaMemcpyHostToDevice, st));
-    } else {
-        TW_TRY(upload(ctx, d_ctr, h_ctr, sizeof(double) * 3 * n, st));
-        TW_TRY(upload(ctx, d_Y, hY.data(), sizeof(double) * 4 * n, st));
+        TW_CUDA_TRY(cudaMemcpyAsync(d_ctr, h_stage, sizeof(double) * 7 * n, cudaMemcpyHostToDevice, st));
+    } else {  // (centres and values are consecutive in the workspace)
+        hY.insert(hY.begin(), h_ctr, h_ctr + 3 * (size_t)n);
+        TW_TRY(upload(ctx, d_ctr, hY.data(), sizeof(double) * 7 * n, st));
     }
-    TW_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));
-    TW_CUDA_TRY(cudaMemsetAsync(d_d, 0, sizeof(double) * 16, st));
+    // d, and the status word after it
+    TW_CUDA_TRY(cudaMemsetAsync(d_d, 0, sizeof(double) * 16 + sizeof(int), st));
 
     uint64_t nl = 0;
     k_qr<<<1, kRedThreads, 0, st>>>(d_ctr, n, d_Xw, d_V, d_tau, d_R, d_status);
@@ -678,8 +682,12 @@ tw_status solve_tps_device(tw_ctx *ctx, const double *h_ctr, const double *h_val
     TW_CUDA_TRY(cudaGetLastError());
     count_launch(ctx, nl);
     if (!h_d_out) return TW_OK;  // the caller reads the status later
-    TW_CUDA_TRY(cudaMemcpyAsync(h_d_out, d_d, sizeof(double) * 16, cudaMemcpyDeviceToHost, st));
-    return solve_status(ctx, d_status, st);
+    // d and the status word after it in one copy
+    struct { double d[16]; int status; } h;
+    TW_CUDA_TRY(cudaMemcpyAsync(&h, d_d, sizeof(double) * 16 + sizeof(int), cudaMemcpyDeviceToHost, st));
+    TW_CUDA_TRY(cudaStreamSynchronize(st));
+    std::memcpy(h_d_out, h.d, sizeof(h.d));
+    return status_of(ctx, h.status);
 }
 
 tw_status solve_status(tw_ctx *ctx, const int *d_status, cudaStream_t st)
@@ -687,36 +695,32 @@ tw_status solve_status(tw_ctx *ctx, const int *d_status, cudaStream_t st)
     int status = 0;
     TW_CUDA_TRY(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     TW_CUDA_TRY(cudaStreamSynchronize(st));
-    if (status & kStSingularX)
-        return fail(ctx, TW_ERR_SINGULAR, "TPS centres are degenerate: [1 s] is rank deficient (coplanar or < 4 distinct points)");
-    if (status & kStTimeout)
-        return fail(ctx, TW_ERR_TIMEOUT, "TPS solve: a wait on another block of the solve timed out");
-    if (status & kStNotSPD)
-        return fail(ctx, TW_ERR_SINGULAR, "projected TPS system is not positive definite");
-    return TW_OK;
+    return status_of(ctx, status);
 }
 
 tw_status fit_affine_device(tw_ctx *ctx, const double *h_tar, const double *h_sub, int n, double M[16],
                             cudaStream_t st)
 {
-    DevBuf ws{ctx};
+    StreamBuf ws{ctx, st};
     ws.bytes = sizeof(double) * (6 * (size_t)n + 16 + 2);
-    TW_TRY(dmalloc(ctx, &ws.p, ws.bytes));
+    TW_TRY(dmalloc_on(ctx, &ws.p, ws.bytes, st));
     double *d_tar = static_cast<double *>(ws.p);
     double *d_sub = d_tar + 3 * (size_t)n;
     double *d_out = d_sub + 3 * (size_t)n;
     int *d_status = reinterpret_cast<int *>(d_out + 16);
-    TW_CUDA_TRY(cudaMemcpyAsync(d_tar, h_tar, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-    TW_CUDA_TRY(cudaMemcpyAsync(d_sub, h_sub, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st));
-    TW_CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), st));
+    // landmarks, a zero matrix and a zero status word in one upload
+    std::vector<double> h(6 * (size_t)n + 18, 0.0);
+    std::memcpy(h.data(), h_tar, sizeof(double) * 3 * n);
+    std::memcpy(h.data() + 3 * (size_t)n, h_sub, sizeof(double) * 3 * n);
+    TW_TRY(upload(ctx, ws.p, h.data(), ws.bytes, st));
     k_affine_fit<<<1, kFitThreads, 0, st>>>(d_tar, d_sub, n, d_out, d_status);
     TW_CUDA_TRY(cudaGetLastError());
     count_launch(ctx, 1);
-    int status = 0;
-    TW_CUDA_TRY(cudaMemcpyAsync(M, d_out, sizeof(double) * 16, cudaMemcpyDeviceToHost, st));
-    TW_CUDA_TRY(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    struct { double M[16]; int status; } r;
+    TW_CUDA_TRY(cudaMemcpyAsync(&r, d_out, sizeof(double) * 16 + sizeof(int), cudaMemcpyDeviceToHost, st));
     TW_CUDA_TRY(cudaStreamSynchronize(st));
-    if (status) return fail(ctx, TW_ERR_SINGULAR, "affine DLT is degenerate (h13 = 0)");
+    std::memcpy(M, r.M, sizeof(r.M));
+    if (r.status) return fail(ctx, TW_ERR_SINGULAR, "affine DLT is degenerate (h13 = 0)");
     return TW_OK;
 }
 
