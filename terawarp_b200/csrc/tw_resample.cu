@@ -296,11 +296,13 @@ __device__ __forceinline__ void store_packed(T *p, uint32_t w, bool pair_ok, int
     }
 }
 
-// Magic float 2^23 + v for a loaded voxel value v (exact for v < 2^23).
+// A voxel value taken as it is loaded, as the bits of a float: the subnormal
+// v 2^-149, exact.  The x lerps scale it (see trilerp2), so no instruction
+// converts it; FP32 multiply-adds take subnormals at full rate.
 template <typename T>
-__device__ __forceinline__ float mag(const T *p)
+__device__ __forceinline__ float raw(const T *p)
 {
-    return __int_as_float(0x4B000000 | (int)(uint32_t)__ldg(p));
+    return __int_as_float((int)(uint32_t)__ldg(p));
 }
 
 // The four source rows a trilinear sample reads, (dy, dz) = (r & 1, r >> 1),
@@ -354,18 +356,28 @@ __device__ __forceinline__ const T *wide_addr(const T *base, uint32_t o)
     return p;
 }
 
-// Trilinear value of a voxel pair from the magic floats 2^23 + v of its taps:
-// lo[r] / hi[r] hold the x and x+1 taps of source row r = (dy, dz) =
-// (r & 1, r >> 1), as (voxel 0, voxel 1).  Every sampler (global gathers,
-// staged shared memory, checked or not) ends in this one sequence of
+// Trilinear value of a voxel pair from its raw taps: lo[r] / hi[r] hold the x
+// and x+1 taps of source row r = (dy, dz) = (r & 1, r >> 1), as (voxel 0,
+// voxel 1); nfx is minus the x fraction.  The result is -v 2^-23: the taps
+// come in scaled by 2^-149, the x lerps multiply them by 2^126 on the way, and
+// the sign lets every product take its operands as they are (FP32x2 has no
+// negated operands).  Scaling by a power of two and negation are exact and
+// commute with rounding, so this is the trilinear sample of the voxel values
+// to the last bit.  Against taps turned into 2^23 + v by an integer OR each, a
+// voxel pair takes 16 instructions of 133 less.  Every sampler (global
+// gathers, staged shared memory, checked or not) ends in this one sequence of
 // operations, so a voxel's value does not depend on which path produced it.
-__device__ __forceinline__ float2 trilerp2(const float2 (&lo)[4], const float2 (&hi)[4], float2 fx, float2 fy,
+constexpr float kTapScale = 8.507059173023462e37f;  // 2^126
+constexpr float kOutScale = 8388608.0f;             // 2^23
+__device__ __forceinline__ float2 trilerp2(const float2 (&lo)[4], const float2 (&hi)[4], float2 nfx, float2 fy,
                                            float2 fz)
 {
     float2 ax[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)  // (2^23 + b) - (2^23 + a) = b - a exactly
-        ax[r] = fma2(fx, sub2(hi[r], lo[r]), sub2(lo[r], f2(8388608.f, 8388608.f)));
+    for (int r = 0; r < 4; ++r) {
+        const float2 nb = __fmul2_rn(lo[r], f2(-kTapScale, -kTapScale));
+        ax[r] = fma2(nfx, fma2(hi[r], f2(kTapScale, kTapScale), nb), nb);  // -(lo + fx (hi - lo))
+    }
     const float2 b0 = fma2(fy, sub2(ax[1], ax[0]), ax[0]);
     const float2 b1 = fma2(fy, sub2(ax[3], ax[2]), ax[2]);
     return fma2(fz, sub2(b1, b0), b0);
@@ -374,12 +386,12 @@ __device__ __forceinline__ float2 trilerp2(const float2 (&lo)[4], const float2 (
 // Unchecked sample of a voxel pair at positions (p0, p1, pz2): every tap is
 // known to be inside the volume and the buffer (hull test), offsets fit int32.
 // Trilinear value of a voxel pair from the offsets of its (0,0,0) taps and
-// its fractions (fx, fy, fz), as a pair (voxel 0, voxel 1).
+// its fractions (nfx = -fx, fy, fz), as a pair (voxel 0, voxel 1).
 template <typename T>
-__device__ __forceinline__ float2 lerp_pair(const Rows<T> &R, uint32_t off0, uint32_t off1, float2 fx, float2 fy,
+__device__ __forceinline__ float2 lerp_pair(const Rows<T> &R, uint32_t off0, uint32_t off1, float2 nfx, float2 fy,
                                             float2 fz)
 {
-    // magic floats of the 8 taps of both voxels: one wide address per voxel,
+    // the 8 taps of both voxels: one wide address per voxel,
     // the other rows at the brick's constant row / plane offsets
     float2 lo[4], hi[4];
     const T *a0 = wide_addr(R.rb[0], off0), *a1 = wide_addr(R.rb[0], off1);
@@ -387,21 +399,22 @@ __device__ __forceinline__ float2 lerp_pair(const Rows<T> &R, uint32_t off0, uin
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const T *q0 = a0 + rofs[r], *q1 = a1 + rofs[r];
-        lo[r] = f2(mag(q0), mag(q1));
-        hi[r] = f2(mag(q0 + 1), mag(q1 + 1));
+        lo[r] = f2(raw(q0), raw(q1));
+        hi[r] = f2(raw(q0 + 1), raw(q1 + 1));
     }
-    return trilerp2(lo, hi, fx, fy, fz);
+    return trilerp2(lo, hi, nfx, fy, fz);
 }
 
-// Output words of a voxel pair: TPS rounds (+0.5), affine truncates; v is a
-// convex combination of voxel values (rounding can leave -0.0x), so
-// 2^23 + floor(v) has the output in its low bits.
+// Output words of a voxel pair from trilerp2's -v 2^-23: TPS rounds (+0.5),
+// affine truncates; v is a convex combination of voxel values (rounding can
+// leave -0.0x), so 2^23 + floor(v) has the output in its low bits.
 template <typename T, bool ROUND>
-__device__ __forceinline__ float2 out_pair(float2 v)
+__device__ __forceinline__ float2 out_pair(float2 nv)
 {
-    if (ROUND) v = add2(v, f2(0.5f, 0.5f));
-    else v = f2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f));
-    return __fadd2_rd(v, f2(8388608.f, 8388608.f));
+    const float2 S = f2(-kOutScale, -kOutScale);
+    if (ROUND) return __fadd2_rd(fma2(nv, S, f2(0.5f, 0.5f)), f2(8388608.f, 8388608.f));
+    nv = f2(fminf(nv.x, 0.f), fminf(nv.y, 0.f));
+    return __ffma2_rd(nv, S, f2(8388608.f, 8388608.f));
 }
 
 template <typename T, bool ROUND>
@@ -413,7 +426,7 @@ __device__ __forceinline__ void pair_fast2(float2 p0, float2 p1, float2 pz2, con
     const float2 f0 = sub2(p0, sub2(m0, MM)), f1 = sub2(p1, sub2(m1, MM)), fz = sub2(pz2, sub2(mz, MM));
     const uint32_t off0 = tap_offset(R, m0.x, m0.y, mz.x);
     const uint32_t off1 = tap_offset(R, m1.x, m1.y, mz.y);
-    const float2 t = out_pair<T, ROUND>(lerp_pair(R, off0, off1, f2(f0.x, f1.x), f2(f0.y, f1.y), fz));
+    const float2 t = out_pair<T, ROUND>(lerp_pair(R, off0, off1, f2(-f0.x, -f1.x), f2(f0.y, f1.y), fz));
     packed = pack_pair<T>(__float_as_uint(t.x), __float_as_uint(t.y));
 }
 
@@ -445,7 +458,7 @@ __device__ __forceinline__ void pair_clamped2(float2 p0, float2 p1, float2 pz2, 
     const float2 m0 = add2(l0, MM), m1 = add2(l1, MM), mz = add2(lz2, MM);  // exact: integers
     const uint32_t off0 = tap_offset(R, m0.x, m0.y, mz.x);
     const uint32_t off1 = tap_offset(R, m1.x, m1.y, mz.y);
-    const float2 t = out_pair<T, ROUND>(lerp_pair(R, off0, off1, f2(f0.x, f1.x), f2(f0.y, f1.y), fz));
+    const float2 t = out_pair<T, ROUND>(lerp_pair(R, off0, off1, f2(-f0.x, -f1.x), f2(f0.y, f1.y), fz));
     // a rejected voxel writes 0: the bits of 2^23 have zero low bits
     packed = pack_pair<T>(ok0 ? __float_as_uint(t.x) : 0x4B000000u, ok1 ? __float_as_uint(t.y) : 0x4B000000u);
 }
@@ -486,10 +499,10 @@ __device__ __forceinline__ void pair_checked2(float2 p0, float2 p1, float2 pz2, 
     for (int r = 0; r < 4; ++r) {
         const T *r0 = base + ((OFF)zs0[r >> 1] * pz + (OFF)ys0[r & 1] * py);
         const T *r1 = base + ((OFF)zs1[r >> 1] * pz + (OFF)ys1[r & 1] * py);
-        lo[r] = f2(mag(r0 + xa0), mag(r1 + xa1));
-        hi[r] = f2(mag(r0 + xb0), mag(r1 + xb1));
+        lo[r] = f2(raw(r0 + xa0), raw(r1 + xa1));
+        hi[r] = f2(raw(r0 + xb0), raw(r1 + xb1));
     }
-    const float2 t = out_pair<T, ROUND>(trilerp2(lo, hi, f2(f0.x, f1.x), f2(f0.y, f1.y), fz));
+    const float2 t = out_pair<T, ROUND>(trilerp2(lo, hi, f2(-f0.x, -f1.x), f2(f0.y, f1.y), fz));
     // a rejected voxel writes 0: the bits of 2^23 have zero low bits
     packed = pack_pair<T>(ok0 ? __float_as_uint(t.x) : 0x4B000000u, ok1 ? __float_as_uint(t.y) : 0x4B000000u);
 }
@@ -1092,30 +1105,25 @@ __device__ __forceinline__ void plane_positions(const RowLayer &L, float4 wz, fl
     pz = fma2(w0, L.P[0][2], fma2(w1, L.P[1][2], fma2(w2, L.P[2][2], fma2(w3, L.P[3][2], f2(0.f, 0.f)))));
 }
 
-// Offset (from the ring base) of the (x, y, z) = floor tap of a staged
-// sample: the in-plane byte offset comes as the magic float kMagic + offset
-// (exact for offsets below 2^22 in magnitude, and every tap of the staged
-// window is), the slot from the z floor's magic bit pattern; cz maps a tap
-// plane to its plane sequence (mod kRing: the slot).  Clamped so that all 8
-// taps stay in the ring whatever the position (an out-of-range or NaN
-// position gives some offset in the ring, for a sample whose value the
-// range rule discards).
+// Offset of the floor tap of a staged sample at frame floors (x, y, z): byte
+// z PLANE_B + y ROW_B + x ES + k of the ring, taken modulo the ring's size (a
+// power of two: plane sequence s is slot s mod kRing).  The sum is formed in
+// floating point on both voxels at once, as kMagic + offset, whose bit
+// pattern's low bits are the offset (exact: every tap of a walk is within 2^22
+// bytes of its layer's frame).  Whatever the position -- NaN included -- the
+// masked offset is an element of the ring and its taps lie in shared memory
+// (the last plane's past it, in the mirror of slot 0 and the barriers after).
+//
+// layer_k: kMagic + k for the cell layer with frame origin Oz of a walk whose
+// first plane (output plane z0 + a) has sequence seq0: the source plane Oz + z
+// has sequence seq0 + (Oz + z) - (z0 + a); DY, DX: row / column of frame (0, 0)
+// in the staged box.
 template <typename T>
-__device__ __forceinline__ uint32_t staged_off(uint32_t omax, uint32_t cz, float mz, float mxy)
+__device__ __forceinline__ float layer_k(uint32_t seq0, int64_t Oz, int64_t z0, const Plan &P)
 {
-    constexpr uint32_t PLANE_B = kHMax * kBoxW * sizeof(T);
-    const uint32_t slot = (__float_as_uint(mz) + cz) & (uint32_t)(kRing - 1);
-    const uint32_t o = slot * PLANE_B + (__float_as_uint(mxy) - (uint32_t)kMagicBits);
-    return min(o, omax);
-}
-
-// cz of staged_off for the cell layer with frame origin Oz of a walk whose
-// first plane (output plane z0 + a) has sequence seq0: the source plane
-// Oz + iz has sequence seq0 + (Oz + iz) - (z0 + a), and the magic floor's
-// bit pattern of iz is kMagicBits + iz (2^32 wrap arithmetic).
-__device__ __forceinline__ uint32_t layer_cz(uint32_t seq0, int64_t Oz, int64_t z0, int a)
-{
-    return seq0 + (uint32_t)(Oz - z0) - (uint32_t)a - (uint32_t)kMagicBits;
+    constexpr int ES = sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
+    const uint32_t slot = (seq0 + (uint32_t)(Oz - z0) - (uint32_t)P.a) & (uint32_t)(kRing - 1);
+    return kMagic + (float)((int)slot * PLANE_B + P.DY * ROW_B + P.DX * ES);
 }
 
 // A voxel pair of an interior walk from the staged planes, in three steps
@@ -1127,64 +1135,61 @@ __device__ __forceinline__ uint32_t layer_cz(uint32_t seq0, int64_t Oz, int64_t 
 // same floors, fractions and trilinear arithmetic (trilerp2) as the gather
 // kernel's samplers.
 struct PairPrep {
-    float2 fx, fy, fz;
-    uint32_t a0, a1;  // shared-window addresses of the floor taps of voxel 0 / 1 in the ring
+    float2 nfx, fy, fz;  // fractions (x negated, as trilerp2 takes it)
+    uint32_t a0, a1;     // shared-window addresses of the floor taps of voxel 0 / 1 in the ring
 };
 
-// ring: shared-window address of slot 0; kc = kMagic + the byte offset of
-// frame (0, 0) in a plane slot.  The floors are integers below 2^22 in
-// magnitude, so fly ROW_B + flx ES + kc is exact whenever the tap lies in
-// the staged window.
+// ring: shared-window address of slot 0; k: layer_k of the cell layer.
 template <typename T>
-__device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float kc, uint32_t omax, uint32_t cz, float2 px,
-                                              float2 py, float2 pz)
+__device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px, float2 py, float2 pz)
 {
-    constexpr float ROW_B = (float)(kBoxW * sizeof(T)), ES = (float)sizeof(T);
+    constexpr float ES = (float)sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
+    constexpr uint32_t RING = kRing * kHMax * kBoxW * (uint32_t)sizeof(T), MASK = RING - (uint32_t)sizeof(T);
+    static_assert((RING & (RING - 1)) == 0 && (kMagicBits & (RING - 1)) == 0, "the ring is a power of two of bytes");
     const float2 MM = f2(kMagic, kMagic);
     const float2 mx = __fadd2_rd(px, MM), my = __fadd2_rd(py, MM), mz = __fadd2_rd(pz, MM);
-    const float2 flx = sub2(mx, MM), fly = sub2(my, MM);
+    const float2 flx = sub2(mx, MM), fly = sub2(my, MM), flz = sub2(mz, MM);
     PairPrep q;
-    q.fx = sub2(px, flx);
+    q.nfx = sub2(flx, px);
     q.fy = sub2(py, fly);
-    q.fz = sub2(pz, sub2(mz, MM));
-    const float2 mxy = fma2(fly, f2(ROW_B, ROW_B), fma2(flx, f2(ES, ES), f2(kc, kc)));
-    q.a0 = ring + staged_off<T>(omax, cz, mz.x, mxy.x);
-    q.a1 = ring + staged_off<T>(omax, cz, mz.y, mxy.y);
+    q.fz = sub2(pz, flz);
+    const float2 o = fma2(flz, f2(PLANE_B, PLANE_B), fma2(fly, f2(ROW_B, ROW_B), fma2(flx, f2(ES, ES), f2(k, k))));
+    q.a0 = ring + (__float_as_uint(o.x) & MASK);
+    q.a1 = ring + (__float_as_uint(o.y) & MASK);
     return q;
 }
 
-// Magic float 2^23 + v of the staged voxel at shared-window address a + OFF:
-// a 32-bit address with the constant offset folded into the load.  Volatile,
+// The staged voxel at shared-window address a + OFF as raw() takes it: a 32-bit address with the constant offset folded into the load.  Volatile,
 // so it stays after the wait for its plane.
 template <typename T, int OFF>
-__device__ __forceinline__ float lds_mag(uint32_t a)
+__device__ __forceinline__ float lds_raw(uint32_t a)
 {
     uint32_t v;
     if (sizeof(T) == 2) asm volatile("ld.shared.u16 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
     else asm volatile("ld.shared.u8 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
-    return __int_as_float(0x4B000000 | (int)v);
+    return __int_as_float((int)v);
 }
 
-// The eight taps of both voxels as magic floats: constant row, plane and
+// The eight taps of both voxels: constant row, plane and
 // element offsets from each voxel's floor tap.
 template <typename T>
 __device__ __forceinline__ void taps_pair(const PairPrep &q, float2 (&lo)[4], float2 (&hi)[4])
 {
     constexpr int ES = sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
-    lo[0] = f2(lds_mag<T, 0>(q.a0), lds_mag<T, 0>(q.a1));
-    hi[0] = f2(lds_mag<T, ES>(q.a0), lds_mag<T, ES>(q.a1));
-    lo[1] = f2(lds_mag<T, ROW_B>(q.a0), lds_mag<T, ROW_B>(q.a1));
-    hi[1] = f2(lds_mag<T, ROW_B + ES>(q.a0), lds_mag<T, ROW_B + ES>(q.a1));
-    lo[2] = f2(lds_mag<T, PLANE_B>(q.a0), lds_mag<T, PLANE_B>(q.a1));
-    hi[2] = f2(lds_mag<T, PLANE_B + ES>(q.a0), lds_mag<T, PLANE_B + ES>(q.a1));
-    lo[3] = f2(lds_mag<T, PLANE_B + ROW_B>(q.a0), lds_mag<T, PLANE_B + ROW_B>(q.a1));
-    hi[3] = f2(lds_mag<T, PLANE_B + ROW_B + ES>(q.a0), lds_mag<T, PLANE_B + ROW_B + ES>(q.a1));
+    lo[0] = f2(lds_raw<T, 0>(q.a0), lds_raw<T, 0>(q.a1));
+    hi[0] = f2(lds_raw<T, ES>(q.a0), lds_raw<T, ES>(q.a1));
+    lo[1] = f2(lds_raw<T, ROW_B>(q.a0), lds_raw<T, ROW_B>(q.a1));
+    hi[1] = f2(lds_raw<T, ROW_B + ES>(q.a0), lds_raw<T, ROW_B + ES>(q.a1));
+    lo[2] = f2(lds_raw<T, PLANE_B>(q.a0), lds_raw<T, PLANE_B>(q.a1));
+    hi[2] = f2(lds_raw<T, PLANE_B + ES>(q.a0), lds_raw<T, PLANE_B + ES>(q.a1));
+    lo[3] = f2(lds_raw<T, PLANE_B + ROW_B>(q.a0), lds_raw<T, PLANE_B + ROW_B>(q.a1));
+    hi[3] = f2(lds_raw<T, PLANE_B + ROW_B + ES>(q.a0), lds_raw<T, PLANE_B + ROW_B + ES>(q.a1));
 }
 
 template <typename T>
 __device__ __forceinline__ uint32_t finish_pair(const PairPrep &q, const float2 (&lo)[4], const float2 (&hi)[4])
 {
-    const float2 t = out_pair<T, true>(trilerp2(lo, hi, q.fx, q.fy, q.fz));
+    const float2 t = out_pair<T, true>(trilerp2(lo, hi, q.nfx, q.fy, q.fz));
     return pack_pair<T>(__float_as_uint(t.x), __float_as_uint(t.y));
 }
 
@@ -1323,7 +1328,7 @@ __device__ __forceinline__ void pair_positions(const float2 (&w)[4], const float
 // region.  This gives the checked sample's bits for every voxel:
 //  - the staged window holds the floor tap and the +1 tap of every sample of
 //    the walk, zero-filled where it reaches past the source, and a tap
-//    offset is clamped into the ring whatever the position, so no position
+//    offset is masked into the ring whatever the position, so no position
 //    reads outside shared memory;
 //  - a valid sample's taps are inside the volume and the source buffer, but
 //    for q = sz - 1 exactly, whose +1 tap has weight 0 (lo + 0 (hi - lo) =
@@ -1353,10 +1358,6 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
     const int xe = BORDER ? (int)min(J.out_o[0] + J.out_n[0] - w.Ox, (int64_t)kTBX) : kTBX;
     const bool pair_ok =
         !BORDER || ((((uintptr_t)J.dst) % (2 * sizeof(T))) == 0 && (J.dst_py % 2 == 0) && (J.dst_pz % 2 == 0));
-    // kMagic + the byte offset of frame (0, 0) in a plane slot (an integer
-    // below 2^14: exact)
-    const float kc = kMagic + (float)(P.DY * Gm::ROW_B + P.DX * Gm::ES);
-    const uint32_t omax = (uint32_t)(kRing * Gm::PLANE_B - Gm::ROW_B - 2 * Gm::ES);
     for (int64_t zf = w.z0; zf < w.z1;) {
         const int64_t ze = min(w.z1, (zf / G + 1) * G);
         const int64_t Oz = (zf / G) * G;
@@ -1371,7 +1372,7 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
             const int64_t O[3] = {w.Ox, w.Oy, Oz};
             fr = make_frame(J, O);
         }
-        const uint32_t cz = layer_cz(seq0, Oz, w.z0, P.a);
+        const float lk = layer_k<T>(seq0, Oz, w.z0, P);
         auto prep = [&](int p, PairPrep (&q)[NR], uint32_t (&keep)[NR]) {
             const float4 wa = S.W2[2 * p], wb = S.W2[2 * p + 1];
             const float2 wz[4] = {f2(wa.x, wa.y), f2(wa.z, wa.w), f2(wb.x, wb.y), f2(wb.z, wb.w)};
@@ -1379,7 +1380,7 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
             for (int k = 0; k < NR; ++k) {
                 float2 px, py, pz;
                 pair_positions(wz, PX[k], PY[k], PZ[k], px, py, pz);
-                q[k] = prep_pair<T>(S.sring, kc, omax, cz, px, py, pz);
+                q[k] = prep_pair<T>(S.sring, lk, px, py, pz);
                 if (BORDER) {
                     const bool ok0 = px.x >= fr.lo[0] && px.x <= fr.hi[0] && py.x >= fr.lo[1] && py.x <= fr.hi[1] &&
                                      pz.x >= fr.lo[2] && pz.x <= fr.hi[2];
@@ -1761,12 +1762,13 @@ __global__ void __launch_bounds__(kTpsThreads, 1) k_tps_gather(const RJob *__res
     __shared__ float4 W[G];
     __shared__ float4 Rw[kTBY * Gm::NRW];
     const int tid = threadIdx.x;
+    const int64_t n = fb ? fb[0] : total_units;
+    if (blockIdx.x >= n) return;  // most launches have no unit left over
     if (tid < G) W[tid] = bspline_w(tid, G);
     __syncthreads();
     const int x = 2 * (tid & 31);
     const float4 wx[2] = {W[x % G], W[(x + 1) % G]};
     float4 *rw = Rw + (tid >> 5) * Gm::NRW;
-    const int64_t n = fb ? fb[0] : total_units;
     for (int64_t i = blockIdx.x; i < n; i += gridDim.x)
         rows_gather<T, G, INTERP>(jobs, njobs, fb ? fb[1 + i] : i, W, rw, wx);
 }
