@@ -424,11 +424,7 @@ tw_status tw_warp_tps_device(tw_ctx *ctx, const void *dev_nodes, int g, int dtyp
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     RJob j = tps_job(dev_src, sz, dev_dst, sz, static_cast<const float4 *>(dev_nodes), g, dtype, interp);
     TW_TRY(run_jobs(ctx, &j, 1, st));
-    if (!stream) {
-        TW_CUDA_TRY(cudaStreamSynchronize(st));
-        return check_kernel_errors(ctx);
-    }
-    return TW_OK;
+    return stream ? TW_OK : check_kernel_errors(ctx);  // (waits for the context's stream)
 }
 
 tw_status tw_warp_affine_device(tw_ctx *ctx, const double M[16], int dtype, int interp, const void *dev_src,
@@ -442,8 +438,7 @@ tw_status tw_warp_affine_device(tw_ctx *ctx, const double M[16], int dtype, int 
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     RJob j = affine_job(dev_src, src_sz, dev_dst, dst_sz, M, dtype, interp);
     TW_TRY(run_jobs(ctx, &j, 1, st));
-    if (!stream) TW_CUDA_TRY(cudaStreamSynchronize(st));
-    return TW_OK;
+    return stream ? TW_OK : check_kernel_errors(ctx);  // (waits for the context's stream)
 }
 
 tw_status tw_fit_affine(tw_ctx *ctx, const tw_marker *tar, const tw_marker *sub, int n, double M[16])

@@ -58,7 +58,10 @@ struct alignas(128) RJob {
     int64_t brick_begin;   // first flattened brick index of this job in its launch
     int g;                 // grid spacing (TPS)
     int zs;                // output planes per TPS work unit (divides g or is a multiple of it; set by run_jobs)
-    int tma_ok;            // tmap is valid: TPS units may stage their source footprint in shared memory
+    int tma_ok;            // units may stage their source footprint in shared memory: 1 through tmap, 2
+                           // (affine) row by row
+    int st_w, st_h, st_d;  // affine: staged box, elements (row by row) or the TMA box
+    int st_pr, st_pp;      // affine: its row and plane pitch in shared memory, bytes
     int dtype;             // 1 u8, 2 u16
     int kind;              // 0 affine, 1 TPS
     int interp;            // 0 trilinear, 1 nearest
@@ -75,6 +78,12 @@ struct alignas(128) RJob {
 cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_bricks, int dtype,
                             int kind, int g, int interp, cudaStream_t st, int sm_count, int *err,
                             void *stage_ws);
+// Trilinear affine jobs whose tiles are staged (encode_affine_box gave each a box), in
+// units of kAffineTile output voxels; stage_bytes: the largest of their boxes.
+cudaError_t launch_affine_staged(const RJob *jobs_dev, int njobs, int64_t total_tiles, int dtype, uint32_t stage_bytes,
+                                 cudaStream_t st, int sm_count, int *err);
+constexpr int kAffineTile[3] = {32, 16, 16};
+constexpr int kAffineSmem = 220 * 1024;  // shared memory for the boxes of one CTA
 size_t tps_stage_ws_bytes(int64_t total_bricks);
 // Brick extents for a (kind, g) pair: x, y and the z extent a unit's frame
 // is anchored to (a control cell layer for TPS).
@@ -82,6 +91,10 @@ void brick_dims(int kind, int g, int64_t out[3]);
 // Fills j.tmap / j.tma_ok for a TPS job (false when the source buffer's
 // address or pitches do not meet the TMA rules; the job then gathers).
 bool encode_source_map(RJob &j);
+// The staged box of an affine job's tiles: its geometry, and the descriptor
+// where TMA can describe the source; returns its bytes (a multiple of 128), 0
+// when the job has to gather.
+uint32_t encode_affine_box(RJob &j);
 // Device error word bits set by the resample kernels.
 constexpr int kKernErrTimeout = 1;
 // The TMA box of the staged TPS path: source elements per staged row and rows

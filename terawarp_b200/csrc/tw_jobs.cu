@@ -83,9 +83,36 @@ struct PoolBlock {
 
 }  // namespace
 
+namespace {
+
+tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cudaStream_t st);
+
+}  // namespace
+
 tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
 {
     if (njobs <= 0) return TW_OK;
+    if (jobs[0].kind == 1) return run_group(ctx, jobs, njobs, 0, st);
+    // affine jobs whose tiles can be staged first, the others gather
+    uint32_t box = 0;
+    const bool staging = ctx->resample_staging.load() != 0;
+    RJob *const mid = std::stable_partition(jobs, jobs + njobs, [&](RJob &j) {
+        const uint32_t b = staging ? encode_affine_box(j) : 0u;
+        box = std::max(box, b);
+        return b != 0;
+    });
+    const int ns = (int)(mid - jobs);
+    if (ns > 0) TW_TRY(run_group(ctx, jobs, ns, box, st));
+    if (ns < njobs) TW_TRY(run_group(ctx, mid, njobs - ns, 0, st));
+    return TW_OK;
+}
+
+namespace {
+
+// One launch over jobs that share (dtype, kind, g, interp); affine_box: bytes
+// of the largest staged box when the jobs are staged affine jobs, else 0.
+tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cudaStream_t st)
+{
     int64_t total = 0;
     auto count = [&](int zs) {
         total = 0;
@@ -93,6 +120,8 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
             int64_t bd[3];
             brick_dims(jobs[i].kind, jobs[i].g, bd);
             if (jobs[i].kind == 1) bd[2] = zs;
+            else if (affine_box)
+                for (int a = 0; a < 3; ++a) bd[a] = kAffineTile[a];
             jobs[i].zs = zs;
             for (int a = 0; a < 3; ++a) jobs[i].bricks[a] = (jobs[i].out_n[a] + bd[a] - 1) / bd[a];
             jobs[i].brick_begin = total;
@@ -126,6 +155,11 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
     void *d_fb = fb.p;
     // plan, walk lists, staged (interior walks), staged (other walks), gather
     const uint64_t launches = staged ? 5 : 1;
+    const auto launch = [&](const RJob *d) {
+        return affine_box ? launch_affine_staged(d, njobs, total, jobs[0].dtype, affine_box, st, ctx->sm_count, ctx->d_err)
+                          : launch_resample(d, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
+                                            ctx->sm_count, ctx->d_err, d_fb);
+    };
     const size_t bytes = sizeof(RJob) * (size_t)njobs;
     if (njobs <= tw_ctx::kJobsPerSlot && ctx->job_d) {
         // descriptors through the context's slot ring: an asynchronous copy
@@ -138,8 +172,7 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
         RJob *d = ctx->job_d + (size_t)s * tw_ctx::kJobsPerSlot;
         std::memcpy(h, jobs, bytes);
         TW_CUDA_TRY(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st));
-        cudaError_t e = launch_resample(d, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
-                                        ctx->sm_count, ctx->d_err, d_fb);
+        cudaError_t e = launch(d);
         if (e != cudaSuccess) return fail(ctx, TW_ERR_CUDA, std::string("resample launch: ") + cudaGetErrorString(e));
         TW_CUDA_TRY(cudaEventRecord(ctx->job_ev[s], st));
         count_launch(ctx, launches);
@@ -148,13 +181,14 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
     RJob *d_jobs = nullptr;
     TW_CUDA_TRY(cudaMallocFromPoolAsync((void **)&d_jobs, bytes, ctx->pool, st));
     TW_CUDA_TRY(cudaMemcpyAsync(d_jobs, jobs, bytes, cudaMemcpyHostToDevice, st));
-    cudaError_t e = launch_resample(d_jobs, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
-                                    ctx->sm_count, ctx->d_err, d_fb);
+    cudaError_t e = launch(d_jobs);
     cudaFreeAsync(d_jobs, st);
     if (e != cudaSuccess) return fail(ctx, TW_ERR_CUDA, std::string("resample launch: ") + cudaGetErrorString(e));
     count_launch(ctx, launches);
     return TW_OK;
 }
+
+}  // namespace
 
 // ------------------------------------------------------- TMA descriptors
 
@@ -207,6 +241,138 @@ bool encode_source_map(RJob &j)
     if (r != CUDA_SUCCESS) return false;
     j.tma_ok = 1;
     return true;
+}
+
+namespace {
+
+// How a warp's tap loads of a staged affine tile meet the 32 banks: floors of
+// the positions of a few of its rows (two rows of 16 lanes, a voxel pair
+// each).
+struct TapRows {
+    static constexpr int kRows = 4;
+    int q[kRows][32][3];
+    explicit TapRows(const double M[12])
+    {
+        const double at[kRows][5] = {{0, 0, .31, .62, .13}, {6, 5, .77, .05, .48}, {10, 9, .52, .89, .95}, {14, 15, .16, .4, .7}};
+        for (int r = 0; r < kRows; ++r)
+            for (int l = 0; l < 32; ++l) {
+                const double p[3] = {2.0 * (l & 15), at[r][0] + (l >> 4), at[r][1]};
+                for (int a = 0; a < 3; ++a)
+                    q[r][l][a] = (int)std::floor(M[a * 4] * p[0] + M[a * 4 + 1] * p[1] + M[a * 4 + 2] * p[2] + at[r][2 + a]);
+            }
+    }
+    // shared-memory passes per load, summed over the rows: the most distinct
+    // words any bank is asked for
+    int passes(int pr, int pp, int es) const
+    {
+        int sum = 0;
+        for (int r = 0; r < kRows; ++r) {
+            int word[32], depth[32] = {0}, chain[32], head[32], worst = 1;
+            for (int k = 0; k < 32; ++k) head[k] = -1;
+            for (int l = 0; l < 32; ++l) {
+                const int w = (q[r][l][2] * pp + q[r][l][1] * pr + q[r][l][0] * es) >> 2, bank = w & 31;
+                int k = head[bank];
+                while (k >= 0 && word[k] != w) k = chain[k];
+                if (k >= 0) continue;
+                word[l] = w;
+                chain[l] = head[bank];
+                head[bank] = l;
+                worst = std::max(worst, ++depth[bank]);
+            }
+            sum += worst;
+        }
+        return sum;
+    }
+};
+
+}  // namespace
+
+uint32_t encode_affine_box(RJob &j)
+{
+    j.tma_ok = 0;
+    const int es = j.dtype == TW_U8 ? 1 : 2;
+    // a nearest-neighbour sample reads one element: gathered it takes less
+    // than its share of a staged box (406 against 1050 us, 700 x 600 x 300 u16)
+    if (j.interp == 1 || reinterpret_cast<uintptr_t>(j.src) % 16 != 0) return 0;
+    // extents of a tile's samples, their +1 taps, and a margin for rounding
+    int box[3];
+    double reach[3];  // largest positions relative to their brick's origin
+    for (int r = 0; r < 3; ++r) {
+        double ext = 0.0, far = 0.0;
+        const int brick[3] = {256, 8, 8};
+        for (int a = 0; a < 3; ++a) {
+            const double m = std::fabs(j.M[r * 4 + a]);
+            ext += m * (kAffineTile[a] - 1);
+            far += m * brick[a];
+        }
+        if (!(ext < 240.0) || !(std::fabs(j.M[r * 4 + 3]) < 1e9)) return 0;  // (NaN and infinity included)
+        box[r] = (int)std::floor(ext + 2.0 / 64.0) + 4;
+        reach[r] = far + box[r];
+    }
+    for (int a = 0; a < 3; ++a) {
+        const int64_t lim = (int64_t)1 << 28;  // TMA coordinates are int32
+        if (j.out_o[a] < -lim || j.out_o[a] + j.out_n[a] > lim || j.src_o[a] < -lim || j.src_o[a] > lim || j.glob[a] > lim) return 0;
+    }
+    double tiles = 1.0;
+    for (int a = 0; a < 3; ++a) tiles *= (double)((j.out_n[a] + kAffineTile[a] - 1) / kAffineTile[a]);
+    if (tiles >= 2147483648.0) return 0;
+    // The box's pitches: the smallest that copies allow, padded (planes by up
+    // to seven steps, then rows by one) until a tap load takes close to its two
+    // passes -- unpadded, some matrices put most lanes in a few banks (8.8
+    // passes at 10 degrees about each axis with rows of 1034 bytes, 16 at a
+    // quarter turn about z).
+    const EncodeTiled fn = encode_fn();
+    const int A = 16 / es, w1 = (box[0] + A - 1 + A - 1) / A * A;  // starts on a 16-byte boundary
+    const bool tma = fn && (j.src_py * es) % 16 == 0 && (j.src_pz * es) % 16 == 0 && w1 + A <= std::min<int64_t>(256, j.src_n[0]) &&
+                     box[1] + 7 <= j.src_n[1] && box[2] <= j.src_n[2] && (uint64_t)j.src_pz * es < (1ull << 40);
+    const int dy = (int)((j.src_py * es) & 15), dz = (int)((j.src_pz * es) & 15);
+    const TapRows rows(j.M);
+    const int good = 9 * TapRows::kRows / 4;  // 2.25 passes
+    int best = 1 << 30;
+    int64_t bytes = 0;
+    for (int pad = 0; pad < 16 && best > good; ++pad) {
+        const int i = pad >> 3, k = pad & 7;
+        int pr, pp;
+        if (tma) {
+            pr = (w1 + A * i) * es;
+            pp = pr * (box[1] + k);
+        } else {
+            // congruent to the source's pitches modulo 16, rows at least 30
+            // bytes apart: each is copied in whole 16-byte granules
+            pr = ((box[0] * es + 30 - dy + 15) & ~15) + dy + 16 * i;
+            pp = ((pr * box[1] - dz + 15) & ~15) + dz + 16 * k;
+        }
+        const int64_t need = ((int64_t)pp * box[2] + 32 + 127) / 128 * 128;
+        if (need > kAffineSmem) continue;
+        if (bytes && 2 * bytes <= kAffineSmem && 2 * need > kAffineSmem) continue;  // two stages are worth more
+        const int p = rows.passes(pr, pp, es);
+        if (p >= best) continue;
+        best = p;
+        bytes = need;
+        j.st_w = tma ? w1 + A * i : box[0];
+        j.st_h = tma ? box[1] + k : box[1];
+        j.st_pr = pr;
+        j.st_pp = pp;
+    }
+    j.st_d = box[2];
+    // the box fits, and tap offsets and their partial sums (floating point,
+    // exact below 2^22) stay small
+    if (!bytes || reach[2] * j.st_pp + reach[1] * j.st_pr + reach[0] * es > 2097152.0) return 0;
+    j.tma_ok = 2;
+    if (tma) {
+        const cuuint64_t dims[3] = {(cuuint64_t)j.src_n[0], (cuuint64_t)j.src_n[1], (cuuint64_t)j.src_n[2]};
+        const cuuint64_t strides[2] = {(cuuint64_t)j.src_py * es, (cuuint64_t)j.src_pz * es};
+        const cuuint32_t b[3] = {(cuuint32_t)j.st_w, (cuuint32_t)j.st_h, (cuuint32_t)j.st_d};
+        const cuuint32_t estr[3] = {1, 1, 1};
+        if (fn(&j.tmap, es == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void *>(j.src),
+               dims, strides, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+            j.tma_ok = 0;
+            return 0;
+        }
+        j.tma_ok = 1;
+    }
+    return (uint32_t)bytes;
 }
 
 // ------------------------------------------------------------ sample hulls

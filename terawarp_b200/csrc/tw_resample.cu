@@ -1610,6 +1610,380 @@ __device__ void affine_brick(const RJob &J, int64_t bx, int64_t by, int64_t bz, 
                                       frame, cw, dst + dbase0, J.dst_py, J.dst_pz, pair_ok, rows);
 }
 
+// ------------------------------------------------------- staged affine tiles
+//
+// The sample positions of an output tile fill a box of the source, the same
+// size for every tile of a job.  A tile of 32 x 16 x 16 output voxels reads a
+// box of about 45 x 29 x 29 elements at 15 degrees about each axis, 4.6
+// elements per voxel, so the box is copied into shared memory once and the
+// eight taps of every voxel are shared-memory loads.  (Gathered from global
+// memory through L1 the taps hit in it, but a tap load of a rotated row
+// touches a different line every few lanes and takes 7.7 cycles: 124 cycles
+// per 64 voxels at 15 degrees, whatever shape of voxel patch a warp takes.
+// In shared memory the same load takes 2.8 cycles for uint16, 2.2 for uint8,
+// with the densest row pitch that copies allow; pitches that are multiples of
+// 128 bytes conflict more under rotation.)
+//
+// One CTA per SM, 16 warps that sample (warp w the tile's plane w, two rows of
+// 32 voxels at a time) and four that copy tiles ahead, in up to four stages.
+// A source whose base and pitches are multiples of 16 bytes is copied by one
+// TMA box per tile.  Any other is copied in 16-byte granules (cp.async): row
+// and plane pitches in shared memory are congruent to the
+// source's modulo 16 bytes, so that every row's shared address is congruent to
+// its global address and the tap of (x, y, z) still sits at one linear offset.
+//
+// Positions come from the same bricks, with the same arithmetic, as the
+// gathered path's, so both give the same bits.
+//
+// Measured on 512 x 512 x 256, us, gathered and staged (uint16 / uint8): no
+// rotation 289 -> 220 / 273 -> 207, 15 degrees about each axis 603 -> 236 / 622
+// -> 230, a quarter turn about z 1990 -> 324 / 1953 -> 317; with odd pitches
+// (517 x 389 x 203 uint16) 251 -> 251, 529 -> 337, 517 -> 231.
+
+constexpr int kATX = kAffineTile[0], kATY = kAffineTile[1], kATZ = kAffineTile[2];
+constexpr int kAWarps = kATZ;
+constexpr int kACopyWarps = 4;
+constexpr int kAStages = 4;
+constexpr int kAStagedThreads = 32 * (kAWarps + kACopyWarps);
+constexpr int kAFrames = (kATY / kABY) * (kATZ / kABZ);
+static_assert(kBX % kATX == 0 && kATY % kABY == 0 && kATZ % kABZ == 0 && kAFrames <= 32, "a tile is made of whole brick parts");
+
+// What a tile's samplers need besides the staged box, per brick it crosses.
+struct AFrame {
+    float fo[3];         // position of the brick's origin, relative to floor of it
+    float k;             // kMagic + byte offset of that floor in the stage
+    float lo[3], hi[3];  // valid positions
+    // the source's last element: a sample exactly on it takes floor top - 1
+    // and fraction 1 where the gathered path does (pair_clamped2), since b0 +
+    // 1 (b1 - b0) is not always b1 in floating point.  (The tap before it is
+    // staged: a box starts 1/64 below its lowest sample.)
+    float top[3];
+};
+struct AStage {
+    AFrame f[kAFrames];
+    int job, whole, check;  // whole: every voxel inside the output, paired stores; check: bit a: samples may leave
+                            // the source along axis a
+    int x0, nx, ny, nz;     // first voxel within its brick along x; the tile's voxels inside the output
+    long long dst;          // element offset of the tile in the output
+    long long box[3];       // the box's first element
+};
+
+// Arrives on the mbarrier once every copy this thread has begun has landed.
+__device__ __forceinline__ void mbar_arrive_copies(uint32_t a)
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(a) : "memory");
+}
+
+// 16 bytes, of which the first `bytes` come from src and the rest are zero.
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src, int bytes)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Copies rows [0, h) of planes [0, d) of the box at source-buffer element (bx,
+// by, bz), w elements wide, to shared address `stage` + (row pitch pr, plane
+// pitch pp) at byte (row 0's global address mod 16), planes part, part +
+// parts, ... of it, by one warp.  A lane takes one 16-byte granule of a row at
+// a time (a bulk copy per row took 35 cycles each, which made a tile's copies
+// slower than its sampling).  Only bytes of the buffer are read: rows outside
+// it and granules before its start are left out, its last granule is read in
+// part.
+template <typename T>
+__device__ void copy_rows(const RJob &J, uint32_t stage, int pr, int pp, int64_t bx, int64_t by, int64_t bz, int w,
+                          int h, int d, int part, int parts)
+{
+    constexpr int ES = (int)sizeof(T);
+    const int lane = threadIdx.x & 31;
+    const char *src = static_cast<const char *>(J.src);
+    const int64_t total = ((J.src_n[2] - 1) * J.src_pz + (J.src_n[1] - 1) * J.src_py + J.src_n[0]) * ES;
+    const int wb = w * ES, per_row = (wb + 30) / 16;  // granules a row may touch
+    const int lpr = per_row <= 4 ? 4 : per_row <= 8 ? 8 : per_row <= 16 ? 16 : 32;  // lanes per row
+    const int sub = 16 * (lane & (lpr - 1)), rows = 32 / lpr;
+    const int64_t pyb = J.src_py * ES, pzb = J.src_pz * ES;
+    const int64_t g00 = bz * pzb + by * pyb + bx * ES;
+    const uint32_t to0 = stage + (uint32_t)(g00 & 15);
+    // rows and planes of the box inside the buffer
+    const int y0 = (int)max((int64_t)0, min(-by, (int64_t)h)), y1 = (int)max((int64_t)0, min(J.src_n[1] - by, (int64_t)h));
+    const int p0 = (int)max((int64_t)0, min(-bz, (int64_t)d)), p1 = (int)max((int64_t)0, min(J.src_n[2] - bz, (int64_t)d));
+    const bool edge = g00 + y0 * pyb + p0 * pzb < 16 || g00 + y1 * pyb + p1 * pzb + wb + 16 > total;
+    const int y_first = y0 + lane / lpr;
+    const int64_t dy = rows * pyb;
+    for (int p = p0 + ((part - p0) % parts + parts) % parts; p < p1; p += parts) {
+        int64_t g = g00 + p * pzb + y_first * pyb;
+        uint32_t to = to0 + (uint32_t)(p * pp + y_first * pr + sub);
+        for (int y = y_first; y < y1; y += rows, g += dy, to += (uint32_t)(rows * pr)) {
+            const int head = (int)g & 15;
+            for (int c = sub; c < head + wb; c += 16 * lpr) {
+                const int64_t at = g + (c - head);
+                const uint32_t dst = to + (uint32_t)(c - sub - head);
+                if (!edge) copy16(dst, src + at, 16);
+                else if (at >= 0 && at < total) copy16(dst, src + at, (int)min((int64_t)16, total - at));
+            }
+        }
+    }
+}
+
+// A tile as a lane of the first copying warp holds it: its box (first element,
+// source-buffer coordinates), lane l's frame l, and the rest.
+struct ATile {
+    AFrame f;
+    int64_t box[3];
+    long long dst;
+    int job, whole, check, x0, nx, ny, nz;
+};
+
+template <typename T>
+__device__ __forceinline__ void affine_tile_setup(const RJob &J, int64_t lb, ATile &S)
+{
+    constexpr int ES = (int)sizeof(T);
+    const int lane = threadIdx.x & 31;
+    // tiles of a job are below 2^31 (the host stages no larger job)
+    const uint32_t b0 = (uint32_t)J.bricks[0], b1 = (uint32_t)J.bricks[1], l32 = (uint32_t)lb;
+    const uint32_t t = l32 / b0;
+    const int64_t t0[3] = {(int64_t)(l32 % b0) * kATX, (int64_t)(t % b1) * kATY, (int64_t)(t / b1) * kATZ};
+    const double e = 1.0 / 64.0;
+    S.check = 0;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        double q = J.M[r * 4 + 3], lo = 0.0, hi = 0.0;
+        const double ext[3] = {kATX - 1.0, kATY - 1.0, kATZ - 1.0};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            q += J.M[r * 4 + a] * (double)(J.out_o[a] + t0[a]);
+            const double v = J.M[r * 4 + a] * ext[a];
+            if (v < 0) lo += v; else hi += v;
+        }
+        lo += q - e;
+        hi += q + e;
+        S.box[r] = (int64_t)floor(lo) - J.src_o[r];
+        const bool in = lo >= (double)max((int64_t)0, J.src_o[r]) && hi < (double)min(J.glob[r] - 1, J.src_o[r] + J.src_n[r] - 1);
+        S.check |= in ? 0 : 1 << r;
+    }
+    // a TMA box starts on a 16-byte boundary along x
+    if (J.tma_ok == 1) S.box[0] &= ~(int64_t)(16 / ES - 1);
+    const int sigma = J.tma_ok == 1 ? 0 : (int)(((S.box[2] * J.src_pz + S.box[1] * J.src_py + S.box[0]) * ES) & 15);
+    if (lane < kAFrames) {
+        const int64_t O[3] = {J.out_o[0] + t0[0] / kBX * kBX, J.out_o[1] + t0[1] + (lane % (kATY / kABY)) * kABY,
+                              J.out_o[2] + t0[2] + (lane / (kATY / kABY)) * kABZ};
+        AFrame &F = S.f;
+        int64_t qf[3];
+        float mn[3], mx[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            // the brick's origin and hull as affine_brick computes them
+            const double q = fma(J.M[r * 4 + 2], (double)O[2],
+                                 fma(J.M[r * 4 + 0], (double)O[0], __dmul_rn(J.M[r * 4 + 1], (double)O[1]))) + J.M[r * 4 + 3];
+            const double f = floor(q);
+            qf[r] = (int64_t)f;
+            F.fo[r] = (float)(q - f);
+            double l = 0, h = 0;
+            const double ext[3] = {kBX - 1.0, kABY - 1.0, kABZ - 1.0};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const double v = J.M[r * 4 + a] * ext[a];
+                if (v < 0) l += v; else h += v;
+            }
+            mn[r] = (float)(F.fo[r] + l);
+            mx[r] = (float)(F.fo[r] + h);
+        }
+        const Frame fr = make_frame(J, qf);
+        const Clamp cw = make_clamp(J, fr, mn, mx);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            F.lo[r] = fr.lo[r];
+            F.hi[r] = fr.hi[r];
+            F.top[r] = cw.clamped ? (float)cw.ch[r] : 3.0e38f;
+        }
+        const int64_t off = (qf[2] - J.src_o[2] - S.box[2]) * J.st_pp + (qf[1] - J.src_o[1] - S.box[1]) * J.st_pr +
+                            (qf[0] - J.src_o[0] - S.box[0]) * ES + sigma;
+        F.k = kMagic + (float)off;  // (exact: the host stages a job only when offsets stay below 2^21)
+    }
+    S.x0 = (int)(t0[0] % kBX);
+    S.nx = (int)min((int64_t)kATX, J.out_n[0] - t0[0]);
+    S.ny = (int)min((int64_t)kATY, J.out_n[1] - t0[1]);
+    S.nz = (int)min((int64_t)kATZ, J.out_n[2] - t0[2]);
+    S.dst = t0[2] * J.dst_pz + t0[1] * J.dst_py + t0[0];
+    S.whole = S.nx == kATX && S.ny == kATY && S.nz == kATZ && ((uintptr_t)J.dst) % (2 * sizeof(T)) == 0 &&
+              J.dst_py % 2 == 0 && J.dst_pz % 2 == 0;
+}
+
+// Warp w's plane of a staged tile.  IN: every sample inside, whole tile,
+// paired stores.
+template <typename T, bool IN>
+__device__ __forceinline__ void affine_tile_rows(const RJob &J, const AStage &S, uint32_t stage, int z)
+{
+    constexpr float ES = (float)sizeof(T);
+    const int lane = threadIdx.x & 31;
+    const int x = 2 * (lane & 15);
+    if (!IN && z >= S.nz) return;
+    const float m00 = (float)J.M[0], m01 = (float)J.M[1], m02 = (float)J.M[2];
+    const float m10 = (float)J.M[4], m11 = (float)J.M[5], m12 = (float)J.M[6];
+    const float m20 = (float)J.M[8], m21 = (float)J.M[9], m22 = (float)J.M[10];
+    const float lx = (float)(S.x0 + x), zz = (float)(z % kABZ);
+    const float PR = (float)J.st_pr, PP = (float)J.st_pp;
+    const uint32_t pr = (uint32_t)J.st_pr, pp = (uint32_t)J.st_pp;
+    const int check = IN ? 0 : S.check;
+    const bool pair_ok = IN || ((((uintptr_t)J.dst) % (2 * sizeof(T))) == 0 && S.dst % 2 == 0 && J.dst_py % 2 == 0 &&
+                                J.dst_pz % 2 == 0);
+    T *dp = static_cast<T *>(J.dst) + S.dst + (int64_t)z * J.dst_pz + (int64_t)(lane >> 4) * J.dst_py + x;
+    const int64_t step = 2 * J.dst_py;
+#pragma unroll 1
+    for (int fy = 0; fy < kATY / kABY; ++fy) {
+        const AFrame &F = S.f[z / kABZ * (kATY / kABY) + fy];
+        const float fo0 = F.fo[0], fo1 = F.fo[1], fo2 = F.fo[2], k = F.k;
+#pragma unroll 2
+        for (int i = 0; i < kABY / 2; ++i, dp += step) {
+            const int yb = 2 * i + (lane >> 4);  // row within the brick
+            if (!IN && (fy * kABY + yb >= S.ny || x >= S.nx)) continue;
+            const float yy = (float)yb;
+            const float bx0 = fmaf(m02, zz, fmaf(m01, yy, fo0)), by0 = fmaf(m12, zz, fmaf(m11, yy, fo1));
+            const float bz0 = fmaf(m22, zz, fmaf(m21, yy, fo2));
+            float2 px, py, pz;
+            px.x = fmaf(m00, lx, bx0);
+            py.x = fmaf(m10, lx, by0);
+            pz.x = fmaf(m20, lx, bz0);
+            px.y = px.x + m00;
+            py.y = py.x + m10;
+            pz.y = pz.x + m20;
+            const float2 MM = f2(kMagic, kMagic);
+            const float2 mx = __fadd2_rd(px, MM), my = __fadd2_rd(py, MM), mz = __fadd2_rd(pz, MM);
+            float2 flx = sub2(mx, MM), fly = sub2(my, MM), flz = sub2(mz, MM);
+            bool ok0 = true, ok1 = true;
+            if (!IN) {  // only along the axes where the tile's samples may leave the source
+                auto axis = [&](int a, float2 q, float2 &fl) {
+                    const float l = F.lo[a], h = F.hi[a], top = F.top[a];
+                    ok0 = ok0 && q.x >= l && q.x <= h;
+                    ok1 = ok1 && q.y >= l && q.y <= h;
+                    fl = f2(q.x == top ? top - 1.f : fl.x, q.y == top ? top - 1.f : fl.y);
+                };
+                if (check & 1) axis(0, px, flx);
+                if (check & 2) axis(1, py, fly);
+                if (check & 4) axis(2, pz, flz);
+            }
+            const float2 o = fma2(flz, f2(PP, PP), fma2(fly, f2(PR, PR), fma2(flx, f2(ES, ES), f2(k, k))));
+            const uint32_t c = stage - (uint32_t)kMagicBits;
+            const uint32_t a0 = c + __float_as_uint(o.x), a1 = c + __float_as_uint(o.y);
+            float2 lo[4], hi[4];
+            constexpr int E = (int)sizeof(T);
+            const uint32_t r0[4] = {a0, a0 + pr, a0 + pp, a0 + pp + pr}, r1[4] = {a1, a1 + pr, a1 + pp, a1 + pp + pr};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                lo[r] = f2(lds_raw<T, 0>(r0[r]), lds_raw<T, 0>(r1[r]));
+                hi[r] = f2(lds_raw<T, E>(r0[r]), lds_raw<T, E>(r1[r]));
+            }
+            const float2 o2 = out_pair<T, false>(trilerp2(lo, hi, sub2(flx, px), sub2(py, fly), sub2(pz, flz)));
+            const uint32_t v = pack_pair<T>(__float_as_uint(o2.x), __float_as_uint(o2.y));
+            if (IN) {
+                if (sizeof(T) == 2) *reinterpret_cast<uint32_t *>(dp) = v;
+                else *reinterpret_cast<uint16_t *>(dp) = (uint16_t)v;
+            } else {
+                constexpr uint32_t M0 = sizeof(T) == 2 ? 0xFFFFu : 0xFFu, M1 = M0 << (8 * sizeof(T));
+                store_packed<T>(dp, v & ((ok0 ? M0 : 0u) | (ok1 ? M1 : 0u)), pair_ok, S.nx - x);
+            }
+        }
+    }
+}
+
+// stages: buffers of stage_b bytes (a multiple of 128), at most kAStages.
+template <typename T>
+__global__ void __launch_bounds__(kAStagedThreads, 1) k_affine_staged(const RJob *__restrict__ jobs, int njobs,
+                                                                       int64_t total, int stages, uint32_t stage_b, int *err)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ AStage st[kAStages];
+    __shared__ unsigned long long bars[2 * kAStages];  // full, empty
+    __shared__ int abort_sh, copy_abort[2];  // copy_abort: of this and the next tile
+    const uint32_t raw0 = (uint32_t)__cvta_generic_to_shared(smem_raw);
+    const uint32_t base = (raw0 + 127u) & ~127u;
+    const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < kAStages; ++s) {
+            mbar_init(bar0 + 8 * s, 32 * kACopyWarps);
+            mbar_init(bar0 + 8 * (kAStages + s), kAWarps);
+        }
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    uint32_t n = 0;  // tiles so far: tile n is the (n / stages)-th of stage n % stages
+    if (warp >= kAWarps) {  // the copying warps
+        int last_job = -1;
+        for (int64_t b = blockIdx.x; b < total; b += gridDim.x, ++n) {
+            const int j = find_job(jobs, njobs, b);
+            const RJob &J = jobs[j];
+            const int s = (int)(n % (uint32_t)stages);
+            const uint32_t use = n / (uint32_t)stages, full = bar0 + 8 * s;
+            const uint32_t to = base + (uint32_t)s * stage_b;
+            const bool first = warp == kAWarps;
+            ATile t;  // worked out while its stage is still in use
+            if (first) affine_tile_setup<T>(J, b - J.brick_begin, t);
+            if (use > 0) {
+                const bool ok = mbar_wait_producer(bar0 + 8 * (kAStages + s), (use - 1u) & 1u, &abort_sh);
+                if (!__all_sync(0xffffffffu, ok) && lane == 0) {
+                    *reinterpret_cast<volatile int *>(&abort_sh) = 1;
+                    if (err) atomicOr(err, kKernErrTimeout);
+                }
+            }
+            AStage &S = st[s];
+            if (first) {
+                if (lane < kAFrames) S.f[lane] = t.f;
+                if (lane == 0) {
+                    S.job = j;
+                    S.whole = t.whole;
+                    S.check = t.check;
+                    S.x0 = t.x0;
+                    S.nx = t.nx;
+                    S.ny = t.ny;
+                    S.nz = t.nz;
+                    S.dst = t.dst;
+                    for (int r = 0; r < 3; ++r) S.box[r] = t.box[r];
+                    copy_abort[n & 1u] = *reinterpret_cast<volatile int *>(&abort_sh);
+                }
+            }
+            __syncwarp();
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * kACopyWarps) : "memory");  // S is written
+            if (copy_abort[n & 1u]) break;  // (every copying warp sees the same)
+            if (J.tma_ok == 2) {
+                copy_rows<T>(J, to, J.st_pr, J.st_pp, S.box[0], S.box[1], S.box[2], J.st_w, J.st_h, J.st_d, warp - kAWarps,
+                             kACopyWarps);
+                mbar_arrive_copies(full);
+            } else if (first && lane == 0) {
+                if (j != last_job)  // the descriptor was written by a copy
+                    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&J.tmap) : "memory");
+                last_job = j;
+                mbar_expect_tx(full, (uint32_t)(J.st_pp * J.st_d));
+                tma_plane(to, &J.tmap, (int)t.box[0], (int)t.box[1], (int)t.box[2], full);
+            } else {
+                mbar_arrive(full);
+            }
+        }
+        // every copy has landed before the CTA exits (the samplers have waited
+        // for all of them unless a wait gave up; bounded)
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (warp == kAWarps && lane == 0)
+            for (uint32_t i = n > (uint32_t)stages ? n - stages : 0u; i < n; ++i) {
+                const uint32_t full = bar0 + 8 * (i % (uint32_t)stages), ph = (i / (uint32_t)stages) & 1u;
+                if (!mbar_try(full, ph)) mbar_wait_slow(full, ph, &abort_sh, true);
+            }
+        return;
+    }
+    for (int64_t b = blockIdx.x; b < total; b += gridDim.x, ++n) {
+        const int s = (int)(n % (uint32_t)stages);
+        const bool ok = mbar_wait(bar0 + 8 * s, (n / (uint32_t)stages) & 1u, &abort_sh);
+        if (!__all_sync(0xffffffffu, ok)) {
+            *reinterpret_cast<volatile int *>(&abort_sh) = 1;
+            if (lane == 0 && err) atomicOr(err, kKernErrTimeout);
+            return;
+        }
+        const RJob &J = jobs[st[s].job];
+        if (st[s].whole && !st[s].check) affine_tile_rows<T, true>(J, st[s], base + (uint32_t)s * stage_b, warp);
+        else affine_tile_rows<T, false>(J, st[s], base + (uint32_t)s * stage_b, warp);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar0 + 8 * (kAStages + s));
+    }
+}
+
 // ---------------------------------------------------------------- kernels
 
 // Plans every unit (one warp each, 8 per CTA): plans[u], and the units that
@@ -1843,6 +2217,21 @@ cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_
     return cudaGetLastError();
 }
 
+// Affine jobs whose boxes are staged (tma_ok != 0 for every job of the launch).
+template <typename T>
+cudaError_t launch_affine_staged_t(const RJob *jobs, int njobs, int64_t total, uint32_t stage_b, cudaStream_t st, int sms,
+                                   int *err)
+{
+    const auto k = k_affine_staged<T>;
+    const int stages = (int)min((uint32_t)kAStages, (uint32_t)kAffineSmem / stage_b);
+    const int smem = (int)(stage_b * (uint32_t)stages) + 128;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t grid = total < sms ? total : sms;
+    k<<<(unsigned)grid, kAStagedThreads, smem, st>>>(jobs, njobs, total, stages, stage_b, err);
+    return cudaGetLastError();
+}
+
 template <typename T, int INTERP>
 cudaError_t launch_affine_t(const RJob *jobs, int njobs, int64_t total, cudaStream_t st, int sms)
 {
@@ -1892,6 +2281,14 @@ void brick_dims(int kind, int g, int64_t out[3])
     out[0] = kTBX;
     out[1] = kTBY;
     out[2] = g;
+}
+
+cudaError_t launch_affine_staged(const RJob *jobs_dev, int njobs, int64_t total_tiles, int dtype, uint32_t stage_bytes,
+                                 cudaStream_t st, int sm_count, int *err)
+{
+    if (total_tiles <= 0) return cudaSuccess;
+    return dtype == 1 ? launch_affine_staged_t<uint8_t>(jobs_dev, njobs, total_tiles, stage_bytes, st, sm_count, err)
+                      : launch_affine_staged_t<uint16_t>(jobs_dev, njobs, total_tiles, stage_bytes, st, sm_count, err);
 }
 
 cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_bricks, int dtype, int kind, int g,
