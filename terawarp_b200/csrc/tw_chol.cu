@@ -994,24 +994,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_chol_solve(Ctl C)
     __syncthreads();
 }
 
-// A, upper part included only inside the diagonal tiles' padding: tile (i, j)
-// of (Q'KQ)(4:,4:) + lambda I, i >= j, or the right-hand-side tile j, z(4:)'.
-// One CTA per tile, 256 threads; rows and columns past m are zero, with ones
-// on the diagonal.
+// Tile (i, j), i >= j, of (Q'KQ)(4:,4:) + lambda I (lower triangle; rows and
+// columns past m zero, with ones on the diagonal), or the right-hand-side tile
+// j, z(4:)'.  kFillParts CTAs per tile, 256 threads: a thread keeps its
+// column's landmark and vectors in registers and takes a few rows, whose own
+// come from shared memory.
+constexpr int kFillParts = 4;
 __global__ void __launch_bounds__(256) k_fill_tiles(const double *__restrict__ ctr, int n, const double *__restrict__ V,
                                                     const double *__restrict__ W, const double *__restrict__ Z,
                                                     double lambda, Ctl C)
 {
+    constexpr int ROWS = kNB / kFillParts;
+    __shared__ double row[ROWS][11];
     const int m = C.m, nblk = C.nblk;
     const int ntri = nblk * (nblk + 1) / 2;
-    int t = (int)blockIdx.x;
+    int t = (int)blockIdx.x / kFillParts;
+    const int part = (int)blockIdx.x % kFillParts;
     if (t >= ntri) {
         const int j = t - ntri;
         double *R = C.rhs + (size_t)j * kRhsD;
-        for (int e = threadIdx.x; e < kRhsD; e += blockDim.x) {
-            const int r = e / kTP, c = j * kNB + e % kTP;
-            R[e] = e % kTP < kNB && c < m ? Z[(size_t)(c + 4) * 4 + r] : 0.0;
-        }
+        if (part == 0)
+            for (int e = threadIdx.x; e < kRhsD; e += blockDim.x) {
+                const int r = e / kTP, c = j * kNB + e % kTP;
+                R[e] = e % kTP < kNB && c < m ? Z[(size_t)(c + 4) * 4 + r] : 0.0;
+            }
         return;
     }
     int j = 0;
@@ -1019,22 +1025,35 @@ __global__ void __launch_bounds__(256) k_fill_tiles(const double *__restrict__ c
         t -= nblk - j;
         ++j;
     }
-    const int i = j + t;
-    double *T = tile_ptr(C, i, j);
-    for (int e = threadIdx.x; e < kTileD; e += blockDim.x) {
-        const int r = e / kTP, c = e % kTP;
-        const int ri = i * kNB + r, cj = j * kNB + c;
-        double v = 0.0;
-        if (c < kNB && ri < m && cj < m && ri >= cj) {
-            const int gi = ri + 4, gj = cj + 4;
-            v = kdist(ctr, gi, gj);
+    const int i = j + t, r0 = part * ROWS;
+    for (int e = threadIdx.x; e < ROWS * 11; e += blockDim.x) {
+        const int q = e % 11, g = min(i * kNB + r0 + e / 11, m - 1) + 4;
+        row[e / 11][q] = q < 3 ? ctr[3 * g + q] : q < 7 ? V[4 * g + q - 3] : W[4 * g + q - 7];
+    }
+    const int c = threadIdx.x & (kNB - 1), cj = j * kNB + c, gj = min(cj, m - 1) + 4;
+    const double x = ctr[3 * gj], y = ctr[3 * gj + 1], z = ctr[3 * gj + 2];
+    double vj[4], wj[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) v -= V[gi * 4 + k] * W[gj * 4 + k] + W[gi * 4 + k] * V[gj * 4 + k];
+    for (int k = 0; k < 4; ++k) {
+        vj[k] = V[gj * 4 + k];
+        wj[k] = W[gj * 4 + k];
+    }
+    __syncthreads();
+    double *T = tile_ptr(C, i, j);
+    for (int r = threadIdx.x / kNB; r < ROWS; r += 256 / kNB) {
+        const int ri = i * kNB + r0 + r;
+        const double *q = row[r];
+        double v = 0.0;
+        if (ri < m && cj < m && ri >= cj) {
+            v = kdist(q[0], q[1], q[2], x, y, z);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v -= q[3 + k] * wj[k] + q[7 + k] * vj[k];
             if (ri == cj) v += lambda;
-        } else if (i == j && r == c) {
+        } else if (ri == cj) {
             v = 1.0;
         }
-        T[e] = v;
+        T[(r0 + r) * kTP + c] = v;
+        if (c < kTP - kNB) T[(r0 + r) * kTP + kNB + c] = 0.0;
     }
 }
 
@@ -1070,7 +1089,7 @@ cudaError_t launch_chol_solve(const double *ctr, int n, const double *V, const d
     cudaError_t e = cudaMemsetAsync(flags, 0, flag_ints(C.nblk) * sizeof(int), st);
     if (e != cudaSuccess) return e;
     const size_t fill = tri_tiles(C.nblk) + (size_t)C.nblk;
-    k_fill_tiles<<<(unsigned)fill, 256, 0, st>>>(ctr, n, V, W, Z, lambda, C);
+    k_fill_tiles<<<(unsigned)(fill * kFillParts), 256, 0, st>>>(ctr, n, V, W, Z, lambda, C);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_chol_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));

@@ -4,12 +4,12 @@
 
 namespace tw {
 
-// K_ij = -|s_i - s_j|
-__device__ __forceinline__ double kdist(const double *ctr, int i, int j)
+// -|a - b|
+__device__ __forceinline__ double kdist(double ax, double ay, double az, double bx, double by, double bz)
 {
-    double dx = ctr[3 * i] - ctr[3 * j];
-    double dy = ctr[3 * i + 1] - ctr[3 * j + 1];
-    double dz = ctr[3 * i + 2] - ctr[3 * j + 2];
+    double dx = ax - bx;
+    double dy = ay - by;
+    double dz = az - bz;
     return -sqrt(dx * dx + dy * dy + dz * dz);
 }
 

@@ -52,81 +52,148 @@ constexpr int kStSingularX = 1;
 constexpr int kStNotSPD = 2;   // set by the Cholesky kernel (tw_chol.cu)
 constexpr int kStTimeout = 4;
 
-__device__ double block_sum(double v, double *sh)
+// The vector kernels below run as one CTA and are a chain of block-wide sums;
+// their time is the latency of those rounds.  Sums that do not depend on one
+// another share a round (the four right-hand sides, the dot products of one
+// reflector), and one thread per sum adds the warps' parts, where every thread
+// adding all 32 of them took 2000 cycles a round in shared-memory loads.  Each
+// sum still adds the same terms in the same order: lanes as a tree, then warps
+// 0, 1, ... (warps past the last landmark hold zeros and are left out).
+constexpr int kMostSums = 12;
+struct SumSmem {
+    double part[kMostSums][33];
+    double sum[kMostSums];
+};
+
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N], int n, SumSmem &S)
 {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    static_assert(N <= kMostSums, "sums per round");
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0)
+#pragma unroll
+        for (int i = 0; i < N; ++i) S.part[i][warp] = v[i];
     __syncthreads();
-    if (lane == 0) sh[warp] = v;
+    if (threadIdx.x < N) {
+        double t = 0.0;
+        const int nw = min((int)blockDim.x >> 5, (n + 31) >> 5);
+#pragma unroll 8
+        for (int w = 0; w < nw; ++w) t += S.part[threadIdx.x][w];
+        S.sum[threadIdx.x] = t;
+    }
     __syncthreads();
-    double t = 0.0;
-    const int nw = (blockDim.x + 31) >> 5;
-    for (int i = 0; i < nw; ++i) t += sh[i];
-    return t;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = S.sum[i];
+}
+
+// Reflector k of the QR below: the rows' column k is turned into V's, and the
+// columns from k on are updated.
+template <int K>
+__device__ __forceinline__ void qr_step(int n, double nrm2, double colnorm, double *Xw, double *V, double *tau, double *R,
+                                        int *status, SumSmem &S)
+{
+    const double nrm = sqrt(nrm2);
+    const double xkk = Xw[K * 4 + K];
+    const double alpha = xkk > 0 ? -nrm : nrm;
+    const double vk = xkk - alpha;
+    const double vv = nrm2 - xkk * xkk + vk * vk;
+    const double t = vv > 0 ? 2.0 / vv : 0.0;
+    double d[4 - K];
+#pragma unroll
+    for (int j = 0; j < 4 - K; ++j) d[j] = 0.0;
+#pragma unroll 4
+    for (int i = K + threadIdx.x; i < n; i += blockDim.x) {
+        const double v = i == K ? vk : Xw[i * 4 + K];
+        V[i * 4 + K] = v;
+#pragma unroll
+        for (int j = 0; j < 4 - K; ++j) d[j] += v * Xw[i * 4 + K + j];
+    }
+    if (threadIdx.x < K) V[threadIdx.x * 4 + K] = 0.0;
+    block_sums(d, n, S);
+    if (threadIdx.x == 0) {
+        tau[K] = t;
+        R[K * 4 + K] = alpha;
+        for (int j = 0; j < K; ++j) R[K * 4 + j] = 0.0;
+        if (!(fabs(alpha) > 1e-10 * (colnorm + 1e-300))) atomicOr(status, kStSingularX);
+    }
+#pragma unroll 4
+    for (int i = K + threadIdx.x; i < n; i += blockDim.x) {
+        const double v = i == K ? vk : Xw[i * 4 + K];
+#pragma unroll
+        for (int j = 4 - K - 1; j >= 0; --j) {  // column K last: it is v itself
+            const double sj = t * d[j];
+            const double x = Xw[i * 4 + K + j] - sj * v;
+            Xw[i * 4 + K + j] = x;
+            if (i == K && j > 0) R[K * 4 + K + j] = x;
+        }
+    }
+    __syncthreads();
 }
 
 // 1. Householder QR of X = [1 s].  Xw (n x 4) is a work copy; V (n x 4) gets
 // the reflectors (zeros above the diagonal), tau[4], R[16].
 __global__ void k_qr(const double *ctr, int n, double *Xw, double *V, double *tau, double *R, int *status)
 {
-    __shared__ double sh[32];
+    __shared__ SumSmem S;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};  // squared column norms; the first is also the first reflector's
+#pragma unroll 4
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        Xw[i * 4 + 0] = 1.0;
-        Xw[i * 4 + 1] = ctr[3 * i];
-        Xw[i * 4 + 2] = ctr[3 * i + 1];
-        Xw[i * 4 + 3] = ctr[3 * i + 2];
-    }
-    __syncthreads();
-    double colnorm[4];
-    for (int j = 0; j < 4; ++j) {
-        double s = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) s += Xw[i * 4 + j] * Xw[i * 4 + j];
-        colnorm[j] = sqrt(block_sum(s, sh));
-    }
-    for (int k = 0; k < 4; ++k) {
-        double s = 0.0;
-        for (int i = k + threadIdx.x; i < n; i += blockDim.x) s += Xw[i * 4 + k] * Xw[i * 4 + k];
-        const double nrm2 = block_sum(s, sh);
-        const double nrm = sqrt(nrm2);
-        const double xkk = Xw[k * 4 + k];
-        const double alpha = xkk > 0 ? -nrm : nrm;
-        const double vk = xkk - alpha;
-        const double vv = nrm2 - xkk * xkk + vk * vk;
-        const double t = vv > 0 ? 2.0 / vv : 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x)
-            V[i * 4 + k] = i < k ? 0.0 : (i == k ? vk : Xw[i * 4 + k]);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            tau[k] = t;
-            R[k * 4 + k] = alpha;
-            for (int j = 0; j < k; ++j) R[k * 4 + j] = 0.0;
-            if (!(fabs(alpha) > 1e-10 * (colnorm[k] + 1e-300))) atomicOr(status, kStSingularX);
+        const double x[4] = {1.0, ctr[3 * i], ctr[3 * i + 1], ctr[3 * i + 2]};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            Xw[i * 4 + j] = x[j];
+            s[j] += x[j] * x[j];
         }
-        for (int j = k; j < 4; ++j) {
-            double d = 0.0;
-            for (int i = k + threadIdx.x; i < n; i += blockDim.x) d += V[i * 4 + k] * Xw[i * 4 + j];
-            const double sj = t * block_sum(d, sh);
-            for (int i = k + threadIdx.x; i < n; i += blockDim.x) Xw[i * 4 + j] -= sj * V[i * 4 + k];
-            __syncthreads();
-            if (threadIdx.x == 0 && j > k) R[k * 4 + j] = Xw[k * 4 + j];
-        }
-        __syncthreads();
     }
+    block_sums(s, n, S);
+    double c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = sqrt(s[j]);
+    qr_step<0>(n, s[0], c[0], Xw, V, tau, R, status, S);
+    auto norm2 = [&](int k) {
+        double q[1] = {0.0};
+        for (int i = k + threadIdx.x; i < n; i += blockDim.x) q[0] += Xw[i * 4 + k] * Xw[i * 4 + k];
+        block_sums(q, n, S);
+        return q[0];
+    };
+    qr_step<1>(n, norm2(1), c[1], Xw, V, tau, R, status, S);
+    qr_step<2>(n, norm2(2), c[2], Xw, V, tau, R, status, S);
+    qr_step<3>(n, norm2(3), c[3], Xw, V, tau, R, status, S);
 }
 
 // out (n x 4) = K B for the implicit K_ij = -|s_i - s_j|; one warp per row.
-__global__ void k_kmul(const double *ctr, int n, const double *B, double *out)
+// The eight rows of a CTA share the other side's landmarks and B, staged in
+// shared memory component by component (read from global memory, each lane's
+// seven strided loads per term bounded it: 91 us at n = 4096); what is left is
+// the FP64 pipe's square roots.
+constexpr int kKmulTile = 256;
+__global__ void __launch_bounds__(256) k_kmul(const double *__restrict__ ctr, int n, const double *__restrict__ B,
+                                              double *__restrict__ out)
 {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    __shared__ double c[3][kKmulTile], q[4][kKmulTile];
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
+    const int r = min(row, n - 1);
+    const double x = ctr[3 * r], y = ctr[3 * r + 1], z = ctr[3 * r + 2];
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    for (int j = lane; j < n; j += 32) {
-        const double k = kdist(ctr, warp, j);
-        a0 += k * B[j * 4 + 0];
-        a1 += k * B[j * 4 + 1];
-        a2 += k * B[j * 4 + 2];
-        a3 += k * B[j * 4 + 3];
+    for (int j0 = 0; j0 < n; j0 += kKmulTile) {
+        const int cnt = min(kKmulTile, n - j0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < 3 * cnt; e += 256) c[e % 3][e / 3] = ctr[3 * (size_t)j0 + e];
+        for (int e = threadIdx.x; e < 4 * cnt; e += 256) q[e & 3][e >> 2] = B[4 * (size_t)j0 + e];
+        __syncthreads();
+#pragma unroll 4
+        for (int j = lane; j < cnt; j += 32) {
+            const double k = kdist(x, y, z, c[0][j], c[1][j], c[2][j]);
+            a0 += k * q[0][j];
+            a1 += k * q[1][j];
+            a2 += k * q[2][j];
+            a3 += k * q[3][j];
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         a0 += __shfl_xor_sync(0xffffffffu, a0, o);
@@ -134,76 +201,101 @@ __global__ void k_kmul(const double *ctr, int n, const double *B, double *out)
         a2 += __shfl_xor_sync(0xffffffffu, a2, o);
         a3 += __shfl_xor_sync(0xffffffffu, a3, o);
     }
-    if (lane == 0) {
-        out[warp * 4 + 0] = a0;
-        out[warp * 4 + 1] = a1;
-        out[warp * 4 + 2] = a2;
-        out[warp * 4 + 3] = a3;
+    if (lane == 0 && row < n) {
+        out[row * 4 + 0] = a0;
+        out[row * 4 + 1] = a1;
+        out[row * 4 + 2] = a2;
+        out[row * 4 + 3] = a3;
     }
 }
 
+// Applies reflector k to the four columns of Z's rows; d: its sums V_k . Z_c.
+__device__ __forceinline__ void reflect(int n, int k, const double *V, double tau, const double (&d)[4], double *Z)
+{
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double v = V[i * 4 + k];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) Z[i * 4 + c] -= tau * d[c] * v;
+    }
+}
+
+// Step K of k_wvec: w_K, and reflector K applied to Z.
+template <int K>
+__device__ __forceinline__ void wvec_step(int n, const double *V, const double *tau, const double *P0, double *W, double *Z,
+                                          SumSmem &S)
+{
+    // p_K = P0_K - sum_{j<K} [ v_j (w_j . v_K) + w_j (v_j . v_K) ]; the sums
+    // V_K . Z_c ride along
+    double s[2 * K + 4];
+#pragma unroll
+    for (int j = 0; j < 2 * K + 4; ++j) s[j] = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double v = V[i * 4 + K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            s[2 * j] += W[i * 4 + j] * v;
+            s[2 * j + 1] += V[i * 4 + j] * v;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[2 * K + c] += v * Z[i * 4 + c];
+    }
+    block_sums(s, n, S);
+    double beta[1] = {0.0};
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        double p = P0[i * 4 + K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) p -= V[i * 4 + j] * s[2 * j] + W[i * 4 + j] * s[2 * j + 1];
+        W[i * 4 + K] = p;  // temporarily p
+        beta[0] += V[i * 4 + K] * p;
+    }
+    const double d[4] = {s[2 * K], s[2 * K + 1], s[2 * K + 2], s[2 * K + 3]};
+    reflect(n, K, V, tau[K], d, Z);
+    block_sums(beta, n, S);
+    const double t = tau[K];
+    const double cf = 0.5 * t * t * beta[0];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) W[i * 4 + K] = t * W[i * 4 + K] - cf * V[i * 4 + K];
+}
+
 // 2. From P0 = K V derive the rank-2 update vectors W (n x 4), and Z = Q' Y.
+// (A thread reads only rows that it wrote.)
 __global__ void k_wvec(int n, const double *V, const double *tau, const double *P0, double *W, const double *Y,
                        double *Z)
 {
-    __shared__ double sh[32];
-    __shared__ double wv[4][4], vvd[4][4];  // w_j . v_k, v_j . v_k
-    for (int k = 0; k < 4; ++k) {
-        // p_k = P0_k - sum_{j<k} [ v_j (w_j . v_k) + w_j (v_j . v_k) ]
-        for (int j = 0; j < k; ++j) {
-            double a = 0, b = 0;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                a += W[i * 4 + j] * V[i * 4 + k];
-                b += V[i * 4 + j] * V[i * 4 + k];
-            }
-            a = block_sum(a, sh);
-            b = block_sum(b, sh);
-            if (threadIdx.x == 0) { wv[j][k] = a; vvd[j][k] = b; }
-        }
-        __syncthreads();
-        double beta = 0.0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            double p = P0[i * 4 + k];
-            for (int j = 0; j < k; ++j) p -= V[i * 4 + j] * wv[j][k] + W[i * 4 + j] * vvd[j][k];
-            W[i * 4 + k] = p;  // temporarily p
-            beta += V[i * 4 + k] * p;
-        }
-        beta = block_sum(beta, sh);
-        const double t = tau[k];
-        const double cf = 0.5 * t * t * beta;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) W[i * 4 + k] = t * W[i * 4 + k] - cf * V[i * 4 + k];
-        __syncthreads();
-    }
-    // Z = H4 H3 H2 H1 Y
+    __shared__ SumSmem S;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         for (int c = 0; c < 4; ++c) Z[i * 4 + c] = Y[i * 4 + c];
-    __syncthreads();
-    for (int k = 0; k < 4; ++k) {
-        for (int c = 0; c < 4; ++c) {
-            double d = 0.0;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) d += V[i * 4 + k] * Z[i * 4 + c];
-            d = tau[k] * block_sum(d, sh);
-            for (int i = threadIdx.x; i < n; i += blockDim.x) Z[i * 4 + c] -= d * V[i * 4 + k];
-            __syncthreads();
-        }
+    wvec_step<0>(n, V, tau, P0, W, Z, S);
+    wvec_step<1>(n, V, tau, P0, W, Z, S);
+    wvec_step<2>(n, V, tau, P0, W, Z, S);
+    wvec_step<3>(n, V, tau, P0, W, Z, S);
+}
+
+__device__ __forceinline__ void reflector_sums(int n, int k, const double *V, const double *Z, double (&d)[4], SumSmem &S)
+{
+#pragma unroll
+    for (int c = 0; c < 4; ++c) d[c] = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const double v = V[i * 4 + k];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d[c] += v * Z[i * 4 + c];
     }
+    block_sums(d, n, S);
 }
 
 // 4c. c = H1 H2 H3 H4 [0; w]  (Z rows 0..3 are replaced by zeros)
 __global__ void k_apply_q(int n, const double *V, const double *tau, const double *Z, double *C)
 {
-    __shared__ double sh[32];
+    __shared__ SumSmem S;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         for (int c = 0; c < 4; ++c) C[i * 4 + c] = i < 4 ? 0.0 : Z[i * 4 + c];
-    __syncthreads();
     for (int k = 3; k >= 0; --k) {
-        for (int c = 0; c < 4; ++c) {
-            double d = 0.0;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) d += V[i * 4 + k] * C[i * 4 + c];
-            d = tau[k] * block_sum(d, sh);
-            for (int i = threadIdx.x; i < n; i += blockDim.x) C[i * 4 + c] -= d * V[i * 4 + k];
-            __syncthreads();
-        }
+        double d[4];
+        reflector_sums(n, k, V, C, d, S);
+        reflect(n, k, V, tau[k], d, C);
     }
 }
 
@@ -211,26 +303,26 @@ __global__ void k_apply_q(int n, const double *V, const double *tau, const doubl
 __global__ void k_finish_d(int n, const double *V, const double *tau, const double *R, const double *Y, double *KC,
                            double *d_out)
 {
-    __shared__ double sh[32];
+    __shared__ SumSmem S;
     for (int i = threadIdx.x; i < n; i += blockDim.x)
         for (int c = 0; c < 4; ++c) KC[i * 4 + c] = Y[i * 4 + c] - KC[i * 4 + c];
-    __syncthreads();
     for (int k = 0; k < 4; ++k) {
-        for (int c = 0; c < 4; ++c) {
-            double d = 0.0;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) d += V[i * 4 + k] * KC[i * 4 + c];
-            d = tau[k] * block_sum(d, sh);
-            for (int i = threadIdx.x; i < n; i += blockDim.x) KC[i * 4 + c] -= d * V[i * 4 + k];
-            __syncthreads();
-        }
+        double d[4];
+        reflector_sums(n, k, V, KC, d, S);
+        reflect(n, k, V, tau[k], d, KC);
     }
-    if (threadIdx.x == 0) {
-        for (int c = 0; c < 4; ++c)
-            for (int a = 3; a >= 0; --a) {
-                double s = KC[a * 4 + c];
-                for (int b = a + 1; b < 4; ++b) s -= R[a * 4 + b] * d_out[b * 4 + c];
-                d_out[a * 4 + c] = s / R[a * 4 + a];
-            }
+    __syncthreads();
+    if (threadIdx.x < 4) {  // one thread per right-hand side
+        const int c = threadIdx.x;
+        double x[4];
+#pragma unroll
+        for (int a = 3; a >= 0; --a) {
+            double s = KC[a * 4 + c];
+#pragma unroll
+            for (int b = a + 1; b < 4; ++b) s -= R[a * 4 + b] * x[b];
+            x[a] = s / R[a * 4 + a];
+            d_out[a * 4 + c] = x[a];
+        }
     }
 }
 
