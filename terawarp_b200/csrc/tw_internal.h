@@ -59,7 +59,8 @@ struct alignas(128) RJob {
     int g;                 // grid spacing (TPS)
     int zs;                // output planes per TPS work unit (divides g or is a multiple of it; set by run_jobs)
     int tma_ok;            // units may stage their source footprint in shared memory: 1 through tmap, 2
-                           // (affine) row by row
+                           // (affine) by granules
+    int ragged;            // TPS: src is a copy with padded rows of a source TMA cannot describe
     int st_w, st_h, st_d;  // affine: staged box, elements (row by row) or the TMA box
     int st_pr, st_pp;      // affine: its row and plane pitch in shared memory, bytes
     int dtype;             // 1 u8, 2 u16
@@ -74,10 +75,13 @@ struct alignas(128) RJob {
 // gave up); may be null.  stage_ws: for trilinear TPS, device memory of
 // tps_stage_ws_bytes(total_bricks) whose first 8 bytes are zero: the units
 // are planned, staged units run the TMA-staged kernel and the rest the
-// gather kernel; null: the gather kernel takes every unit.
+// gather kernel; null: the gather kernel takes every unit.  ragged: the jobs'
+// sources are padded copies (every job's `ragged` is set).
 cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_bricks, int dtype,
                             int kind, int g, int interp, cudaStream_t st, int sm_count, int *err,
-                            void *stage_ws);
+                            void *stage_ws, bool ragged);
+// A copy of the job's source with rows of row_bytes (a multiple of 16).
+cudaError_t launch_repitch(const RJob &j, void *dst, int64_t row_bytes, cudaStream_t st, int sm_count);
 // Trilinear affine jobs whose tiles are staged (encode_affine_box gave each a box), in
 // units of kAffineTile output voxels; stage_bytes: the largest of their boxes.
 cudaError_t launch_affine_staged(const RJob *jobs_dev, int njobs, int64_t total_tiles, int dtype, uint32_t stage_bytes,

@@ -87,15 +87,76 @@ namespace {
 
 tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cudaStream_t st);
 
+// Copies the sources of those jobs of [first, end) that gain by it into rows
+// padded to 16 bytes (one block, `copy`), moves these jobs to the front and
+// returns their end.  A small launch gathers in the same or less time (517 x
+// 389 x 203 uint16: 367 us gathered, 370 copied and staged; 801 x 601 x 301:
+// 1091 and 850), and the copies are held to 512 MiB, which the context's pool
+// then keeps, and to what the budget has left.
+RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaStream_t st)
+{
+    constexpr int64_t kMinVoxels = 48 << 20;
+    constexpr size_t kMostBytes = (size_t)512 << 20;
+    int64_t vox = 0;
+    size_t bytes = 0;
+    const auto row_bytes = [](const RJob &j) { return (size_t)((j.src_n[0] * (j.dtype == TW_U8 ? 1 : 2) + 15) / 16 * 16); };
+    const auto size = [&](const RJob &j) { return (row_bytes(j) * (size_t)(j.src_n[1] * j.src_n[2]) + 255) / 256 * 256; };
+    RJob *const last = std::stable_partition(first, end, [&](const RJob &j) {
+        const int64_t out = j.out_n[0] * j.out_n[1] * j.out_n[2];
+        if (j.src_n[0] < kStageBoxW || j.src_n[1] < kStageBoxH || j.src_n[2] < 2 || bytes + size(j) > kMostBytes) return false;
+        if (2 * out < j.src_n[0] * j.src_n[1] * j.src_n[2]) return false;  // (a slab: the copy takes the whole source)
+        bytes += size(j);
+        vox += out;
+        return true;
+    });
+    if (last == first || vox < kMinVoxels || dmalloc_on(ctx, &copy.p, bytes, st) != TW_OK) return first;
+    copy.bytes = bytes;
+    unsigned char *to = static_cast<unsigned char *>(copy.p);
+    for (RJob *j = first; j < last; ++j) {
+        RJob padded = *j;
+        padded.src = to;
+        padded.src_py = (int64_t)row_bytes(*j) / (j->dtype == TW_U8 ? 1 : 2);
+        padded.src_pz = padded.src_py * j->src_n[1];
+        padded.ragged = 1;
+        if (!encode_source_map(padded) || launch_repitch(*j, to, (int64_t)row_bytes(*j), st, ctx->sm_count) != cudaSuccess) {
+            cudaGetLastError();  // (a descriptor the driver refuses: it and the rest gather)
+            return j;
+        }
+        to += size(*j);
+        *j = padded;
+        count_launch(ctx);
+    }
+    return last;
+}
+
 }  // namespace
 
 tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
 {
     if (njobs <= 0) return TW_OK;
-    if (jobs[0].kind == 1) return run_group(ctx, jobs, njobs, 0, st);
+    const bool staging = ctx->resample_staging.load() != 0;
+    if (jobs[0].kind == 1) {
+        // trilinear TPS jobs: those whose source TMA can describe, those that
+        // are resampled from a padded copy, and the rest, which gather
+        if (!staging || jobs[0].interp != 0) return run_group(ctx, jobs, njobs, 0, st);
+        RJob *const end = jobs + njobs;
+        RJob *const mid = std::stable_partition(jobs, end, [](RJob &j) { return encode_source_map(j); });
+        if (mid > jobs) TW_TRY(run_group(ctx, jobs, (int)(mid - jobs), 0, st));
+        StreamBlock copy{ctx, st};
+        RJob *const last = pad_sources(ctx, mid, end, copy, st);
+        if (last > mid) {
+            tw_status s = run_group(ctx, mid, (int)(last - mid), 0, st);
+            if (s == TW_ERR_OOM) {  // no room for the plans: gather, from the copies
+                for (RJob *j = mid; j < last; ++j) j->tma_ok = 0;
+                s = run_group(ctx, mid, (int)(last - mid), 0, st);
+            }
+            if (s != TW_OK) return s;
+        }
+        if (end > last) TW_TRY(run_group(ctx, last, (int)(end - last), 0, st));
+        return TW_OK;
+    }
     // affine jobs whose tiles can be staged first, the others gather
     uint32_t box = 0;
-    const bool staging = ctx->resample_staging.load() != 0;
     RJob *const mid = std::stable_partition(jobs, jobs + njobs, [&](RJob &j) {
         const uint32_t b = staging ? encode_affine_box(j) : 0u;
         box = std::max(box, b);
@@ -130,21 +191,18 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
     };
     // TPS units walk 64 output planes (several cell layers: the staged source
     // window is loaded once per walk); when a launch has too few units to
-    // fill every SM a few times, they get shorter, down to parts of a layer
+    // balance, they get shorter, down to 16 planes -- below that the windows
+    // and the per-layer set-up cost more than an even last wave gives (256 x 256
+    // x 128 uint8: 109 us at 4 planes, 91 at 16; 512^3 uint16: 573 at 64, 513 at
+    // 16; 1024 x 1024 x 256 uint8, spacing 4: 2114 at 64, 2011 at 32)
     int zs = jobs[0].kind == 1 ? std::max(64, jobs[0].g) : 8;
     count(zs);
-    while (jobs[0].kind == 1 && zs > 1 && total < 8 * (int64_t)ctx->sm_count) {
+    while (jobs[0].kind == 1 && zs > 16 && total < 32 * (int64_t)ctx->sm_count) {
         zs /= 2;
         count(zs);
     }
     if (total == 0) return TW_OK;
-    bool staged = false;  // some job's source can be staged by TMA
-    if (jobs[0].kind == 1 && jobs[0].interp == 0)
-        for (int i = 0; i < njobs; ++i) {
-            if (ctx->resample_staging.load()) encode_source_map(jobs[i]);
-            else jobs[i].tma_ok = 0;
-            staged = staged || jobs[i].tma_ok;
-        }
+    const bool staged = jobs[0].kind == 1 && jobs[0].tma_ok != 0, ragged = staged && jobs[0].ragged;
     // the units' staging plans and the list of units left to the gather kernel
     StreamBlock fb{ctx, st};
     if (staged) {
@@ -158,7 +216,7 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
     const auto launch = [&](const RJob *d) {
         return affine_box ? launch_affine_staged(d, njobs, total, jobs[0].dtype, affine_box, st, ctx->sm_count, ctx->d_err)
                           : launch_resample(d, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
-                                            ctx->sm_count, ctx->d_err, d_fb);
+                                            ctx->sm_count, ctx->d_err, d_fb, ragged);
     };
     const size_t bytes = sizeof(RJob) * (size_t)njobs;
     if (njobs <= tw_ctx::kJobsPerSlot && ctx->job_d) {

@@ -31,6 +31,7 @@
 
 #include "tw_internal.h"
 
+#include <algorithm>
 #include <cstdint>
 
 namespace tw {
@@ -598,9 +599,11 @@ constexpr int kRowWarps = kTBY / kRowsPerWarp;  // row warp y owns rows y + k kR
 constexpr int kStagedThreads = 32 * kRowWarps + 32;  // row warps + the producer warp
 constexpr int kBoxW = kStageBoxW;            // TMA box: source elements per row copy
 constexpr int kHMax = kStageBoxH;            // TMA box: rows per staged plane
-constexpr int kRing = 16;                    // plane slots (plus the mirror of slot 0); a power of 2
+// plane slots (plus the mirror of slot 0), a power of 2: 128 KB of them
+template <typename T>
+constexpr int kRing = 32 / (int)sizeof(T);
+constexpr int kGatherParts = 8;              // parts of a leftover walk in the gather kernel
 constexpr int kMinAhead = 3;                 // slots a walk's window leaves for copies in flight
-static_assert((kRing & (kRing - 1)) == 0, "slot = sequence & (kRing - 1)");
 // a wait on a copy or on another warp that has not ended after this long is
 // an error (the kernel reports kKernErrTimeout and returns)
 constexpr unsigned long long kStageWaitNs = 2000000000ull;
@@ -629,8 +632,8 @@ struct TGeom {
     static constexpr int ES = (int)sizeof(T);
     static constexpr int ROW_B = kBoxW * ES;
     static constexpr int PLANE_B = kHMax * ROW_B;
-    static constexpr int RING_B = (kRing + 1) * PLANE_B;
-    static constexpr int NBAR = 2 * kRing;        // full[kRing], empty[kRing]
+    static constexpr int RING_B = (kRing<T> + 1) * PLANE_B;
+    static constexpr int NBAR = 2 * kRing<T>;        // full, empty
     // ring, barriers, then the weight tables: W[G] (float4) and W2[G][2]
     // (float4 pairs (w0, w0, w1, w1), (w2, w2, w3, w3)), then the row warps'
     // nodes (two float4 per y-contracted node: the interior walks keep them
@@ -828,12 +831,21 @@ __device__ Plan plan_walk(const RJob &J, const Walk &w)
     const int rows = kTBY + fy1 - fy0 + 1;
     if (rows > kHMax) return P;
     const int a = fz0, b = fz1 + 1;
-    if (b - a + 1 + kMinAhead > kRing) return P;
+    if (b - a + 1 + kMinAhead > kRing<T>) return P;
     const int64_t ry0 = w.Oy - J.src_o[1] + fy0;
     const int64_t p0 = w.z0 + a - J.src_o[2], p1 = w.z1 - 1 + b - J.src_o[2];
     const int64_t lim = (int64_t)1 << 30;  // TMA coordinates and the plan's coordinates are int32
     if (rx0 < -lim || rx0 > lim || ry0 < -lim || ry0 + rows > lim || p0 < -lim || p1 > lim) return P;
     if (w.Ox > lim || w.Oy > lim || w.z1 > lim) return P;
+    if (J.ragged) {
+        // a sample on the source's last element takes the gathered path's floor
+        // (see walk_rows), which for such sources is the clamped one: at least
+        // two elements along every axis, offsets of a layer's taps below 1e9
+        const double far = fmax(fabs((double)fx0) + 2.0, kTBX + fabs((double)fx1) + 3.0) +
+                           fmax(fabs((double)fy0) + 2.0, kTBY + fabs((double)fy1) + 3.0) * (double)J.src_py +
+                           fmax(fabs((double)fz0) + 2.0, G + fabs((double)fz1) + 3.0) * (double)J.src_pz;
+        if (J.src_n[0] < 2 || J.src_n[1] < 2 || J.src_n[2] < 2 || far >= 0.9e9) return P;
+    }
     // staged walks index the node grid with 32 bits
     if (J.gsz[0] * J.gsz[1] * J.gsz[2] >= ((int64_t)1 << 31)) return P;
     P.staged = 1;
@@ -851,13 +863,14 @@ __device__ Plan plan_walk(const RJob &J, const Walk &w)
     P.z0 = (int)w.z0;
     P.z1 = (int)w.z1;
     // interior: the unit lies wholly inside the output region, its voxel
-    // pairs can be stored as one word each, and every sample q (with the
+    // pairs can be stored as one word each (walks of ragged sources can also
+    // store element by element), and every sample q (with the
     // margin) has 0 <= floor(q) and floor(q) + 1 <= sz - 1 inside both the
     // subject volume and the source buffer, so no range test can fail
     const int64_t pe[3] = {w.Ox + kTBX - 1, w.Oy + kTBY - 1, w.z1 - 1};
     const int64_t ps[3] = {w.Ox, w.Oy, w.z0};
     bool in = w.Ox + kTBX <= J.out_o[0] + J.out_n[0] && w.Oy + kTBY <= J.out_o[1] + J.out_n[1];
-    in = in && ((uintptr_t)J.dst) % (2 * sizeof(T)) == 0 && J.dst_py % 2 == 0 && J.dst_pz % 2 == 0;
+    in = in && (J.ragged || (((uintptr_t)J.dst) % (2 * sizeof(T)) == 0 && J.dst_py % 2 == 0 && J.dst_pz % 2 == 0));
     for (int ax = 0; ax < 3; ++ax) {
         const double lo = (double)ps[ax] + (double)mn[ax] - (double)e;
         const double hi = (double)pe[ax] + (double)mx[ax] + (double)e;
@@ -882,16 +895,19 @@ __device__ __forceinline__ int list_count(const int *list) { return list[0]; }
 // Ring barriers come in plane pairs: planes 2p and 2p + 1 (sequence numbers)
 // share the "full" and "empty" mbarriers of pair slot p & (kPairs - 1), so a
 // row warp waits and releases once per two planes.
-constexpr int kPairs = kRing / 2;
+template <typename T>
+constexpr int kPairs = kRing<T> / 2;
 
+template <typename T>
 __device__ __forceinline__ uint32_t full_bar(const TSmem &S, uint32_t pair)
 {
-    return S.sfull + 8u * (pair & (uint32_t)(kPairs - 1));
+    return S.sfull + 8u * (pair & (uint32_t)(kPairs<T> - 1));
 }
 
+template <typename T>
 __device__ __forceinline__ uint32_t empty_bar(const TSmem &S, uint32_t pair)
 {
-    return S.sfull + 8u * (kRing + (pair & (uint32_t)(kPairs - 1)));
+    return S.sfull + 8u * (kRing<T> + (pair & (uint32_t)(kPairs<T> - 1)));
 }
 
 // The producer (lane 0 of the producer warp): copies every source plane of
@@ -920,15 +936,15 @@ __device__ bool produce(const RJob *__restrict__ jobs, const int *__restrict__ l
         }
         const int pfirst = (int)((int64_t)P.z0 + P.a - J.src_o[2]);
         for (int i = 0; i < P.nplanes; ++i, ++seq) {
-            const uint32_t slot = seq & (uint32_t)(kRing - 1), pair = seq >> 1;
-            const uint32_t full = full_bar(S, pair);
-            if ((seq & 1u) == 0 && pair >= (uint32_t)kPairs &&
-                !mbar_wait_producer(empty_bar(S, pair), ((pair / kPairs) - 1u) & 1u, S.abort))
+            const uint32_t slot = seq & (uint32_t)(kRing<T> - 1), pair = seq >> 1;
+            const uint32_t full = full_bar<T>(S, pair);
+            if ((seq & 1u) == 0 && pair >= (uint32_t)kPairs<T> &&
+                !mbar_wait_producer(empty_bar<T>(S, pair), ((pair / kPairs<T>) - 1u) & 1u, S.abort))
                 return false;
             mbar_expect_tx(full, (uint32_t)(slot == 0 ? 2 : 1) * (uint32_t)Gm::PLANE_B);
             const uint32_t d = S.sring + slot * (uint32_t)Gm::PLANE_B;
             tma_plane(d, &J.tmap, P.rx0, P.ry0, pfirst + i, full);
-            if (slot == 0) tma_plane(d + (uint32_t)(kRing * Gm::PLANE_B), &J.tmap, P.rx0, P.ry0, pfirst + i, full);
+            if (slot == 0) tma_plane(d + (uint32_t)(kRing<T> * Gm::PLANE_B), &J.tmap, P.rx0, P.ry0, pfirst + i, full);
         }
     }
     return true;
@@ -939,14 +955,15 @@ __device__ bool produce(const RJob *__restrict__ jobs, const int *__restrict__ l
 // completes once the copy lands.  Then every copy issued has landed before
 // the CTA exits (the row warps waited for all of them unless a wait gave
 // up; bounded waits).
+template <typename T>
 __device__ void drain_copies(const TSmem &S, uint32_t seq)
 {
-    if (seq & 1u) mbar_arrive(full_bar(S, seq >> 1));
+    if (seq & 1u) mbar_arrive(full_bar<T>(S, seq >> 1));
     const uint32_t npairs = (seq + 1u) >> 1;
-    const uint32_t n0 = npairs > (uint32_t)kPairs ? npairs - kPairs : 0u;
+    const uint32_t n0 = npairs > (uint32_t)kPairs<T> ? npairs - kPairs<T> : 0u;
     for (uint32_t n = n0; n < npairs; ++n)
-        if (!mbar_try(full_bar(S, n), (n / kPairs) & 1u))
-            mbar_wait_slow(full_bar(S, n), (n / kPairs) & 1u, S.abort, true);
+        if (!mbar_try(full_bar<T>(S, n), (n / kPairs<T>) & 1u))
+            mbar_wait_slow(full_bar<T>(S, n), (n / kPairs<T>) & 1u, S.abort, true);
 }
 
 // A row warp's place in the ring: the next plane pair to wait for and the
@@ -960,11 +977,12 @@ struct RingPos {
 // Waits (bounded) for the planes before sequence `need` (their pairs);
 // false if a wait gave up.  Every lane waits; the outcome is made uniform
 // across the warp.
+template <typename T>
 __device__ __forceinline__ bool wait_planes(const TSmem &S, RingPos &R, uint32_t need)
 {
     const uint32_t last = (need - 1u) >> 1;  // the pair of plane need - 1
     for (; R.wpair <= last; ++R.wpair) {
-        const bool ok = mbar_wait(full_bar(S, R.wpair), (R.wpair / kPairs) & 1u, S.abort);
+        const bool ok = mbar_wait(full_bar<T>(S, R.wpair), (R.wpair / kPairs<T>) & 1u, S.abort);
         if (!__all_sync(0xffffffffu, ok)) return false;
     }
     return true;
@@ -973,9 +991,10 @@ __device__ __forceinline__ bool wait_planes(const TSmem &S, RingPos &R, uint32_t
 // Releases the oldest plane the warp holds.  When it is the second plane of
 // its pair, every lane arrives on the pair's "empty" barrier (32 arrivals
 // per row warp), each arrival a release of that lane's reads of both planes.
+template <typename T>
 __device__ __forceinline__ void release_plane(const TSmem &S, RingPos &R)
 {
-    if (R.rseq & 1u) mbar_arrive(empty_bar(S, R.rseq >> 1));
+    if (R.rseq & 1u) mbar_arrive(empty_bar<T>(S, R.rseq >> 1));
     ++R.rseq;
 }
 
@@ -985,9 +1004,10 @@ __device__ __forceinline__ void release_plane(const TSmem &S, RingPos &R)
 // before, and s when s is odd), and every lane arrives on that pair's
 // "empty" barrier.  A pair is completed by exactly one release, single or
 // double, so each lane arrives once per pair.
+template <typename T>
 __device__ __forceinline__ void release_two_planes(const TSmem &S, RingPos &R)
 {
-    mbar_arrive(empty_bar(S, R.rseq >> 1));
+    mbar_arrive(empty_bar<T>(S, R.rseq >> 1));
     R.rseq += 2;
 }
 
@@ -1122,7 +1142,7 @@ template <typename T>
 __device__ __forceinline__ float layer_k(uint32_t seq0, int64_t Oz, int64_t z0, const Plan &P)
 {
     constexpr int ES = sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
-    const uint32_t slot = (seq0 + (uint32_t)(Oz - z0) - (uint32_t)P.a) & (uint32_t)(kRing - 1);
+    const uint32_t slot = (seq0 + (uint32_t)(Oz - z0) - (uint32_t)P.a) & (uint32_t)(kRing<T> - 1);
     return kMagic + (float)((int)slot * PLANE_B + P.DY * ROW_B + P.DX * ES);
 }
 
@@ -1139,16 +1159,23 @@ struct PairPrep {
     uint32_t a0, a1;     // shared-window addresses of the floor taps of voxel 0 / 1 in the ring
 };
 
-// ring: shared-window address of slot 0; k: layer_k of the cell layer.
-template <typename T>
-__device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px, float2 py, float2 pz)
+// ring: shared-window address of slot 0; k: layer_k of the cell layer; LAST
+// (RAGGED border walks) with the layer's frame.
+template <typename T, bool LAST>
+__device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px, float2 py, float2 pz, const Frame &fr)
 {
     constexpr float ES = (float)sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
-    constexpr uint32_t RING = kRing * kHMax * kBoxW * (uint32_t)sizeof(T), MASK = RING - (uint32_t)sizeof(T);
+    constexpr uint32_t RING = kRing<T> * kHMax * kBoxW * (uint32_t)sizeof(T), MASK = RING - (uint32_t)sizeof(T);
     static_assert((RING & (RING - 1)) == 0 && (kMagicBits & (RING - 1)) == 0, "the ring is a power of two of bytes");
     const float2 MM = f2(kMagic, kMagic);
     const float2 mx = __fadd2_rd(px, MM), my = __fadd2_rd(py, MM), mz = __fadd2_rd(pz, MM);
-    const float2 flx = sub2(mx, MM), fly = sub2(my, MM), flz = sub2(mz, MM);
+    float2 flx = sub2(mx, MM), fly = sub2(my, MM), flz = sub2(mz, MM);
+    if (LAST) {
+        const float tx = (float)fr.bh[0], ty = (float)fr.bh[1], tz = (float)fr.bh[2];
+        flx = f2(px.x == tx ? tx - 1.f : flx.x, px.y == tx ? tx - 1.f : flx.y);
+        fly = f2(py.x == ty ? ty - 1.f : fly.x, py.y == ty ? ty - 1.f : fly.y);
+        flz = f2(pz.x == tz ? tz - 1.f : flz.x, pz.y == tz ? tz - 1.f : flz.y);
+    }
     PairPrep q;
     q.nfx = sub2(flx, px);
     q.fy = sub2(py, fly);
@@ -1335,7 +1362,14 @@ __device__ __forceinline__ void pair_positions(const float2 (&w)[4], const float
 //    lo exactly, as the clamped floor sz - 2 with fraction 1 gives hi);
 //  - an invalid sample (NaN included: every comparison fails) is masked.
 // false if a wait gave up.
-template <typename T, int G, bool BORDER>
+//
+// RAGGED (a job resampled from a padded copy of its source): a sample exactly
+// on the source's last element along an axis takes the floor before it and
+// fraction 1, as the gathered path does (pair_clamped2), where other staged
+// walks take floor sz - 1 and fraction 0: b0 + 1 (b1 - b0) is not always b1 in
+// floating point.  (The tap before is staged: the window starts 1/64 below its
+// lowest sample.)  The output's rows may start at odd elements.
+template <typename T, int G, bool BORDER, bool RAGGED>
 __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSmem &S, float4 *Rw,
                           const float4 (&wx)[2], RingPos &R)
 {
@@ -1356,8 +1390,8 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
 #pragma unroll
     for (int k = 0; k < NR; ++k) rowv[k] = !BORDER || (int64_t)(y + k * kRowWarps) < J.out_o[1] + J.out_n[1] - w.Oy;
     const int xe = BORDER ? (int)min(J.out_o[0] + J.out_n[0] - w.Ox, (int64_t)kTBX) : kTBX;
-    const bool pair_ok =
-        !BORDER || ((((uintptr_t)J.dst) % (2 * sizeof(T))) == 0 && (J.dst_py % 2 == 0) && (J.dst_pz % 2 == 0));
+    const bool pair_ok = (!BORDER && !RAGGED) || ((((uintptr_t)J.dst) % (2 * sizeof(T))) == 0 && (J.dst_py % 2 == 0) &&
+                                                (J.dst_pz % 2 == 0));
     for (int64_t zf = w.z0; zf < w.z1;) {
         const int64_t ze = min(w.z1, (zf / G + 1) * G);
         const int64_t Oz = (zf / G) * G;
@@ -1380,7 +1414,7 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
             for (int k = 0; k < NR; ++k) {
                 float2 px, py, pz;
                 pair_positions(wz, PX[k], PY[k], PZ[k], px, py, pz);
-                q[k] = prep_pair<T>(S.sring, lk, px, py, pz);
+                q[k] = prep_pair<T, BORDER && RAGGED>(S.sring, lk, px, py, pz, fr);
                 if (BORDER) {
                     const bool ok0 = px.x >= fr.lo[0] && px.x <= fr.hi[0] && py.x >= fr.lo[1] && py.x <= fr.hi[1] &&
                                      pz.x >= fr.lo[2] && pz.x <= fr.hi[2];
@@ -1407,8 +1441,14 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
             for (int k = 0; k < NR; ++k) {
                 const uint32_t v = finish_pair<T>(q[k], lo[k], hi[k]);
                 if (!BORDER) {
-                    if (sizeof(T) == 2) *reinterpret_cast<uint32_t *>(dp + k * drow2) = v;
-                    else *reinterpret_cast<uint16_t *>(dp + k * drow2) = (uint16_t)v;
+                    T *d = dp + k * drow2;
+                    if (pair_ok) {
+                        if (sizeof(T) == 2) *reinterpret_cast<uint32_t *>(d) = v;
+                        else *reinterpret_cast<uint16_t *>(d) = (uint16_t)v;
+                    } else {
+                        d[0] = (T)v;
+                        d[1] = (T)(v >> (8 * sizeof(T)));
+                    }
                 } else if (rowv[k] && x < xe) {
                     store_packed<T>(dp + k * drow2, v & keep[k], pair_ok, xe - x);
                 }
@@ -1424,32 +1464,38 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
         int pz = zoff;
         if constexpr (!BORDER) {
             for (; pz + 1 < zend; pz += 2, need += 2) {
-                if (!wait_planes(S, R, need + 1)) return false;
+                if (!wait_planes<T>(S, R, need + 1)) return false;
                 plane(pz);
                 plane(pz + 1);
-                release_two_planes(S, R);
+                release_two_planes<T>(S, R);
             }
         }
         for (; pz < zend; ++pz, ++need) {
-            if (!wait_planes(S, R, need)) return false;
+            if (!wait_planes<T>(S, R, need)) return false;
             plane(pz);
-            release_plane(S, R);
+            release_plane<T>(S, R);
         }
         zf = ze;
     }
-    for (uint32_t i = 1; i < Wn; ++i) release_plane(S, R);  // the rest of the last window
+    for (uint32_t i = 1; i < Wn; ++i) release_plane<T>(S, R);  // the rest of the last window
     return true;
 }
 
-// One unit gathered from global memory (gather kernel): warp y computes
-// output row y of the unit at flattened index u.
+// One unit gathered from global memory (gather kernel), or part `part` of
+// `parts` of its planes: warp y computes output row y of the unit at flattened
+// index u.
 template <typename T, int G, int INTERP>
-__device__ void rows_gather(const RJob *__restrict__ jobs, int njobs, int64_t u, const float4 *W, float4 *Rw,
-                            const float4 (&wx)[2])
+__device__ void rows_gather(const RJob *__restrict__ jobs, int njobs, int64_t u, int part, int parts, const float4 *W,
+                            float4 *Rw, const float4 (&wx)[2])
 {
     const int y = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x = 2 * lane;
-    const Walk w = walk_of(jobs, njobs, u);
+    Walk w = walk_of(jobs, njobs, u);
+    if (parts > 1) {
+        const int64_t n = w.z1 - w.z0, z0 = w.z0;
+        w.z0 = z0 + n * part / parts;
+        w.z1 = z0 + n * (part + 1) / parts;
+    }
     const RJob &J = jobs[w.j];
     const int xe = (int)min(J.out_o[0] + J.out_n[0] - w.Ox, (int64_t)kTBX);
     if ((int64_t)y >= J.out_o[1] + J.out_n[1] - w.Oy) return;
@@ -1984,6 +2030,85 @@ __global__ void __launch_bounds__(kAStagedThreads, 1) k_affine_staged(const RJob
     }
 }
 
+// ------------------------------------------------------- ragged sources
+//
+// TMA describes a source whose base and pitches are multiples of 16 bytes.  A
+// trilinear TPS job with any other source is resampled from a copy with rows
+// padded to 16 bytes: one read and one write of the source at memory speed,
+// against a resample that stages its taps instead of gathering them (801 x 601
+// x 301 uint16: gathered 1076 us).  Copying into the staged planes directly,
+// each row shifted into place by four more warps, took 1016 us there: the
+// shifts and the unaligned loads hold the row warps back.
+
+// 16 bytes of the source at p, which need not be aligned: two aligned loads
+// and a funnel shift, or, where those would leave the buffer [lo, hi), its
+// elements one by one (zeros past it).
+struct Granule {
+    uint4 a, b;
+    int head;  // bytes of a before p
+};
+
+template <typename T>
+__device__ __forceinline__ Granule load_granule(const char *p, const char *lo, const char *hi)
+{
+    Granule g;
+    g.head = (int)(reinterpret_cast<uintptr_t>(p) & 15);
+    const char *q = p - g.head;
+    if (q >= lo && q + (g.head ? 32 : 16) <= hi) {
+        g.a = __ldg(reinterpret_cast<const uint4 *>(q));
+        g.b = g.head ? __ldg(reinterpret_cast<const uint4 *>(q) + 1) : make_uint4(0, 0, 0, 0);
+    } else {
+        uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int e = 0; e < 16; e += (int)sizeof(T))
+            if (p + e >= lo && p + e + (int)sizeof(T) <= hi)
+                w[e >> 2] |= (uint32_t)*reinterpret_cast<const T *>(p + e) << (8 * (e & 3));
+        g.a = make_uint4(w[0], w[1], w[2], w[3]);
+        g.b = make_uint4(0, 0, 0, 0);
+        g.head = 0;
+    }
+    return g;
+}
+
+__device__ __forceinline__ uint4 shifted(const Granule &g)
+{
+    const bool s2 = (g.head & 8) != 0, s1 = (g.head & 4) != 0;
+    const uint32_t t0 = s2 ? g.a.z : g.a.x, t1 = s2 ? g.a.w : g.a.y, t2 = s2 ? g.b.x : g.a.z, t3 = s2 ? g.b.y : g.a.w;
+    const uint32_t t4 = s2 ? g.b.z : g.b.x, t5 = s2 ? g.b.w : g.b.y;
+    const uint32_t u0 = s1 ? t1 : t0, u1 = s1 ? t2 : t1, u2 = s1 ? t3 : t2, u3 = s1 ? t4 : t3, u4 = s1 ? t5 : t4;
+    const int sh = 8 * (g.head & 3);
+    return make_uint4(__funnelshift_r(u0, u1, sh), __funnelshift_r(u1, u2, sh), __funnelshift_r(u2, u3, sh),
+                      __funnelshift_r(u3, u4, sh));
+}
+
+// Copies an nx x ny x nz volume of T (row / plane pitches spy / spz elements)
+// to rows of dpb bytes, a multiple of 16; a thread copies 16 bytes at a time.
+template <typename T>
+__global__ void __launch_bounds__(256) k_repitch(const T *__restrict__ src, int64_t nx, int64_t ny, int64_t nz, int64_t spy,
+                                                 int64_t spz, unsigned char *__restrict__ dst, int64_t dpb)
+{
+    constexpr int ES = (int)sizeof(T);
+    const char *lo = reinterpret_cast<const char *>(src);
+    const char *hi = lo + ((nz - 1) * spz + (ny - 1) * spy + nx) * ES;
+    const int64_t rows = ny * nz;
+    const int per_row = (int)(dpb / 16);
+    // a CTA takes four rows at a time, its threads their granules in order
+    for (int64_t r0 = (int64_t)blockIdx.x * 4; r0 < rows; r0 += (int64_t)gridDim.x * 4) {
+        const int nr = (int)min((int64_t)4, rows - r0);
+        const int64_t y0 = r0 % ny, z0 = r0 / ny;
+        for (int i = threadIdx.x; i < nr * per_row; i += 256) {
+            const int k = i / per_row, c = i - k * per_row;
+            int64_t y = y0 + k, z = z0;
+            while (y >= ny) {
+                y -= ny;
+                ++z;
+            }
+            const Granule g = load_granule<T>(lo + (z * spz + y * spy) * ES + 16 * c, lo, hi);
+            *reinterpret_cast<uint4 *>(dst + (r0 + k) * dpb + 16 * c) = shifted(g);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- kernels
 
 // Plans every unit (one warp each, 8 per CTA): plans[u], and the units that
@@ -2054,7 +2179,7 @@ __global__ void __launch_bounds__(1024) k_tps_lists(const Plan *__restrict__ pla
 
 // TPS units whose source footprint is staged by TMA (trilinear), with the
 // plans of k_tps_plan; units without a staged plan are left to k_tps_gather.
-template <typename T, int G, int MODE>
+template <typename T, int G, int MODE, bool RAGGED>
 __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__restrict__ jobs,
                                                                    const int *__restrict__ list,
                                                                    const Plan *__restrict__ plans, int *err)
@@ -2081,9 +2206,9 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__
         S.W2[2 * tid] = make_float4(w.x, w.x, w.y, w.y);
         S.W2[2 * tid + 1] = make_float4(w.z, w.z, w.w, w.w);
     }
-    if (tid < kPairs) {
-        mbar_init(full_bar(S, tid), 2);                       // one arrival per plane of the pair
-        mbar_init(empty_bar(S, tid), 32 * kRowWarps);         // every lane of every row warp
+    if (tid < kPairs<T>) {
+        mbar_init(full_bar<T>(S, tid), 2);                       // one arrival per plane of the pair
+        mbar_init(empty_bar<T>(S, tid), 32 * kRowWarps);         // every lane of every row warp
     }
     if (tid == 0) {
         abort_sh = 0;
@@ -2098,7 +2223,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__
                 *reinterpret_cast<volatile int *>(&abort_sh) = 1;  // the row warps see it in their waits
                 if (err) atomicOr(err, kKernErrTimeout);
             }
-            drain_copies(S, seq);
+            drain_copies<T>(S, seq);
         }
         return;
     }
@@ -2116,7 +2241,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__
         w.z0 = P.z0;
         w.z1 = P.z1;
         const RJob &J = jobs[w.j];
-        const bool ok = walk_rows<T, G, MODE == 1>(J, w, P, S, Rw, wx, R);
+        const bool ok = walk_rows<T, G, MODE == 1, RAGGED>(J, w, P, S, Rw, wx, R);
         if (!ok) {
             // the other warps see the flag in their waits and return
             *reinterpret_cast<volatile int *>(&abort_sh) = 1;
@@ -2137,14 +2262,20 @@ __global__ void __launch_bounds__(kTpsThreads, 1) k_tps_gather(const RJob *__res
     __shared__ float4 Rw[kTBY * Gm::NRW];
     const int tid = threadIdx.x;
     const int64_t n = fb ? fb[0] : total_units;
-    if (blockIdx.x >= n) return;  // most launches have no unit left over
+    if (blockIdx.x >= (fb ? n * kGatherParts : n)) return;  // most launches have no unit left over
     if (tid < G) W[tid] = bspline_w(tid, G);
     __syncthreads();
     const int x = 2 * (tid & 31);
     const float4 wx[2] = {W[x % G], W[(x + 1) % G]};
     float4 *rw = Rw + (tid >> 5) * Gm::NRW;
-    for (int64_t i = blockIdx.x; i < n; i += gridDim.x)
-        rows_gather<T, G, INTERP>(jobs, njobs, fb ? fb[1 + i] : i, W, rw, wx);
+    // a few leftover walks are cut along z, so that they do not run on as many
+    // CTAs alone (65 us for the leftovers of a 999 x 501 x 301 uint8 job, 26 us
+    // in parts)
+    const int parts = fb && n < 4 * (int64_t)gridDim.x ? kGatherParts : 1;
+    for (int64_t i = blockIdx.x; i < n * parts; i += gridDim.x) {
+        const int64_t k = i / parts;
+        rows_gather<T, G, INTERP>(jobs, njobs, fb ? fb[1 + k] : k, (int)(i % parts), parts, W, rw, wx);
+    }
 }
 
 template <typename T, int INTERP>
@@ -2164,17 +2295,18 @@ __global__ void __launch_bounds__(kThreads) k_resample_affine(const RJob *__rest
     }
 }
 
+// ragged: the jobs are resampled from padded copies (see walk_rows).
 // TPS launches: trilinear jobs run the planning kernel, the staged kernel
 // and the gather kernel over the planning kernel's fallback list (ws: the
 // list, 1 + total int64 with the count zeroed by the caller, then the plans
 // on a 16-byte boundary); nearest-neighbour jobs, or a launch without ws, run
 // the gather kernel over every unit.
 template <typename T, int G, int INTERP>
-cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_t st, int sms, int *err, void *ws)
+cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_t st, int sms, int *err, void *ws, bool ragged)
 {
-    using Gm = TGeom<T, G>;
     int64_t *fb = static_cast<int64_t *>(ws);
-    if (INTERP == 0 && fb) {
+    if constexpr (INTERP == 0) if (fb) {
+        using Gm = TGeom<T, G>;
         Plan *plans = reinterpret_cast<Plan *>(fb + ((1 + total + 1) & ~(int64_t)1));
         int64_t pgrid = (total + 7) / 8;
         if (pgrid > (int64_t)sms * 8) pgrid = (int64_t)sms * 8;
@@ -2187,16 +2319,13 @@ cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_
         k_tps_lists<<<1, 1024, 0, st>>>(plans, total, l0, l1);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        const auto k0 = k_tps_staged<T, G, 0>, k1 = k_tps_staged<T, G, 1>;
+        const auto k0 = ragged ? k_tps_staged<T, G, 0, true> : k_tps_staged<T, G, 0, false>;
+        const auto k1 = ragged ? k_tps_staged<T, G, 1, true> : k_tps_staged<T, G, 1, false>;
         for (int mode = 0; mode < 2; ++mode) {  // interior walks, then the others
             const auto k = mode == 0 ? k0 : k1;
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Gm::smem_bytes);
             if (e != cudaSuccess) return e;
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kStagedThreads, Gm::smem_bytes);
-            if (e != cudaSuccess) return e;
-            if (per_sm < 1) return cudaErrorInvalidConfiguration;
-            int64_t grid = (int64_t)sms * per_sm;
+            int64_t grid = sms;  // one CTA per SM: 17 warps of 96 registers
             if (grid > total) grid = total;
             if (grid < 1) grid = 1;
             k<<<(unsigned)grid, kStagedThreads, Gm::smem_bytes, st>>>(jobs, mode == 0 ? l0 : l1, plans, err);
@@ -2249,14 +2378,14 @@ cudaError_t launch_affine_t(const RJob *jobs, int njobs, int64_t total, cudaStre
 
 template <typename T, int INTERP>
 cudaError_t dispatch_g(const RJob *jobs, int njobs, int64_t total, int g, cudaStream_t st, int sms, int *err,
-                       void *fb)
+                       void *fb, bool ragged)
 {
     switch (g) {
-    case 4: return launch_tps_t<T, 4, INTERP>(jobs, njobs, total, st, sms, err, fb);
-    case 8: return launch_tps_t<T, 8, INTERP>(jobs, njobs, total, st, sms, err, fb);
-    case 16: return launch_tps_t<T, 16, INTERP>(jobs, njobs, total, st, sms, err, fb);
-    case 32: return launch_tps_t<T, 32, INTERP>(jobs, njobs, total, st, sms, err, fb);
-    case 64: return launch_tps_t<T, 64, INTERP>(jobs, njobs, total, st, sms, err, fb);
+    case 4: return launch_tps_t<T, 4, INTERP>(jobs, njobs, total, st, sms, err, fb, ragged);
+    case 8: return launch_tps_t<T, 8, INTERP>(jobs, njobs, total, st, sms, err, fb, ragged);
+    case 16: return launch_tps_t<T, 16, INTERP>(jobs, njobs, total, st, sms, err, fb, ragged);
+    case 32: return launch_tps_t<T, 32, INTERP>(jobs, njobs, total, st, sms, err, fb, ragged);
+    case 64: return launch_tps_t<T, 64, INTERP>(jobs, njobs, total, st, sms, err, fb, ragged);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -2268,6 +2397,20 @@ size_t tps_stage_ws_bytes(int64_t total_bricks)
     // fallback list, plans, the two staged-walk lists
     return sizeof(int64_t) * (size_t)((1 + total_bricks + 1) & ~(int64_t)1) + sizeof(Plan) * (size_t)total_bricks +
            sizeof(int) * (size_t)(2 * (1 + total_bricks));
+}
+
+cudaError_t launch_repitch(const RJob &j, void *dst, int64_t row_bytes, cudaStream_t st, int sm_count)
+{
+    const int64_t rows = j.src_n[1] * j.src_n[2];
+    const int64_t grid = std::min<int64_t>((rows + 3) / 4, (int64_t)sm_count * 8);
+    if (j.dtype == 1)
+        k_repitch<uint8_t><<<(unsigned)grid, 256, 0, st>>>(static_cast<const uint8_t *>(j.src), j.src_n[0], j.src_n[1], j.src_n[2],
+                                                           j.src_py, j.src_pz, static_cast<unsigned char *>(dst), row_bytes);
+    else
+        k_repitch<uint16_t><<<(unsigned)grid, 256, 0, st>>>(static_cast<const uint16_t *>(j.src), j.src_n[0], j.src_n[1],
+                                                            j.src_n[2], j.src_py, j.src_pz, static_cast<unsigned char *>(dst),
+                                                            row_bytes);
+    return cudaGetLastError();
 }
 
 bool g_supported(int g) { return g == 4 || g == 8 || g == 16 || g == 32 || g == 64; }
@@ -2292,7 +2435,7 @@ cudaError_t launch_affine_staged(const RJob *jobs_dev, int njobs, int64_t total_
 }
 
 cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_bricks, int dtype, int kind, int g,
-                            int interp, cudaStream_t st, int sm_count, int *err, void *stage_ws)
+                            int interp, cudaStream_t st, int sm_count, int *err, void *stage_ws, bool ragged)
 {
     if (total_bricks <= 0) return cudaSuccess;
     if (kind == 0) {
@@ -2302,10 +2445,10 @@ cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_brick
                       : launch_affine_t<uint16_t, 0>(jobs_dev, njobs, total_bricks, st, sm_count);
     }
     if (dtype == 1)
-        return interp ? dispatch_g<uint8_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr)
-                      : dispatch_g<uint8_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws);
-    return interp ? dispatch_g<uint16_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr)
-                  : dispatch_g<uint16_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws);
+        return interp ? dispatch_g<uint8_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr, false)
+                      : dispatch_g<uint8_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, ragged);
+    return interp ? dispatch_g<uint16_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr, false)
+                  : dispatch_g<uint16_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, ragged);
 }
 
 }  // namespace tw
