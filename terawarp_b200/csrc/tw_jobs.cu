@@ -136,22 +136,30 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
     if (njobs <= 0) return TW_OK;
     const bool staging = ctx->resample_staging.load() != 0;
     if (jobs[0].kind == 1) {
-        // trilinear TPS jobs: those whose source TMA can describe, those that
+        // TPS jobs: those whose source TMA can describe, trilinear ones that
         // are resampled from a padded copy, and the rest, which gather
-        if (!staging || jobs[0].interp != 0) return run_group(ctx, jobs, njobs, 0, st);
+        // (below 16 M voxels a nearest-neighbour launch gathers: one launch
+        // instead of five; 208 x 144 x 131 uint8, call: 81 us gathered, 91
+        // staged; 256 x 256 x 128: 97 and 104; 400 x 224 x 128: 116 and 114)
+        const bool nearest = jobs[0].interp != 0;
+        int64_t vox = 0;
+        for (int i = 0; i < njobs; ++i) vox += jobs[i].out_n[0] * jobs[i].out_n[1] * jobs[i].out_n[2];
+        if (!staging || (nearest && vox < (int64_t)16 << 20)) return run_group(ctx, jobs, njobs, 0, st);
         RJob *const end = jobs + njobs;
         RJob *const mid = std::stable_partition(jobs, end, [](RJob &j) { return encode_source_map(j); });
-        if (mid > jobs) TW_TRY(run_group(ctx, jobs, (int)(mid - jobs), 0, st));
-        StreamBlock copy{ctx, st};
-        RJob *const last = pad_sources(ctx, mid, end, copy, st);
-        if (last > mid) {
-            tw_status s = run_group(ctx, mid, (int)(last - mid), 0, st);
-            if (s == TW_ERR_OOM) {  // no room for the plans: gather, from the copies
-                for (RJob *j = mid; j < last; ++j) j->tma_ok = 0;
-                s = run_group(ctx, mid, (int)(last - mid), 0, st);
+        const auto run_tps = [&](RJob *b, RJob *e, bool gathers) -> tw_status {
+            if (e == b) return TW_OK;
+            tw_status s = run_group(ctx, b, (int)(e - b), 0, st);
+            if (s == TW_ERR_OOM && gathers) {  // no room for the plans: gathering needs none
+                for (RJob *j = b; j < e; ++j) j->tma_ok = 0;
+                s = run_group(ctx, b, (int)(e - b), 0, st);
             }
-            if (s != TW_OK) return s;
-        }
+            return s;
+        };
+        TW_TRY(run_tps(jobs, mid, nearest));
+        StreamBlock copy{ctx, st};
+        RJob *const last = jobs[0].interp == 0 ? pad_sources(ctx, mid, end, copy, st) : mid;
+        TW_TRY(run_tps(mid, last, true));
         if (end > last) TW_TRY(run_group(ctx, last, (int)(end - last), 0, st));
         return TW_OK;
     }
@@ -194,15 +202,16 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
     // balance, they get shorter, down to 16 planes -- below that the windows
     // and the per-layer set-up cost more than an even last wave gives (256 x 256
     // x 128 uint8: 109 us at 4 planes, 91 at 16; 512^3 uint16: 573 at 64, 513 at
-    // 16; 1024 x 1024 x 256 uint8, spacing 4: 2114 at 64, 2011 at 32)
+    // 16; 1024 x 1024 x 256 uint8, spacing 4: 2114 at 64, 2011 at 32).  Gathered
+    // units keep no window and need fewer to balance.
     int zs = jobs[0].kind == 1 ? std::max(64, jobs[0].g) : 8;
     count(zs);
-    while (jobs[0].kind == 1 && zs > 16 && total < 32 * (int64_t)ctx->sm_count) {
+    const bool staged = jobs[0].kind == 1 && jobs[0].tma_ok != 0, ragged = staged && jobs[0].ragged;
+    while (jobs[0].kind == 1 && zs > 16 && total < (staged ? 32 : 8) * (int64_t)ctx->sm_count) {
         zs /= 2;
         count(zs);
     }
     if (total == 0) return TW_OK;
-    const bool staged = jobs[0].kind == 1 && jobs[0].tma_ok != 0, ragged = staged && jobs[0].ragged;
     // the units' staging plans and the list of units left to the gather kernel
     StreamBlock fb{ctx, st};
     if (staged) {

@@ -574,7 +574,7 @@ __device__ __forceinline__ Clamp make_clamp(const RJob &J, const Frame &f, const
 // and each source plane comes from DRAM about once.  (Numbered z-fastest,
 // the walks in flight were a few columns at 16 depths and the y-neighbours'
 // halo rows were fetched again later: 3x the source bytes read from DRAM on
-// a 1024^3 u16 job.)  A walk whose box or window does not fit, a nearest-neighbour job,
+// a 1024^3 u16 job.)  A walk whose box or window does not fit
 // or a source buffer TMA cannot describe gathers from global memory instead
 // (the gather kernel), with the same positions and the same trilinear
 // arithmetic (trilerp2).
@@ -1161,13 +1161,22 @@ struct PairPrep {
 
 // ring: shared-window address of slot 0; k: layer_k of the cell layer; LAST
 // (RAGGED border walks) with the layer's frame.
-template <typename T, bool LAST>
+// NEAR: nearest neighbour, the only tap is the floor of q + 0.5 (which the
+// window holds: it is floor(q) or the element after) and the fractions are
+// not used.
+template <typename T, bool LAST, bool NEAR>
 __device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px, float2 py, float2 pz, const Frame &fr)
 {
     constexpr float ES = (float)sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
     constexpr uint32_t RING = kRing<T> * kHMax * kBoxW * (uint32_t)sizeof(T), MASK = RING - (uint32_t)sizeof(T);
     static_assert((RING & (RING - 1)) == 0 && (kMagicBits & (RING - 1)) == 0, "the ring is a power of two of bytes");
     const float2 MM = f2(kMagic, kMagic);
+    if (NEAR) {
+        const float2 half = f2(0.5f, 0.5f);
+        px = add2(px, half);
+        py = add2(py, half);
+        pz = add2(pz, half);
+    }
     const float2 mx = __fadd2_rd(px, MM), my = __fadd2_rd(py, MM), mz = __fadd2_rd(pz, MM);
     float2 flx = sub2(mx, MM), fly = sub2(my, MM), flz = sub2(mz, MM);
     if (LAST) {
@@ -1177,9 +1186,11 @@ __device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px,
         flz = f2(pz.x == tz ? tz - 1.f : flz.x, pz.y == tz ? tz - 1.f : flz.y);
     }
     PairPrep q;
-    q.nfx = sub2(flx, px);
-    q.fy = sub2(py, fly);
-    q.fz = sub2(pz, flz);
+    if (!NEAR) {
+        q.nfx = sub2(flx, px);
+        q.fy = sub2(py, fly);
+        q.fz = sub2(pz, flz);
+    }
     const float2 o = fma2(flz, f2(PLANE_B, PLANE_B), fma2(fly, f2(ROW_B, ROW_B), fma2(flx, f2(ES, ES), f2(k, k))));
     q.a0 = ring + (__float_as_uint(o.x) & MASK);
     q.a1 = ring + (__float_as_uint(o.y) & MASK);
@@ -1369,7 +1380,7 @@ __device__ __forceinline__ void pair_positions(const float2 (&w)[4], const float
 // walks take floor sz - 1 and fraction 0: b0 + 1 (b1 - b0) is not always b1 in
 // floating point.  (The tap before is staged: the window starts 1/64 below its
 // lowest sample.)  The output's rows may start at odd elements.
-template <typename T, int G, bool BORDER, bool RAGGED>
+template <typename T, int G, bool BORDER, bool RAGGED, bool NEAR>
 __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSmem &S, float4 *Rw,
                           const float4 (&wx)[2], RingPos &R)
 {
@@ -1414,7 +1425,7 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
             for (int k = 0; k < NR; ++k) {
                 float2 px, py, pz;
                 pair_positions(wz, PX[k], PY[k], PZ[k], px, py, pz);
-                q[k] = prep_pair<T, BORDER && RAGGED>(S.sring, lk, px, py, pz, fr);
+                q[k] = prep_pair<T, BORDER && RAGGED, NEAR>(S.sring, lk, px, py, pz, fr);
                 if (BORDER) {
                     const bool ok0 = px.x >= fr.lo[0] && px.x <= fr.hi[0] && py.x >= fr.lo[1] && py.x <= fr.hi[1] &&
                                      pz.x >= fr.lo[2] && pz.x <= fr.hi[2];
@@ -1433,13 +1444,18 @@ __device__ bool walk_rows(const RJob &J, const Walk &w, const Plan &P, const TSm
         auto plane = [&](int pz) {
             float2 lo[NR][4], hi[NR][4];
 #pragma unroll
-            for (int k = 0; k < NR; ++k) taps_pair<T>(q[k], lo[k], hi[k]);
+            for (int k = 0; k < NR; ++k) {
+                if constexpr (NEAR) lo[k][0] = f2(lds_raw<T, 0>(q[k].a0), lds_raw<T, 0>(q[k].a1));
+                else taps_pair<T>(q[k], lo[k], hi[k]);
+            }
             PairPrep nq[NR];
             uint32_t nkeep[NR];
             prep(min(pz + 1, G - 1), nq, nkeep);  // (the last plane's is not used)
 #pragma unroll
             for (int k = 0; k < NR; ++k) {
-                const uint32_t v = finish_pair<T>(q[k], lo[k], hi[k]);
+                uint32_t v;
+                if constexpr (NEAR) v = pack_pair<T>(__float_as_uint(lo[k][0].x), __float_as_uint(lo[k][0].y));
+                else v = finish_pair<T>(q[k], lo[k], hi[k]);
                 if (!BORDER) {
                     T *d = dp + k * drow2;
                     if (pair_ok) {
@@ -2177,9 +2193,9 @@ __global__ void __launch_bounds__(1024) k_tps_lists(const Plan *__restrict__ pla
     }
 }
 
-// TPS units whose source footprint is staged by TMA (trilinear), with the
+// TPS units whose source footprint is staged by TMA, with the
 // plans of k_tps_plan; units without a staged plan are left to k_tps_gather.
-template <typename T, int G, int MODE, bool RAGGED>
+template <typename T, int G, int MODE, bool RAGGED, bool NEAR>
 __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__restrict__ jobs,
                                                                    const int *__restrict__ list,
                                                                    const Plan *__restrict__ plans, int *err)
@@ -2241,7 +2257,7 @@ __global__ void __launch_bounds__(kStagedThreads, 1) k_tps_staged(const RJob *__
         w.z0 = P.z0;
         w.z1 = P.z1;
         const RJob &J = jobs[w.j];
-        const bool ok = walk_rows<T, G, MODE == 1, RAGGED>(J, w, P, S, Rw, wx, R);
+        const bool ok = walk_rows<T, G, MODE == 1, RAGGED, NEAR>(J, w, P, S, Rw, wx, R);
         if (!ok) {
             // the other warps see the flag in their waits and return
             *reinterpret_cast<volatile int *>(&abort_sh) = 1;
@@ -2296,16 +2312,19 @@ __global__ void __launch_bounds__(kThreads) k_resample_affine(const RJob *__rest
 }
 
 // ragged: the jobs are resampled from padded copies (see walk_rows).
-// TPS launches: trilinear jobs run the planning kernel, the staged kernel
+// TPS launches: jobs with ws run the planning kernel, the staged kernel
 // and the gather kernel over the planning kernel's fallback list (ws: the
 // list, 1 + total int64 with the count zeroed by the caller, then the plans
-// on a 16-byte boundary); nearest-neighbour jobs, or a launch without ws, run
-// the gather kernel over every unit.
+// on a 16-byte boundary); a launch without ws runs the gather kernel over
+// every unit.  Nearest-neighbour jobs take the staged kernels too: their one
+// tap per voxel then is a shared-memory load instead of a gathered one that
+// costs an L1 wavefront per line (512^3 uint8 labels, call: 726 us gathered,
+// 418 staged; 1024 x 512 x 300: 845 and 435).
 template <typename T, int G, int INTERP>
 cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_t st, int sms, int *err, void *ws, bool ragged)
 {
     int64_t *fb = static_cast<int64_t *>(ws);
-    if constexpr (INTERP == 0) if (fb) {
+    if (fb) {
         using Gm = TGeom<T, G>;
         Plan *plans = reinterpret_cast<Plan *>(fb + ((1 + total + 1) & ~(int64_t)1));
         int64_t pgrid = (total + 7) / 8;
@@ -2319,8 +2338,9 @@ cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_
         k_tps_lists<<<1, 1024, 0, st>>>(plans, total, l0, l1);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-        const auto k0 = ragged ? k_tps_staged<T, G, 0, true> : k_tps_staged<T, G, 0, false>;
-        const auto k1 = ragged ? k_tps_staged<T, G, 1, true> : k_tps_staged<T, G, 1, false>;
+        constexpr bool NEAR = INTERP == 1, RAG = INTERP == 0;  // (nearest-neighbour jobs are never ragged)
+        const auto k0 = ragged ? k_tps_staged<T, G, 0, RAG, NEAR> : k_tps_staged<T, G, 0, false, NEAR>;
+        const auto k1 = ragged ? k_tps_staged<T, G, 1, RAG, NEAR> : k_tps_staged<T, G, 1, false, NEAR>;
         for (int mode = 0; mode < 2; ++mode) {  // interior walks, then the others
             const auto k = mode == 0 ? k0 : k1;
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Gm::smem_bytes);
@@ -2339,7 +2359,7 @@ cudaError_t launch_tps_t(const RJob *jobs, int njobs, int64_t total, cudaStream_
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     int64_t grid = (int64_t)sms * per_sm;
-    const bool listed = INTERP == 0 && fb;
+    const bool listed = fb != nullptr;
     if (!listed && grid > total) grid = total;
     if (grid < 1) grid = 1;
     kg<<<(unsigned)grid, kTpsThreads, 0, st>>>(jobs, njobs, total, listed ? fb : nullptr);
@@ -2445,9 +2465,9 @@ cudaError_t launch_resample(const RJob *jobs_dev, int njobs, int64_t total_brick
                       : launch_affine_t<uint16_t, 0>(jobs_dev, njobs, total_bricks, st, sm_count);
     }
     if (dtype == 1)
-        return interp ? dispatch_g<uint8_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr, false)
+        return interp ? dispatch_g<uint8_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, false)
                       : dispatch_g<uint8_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, ragged);
-    return interp ? dispatch_g<uint16_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, nullptr, false)
+    return interp ? dispatch_g<uint16_t, 1>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, false)
                   : dispatch_g<uint16_t, 0>(jobs_dev, njobs, total_bricks, g, st, sm_count, err, stage_ws, ragged);
 }
 
