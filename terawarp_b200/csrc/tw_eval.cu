@@ -5,15 +5,19 @@
 // per thread (80 KB of local memory) and launches once per z plane; the CPU
 // loops are q_imgwarp_tps_quicksmallmemory.cpp:620-648 and :1117-1146.
 //
-// Here one launch covers the whole grid.  Landmarks (centres and negated
+// Here one launch covers the whole grid.  Landmarks (negated centres and
 // coefficients) are staged through shared memory in tiles and read as
-// warp-wide broadcasts; each thread evaluates kNPT nodes so every shared
-// load feeds kNPT node-landmark pairs.  Per pair: 3 FADD, 1 FMUL, 2 FFMA,
-// 1 sqrt, 3 FFMA, issued as Blackwell FP32x2 instructions over two nodes at a
-// time (the landmark is staged with each component duplicated, negated
-// centre), so a pair costs ~5.5 issue slots.  Sums are two-level: plain FP32
-// FMA chains over 32 landmarks, then Kahan-compensated accumulation of those
-// partials.
+// warp-wide broadcasts; a thread evaluates 2 or 4 nodes of one (x, y) column, so
+// dx^2 + dy^2 is computed once per landmark for all of them.  Per landmark and
+// two nodes what is left is one add, one multiply-add, two square roots and
+// three multiply-adds, the node pairs in FP32x2 instructions.  What bounds it:
+// the square roots, 16 per SM and clock (1.15 M nodes x 2000 landmarks: 0.51
+// ms of them; the call takes 648 us, 826 when each node had its own dx and dy
+// and the landmarks' components were staged twice over: a broadcast of 16
+// bytes to a warp takes 4 cycles of the shared memory's return path, and three
+// of them per landmark and four nodes were more than the square roots).  Sums
+// are two-level: plain FP32 FMA chains over 32 landmarks, then
+// Kahan-compensated accumulation of those partials.
 //
 // Coordinates are taken relative to an origin o near the landmarks so the
 // FP32 magnitudes stay small; the affine part is folded (in FP64, on the
@@ -28,7 +32,6 @@ namespace tw {
 namespace {
 
 constexpr int kEvalThreads = 256;
-constexpr int kNPT = 4;      // nodes per thread
 constexpr int kTile = 256;   // landmarks staged per shared-memory tile
 constexpr int kSub = 32;     // landmarks per plain FP32 partial sum
 
@@ -47,86 +50,103 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
     s = t;
 }
 
+// NPT: nodes per thread, consecutive in z.  SPLIT: groups of threads that
+// share the 32-landmark partial sums of the same nodes out among themselves,
+// turn by turn; the partials then meet in shared memory and are added in
+// landmark order, so the sums are the same whatever the split.
+template <int NPT, int SPLIT>
 __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
 {
-    // per landmark: (-cx, -cx, -cy, -cy), (-cz, -cz, wx, wx), (wy, wy, wz, wz)
-    __shared__ float4 s_lm[kTile][3];
-    const int64_t nnodes = p.gsz[0] * p.gsz[1] * p.gsz[2];
-    const int64_t base = (int64_t)blockIdx.x * (kEvalThreads * kNPT) + threadIdx.x;
-
-    float px[kNPT], py[kNPT], pz[kNPT];
-    float sx[kNPT], sy[kNPT], sz[kNPT], cx[kNPT], cy[kNPT], cz[kNPT];
+    constexpr int UNITS = kEvalThreads / SPLIT, P2 = NPT / 2;
+    static_assert(kTile / kSub == 8 && 8 % SPLIT == 0 && UNITS % 32 == 0, "whole warps, whole turns");
+    __shared__ float4 s_a[kTile];  // -cx, -cy, -cz, wx
+    __shared__ float2 s_b[kTile];  // wy, wz
+    __shared__ float s_part[SPLIT > 1 ? SPLIT : 1][3 * NPT][SPLIT > 1 ? UNITS : 1];
+    const int unit = threadIdx.x % UNITS, grp = threadIdx.x / UNITS;
+    const int64_t U = (int64_t)blockIdx.x * UNITS + unit;
+    // units: x fastest, then y, then runs of NPT planes (past the end: the
+    // last node again, not stored)
+    const int64_t ix = U % p.gsz[0], iy = U / p.gsz[0] % p.gsz[1], iz = U / (p.gsz[0] * p.gsz[1]) * NPT;
+    const float px = (float)(p.node_o[0] + ix * p.g), py = (float)(p.node_o[1] + iy * p.g);
+    float pz[NPT];
+    float s[3][NPT], c[3][NPT];
 #pragma unroll
-    for (int j = 0; j < kNPT; ++j) {
-        int64_t L = base + (int64_t)j * kEvalThreads;
-        if (L >= nnodes) L = nnodes - 1;  // duplicate work, store is skipped below
-        int64_t i = L % p.gsz[0];
-        int64_t t = L / p.gsz[0];
-        int64_t jj = t % p.gsz[1];
-        int64_t k = t / p.gsz[1];
-        px[j] = (float)(p.node_o[0] + i * p.g);
-        py[j] = (float)(p.node_o[1] + jj * p.g);
-        pz[j] = (float)(p.node_o[2] + k * p.g);
-        sx[j] = sy[j] = sz[j] = 0.f;
-        cx[j] = cy[j] = cz[j] = 0.f;
-    }
-
-    float2 px2[kNPT / 2], py2[kNPT / 2], pz2[kNPT / 2];
+    for (int j = 0; j < NPT; ++j) {
+        pz[j] = (float)(p.node_o[2] + (iz + j < p.gsz[2] ? iz + j : p.gsz[2] - 1) * p.g);
 #pragma unroll
-    for (int k = 0; k < kNPT / 2; ++k) {
-        px2[k] = make_float2(px[2 * k], px[2 * k + 1]);
-        py2[k] = make_float2(py[2 * k], py[2 * k + 1]);
-        pz2[k] = make_float2(pz[2 * k], pz[2 * k + 1]);
+        for (int q = 0; q < 3; ++q) s[q][j] = c[q][j] = 0.f;
     }
 
     for (int t0 = 0; t0 < p.n; t0 += kTile) {
         const int cnt = min(kTile, p.n - t0);
         __syncthreads();
         for (int l = threadIdx.x; l < kTile; l += kEvalThreads) {
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f), w = c;  // zero weight pads the tile
+            float4 e = make_float4(0.f, 0.f, 0.f, 0.f), w = e;  // zero weight pads the tile
             if (l < cnt) {
-                c = p.ctr[t0 + l];
+                e = p.ctr[t0 + l];
                 w = p.coef[t0 + l];
             }
-            s_lm[l][0] = make_float4(-c.x, -c.x, -c.y, -c.y);
-            s_lm[l][1] = make_float4(-c.z, -c.z, w.x, w.x);
-            s_lm[l][2] = make_float4(w.y, w.y, w.z, w.z);
+            s_a[l] = make_float4(-e.x, -e.y, -e.z, w.x);
+            s_b[l] = make_float2(w.y, w.z);
         }
         __syncthreads();
         const int nsub = (cnt + kSub - 1) / kSub;
-        for (int sb = 0; sb < nsub; ++sb) {
-            // node pairs (2k, 2k+1); the same operations, in the same order,
-            // as one FP32 instruction per node and landmark
-            float2 ax[kNPT / 2], ay[kNPT / 2], az[kNPT / 2];
+        for (int sb0 = 0; sb0 < nsub; sb0 += SPLIT) {
+            const int sb = sb0 + grp;
+            // two nodes per instruction: the same operations, in the same
+            // order, as one FP32 instruction per node and landmark
+            float2 a[3][P2];
 #pragma unroll
-            for (int k = 0; k < kNPT / 2; ++k) ax[k] = ay[k] = az[k] = make_float2(0.f, 0.f);
+            for (int k = 0; k < P2; ++k) a[0][k] = a[1][k] = a[2][k] = make_float2(0.f, 0.f);
+            if (SPLIT == 1 || sb < nsub) {
 #pragma unroll 4
-            for (int l = sb * kSub; l < sb * kSub + kSub; ++l) {
-                const float4 A = s_lm[l][0], B = s_lm[l][1], Cw = s_lm[l][2];
-                const float2 ncx = make_float2(A.x, A.y), ncy = make_float2(A.z, A.w);
-                const float2 ncz = make_float2(B.x, B.y), wx = make_float2(B.z, B.w);
-                const float2 wy = make_float2(Cw.x, Cw.y), wz = make_float2(Cw.z, Cw.w);
+                for (int l = sb * kSub; l < sb * kSub + kSub; ++l) {
+                    const float4 A = s_a[l];
+                    const float2 B = s_b[l];
+                    const float dx = __fadd_rn(px, A.x), dy = __fadd_rn(py, A.y);
+                    const float r0 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+                    const float2 r02 = make_float2(r0, r0), ncz = make_float2(A.z, A.z);
+                    const float2 wx = make_float2(A.w, A.w), wy = make_float2(B.x, B.x), wz = make_float2(B.y, B.y);
 #pragma unroll
-                for (int k = 0; k < kNPT / 2; ++k) {
-                    const float2 dx = __fadd2_rn(px2[k], ncx), dy = __fadd2_rn(py2[k], ncy);
-                    const float2 dz = __fadd2_rn(pz2[k], ncz);
-                    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-                    const float2 r = make_float2(fast_sqrt(r2.x), fast_sqrt(r2.y));
-                    ax[k] = __ffma2_rn(r, wx, ax[k]);
-                    ay[k] = __ffma2_rn(r, wy, ay[k]);
-                    az[k] = __ffma2_rn(r, wz, az[k]);
+                    for (int k = 0; k < P2; ++k) {
+                        const float2 dz = __fadd2_rn(make_float2(pz[2 * k], pz[2 * k + 1]), ncz);
+                        const float2 r2 = __ffma2_rn(dz, dz, r02);
+                        const float2 r = make_float2(fast_sqrt(r2.x), fast_sqrt(r2.y));
+                        a[0][k] = __ffma2_rn(r, wx, a[0][k]);
+                        a[1][k] = __ffma2_rn(r, wy, a[1][k]);
+                        a[2][k] = __ffma2_rn(r, wz, a[2][k]);
+                    }
                 }
             }
+            if constexpr (SPLIT == 1) {
 #pragma unroll
-            for (int j = 0; j < kNPT; ++j) {
-                const float axj = (j & 1) ? ax[j >> 1].y : ax[j >> 1].x;
-                const float ayj = (j & 1) ? ay[j >> 1].y : ay[j >> 1].x;
-                const float azj = (j & 1) ? az[j >> 1].y : az[j >> 1].x;
-                kahan_add(sx[j], cx[j], axj);
-                kahan_add(sy[j], cy[j], ayj);
-                kahan_add(sz[j], cz[j], azj);
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int j = 0; j < NPT; ++j) kahan_add(s[q][j], c[q][j], (j & 1) ? a[q][j >> 1].y : a[q][j >> 1].x);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int j = 0; j < NPT; ++j) s_part[grp][q * NPT + j][unit] = (j & 1) ? a[q][j >> 1].y : a[q][j >> 1].x;
+                __syncthreads();
+                // sum e of a unit belongs to group e % SPLIT
+                const int have = min(SPLIT, nsub - sb0);
+#pragma unroll
+                for (int e = 0; e < 3 * NPT; e += SPLIT)
+                    if (e + grp < 3 * NPT)
+                        for (int k = 0; k < have; ++k)
+                            kahan_add(s[0][e / SPLIT], c[0][e / SPLIT], s_part[k][e + grp][unit]);
+                __syncthreads();
             }
         }
+    }
+    if constexpr (SPLIT > 1) {  // the sums, less their compensation, to group 0
+        static_assert(3 * NPT <= SPLIT * NPT, "a group's sums fit in s[0]");
+#pragma unroll
+        for (int e = 0; e < 3 * NPT; e += SPLIT)
+            if (e + grp < 3 * NPT) s_part[0][e + grp][unit] = s[0][e / SPLIT] - c[0][e / SPLIT];
+        __syncthreads();
+        if (grp != 0) return;
     }
 
     // affine part: f_c(q) = d[0][c] + sum_r q_r d[r+1][c]; with q = o + p:
@@ -143,32 +163,49 @@ __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
         for (int r = 0; r < 3; ++r) alin[r][c] = (float)__dsub_rn(__ldg(&p.aff[(r + 1) * 4 + c + 1]), r == c ? 1.0 : 0.0);
     }
 #pragma unroll
-    for (int j = 0; j < kNPT; ++j) {
-        const int64_t L = base + (int64_t)j * kEvalThreads;
-        if (L >= nnodes) continue;
-        float dfx = a0[0] + alin[0][0] * px[j] + alin[1][0] * py[j] + alin[2][0] * pz[j];
-        float dfy = a0[1] + alin[0][1] * px[j] + alin[1][1] * py[j] + alin[2][1] * pz[j];
-        float dfz = a0[2] + alin[0][2] * px[j] + alin[1][2] * py[j] + alin[2][2] * pz[j];
+    for (int j = 0; j < NPT; ++j) {
+        if (iz + j >= p.gsz[2]) break;
+        float dfx = a0[0] + alin[0][0] * px + alin[1][0] * py + alin[2][0] * pz[j];
+        float dfy = a0[1] + alin[0][1] * px + alin[1][1] * py + alin[2][1] * pz[j];
+        float dfz = a0[2] + alin[0][2] * px + alin[1][2] * py + alin[2][2] * pz[j];
         // the running compensation holds minus the lost low-order part
-        dfx += sx[j] - cx[j];
-        dfy += sy[j] - cy[j];
-        dfz += sz[j] - cz[j];
-        p.out[L] = make_float4(dfx, dfy, dfz, 0.f);
+        if constexpr (SPLIT > 1) {
+            dfx += s_part[0][j][unit];
+            dfy += s_part[0][NPT + j][unit];
+            dfz += s_part[0][2 * NPT + j][unit];
+        } else {
+            dfx += s[0][j] - c[0][j];
+            dfy += s[1][j] - c[1][j];
+            dfz += s[2][j] - c[2][j];
+        }
+        p.out[((iz + j) * p.gsz[1] + iy) * p.gsz[0] + ix] = make_float4(dfx, dfy, dfz, 0.f);
     }
+}
+
+template <int NPT, int SPLIT>
+cudaError_t launch_eval(const EvalParams &p, cudaStream_t st)
+{
+    const int64_t units = p.gsz[0] * p.gsz[1] * ((p.gsz[2] + NPT - 1) / NPT);
+    const int64_t per = kEvalThreads / SPLIT, grid = (units + per - 1) / per;
+    if (grid > 0x7fffffff) return cudaErrorInvalidValue;
+    k_tps_eval<NPT, SPLIT><<<(unsigned)grid, kEvalThreads, 0, st>>>(p);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_tps_eval(const EvalParams &p, cudaStream_t st, int sm_count)
 {
-    (void)sm_count;
     const int64_t nnodes = p.gsz[0] * p.gsz[1] * p.gsz[2];
     if (nnodes <= 0) return cudaSuccess;
-    const int64_t per_block = (int64_t)kEvalThreads * kNPT;
-    const int64_t grid = (nnodes + per_block - 1) / per_block;
-    if (grid > 0x7fffffff) return cudaErrorInvalidValue;
-    k_tps_eval<<<(unsigned)grid, kEvalThreads, 0, st>>>(p);
-    return cudaGetLastError();
+    // A grid that fills the chip runs one thread per four nodes.  Smaller ones
+    // share the landmarks of 32-node units out over a block's eight warps, if
+    // there are enough of them (calls with 2000 landmarks: 847 nodes 129 us
+    // unsplit, 49 split, 23,000 129 and 58 with two nodes a thread, 61 with
+    // four; 157,000 201, 150 and 134; 1.15 M 649, 793 and 677).
+    if (nnodes >= (int64_t)sm_count * 2048) return launch_eval<4, 1>(p, st);
+    if (nnodes >= (int64_t)sm_count * 256) return p.n > 128 ? launch_eval<4, 8>(p, st) : launch_eval<4, 1>(p, st);
+    return launch_eval<2, 8>(p, st);
 }
 
 }  // namespace tw
