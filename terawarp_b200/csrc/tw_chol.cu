@@ -2,13 +2,13 @@
 // of the projected TPS system, one cooperative kernel.
 //
 // A (m x m, symmetric positive definite) is held as 64 x 64 tiles of its lower
-// triangle, each stored with a row pitch of 66 doubles: a tile is one
-// contiguous 33,792-byte block that a single bulk copy moves between global
+// triangle, each stored with a row pitch of 68 doubles: a tile is one
+// contiguous 34,816-byte block that a single bulk copy moves between global
 // and shared memory, already in the layout whose 16-byte row loads are free of
 // bank conflicts.  Column 64 of a factored diagonal tile holds the reciprocals
 // of its diagonal and its upper triangle the transpose of the lower, so the
 // panel solves read both along rows.  The four right-hand sides are an extra
-// row block of 4 x 66 tiles, so the forward substitution is part of the
+// row block of 4 x 68 tiles, so the forward substitution is part of the
 // factorisation; the back substitution overwrites the same tiles.
 //
 // Roles.  CTA 0 runs the critical chain POTRF(k-1) -> TRSM(k, k-1) ->
@@ -45,7 +45,7 @@ namespace tw {
 namespace {
 
 constexpr int kNB = 64;                        // tile
-constexpr int kTP = 66;                        // tile row pitch, doubles
+constexpr int kTP = 68;                        // tile row pitch, doubles
 constexpr int kTileD = kNB * kTP;              // doubles of a tile
 constexpr uint32_t kTileB = kTileD * 8;        // bytes
 constexpr int kRhsD = 4 * kTP;                 // a right-hand-side tile
@@ -54,12 +54,13 @@ constexpr int kCompute = 256;                  // compute threads
 constexpr int kThreads = kCompute + 64;        // + the fetching warp + the publishing warp
 constexpr int kFetchWarp = kCompute / 32, kPublishWarp = kFetchWarp + 1;
 constexpr int kBufs = 6;                       // tile buffers in shared memory
+constexpr int kPotBars = 23;                   // barriers inside a diagonal tile's factorisation
 
 // status word bits
 constexpr int kStNotSPD = 2;
 constexpr int kStTimeout = 4;
 
-static_assert(kTileB % 16 == 0 && kRhsB % 16 == 0, "bulk copies move multiples of 16 bytes");
+static_assert(kTP - kNB == 4 && kTileB % 16 == 0 && kRhsB % 16 == 0, "bulk copies move multiples of 16 bytes");
 
 // Flags (zeroed before the launch).  tdone[i]: panel tiles of row block i that
 // are final (row block nblk: the right-hand sides); pre_d[j], pre_s[j]: tile
@@ -74,7 +75,7 @@ struct Flags {
 
 struct Ctl {
     double *tiles;  // lower-triangle tiles, column after column
-    double *rhs;    // nblk tiles of 4 x 66
+    double *rhs;    // nblk tiles of 4 x 68
     double *x;      // the solution, 4 per row (rows 0 .. m-1)
     int m, nblk;
     int *status;
@@ -101,6 +102,7 @@ struct Smem {
     unsigned long long zfull[4];
     unsigned long long post[2], freed[2];  // results handed to the publishing warp / their buffers read
     unsigned long long xdone;
+    unsigned long long pot[kPotBars];
     // a result to publish: shared source, global destination, bytes, flag and its value
     struct Mail {
         const double *src;
@@ -114,6 +116,8 @@ struct Smem {
     int abort;
 };
 
+static_assert(sizeof(Smem) <= 232448, "one CTA per SM");
+
 // ------------------------------------------------------------ small helpers
 
 __device__ __forceinline__ unsigned long long now_ns()
@@ -122,6 +126,11 @@ __device__ __forceinline__ unsigned long long now_ns()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// The warp's index through a shuffle, so that the compiler knows it to be the
+// same in all lanes: below a branch on threadIdx.x / 32 it guards every shuffle
+// and matrix instruction against lanes that went the other way, and the 16
+// pivots of factor16 take 3280 cycles instead of 2350.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ int ld_acquire(const int *p)
@@ -143,6 +152,13 @@ __device__ __forceinline__ void bar_init(unsigned long long *b, uint32_t n)
 __device__ __forceinline__ void bar_arrive(unsigned long long *b)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
+}
+// Arrival of lane 0, without a branch.
+__device__ __forceinline__ void bar_arrive_lane0(unsigned long long *b)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(saddr(b)),
+                 "r"(threadIdx.x & 31)
+                 : "memory");
 }
 __device__ __forceinline__ void bar_expect(unsigned long long *b, uint32_t bytes)
 {
@@ -229,7 +245,7 @@ __device__ __forceinline__ void post(Smem &S, int b, const double *src, double *
     fence_async();
     if (threadIdx.x == 0) S.mail[b] = {src, dst, bytes, flag, value};
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) bar_arrive(&S.post[b]);
+    bar_arrive_lane0(&S.post[b]);
 }
 
 // The publishing warp's lane 0: stores the n-th result of mailbox b and
@@ -258,38 +274,146 @@ __device__ bool publish(const Ctl &C, Smem &S, int b, uint32_t n)
 
 // ------------------------------------------------------------- tile kernels
 //
-// Compute thread t owns the elements (tr + 16u, tc + 16v) of a tile, tr = t / 16,
-// tc = t % 16: two rows of a warp's operand loads are broadcast, the other
-// operand's 16 rows are conflict-free 16-byte loads.
+// Tile products run on the FP64 matrix instruction (m8n8k4): each element is
+// the same chain of fused multiply-adds, in ascending order of k, that scalar
+// code would run, so its bits do not depend on which of the two computes it.
+// A compute warp owns eight rows of a tile, row block wr, as eight 8 x 8
+// fragments: lane (lr, lc) = (lane / 4, lane % 4) holds the columns
+// 8 f + 2 lc + {0, 1} of row 8 wr + lr.  The rows of a tile are 68 doubles
+// apart, so the 8 x 4 operand fragments (row lr, column lc) are free of bank
+// conflicts, and per four k's a warp loads nine of them for eight products:
+// 144 of the 256 cycles that the products take.
 
-// acc[u][v] = sum over the 64 columns, in order, of Li(tr + 16u, .) Lj(tc + 16v, .);
-// DIAG: only v <= u.
-template <bool DIAG>
-__device__ __forceinline__ void tile_product(const double *__restrict__ Li, const double *__restrict__ Lj, double (&acc)[4][4])
+using Frags = double[8][2];
+
+// row block of a compute warp; the two warps of a sub-partition (w, w + 4)
+// have nine lower fragments together
+__device__ __forceinline__ int row_block()
 {
-    const int tr = threadIdx.x >> 4, tc = threadIdx.x & 15;
+    const int w = warp_index();
+    return w < 4 ? w : 11 - w;
+}
+// element (row lr, column 2 lc) of row block wr of the tile T
+__device__ __forceinline__ int frag_at(int wr)
+{
+    const int lane = threadIdx.x & 31;
+    return (8 * wr + (lane >> 2)) * kTP + 2 * (lane & 3);
+}
+__device__ __forceinline__ void load_frags(const double *T, int wr, Frags &a)
+{
+    const double *p = T + frag_at(wr);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int f = 0; f < 8; ++f) {
+        const double2 v = *reinterpret_cast<const double2 *>(p + 8 * f);
+        a[f][0] = v.x;
+        a[f][1] = v.y;
+    }
+}
+__device__ __forceinline__ void store_frags(double *T, int wr, const Frags &a)
+{
+    double *p = T + frag_at(wr);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
+    for (int f = 0; f < 8; ++f) *reinterpret_cast<double2 *>(p + 8 * f) = make_double2(a[f][0], a[f][1]);
+}
+// c += A B' for an 8 x 4 A and B fragment
+__device__ __forceinline__ void mma4(double (&c)[2], double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// acc = Li Lj', summed over the 64 columns in order; DIAG: only the lower
+// fragments (f <= wr), the others 0.
+template <bool DIAG>
+__device__ __forceinline__ void tile_product(const double *__restrict__ Li, const double *__restrict__ Lj, int wr, Frags &acc)
+{
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+#pragma unroll
+    for (int f = 0; f < 8; ++f) acc[f][0] = acc[f][1] = 0.0;
+    const double *A = Li + (8 * wr + lr) * kTP + lc, *B = Lj + lr * kTP + lc;
 #pragma unroll 4
-    for (int p = 0; p < kNB; p += 2) {
-        double2 a[4], b[4];
+    for (int p = 0; p < kNB; p += 4) {
+        const double x = A[p];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            a[u] = *reinterpret_cast<const double2 *>(Li + (tr + 16 * u) * kTP + p);
-            b[u] = *reinterpret_cast<const double2 *>(Lj + (tc + 16 * u) * kTP + p);
+        for (int f = 0; f < 8; ++f)
+            if (!DIAG || f <= wr) mma4(acc[f], x, B[8 * f * kTP + p]);
+    }
+}
+
+// Four columns (half h of the fragment `own`, c0 .. c0 + 3 of the tile) of
+// X = A L^-T for the eight rows of a fragment row: a row's four lanes gather
+// its four values, and all solve them against the 4 x 4 block D on L's diagonal
+// (transposed above it; r: the reciprocal pivots).  Returns lane (lr, lc)'s
+// operand element x(row lr, column c0 + lc).
+__device__ __forceinline__ void gather4(const double (&own)[2], int h, double (&w)[4])
+{
+    const unsigned full = 0xffffffffu;
+    const int from = (threadIdx.x & 28) + 2 * h;
+    w[0] = __shfl_sync(full, own[0], from);
+    w[1] = __shfl_sync(full, own[1], from);
+    w[2] = __shfl_sync(full, own[0], from + 1);
+    w[3] = __shfl_sync(full, own[1], from + 1);
+}
+__device__ __forceinline__ double solve4(double (&own)[2], int h, const double (&w)[4], const double *__restrict__ D,
+                                         const double (&r)[4])
+{
+    const int lc = threadIdx.x & 3;
+    double w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
+    w0 = w0 * r[0];
+    w1 = fma(-w0, D[1], w1);
+    w2 = fma(-w0, D[2], w2);
+    w3 = fma(-w0, D[3], w3);
+    w1 = w1 * r[1];
+    w2 = fma(-w1, D[kTP + 2], w2);
+    w3 = fma(-w1, D[kTP + 3], w3);
+    w2 = w2 * r[2];
+    w3 = fma(-w2, D[2 * kTP + 3], w3);
+    w3 = w3 * r[3];
+    const bool odd = (lc & 1) != 0, mine = (lc >> 1) == h;
+    const double lo = odd ? w2 : w0, hi = odd ? w3 : w1;
+    own[0] = mine ? lo : own[0];
+    own[1] = mine ? hi : own[1];
+    return lc == 0 ? w0 : lc == 1 ? w1 : lc == 2 ? w2 : w3;
+}
+// Subtracts solved columns (x: operand elements) from the other half of their
+// own fragment; b: L's element (row lr of the fragment, column c0 + lc).
+__device__ __forceinline__ void other_half(double (&own)[2], int h, double x, double b)
+{
+    const bool mine = ((int)(threadIdx.x & 3) >> 1) == h;
+    double t[2] = {own[0], own[1]};
+    mma4(t, -x, b);
+    own[0] = mine ? own[0] : t[0];
+    own[1] = mine ? own[1] : t[1];
+}
+
+// X = A L^-T for the tile held in fragments, L a factored diagonal tile in
+// shared memory; each warp solves its own rows, so nothing is waited for.  In
+// groups of four columns, each subtracted from the later ones as soon as it is
+// solved: x(c) l(., c) in ascending order of c for every element.  The next
+// group's columns come first; the others' products are issued after the next
+// group's values have been gathered, so that they run under its solution
+// instead of before it.
+__device__ __forceinline__ void tile_solve(Frags &a, const double *__restrict__ L)
+{
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    double x = 0.0;
+#pragma unroll
+    for (int g = 0; g < 16; ++g) {
+        const int f = g >> 1, h = g & 1, c0 = 4 * g;
+        const double *R = L + c0 * kTP + kNB;
+        const double r[4] = {R[0], R[kTP], R[2 * kTP], R[3 * kTP]};
+        double w[4];
+        gather4(a[f], h, w);
+        if (g > 0) {  // the previous group's other fragments
+#pragma unroll
+            for (int k = f + 1; k < 8; ++k) mma4(a[k], -x, L[(8 * k + lr) * kTP + c0 - 4 + lc]);
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                if (!DIAG || v <= u) acc[u][v] = fma(a[u].x, b[v].x, acc[u][v]);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v)
-                if (!DIAG || v <= u) acc[u][v] = fma(a[u].y, b[v].y, acc[u][v]);
+        x = solve4(a[f], h, w, L + c0 * kTP + c0, r);
+        if (g == 15) break;
+        const double *B = L + lr * kTP + c0 + lc;
+        if (h == 0) other_half(a[f], h, x, B[8 * f * kTP]);
+        else mma4(a[f + 1], -x, B[8 * (f + 1) * kTP]);
     }
 }
 
@@ -328,54 +452,6 @@ __device__ __forceinline__ void solve_row16(double *x, const double *D, const do
     for (int k = 0; k < 16; k += 2) *reinterpret_cast<double2 *>(x + k) = make_double2(v[k], v[k + 1]);
 }
 
-// X = X L^-T for the tile held in registers (a), L a factored diagonal tile;
-// the result goes to Xs.  With SYRK also acc = X X' (lower part), summed over
-// the columns in order.  In four 16-column panels: the panel is solved row by
-// row, then subtracted from the later columns.
-template <bool SYRK>
-__device__ __forceinline__ void tile_solve(double (&a)[4][4], const double *__restrict__ L, double *__restrict__ Xs,
-                                           double (&acc)[4][4])
-{
-    const int t = threadIdx.x, tr = t >> 4, tc = t & 15;
-    if (SYRK) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
-    }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        const int c0 = 16 * v;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) Xs[(tr + 16 * u) * kTP + c0 + tc] = a[u][v];
-        sync_compute();
-        if (t < kNB) solve_row16(Xs + t * kTP + c0, L + c0 * kTP + c0, L + c0 * kTP + kNB);
-        sync_compute();
-        if (v < 3 || SYRK) {
-#pragma unroll 4
-            for (int p = c0; p < c0 + 16; p += 2) {
-                double2 x[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) x[u] = *reinterpret_cast<const double2 *>(Xs + (tr + 16 * u) * kTP + p);
-#pragma unroll
-                for (int w = v + 1; w < 4; ++w) {
-                    const double2 l = *reinterpret_cast<const double2 *>(L + (tc + 16 * w) * kTP + p);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) a[u][w] = fma(-x[u].y, l.y, fma(-x[u].x, l.x, a[u][w]));
-                }
-                if (SYRK) {
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const double2 y = *reinterpret_cast<const double2 *>(Xs + (tc + 16 * w) * kTP + p);
-#pragma unroll
-                        for (int u = w; u < 4; ++u) acc[u][w] = fma(x[u].y, y.y, fma(x[u].x, y.x, acc[u][w]));
-                    }
-                }
-            }
-        }
-    }
-}
-
 // Column J onwards of the Cholesky of a 16 x 16 block held by the lanes of
 // one warp, lane l (l = lane % 16) owning row l (v[k] = element (l, k)); d is
 // column J's pivot, in every lane.  The next pivot's own update needs no
@@ -383,9 +459,11 @@ __device__ __forceinline__ void tile_solve(double (&a)[4][4], const double *__re
 // two products and one shuffle; the other columns' shuffles overlap it.  No
 // branches (they cost 235 of 343 cycles a column): every lane updates its whole
 // row, and what lands above the diagonal is never read; `bad` collects pivots
-// that are not positive (each replaced by 1).
+// that are not positive (each replaced by 1).  Each column is stored as it is
+// found (B: the block in shared memory; its transpose above the diagonal), and
+// every four columns are announced on cols[J / 4] (if any).
 template <int J>
-__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, bool &bad)
+__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, bool &bad, double *B, unsigned long long *cols)
 {
     if constexpr (J < 16) {
         const unsigned full = 0xffffffffu;
@@ -397,101 +475,181 @@ __device__ __forceinline__ void factor16(double (&v)[16], double d, int l, bool 
         v[J] = l == J ? piv : col;
         double dn = 1.0;
         if constexpr (J + 1 < 16) dn = __shfl_sync(full, fma(-col, col, v[J + 1]), J + 1);  // lane J + 1: its pivot
+        if (l >= J) {
+            B[J * kTP + l] = v[J];
+            B[l * kTP + J] = v[J];
+        }
+        if constexpr ((J & 3) == 3) {
+            __syncwarp();
+            if (cols) bar_arrive_lane0(cols + J / 4);
+        }
 #pragma unroll
         for (int k = J + 1; k < 16; ++k) {
             const double lkj = __shfl_sync(full, col, k);  // L(k, J), from row k's lane
             v[k] = fma(-v[J], lkj, v[k]);
         }
-        factor16<J + 1>(v, dn, l, bad);
+        factor16<J + 1>(v, dn, l, bad, B, cols);
     }
 }
 
-// Cholesky of the diagonal tile W (shared memory, lower triangle in; out: the
-// factor, its transpose above, the reciprocals in column 64).  Four 16-column
-// panels: warp 0 factors the panel's diagonal block while the other warps
-// finish the previous panel's trailing update; then one thread per row solves
-// the rows below, and all warps update the next diagonal block.
-__device__ void tile_potrf(double *__restrict__ W, int *status)
+// barriers of tile_potrf, each completed once per tile: four columns of panel
+// P factored; rows 16 g .. of panel P solved (P < 2); block (i, j) has all its
+// products subtracted
+__device__ __forceinline__ int pot_cols(int P) { return 4 * P; }
+__device__ __forceinline__ int pot_rows(int P, int g) { return 12 + 3 * P + g - 1; }
+__device__ __forceinline__ int pot_block(int i, int j) { return i == 2 ? 16 + 2 * j : 17 + 2 * j - (j == 3); }
+
+// block (i, j) -= its rows' and columns' parts of panel P (one warp)
+__device__ __forceinline__ void block_update(double *__restrict__ W, int i, int j, int P)
 {
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-#pragma unroll 1
-    for (int c0 = 0; c0 < kNB; c0 += 16) {
-        if (warp == 0) {
-            const int l = lane & 15;
-            double *row = W + (c0 + l) * kTP + c0;
-            double v[16];
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    double acc[2][2][2] = {};
+    const double *A = W + (16 * i + lr) * kTP + 16 * P + lc, *B = W + (16 * j + lr) * kTP + 16 * P + lc;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = k <= l ? row[k] : 0.0;
-            __syncwarp();
-            bool bad = false;
-            factor16<0>(v, __shfl_sync(0xffffffffu, v[0], 0), l, bad);
-            if (bad && lane == 0) atomicOr(status, kStNotSPD);
-            double dl = 1.0;
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                if (k == l) dl = v[k];
-            if (lane < 16) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k)
-                    if (k <= l) {
-                        row[k] = v[k];
-                        W[(c0 + k) * kTP + c0 + l] = v[k];
-                    }
-                row[kNB - c0] = 1.0 / dl;
-            }
-        } else if (c0 > 0) {
-            // trailing update by panel c0 - 16 of the 16 x 16 blocks (bi, bj),
-            // c0 / 16 <= bj <= bi < 4, but for the diagonal block at c0 (done):
-            // half a block per warp and turn, four columns of one row per lane
-            const int b0 = c0 >> 4, nb = 4 - b0, units = nb * (nb + 1) - 2;
-            for (int e = warp - 1; e < units; e += kCompute / 32 - 1) {
-                int f = (e >> 1) + 1, bj = b0;  // f: block in column order
-                while (f >= 4 - bj) {
-                    f -= 4 - bj;
-                    ++bj;
-                }
-                const int bi = bj + f;
-                const int i = 16 * bi + (lane & 15), j0 = 16 * bj + 8 * (e & 1) + 4 * (lane >> 4);
-                const double *ri = W + i * kTP + c0 - 16;
-                double s[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-                for (int p = 0; p < 16; p += 2) {
-                    const double2 x = *reinterpret_cast<const double2 *>(ri + p);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const double2 y = *reinterpret_cast<const double2 *>(W + (j0 + k) * kTP + c0 - 16 + p);
-                        s[k] = fma(x.y, y.y, fma(x.x, y.x, s[k]));
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (j0 + k <= i) W[i * kTP + j0 + k] -= s[k];
-            }
-        }
-        sync_compute();
-        if (c0 + 16 >= kNB) break;
-        if (t < kNB - 16 - c0) {
-            double *x = W + (c0 + 16 + t) * kTP + c0;
-            solve_row16(x, W + c0 * kTP + c0, W + c0 * kTP + kNB);
-        }
-        sync_compute();
-        {
-            // the next diagonal block, one element per thread
-            const int r = t >> 4, c = t & 15, c1 = c0 + 16;
-            if (c <= r) {
-                const double *ri = W + (c1 + r) * kTP + c0, *rj = W + (c1 + c) * kTP + c0;
-                double s = 0.0;
-#pragma unroll
-                for (int p = 0; p < 16; p += 2) {
-                    const double2 x = *reinterpret_cast<const double2 *>(ri + p), y = *reinterpret_cast<const double2 *>(rj + p);
-                    s = fma(x.y, y.y, fma(x.x, y.x, s));
-                }
-                W[(c1 + r) * kTP + c1 + c] -= s;
-            }
-        }
-        sync_compute();
+    for (int p = 0; p < 16; p += 4) {
+        const double a0 = A[p], a1 = A[8 * kTP + p], b0 = B[p], b1 = B[8 * kTP + p];
+        mma4(acc[0][0], a0, b0);
+        mma4(acc[0][1], a0, b1);
+        mma4(acc[1][0], a1, b0);
+        mma4(acc[1][1], a1, b1);
     }
-    // the transpose of the panels below the diagonal blocks is not read
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            double2 *c = reinterpret_cast<double2 *>(W + (16 * i + 8 * a + lr) * kTP + 16 * j + 8 * b + 2 * lc);
+            double2 v = *c;
+            v.x -= acc[a][b][0];
+            v.y -= acc[a][b][1];
+            *c = v;
+        }
+}
+
+// Cholesky of the diagonal tile W (shared memory, lower triangle in; out: the
+// factor, the transposes of its 16 x 16 diagonal blocks above them, the
+// reciprocals in column 64), n tiles having been factored before.  Four panels
+// of 16 columns.  Warp g < 4 owns the rows 16 g ..: it solves them against
+// panel P < g while warp P is still factoring that panel, four columns behind,
+// sums its own diagonal block's part of the last panel (P = g - 1) on the way,
+// and so goes on to factor its own panel a few hundred cycles after the one
+// before: the chain is 64 pivots and little else.  The products for the other
+// blocks are warps 4 .. 7's.  A panel's product is summed over its 16 columns
+// first, then subtracted.  (Panel after panel with barriers of all warps
+// between factoring, solving and updating: 20,800 cycles.)
+__device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__restrict__ W, uint32_t n)
+{
+    const unsigned full = 0xffffffffu;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const auto wait = [&](int b) {
+        bar_wait(C, S, &S.pot[b], n);
+        __syncwarp();
+    };
+    const auto done = [&](int b) {
+        __syncwarp();
+        bar_arrive_lane0(&S.pot[b]);
+    };
+    if (warp < 4) {
+        const int g = warp, l = lane & 15, lr = lane >> 2, lc = lane & 3;
+        double s[3][2] = {};  // fragments (0, 0), (1, 0), (1, 1) of the diagonal block's part of the last panel
+        double *const mine = W + (16 * g + lr) * kTP + 2 * lc;  // row lr, column 2 lc of the warp's rows
+#pragma unroll 1
+        for (int P = 0; P < g; ++P) {
+            if (P > 0) wait(pot_block(g, P));
+            double v[2][2][2];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const double2 x = *reinterpret_cast<const double2 *>(mine + 8 * (e >> 1) * kTP + 16 * P + 8 * (e & 1));
+                v[e >> 1][e & 1][0] = x.x;
+                v[e >> 1][e & 1][1] = x.y;
+            }
+            const double *D = W + 16 * P * kTP + 16 * P;  // panel P's diagonal block, its transpose above
+            const bool last = P == g - 1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int f = q >> 1, h = q & 1, c0 = 4 * q;
+                wait(pot_cols(P) + q);
+                const double rl = 1.0 / D[(c0 + lc) * kTP + c0 + lc];
+                double r[4], x[2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r[k] = __shfl_sync(full, rl, k);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    double w[4];
+                    gather4(v[e][f], h, w);
+                    x[e] = solve4(v[e][f], h, w, D + c0 * kTP + c0, r);
+                }
+                const double *B = D + lr * kTP + c0 + lc;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (h == 0) other_half(v[e][f], h, x[e], B[8 * f * kTP]);
+                    if (f == 0) mma4(v[e][1], -x[e], B[8 * kTP]);
+                }
+                if (last) {  // (a product's second operand is held as its first)
+                    mma4(s[0], x[0], x[0]);
+                    mma4(s[1], x[1], x[0]);
+                    mma4(s[2], x[1], x[1]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                *reinterpret_cast<double2 *>(mine + 8 * (e >> 1) * kTP + 16 * P + 8 * (e & 1)) =
+                    make_double2(v[e >> 1][e & 1][0], v[e >> 1][e & 1][1]);
+            if (P < 2) done(pot_rows(P, g));
+        }
+        if (g >= 2) wait(pot_block(g, g));
+        if (g > 0) {
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                double2 *c = reinterpret_cast<double2 *>(mine + (e > 0 ? 8 * kTP : 0) + 16 * g + (e > 1 ? 8 : 0));
+                double2 x = *c;
+                x.x -= s[e][0];
+                x.y -= s[e][1];
+                *c = x;
+            }
+            __syncwarp();
+        }
+        double v[16];
+        double *row = W + (16 * g + l) * kTP;
+#pragma unroll
+        for (int k = 0; k < 16; k += 2) {
+            const double2 x = *reinterpret_cast<const double2 *>(row + 16 * g + k);
+            v[k] = x.x;
+            v[k + 1] = x.y;
+        }
+        __syncwarp();
+        bool bad = false;
+        factor16<0>(v, __shfl_sync(full, v[0], 0), l, bad, W + 16 * g * kTP + 16 * g,
+                    g < 3 ? &S.pot[pot_cols(g)] : nullptr);
+        if (bad && lane == 0) atomicOr(C.status, kStNotSPD);
+        if (lane < 16) row[kNB] = 1.0 / row[16 * g + l];
+    } else if (warp == 4) {
+        wait(pot_rows(0, 1));
+        wait(pot_rows(0, 2));
+        block_update(W, 2, 1, 0);
+        done(pot_block(2, 1));
+        wait(pot_rows(0, 3));
+        block_update(W, 3, 2, 0);
+        wait(pot_rows(1, 2));
+        wait(pot_rows(1, 3));
+        block_update(W, 3, 2, 1);
+        done(pot_block(3, 2));
+    } else if (warp == 5) {
+        wait(pot_rows(0, 1));
+        wait(pot_rows(0, 3));
+        block_update(W, 3, 1, 0);
+        done(pot_block(3, 1));
+    } else if (warp == 6) {
+        wait(pot_rows(0, 2));
+        block_update(W, 2, 2, 0);
+        done(pot_block(2, 2));
+    } else {
+        wait(pot_rows(0, 3));
+        block_update(W, 3, 3, 0);
+        wait(pot_rows(1, 3));
+        block_update(W, 3, 3, 1);
+        done(pot_block(3, 3));
+    }
+    sync_compute();
 }
 
 // ------------------------------------------------------------------ chain
@@ -615,47 +773,43 @@ __device__ __forceinline__ void back_product(const double *__restrict__ L, const
     }
 }
 
-__device__ void chain_compute(const Ctl &C, Smem &S)
+__device__ __forceinline__ void chain_compute(const Ctl &C, Smem &S)
 {
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31, tr = t >> 4, tc = t & 15;
+    const int t = threadIdx.x, warp = warp_index(), lane = t & 31, wr = row_block();
     const int nblk = C.nblk;
     double *W = S.buf[kBufW], *Xs = S.buf[kBufOut];
-    {
-        const double *src = tile_ptr(C, 0, 0);
-        for (int e = t; e < kTileD / 2; e += kCompute)
-            reinterpret_cast<double2 *>(W)[e] = reinterpret_cast<const double2 *>(src)[e];
+    for (int k = 0; k < nblk; ++k) {
+        if (k == 0) {
+            const double *src = tile_ptr(C, 0, 0);
+            for (int e = t; e < kTileD / 2; e += kCompute)
+                reinterpret_cast<double2 *>(W)[e] = reinterpret_cast<const double2 *>(src)[e];
+        } else {
+            const uint32_t n = (uint32_t)(k - 1);
+            Frags a, acc;
+            bar_wait(C, S, &S.full[kBufX], n);
+            load_frags(S.buf[kBufX], wr, a);
+            __syncwarp();
+            bar_arrive_lane0(&S.empty[kBufX]);
+            tile_solve(a, W);
+            bar_wait_free(C, S, &S.freed[0], n);  // the previous panel tile has been stored
+            store_frags(Xs, wr, a);
+            sync_compute();  // (and every warp has read W)
+            post(S, 0, Xs, tile_ptr(C, k, k - 1), kTileB, &C.tdone[k], k);
+            tile_product<true>(Xs, Xs, wr, acc);
+            bar_wait(C, S, &S.full[kBufD], n);
+            load_frags(S.buf[kBufD], wr, a);
+            __syncwarp();
+            bar_arrive_lane0(&S.empty[kBufD]);
+#pragma unroll
+            for (int f = 0; f < 8; ++f) {
+                a[f][0] -= acc[f][0];
+                a[f][1] -= acc[f][1];
+            }
+            bar_wait(C, S, &S.freed[1], n);  // the previous diagonal tile has been stored
+            store_frags(W, wr, a);           // (what is above the diagonal is not read)
+        }
         sync_compute();
-        tile_potrf(W, C.status);
-        post(S, 1, W, tile_ptr(C, 0, 0), kTileB, &C.F->pdone, 1);
-    }
-    for (int k = 1; k < nblk; ++k) {
-        const uint32_t n = (uint32_t)(k - 1);
-        double a[4][4], ad[4][4], acc[4][4];
-        bar_wait(C, S, &S.full[kBufX], n);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) a[u][v] = S.buf[kBufX][(tr + 16 * u) * kTP + tc + 16 * v];
-        __syncwarp();
-        if (lane == 0) bar_arrive(&S.empty[kBufX]);
-        bar_wait_free(C, S, &S.freed[0], n);  // the previous panel tile has been stored
-        tile_solve<true>(a, W, Xs, acc);
-        post(S, 0, Xs, tile_ptr(C, k, k - 1), kTileB, &C.tdone[k], k);
-        bar_wait(C, S, &S.full[kBufD], n);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v <= u; ++v) ad[u][v] = S.buf[kBufD][(tr + 16 * u) * kTP + tc + 16 * v] - acc[u][v];
-        __syncwarp();
-        if (lane == 0) bar_arrive(&S.empty[kBufD]);
-        bar_wait(C, S, &S.freed[1], n);  // the previous diagonal tile has been stored
-        sync_compute();                  // and every warp has read it
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v <= u; ++v) W[(tr + 16 * u) * kTP + tc + 16 * v] = ad[u][v];
-        sync_compute();
-        tile_potrf(W, C.status);
+        tile_potrf(C, S, W, (uint32_t)k);
         post(S, 1, W, tile_ptr(C, k, k), kTileB, &C.F->pdone, k + 1);
     }
     // back substitution: the fetching warp may overwrite every buffer once
@@ -702,7 +856,7 @@ __device__ void chain_compute(const Ctl &C, Smem &S)
                 }
             }
             __syncwarp();
-            if (lane == 0) bar_arrive(&S.empty[b]);
+            bar_arrive_lane0(&S.empty[b]);
         }
         if (head) {
             S.xs[kb & 3][c * kTP + lane] = b0;
@@ -803,9 +957,9 @@ __device__ void helper_fetch(const Ctl &C, Smem &S, const Task &T, uint32_t &sta
     }
 }
 
-__device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &stage, uint32_t &diags, uint32_t &posts)
+__device__ __forceinline__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &stage, uint32_t &diags, uint32_t &posts)
 {
-    const int t = threadIdx.x, lane = t & 31, tr = t >> 4, tc = t & 15;
+    const int t = threadIdx.x, lane = t & 31, wr = row_block();
     const int nblk = C.nblk;
     double *Xs = S.buf[kBufOut];
     if (T.kind == 1) {
@@ -813,37 +967,31 @@ __device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &s
         const int kn = diag ? T.j - 1 : T.j;
         if (kn <= 0 && T.i <= T.j + 1) return;  // the chain reads the tile as it is
         double *A = tile_ptr(C, T.i, T.j);
-        double a[4][4], acc[4][4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-            for (int v = 0; v < 4; ++v) a[u][v] = A[(tr + 16 * u) * kTP + tc + 16 * v];
+        Frags a, acc;
+        load_frags(A, wr, a);
         for (int k = 0; k < kn; ++k, ++stage) {
             const int b = 2 * (int)(stage & 1u);
             bar_wait(C, S, &S.full[b], stage >> 1);
-            if (diag) tile_product<true>(S.buf[b], S.buf[b], acc);
-            else tile_product<false>(S.buf[b + 1], S.buf[b], acc);
+            if (diag) tile_product<true>(S.buf[b], S.buf[b], wr, acc);
+            else tile_product<false>(S.buf[b + 1], S.buf[b], wr, acc);
             __syncwarp();
-            if (lane == 0) bar_arrive(&S.empty[b]);
+            bar_arrive_lane0(&S.empty[b]);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) a[u][v] -= acc[u][v];
+            for (int f = 0; f < 8; ++f) {
+                a[f][0] -= acc[f][0];
+                a[f][1] -= acc[f][1];
+            }
+        }
+        const bool solved = T.i > T.j + 1;
+        if (solved) {
+            bar_wait(C, S, &S.full[kBufL], diags++);
+            tile_solve(a, S.buf[kBufL]);
+            __syncwarp();
+            bar_arrive_lane0(&S.empty[kBufL]);
         }
         bar_wait_free(C, S, &S.freed[0], posts);
-        if (T.i <= T.j + 1) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Xs[(tr + 16 * u) * kTP + tc + 16 * v] = a[u][v];
-            post(S, 0, Xs, A, kTileB, diag ? &C.pre_d[T.j] : &C.pre_s[T.j], 1);
-        } else {
-            bar_wait(C, S, &S.full[kBufL], diags++);
-            tile_solve<false>(a, S.buf[kBufL], Xs, acc);
-            __syncwarp();
-            if (lane == 0) bar_arrive(&S.empty[kBufL]);
-            post(S, 0, Xs, A, kTileB, &C.tdone[T.i], T.j + 1);
-        }
+        store_frags(Xs, wr, a);
+        post(S, 0, Xs, A, kTileB, solved ? &C.tdone[T.i] : diag ? &C.pre_d[T.j] : &C.pre_s[T.j], solved ? T.j + 1 : 1);
         ++posts;
         return;
     }
@@ -863,7 +1011,7 @@ __device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &s
                 s = fma(x.y, y.y, fma(x.x, y.x, s));
             }
             __syncwarp();
-            if (lane == 0) bar_arrive(&S.empty[b]);
+            bar_arrive_lane0(&S.empty[b]);
             a -= s;
         }
         bar_wait_free(C, S, &S.freed[0], posts);
@@ -882,9 +1030,9 @@ __device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &s
                     a = fma(-x.y, l.y, fma(-x.x, l.x, a));
                 }
         }
-        if (t < 8) Xs[(t >> 1) * kTP + kNB + (t & 1)] = 0.0;  // the pitch's spare columns
+        if (t < 16) Xs[(t >> 2) * kTP + kNB + (t & 3)] = 0.0;  // the pitch's spare columns
         __syncwarp();
-        if (lane == 0) bar_arrive(&S.empty[kBufL]);
+        bar_arrive_lane0(&S.empty[kBufL]);
         post(S, 0, Xs, A, kRhsB, &C.tdone[nblk], T.j + 1);
         ++posts;
         return;
@@ -911,12 +1059,12 @@ __device__ void helper_compute(const Ctl &C, Smem &S, const Task &T, uint32_t &s
             s = fma(L[(p + 1) * kTP], xp.y, s);
         }
         __syncwarp();
-        if (lane == 0) bar_arrive(&S.empty[b]);
+        bar_arrive_lane0(&S.empty[b]);
         a -= s;
     }
     bar_wait_free(C, S, &S.freed[0], posts);
     Xs[r * kTP + c] = a;
-    if (t < 8) Xs[(t >> 1) * kTP + kNB + (t & 1)] = 0.0;
+    if (t < 16) Xs[(t >> 2) * kTP + kNB + (t & 3)] = 0.0;
     post(S, 0, Xs, A, kRhsB, &C.bcnt[T.i], 1);
     ++posts;
 }
@@ -930,11 +1078,11 @@ __device__ void drain(unsigned long long *b, uint32_t n)
         if (now_ns() - t0 > 2000000000ull) return;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_chol_solve(Ctl C)
+__global__ void __launch_bounds__(kThreads, 1) k_chol_solve(const __grid_constant__ Ctl C)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Smem &S = *reinterpret_cast<Smem *>(smem_raw);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int b = 0; b < kBufs; ++b) {
             bar_init(&S.full[b], 1);
@@ -950,6 +1098,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_chol_solve(Ctl C)
             bar_init(&S.freed[b], 1);
         }
         bar_init(&S.xdone, 1);
+        for (int b = 0; b < kPotBars; ++b) bar_init(&S.pot[b], 1);
         S.abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
