@@ -91,12 +91,12 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
 // padded to 16 bytes (one block, `copy`), moves these jobs to the front and
 // returns their end.  A small launch gathers in the same or less time (517 x
 // 389 x 203 uint16: 367 us gathered, 370 copied and staged; 801 x 601 x 301:
-// 1091 and 850), and the copies are held to 512 MiB, which the context's pool
+// 1091 and 850), and the copies are held to 256 MiB, which the context's pool
 // then keeps, and to what the budget has left.
 RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaStream_t st)
 {
     constexpr int64_t kMinVoxels = 48 << 20;
-    constexpr size_t kMostBytes = (size_t)512 << 20;
+    constexpr size_t kMostBytes = (size_t)256 << 20;
     int64_t vox = 0;
     size_t bytes = 0;
     const auto row_bytes = [](const RJob &j) { return (size_t)((j.src_n[0] * (j.dtype == TW_U8 ? 1 : 2) + 15) / 16 * 16); };
