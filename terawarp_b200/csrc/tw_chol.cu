@@ -26,9 +26,13 @@
 // copies into a ring of shared-memory buffers, after the flag that publishes
 // each tile) and one warp stores results and publishes them, so neither a
 // flag's round trip nor a store's completion stands on the compute warps'
-// path.  What bounds it: the chain's latency up to about 3000 landmarks (per
-// 64 columns 16 dependent pivots x 4: reciprocal square root, multiply,
-// multiply-add, shuffle), the FP64 pipe beyond.
+// path.  What bounds it: the chain's latency up to about 3000 landmarks -- per
+// 64 columns some 35,000 cycles: 22,000 in the diagonal tile (64 dependent
+// pivots: reciprocal square root, multiply, multiply-add, shuffle), 7,000 in
+// the panel tile's solution, 4,500 in its product -- and the helpers' FP64
+// matrix instructions beyond (64 multiply-adds per SM and clock).  Kernel at
+// 4096 landmarks: 1.92 ms with scalar multiply-adds for the products and
+// solutions, 1.63 ms with the matrix instruction.
 //
 // Every element sees the operations of the plain right-looking tiled
 // factorisation in the same order, whatever the schedule.
@@ -127,9 +131,9 @@ __device__ __forceinline__ unsigned long long now_ns()
     return t;
 }
 // The warp's index through a shuffle, so that the compiler knows it to be the
-// same in all lanes: below a branch on threadIdx.x / 32 it guards every shuffle
-// and matrix instruction against lanes that went the other way, and the 16
-// pivots of factor16 take 3280 cycles instead of 2350.
+// same in all lanes: below a branch on threadIdx.x / 32 it guards shuffles and
+// matrix instructions against lanes that went the other way (factor16 in a
+// kernel of its own: 3,280 cycles instead of 2,350).
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -534,8 +538,10 @@ __device__ __forceinline__ void block_update(double *__restrict__ W, int i, int 
 // and so goes on to factor its own panel a few hundred cycles after the one
 // before: the chain is 64 pivots and little else.  The products for the other
 // blocks are warps 4 .. 7's.  A panel's product is summed over its 16 columns
-// first, then subtracted.  (Panel after panel with barriers of all warps
-// between factoring, solving and updating: 20,800 cycles.)
+// first, then subtracted.  (21,900 cycles: four times 3,700 in factor16, three
+// times 1,400 from one panel's last column to the next panel's first; 22,900
+// panel after panel, with barriers of all warps between factoring, solving and
+// updating.)
 __device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__restrict__ W, uint32_t n)
 {
     const unsigned full = 0xffffffffu;

@@ -20,7 +20,9 @@
 // by TMA, plane by plane, so that the eight taps of every voxel are
 // shared-memory loads (see "TPS units" below).
 //
-// Affine bricks are 256 x 8 x 8 output voxels gathered from global memory.
+// Affine tiles are 32 x 16 x 16 output voxels whose source box is staged in
+// shared memory; jobs whose box does not fit, and nearest-neighbour ones, run
+// as bricks of 256 x 8 x 8 output voxels gathered from global memory.
 //
 // Sampling follows the reference exactly: a sample with any q_i < 0 or
 // q_i > sz_i - 1 writes 0; weights come from floor(q); TPS rounds with +0.5

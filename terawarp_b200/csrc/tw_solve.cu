@@ -20,12 +20,11 @@
 //      product P0 = K V over the implicit K_ij = -|s_i - s_j|.
 //   3. A = (Q' K Q)(4:,4:) + lambda I is symmetric positive definite (-|r| is
 //      conditionally positive definite of order 1 in 3-D and q2 is orthogonal
-//      to the polynomials), so it is factored by a blocked right-looking
-//      Cholesky: diagonal block in shared memory, panel TRSM, trailing SYRK
-//      in 64 x 64 FP64 tiles.
+//      to the polynomials), so it is factored by a blocked Cholesky in
+//      64 x 64 FP64 tiles (tw_chol.cu).
 //   4. z = Q' Y; w = A^-1 z(4:): the forward substitution rides along in the
 //      factorisation (z(4:)' is an extra row block of the panel solves and
-//      trailing updates), the back substitution is one CTA;
+//      trailing updates), the back substitution follows in the same kernel;
 //      c = Q [0; w]; d = R^-1 (Q' (Y - K c))(0:4).
 //
 // Affine (reference: q_affine_compute_affinmatrix_3D,
