@@ -137,6 +137,16 @@ __device__ __forceinline__ unsigned long long now_ns()
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// c ? a : b as one selection.  Written as a
+// conditional expression it becomes a branch (one side's arithmetic sinks
+// into them), and in the chains below a branch costs more than the arithmetic:
+// solve4 210 cycles with, 86 without.
+__device__ __forceinline__ double sel(int c, double a, double b)
+{
+    double r;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\tselp.f64 %0, %1, %2, p;\n\t}" : "=d"(r) : "d"(a), "d"(b), "r"(c));
+    return r;
+}
 __device__ __forceinline__ int ld_acquire(const int *p)
 {
     int v;
@@ -345,11 +355,24 @@ __device__ __forceinline__ void tile_product(const double *__restrict__ Li, cons
     }
 }
 
-// Four columns (half h of the fragment `own`, c0 .. c0 + 3 of the tile) of
-// X = A L^-T for the eight rows of a fragment row: a row's four lanes gather
-// its four values, and all solve them against the 4 x 4 block D on L's diagonal
-// (transposed above it; r: the reciprocal pivots).  Returns lane (lr, lc)'s
-// operand element x(row lr, column c0 + lc).
+// What a group of four columns c0 .. c0 + 3 is solved with: the reciprocal
+// pivots and the block below the diagonal (its transpose lies above it).
+struct Group {
+    double r[4], l10, l20, l30, l21, l31, l32;
+};
+__device__ __forceinline__ void load_group(Group &G, const double *__restrict__ D)
+{
+    G.l10 = D[1];
+    const double2 t = *reinterpret_cast<const double2 *>(D + 2), u = *reinterpret_cast<const double2 *>(D + kTP + 2);
+    G.l20 = t.x;
+    G.l30 = t.y;
+    G.l21 = u.x;
+    G.l31 = u.y;
+    G.l32 = D[2 * kTP + 3];
+}
+// Four columns (half h of the fragment `own`) of X = A L^-T for the eight rows
+// of a fragment row: a row's four lanes gather its four values, and all solve
+// them.  Returns lane (lr, lc)'s operand element x(row lr, column c0 + lc).
 __device__ __forceinline__ void gather4(const double (&own)[2], int h, double (&w)[4])
 {
     const unsigned full = 0xffffffffu;
@@ -359,36 +382,30 @@ __device__ __forceinline__ void gather4(const double (&own)[2], int h, double (&
     w[2] = __shfl_sync(full, own[0], from + 1);
     w[3] = __shfl_sync(full, own[1], from + 1);
 }
-__device__ __forceinline__ double solve4(double (&own)[2], int h, const double (&w)[4], const double *__restrict__ D,
-                                         const double (&r)[4])
+__device__ __forceinline__ double solve4(double (&own)[2], int h, const double (&w)[4], const Group &G)
 {
-    const int lc = threadIdx.x & 3;
-    double w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
-    w0 = w0 * r[0];
-    w1 = fma(-w0, D[1], w1);
-    w2 = fma(-w0, D[2], w2);
-    w3 = fma(-w0, D[3], w3);
-    w1 = w1 * r[1];
-    w2 = fma(-w1, D[kTP + 2], w2);
-    w3 = fma(-w1, D[kTP + 3], w3);
-    w2 = w2 * r[2];
-    w3 = fma(-w2, D[2 * kTP + 3], w3);
-    w3 = w3 * r[3];
-    const bool odd = (lc & 1) != 0, mine = (lc >> 1) == h;
-    const double lo = odd ? w2 : w0, hi = odd ? w3 : w1;
-    own[0] = mine ? lo : own[0];
-    own[1] = mine ? hi : own[1];
-    return lc == 0 ? w0 : lc == 1 ? w1 : lc == 2 ? w2 : w3;
+    const int odd = threadIdx.x & 1, high = threadIdx.x & 2, mine = (high >> 1) == h;
+    const double w0 = w[0] * G.r[0];
+    double w1 = fma(-w0, G.l10, w[1]), w2 = fma(-w0, G.l20, w[2]), w3 = fma(-w0, G.l30, w[3]);
+    w1 = w1 * G.r[1];
+    w2 = fma(-w1, G.l21, w2);
+    w3 = fma(-w1, G.l31, w3);
+    w2 = w2 * G.r[2];
+    w3 = fma(-w2, G.l32, w3);
+    w3 = w3 * G.r[3];
+    own[0] = sel(mine, sel(odd, w2, w0), own[0]);
+    own[1] = sel(mine, sel(odd, w3, w1), own[1]);
+    return sel(high, sel(odd, w3, w2), sel(odd, w1, w0));
 }
 // Subtracts solved columns (x: operand elements) from the other half of their
 // own fragment; b: L's element (row lr of the fragment, column c0 + lc).
 __device__ __forceinline__ void other_half(double (&own)[2], int h, double x, double b)
 {
-    const bool mine = ((int)(threadIdx.x & 3) >> 1) == h;
+    const int mine = ((int)(threadIdx.x & 3) >> 1) == h;
     double t[2] = {own[0], own[1]};
     mma4(t, -x, b);
-    own[0] = mine ? own[0] : t[0];
-    own[1] = mine ? own[1] : t[1];
+    own[0] = sel(mine, own[0], t[0]);
+    own[1] = sel(mine, own[1], t[1]);
 }
 
 // X = A L^-T for the tile held in fragments, L a factored diagonal tile in
@@ -401,19 +418,26 @@ __device__ __forceinline__ void other_half(double (&own)[2], int h, double x, do
 __device__ __forceinline__ void tile_solve(Frags &a, const double *__restrict__ L)
 {
     const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    const auto load = [&](Group &G, int c0) {
+        const double *R = L + c0 * kTP + kNB;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) G.r[k] = R[k * kTP];
+        load_group(G, L + c0 * kTP + c0);
+    };
+    Group G[2];
+    load(G[0], 0);
     double x = 0.0;
 #pragma unroll
     for (int g = 0; g < 16; ++g) {
         const int f = g >> 1, h = g & 1, c0 = 4 * g;
-        const double *R = L + c0 * kTP + kNB;
-        const double r[4] = {R[0], R[kTP], R[2 * kTP], R[3 * kTP]};
         double w[4];
         gather4(a[f], h, w);
+        if (g < 15) load(G[(g + 1) & 1], c0 + 4);
         if (g > 0) {  // the previous group's other fragments
 #pragma unroll
             for (int k = f + 1; k < 8; ++k) mma4(a[k], -x, L[(8 * k + lr) * kTP + c0 - 4 + lc]);
         }
-        x = solve4(a[f], h, w, L + c0 * kTP + c0, r);
+        x = solve4(a[f], h, w, G[g & 1]);
         if (g == 15) break;
         const double *B = L + lr * kTP + c0 + lc;
         if (h == 0) other_half(a[f], h, x, B[8 * f * kTP]);
@@ -464,25 +488,22 @@ __device__ __forceinline__ void solve_row16(double *x, const double *D, const do
 // branches (they cost 235 of 343 cycles a column): every lane updates its whole
 // row, and what lands above the diagonal is never read; `bad` collects pivots
 // that are not positive (each replaced by 1).  Each column is stored as it is
-// found (B: the block in shared memory; its transpose above the diagonal), and
+// found, above the diagonal of the block B in shared memory (transposed), and
 // every four columns are announced on cols[J / 4] (if any).
 template <int J>
-__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, bool &bad, double *B, unsigned long long *cols)
+__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, int &bad, double *B, unsigned long long *cols)
 {
     if constexpr (J < 16) {
         const unsigned full = 0xffffffffu;
-        const bool ok = d > 0.0;
-        bad = bad || !ok;
-        d = ok ? d : 1.0;
+        const int ok = d > 0.0;
+        bad |= ok ^ 1;
+        d = sel(ok, d, 1.0);
         const double inv = rsqrt(d);
         const double col = v[J] * inv, piv = d * inv;
-        v[J] = l == J ? piv : col;
+        v[J] = sel(l == J, piv, col);
         double dn = 1.0;
         if constexpr (J + 1 < 16) dn = __shfl_sync(full, fma(-col, col, v[J + 1]), J + 1);  // lane J + 1: its pivot
-        if (l >= J) {
-            B[J * kTP + l] = v[J];
-            B[l * kTP + J] = v[J];
-        }
+        B[J * kTP + l] = v[J];  // (lanes l < J: what lies below the diagonal is written at the end)
         if constexpr ((J & 3) == 3) {
             __syncwarp();
             if (cols) bar_arrive_lane0(cols + J / 4);
@@ -575,20 +596,22 @@ __device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__rest
                 const int f = q >> 1, h = q & 1, c0 = 4 * q;
                 wait(pot_cols(P) + q);
                 const double rl = 1.0 / D[(c0 + lc) * kTP + c0 + lc];
-                double r[4], x[2];
+                double x[2];
+                Group G;
+                load_group(G, D + c0 * kTP + c0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) r[k] = __shfl_sync(full, rl, k);
+                for (int k = 0; k < 4; ++k) G.r[k] = __shfl_sync(full, rl, k);
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     double w[4];
                     gather4(v[e][f], h, w);
-                    x[e] = solve4(v[e][f], h, w, D + c0 * kTP + c0, r);
+                    x[e] = solve4(v[e][f], h, w, G);
                 }
-                const double *B = D + lr * kTP + c0 + lc;
+                const double *B = D + (c0 + lc) * kTP + lr;  // (L's elements from their transpose)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    if (h == 0) other_half(v[e][f], h, x[e], B[8 * f * kTP]);
-                    if (f == 0) mma4(v[e][1], -x[e], B[8 * kTP]);
+                    if (h == 0) other_half(v[e][f], h, x[e], B[8 * f]);
+                    if (f == 0) mma4(v[e][1], -x[e], B[8]);
                 }
                 if (last) {  // (a product's second operand is held as its first)
                     mma4(s[0], x[0], x[0]);
@@ -623,10 +646,15 @@ __device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__rest
             v[k + 1] = x.y;
         }
         __syncwarp();
-        bool bad = false;
+        int bad = 0;
         factor16<0>(v, __shfl_sync(full, v[0], 0), l, bad, W + 16 * g * kTP + 16 * g,
                     g < 3 ? &S.pot[pot_cols(g)] : nullptr);
         if (bad && lane == 0) atomicOr(C.status, kStNotSPD);
+        if (lane < 16) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (k < l) row[16 * g + k] = v[k];
+        }
         if (lane < 16) row[kNB] = 1.0 / row[16 * g + l];
     } else if (warp == 4) {
         wait(pot_rows(0, 1));
@@ -746,17 +774,17 @@ __device__ __forceinline__ void back_diag(const double *__restrict__ D, double &
     double x0 = 0.0, x1 = 0.0;
 #pragma unroll 16
     for (int j = kNB - 1; j >= 32; --j) {
-        const double rd = D[j * kTP + kNB], d0 = -D[j * kTP + lane], d1 = lane + 32 < j ? -D[j * kTP + lane + 32] : 0.0;
+        const double rd = D[j * kTP + kNB], d0 = -D[j * kTP + lane], d1 = sel(lane + 32 < j, -D[j * kTP + lane + 32], 0.0);
         const double xj = __shfl_sync(full, b1, j & 31) * rd;
-        x1 = lane == (j & 31) ? xj : x1;
+        x1 = sel(lane == (j & 31), xj, x1);
         b1 = fma(d1, xj, b1);
         b0 = fma(d0, xj, b0);
     }
 #pragma unroll 16
     for (int j = 31; j >= 0; --j) {
-        const double rd = D[j * kTP + kNB], d0 = lane < j ? -D[j * kTP + lane] : 0.0;
+        const double rd = D[j * kTP + kNB], d0 = sel(lane < j, -D[j * kTP + lane], 0.0);
         const double xj = __shfl_sync(full, b0, j) * rd;
-        x0 = lane == j ? xj : x0;
+        x0 = sel(lane == j, xj, x0);
         b0 = fma(d0, xj, b0);
     }
     b0 = x0;
