@@ -480,41 +480,100 @@ __device__ __forceinline__ void solve_row16(double *x, const double *D, const do
     for (int k = 0; k < 16; k += 2) *reinterpret_cast<double2 *>(x + k) = make_double2(v[k], v[k + 1]);
 }
 
-// Column J onwards of the Cholesky of a 16 x 16 block held by the lanes of
-// one warp, lane l (l = lane % 16) owning row l (v[k] = element (l, k)); d is
-// column J's pivot, in every lane.  The next pivot's own update needs no
-// other lane's value, so the chain per column is the reciprocal square root,
-// two products and one shuffle; the other columns' shuffles overlap it.  No
-// branches (they cost 235 of 343 cycles a column): every lane updates its whole
-// row, and what lands above the diagonal is never read; `bad` collects pivots
-// that are not positive (each replaced by 1).  Each column is stored as it is
-// found, above the diagonal of the block B in shared memory (transposed), and
-// every four columns are announced on cols[J / 4] (if any).
-template <int J>
-__device__ __forceinline__ void factor16(double (&v)[16], double d, int l, int &bad, double *B, unsigned long long *cols)
+// Reciprocal square root of a pivot; one that is not positive is replaced by 1.
+__device__ __forceinline__ double pivot_root(double &d, int &bad)
 {
-    if constexpr (J < 16) {
-        const unsigned full = 0xffffffffu;
-        const int ok = d > 0.0;
-        bad |= ok ^ 1;
-        d = sel(ok, d, 1.0);
-        const double inv = rsqrt(d);
-        const double col = v[J] * inv, piv = d * inv;
-        v[J] = sel(l == J, piv, col);
-        double dn = 1.0;
-        if constexpr (J + 1 < 16) dn = __shfl_sync(full, fma(-col, col, v[J + 1]), J + 1);  // lane J + 1: its pivot
-        B[J * kTP + l] = v[J];  // (lanes l < J: what lies below the diagonal is written at the end)
-        if constexpr ((J & 3) == 3) {
-            __syncwarp();
-            if (cols) bar_arrive_lane0(cols + J / 4);
-        }
+    const int ok = d > 0.0;
+    bad |= ok ^ 1;
+    d = sel(ok, d, 1.0);
+    return rsqrt(d);
+}
+
+// Cholesky of a 16 x 16 block held by one warp as the fragments (0, 0), (1, 0),
+// (1, 1).  Four columns at a time: every lane factors the 4 x 4 block on the
+// diagonal for itself, so a pivot costs the chain a reciprocal square root, a
+// product and a multiply-add and no shuffle, all rows are solved against it
+// (times the reciprocal roots), and products subtract the four columns from the
+// later ones.  Solved columns are stored above the diagonal of the block B in
+// shared memory (transposed; what that puts below it is overwritten at the
+// end) and announced on cols[q] (if any).  (2,080 cycles in a kernel of its own,
+// 2,220 with one row per lane and a shuffle per column and element.)
+__device__ __forceinline__ void factor16(double (&a)[3][2], int &bad, double *B, unsigned long long *cols)
+{
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    double x[4][2];
 #pragma unroll
-        for (int k = J + 1; k < 16; ++k) {
-            const double lkj = __shfl_sync(full, col, k);  // L(k, J), from row k's lane
-            v[k] = fma(-v[J], lkj, v[k]);
+    for (int q = 0; q < 4; ++q) {
+        const int h = q & 1, c0 = 4 * q, fd = q < 2 ? 0 : 2, at = 18 * h;  // (lane of the 4 x 4 block's first element)
+        double a00 = __shfl_sync(full, a[fd][0], at);
+        double a10 = __shfl_sync(full, a[fd][0], at + 4), a11 = __shfl_sync(full, a[fd][1], at + 4);
+        double a20 = __shfl_sync(full, a[fd][0], at + 8), a21 = __shfl_sync(full, a[fd][1], at + 8);
+        double a30 = __shfl_sync(full, a[fd][0], at + 12), a31 = __shfl_sync(full, a[fd][1], at + 12);
+        double a22 = __shfl_sync(full, a[fd][0], at + 9), a32 = __shfl_sync(full, a[fd][0], at + 13);
+        double a33 = __shfl_sync(full, a[fd][1], at + 13);
+        double w[2][4];  // each row's four values, rows of fragment row e
+#pragma unroll
+        for (int e = q < 2 ? 0 : 1; e < 2; ++e) gather4(a[q < 2 ? e : 2], h, w[e]);
+        Group G;
+        double p[4];
+        G.r[0] = pivot_root(a00, bad);
+        p[0] = a00 * G.r[0];
+        G.l10 = a10 * G.r[0];
+        G.l20 = a20 * G.r[0];
+        G.l30 = a30 * G.r[0];
+        a11 = fma(-G.l10, G.l10, a11);
+        a21 = fma(-G.l20, G.l10, a21);
+        a31 = fma(-G.l30, G.l10, a31);
+        a22 = fma(-G.l20, G.l20, a22);
+        a32 = fma(-G.l30, G.l20, a32);
+        a33 = fma(-G.l30, G.l30, a33);
+        G.r[1] = pivot_root(a11, bad);
+        p[1] = a11 * G.r[1];
+        G.l21 = a21 * G.r[1];
+        G.l31 = a31 * G.r[1];
+        a22 = fma(-G.l21, G.l21, a22);
+        a32 = fma(-G.l31, G.l21, a32);
+        a33 = fma(-G.l31, G.l31, a33);
+        G.r[2] = pivot_root(a22, bad);
+        p[2] = a22 * G.r[2];
+        G.l32 = a32 * G.r[2];
+        a33 = fma(-G.l32, G.l32, a33);
+        G.r[3] = pivot_root(a33, bad);
+        p[3] = a33 * G.r[3];
+#pragma unroll
+        for (int e = q < 2 ? 0 : 1; e < 2; ++e) {
+            double w0 = w[e][0] * G.r[0];
+            double w1 = fma(-w0, G.l10, w[e][1]), w2 = fma(-w0, G.l20, w[e][2]), w3 = fma(-w0, G.l30, w[e][3]);
+            w1 = w1 * G.r[1];
+            w2 = fma(-w1, G.l21, w2);
+            w3 = fma(-w1, G.l31, w3);
+            w2 = w2 * G.r[2];
+            w3 = fma(-w2, G.l32, w3);
+            w3 = w3 * G.r[3];
+            if (e == fd >> 1) {  // the pivots themselves
+                w0 = sel(lr == 4 * h, p[0], w0);
+                w1 = sel(lr == 4 * h + 1, p[1], w1);
+                w2 = sel(lr == 4 * h + 2, p[2], w2);
+                w3 = sel(lr == 4 * h + 3, p[3], w3);
+            }
+            x[q][e] = sel(lc & 2, sel(lc & 1, w3, w2), sel(lc & 1, w1, w0));
+            B[(c0 + lc) * kTP + 8 * e + lr] = x[q][e];
         }
-        factor16<J + 1>(v, dn, l, bad, B, cols);
+        __syncwarp();
+        if (cols) bar_arrive_lane0(cols + q);
+        if (q == 0) {
+            mma4(a[0], -x[0][0], x[0][0]);
+            mma4(a[1], -x[0][1], x[0][0]);
+        }
+        if (q < 3) mma4(a[2], -x[q][1], x[q][1]);
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = q < 2 ? 0 : 1; e < 2; ++e)
+            if (8 * e + lr > 4 * q + lc) B[(8 * e + lr) * kTP + 4 * q + lc] = x[q][e];
+    __syncwarp();
 }
 
 // barriers of tile_potrf, each completed once per tile: four columns of panel
@@ -626,35 +685,18 @@ __device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__rest
             if (P < 2) done(pot_rows(P, g));
         }
         if (g >= 2) wait(pot_block(g, g));
-        if (g > 0) {
+        double d[3][2];
 #pragma unroll
-            for (int e = 0; e < 3; ++e) {
-                double2 *c = reinterpret_cast<double2 *>(mine + (e > 0 ? 8 * kTP : 0) + 16 * g + (e > 1 ? 8 : 0));
-                double2 x = *c;
-                x.x -= s[e][0];
-                x.y -= s[e][1];
-                *c = x;
-            }
-            __syncwarp();
-        }
-        double v[16];
-        double *row = W + (16 * g + l) * kTP;
-#pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-            const double2 x = *reinterpret_cast<const double2 *>(row + 16 * g + k);
-            v[k] = x.x;
-            v[k + 1] = x.y;
+        for (int e = 0; e < 3; ++e) {
+            const double2 x = *reinterpret_cast<const double2 *>(mine + (e > 0 ? 8 * kTP : 0) + 16 * g + (e > 1 ? 8 : 0));
+            d[e][0] = x.x - s[e][0];
+            d[e][1] = x.y - s[e][1];
         }
         __syncwarp();
         int bad = 0;
-        factor16<0>(v, __shfl_sync(full, v[0], 0), l, bad, W + 16 * g * kTP + 16 * g,
-                    g < 3 ? &S.pot[pot_cols(g)] : nullptr);
+        factor16(d, bad, W + 16 * g * kTP + 16 * g, g < 3 ? &S.pot[pot_cols(g)] : nullptr);
         if (bad && lane == 0) atomicOr(C.status, kStNotSPD);
-        if (lane < 16) {
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                if (k < l) row[16 * g + k] = v[k];
-        }
+        double *row = W + (16 * g + l) * kTP;
         if (lane < 16) row[kNB] = 1.0 / row[16 * g + l];
     } else if (warp == 4) {
         wait(pot_rows(0, 1));
