@@ -26,13 +26,15 @@
 // copies into a ring of shared-memory buffers, after the flag that publishes
 // each tile) and one warp stores results and publishes them, so neither a
 // flag's round trip nor a store's completion stands on the compute warps'
-// path.  What bounds it: the chain's latency up to about 3000 landmarks -- per
-// 64 columns some 35,000 cycles: 22,000 in the diagonal tile (64 dependent
-// pivots: reciprocal square root, multiply, multiply-add, shuffle), 7,000 in
-// the panel tile's solution, 4,500 in its product -- and the helpers' FP64
-// matrix instructions beyond (64 multiply-adds per SM and clock).  Kernel at
-// 4096 landmarks: 1.92 ms with scalar multiply-adds for the products and
-// solutions, 1.63 ms with the matrix instruction.
+// path.  What bounds it: latency up to about 3000 landmarks -- per 64 columns
+// the chain takes some 25,000 cycles (diagonal tile 14,000: 64 dependent
+// pivots, each a reciprocal square root, a product and a multiply-add, and
+// three hand-overs between panels; panel tile's solution 5,000; its product
+// 2,500), and a tile needs about as long from a diagonal tile's publication
+// through a helper's solution and the next helper's product to the chain -- and
+// the helpers' FP64 matrix instructions beyond (64 multiply-adds per SM and
+// clock).  Solve of 500 / 2000 / 4096 landmarks: 337 / 1074 / 2452 us with
+// scalar multiply-adds for products and solutions, 300 / 932 / 1984 now.
 //
 // Every element sees the operations of the plain right-looking tiled
 // factorisation in the same order, whatever the schedule.
@@ -337,21 +339,38 @@ __device__ __forceinline__ void mma4(double (&c)[2], double a, double b)
         : "d"(a), "d"(b));
 }
 
-// acc = Li Lj', summed over the 64 columns in order; DIAG: only the lower
-// fragments (f <= wr), the others 0.
-template <bool DIAG>
-__device__ __forceinline__ void tile_product(const double *__restrict__ Li, const double *__restrict__ Lj, int wr, Frags &acc)
+// The first N fragments of acc = Li Lj', summed over the 64 columns in order;
+// the others 0.
+template <int N>
+__device__ __forceinline__ void product_n(const double *__restrict__ A, const double *__restrict__ B, Frags &acc)
 {
-    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
 #pragma unroll
     for (int f = 0; f < 8; ++f) acc[f][0] = acc[f][1] = 0.0;
-    const double *A = Li + (8 * wr + lr) * kTP + lc, *B = Lj + lr * kTP + lc;
 #pragma unroll 4
     for (int p = 0; p < kNB; p += 4) {
         const double x = A[p];
 #pragma unroll
-        for (int f = 0; f < 8; ++f)
-            if (!DIAG || f <= wr) mma4(acc[f], x, B[8 * f * kTP + p]);
+        for (int f = 0; f < N; ++f) mma4(acc[f], x, B[8 * f * kTP + p]);
+    }
+}
+// DIAG: only the lower fragments (f <= wr), in a loop of their own for each wr
+// (a test per fragment in one loop keeps its loads from moving ahead of the
+// products: 4,800 cycles for the two warps of a sub-partition).
+template <bool DIAG>
+__device__ __forceinline__ void tile_product(const double *__restrict__ Li, const double *__restrict__ Lj, int wr, Frags &acc)
+{
+    const int lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+    const double *A = Li + (8 * wr + lr) * kTP + lc, *B = Lj + lr * kTP + lc;
+    if (!DIAG) return product_n<8>(A, B, acc);
+    switch (wr) {
+    case 0: return product_n<1>(A, B, acc);
+    case 1: return product_n<2>(A, B, acc);
+    case 2: return product_n<3>(A, B, acc);
+    case 3: return product_n<4>(A, B, acc);
+    case 4: return product_n<5>(A, B, acc);
+    case 5: return product_n<6>(A, B, acc);
+    case 6: return product_n<7>(A, B, acc);
+    default: return product_n<8>(A, B, acc);
     }
 }
 
@@ -618,10 +637,10 @@ __device__ __forceinline__ void block_update(double *__restrict__ W, int i, int 
 // and so goes on to factor its own panel a few hundred cycles after the one
 // before: the chain is 64 pivots and little else.  The products for the other
 // blocks are warps 4 .. 7's.  A panel's product is summed over its 16 columns
-// first, then subtracted.  (21,900 cycles: four times 3,700 in factor16, three
-// times 1,400 from one panel's last column to the next panel's first; 22,900
-// panel after panel, with barriers of all warps between factoring, solving and
-// updating.)
+// first, then subtracted.  (14,000 cycles: four times 2,650 in factor16 and
+// three times 850 from one panel's last column to the next panel's first;
+// 22,900 panel after panel, with barriers of all warps between factoring,
+// solving and updating.)
 __device__ __forceinline__ void tile_potrf(const Ctl &C, Smem &S, double *__restrict__ W, uint32_t n)
 {
     const unsigned full = 0xffffffffu;
