@@ -318,7 +318,7 @@ def affine_leg(ctx, device: int, steps: int = 5):
     gbs = vox * 4 / (ms / 1e3) / 1e9
     del src, dst
     return {"workload": "affine_1024x1024x512_u16_n32", "ms_per_warp": ms, "gvoxel_s": vox / (ms / 1e3) / 1e9,
-            "achieved_gbs": gbs, "frac_of_hbm": gbs / peak, "kernel": "k_resample_affine<uint16,trilinear>"}
+            "achieved_gbs": gbs, "frac_of_hbm": gbs / peak, "kernel": "k_affine_staged<uint16>"}
 
 
 def tiled_leg(ctx, device: int, shape_zyx=(512, 2048, 2048)):
