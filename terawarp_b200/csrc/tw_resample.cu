@@ -786,6 +786,35 @@ __device__ __forceinline__ void warp_minmax(float (&mn)[3], float (&mx)[3])
         }
 }
 
+// Bytes of the whole rings at or below source plane `a` (relative to a walk's
+// first output plane): the part of the shift along z that layer_k takes out of
+// the tap offsets.
+template <typename T>
+__device__ __forceinline__ int64_t shift_rings(int a)
+{
+    constexpr int64_t PLANE_B = kHMax * kBoxW * sizeof(T);
+    return (a & ~(kRing<T> - 1)) * PLANE_B;
+}
+
+// Is every partial sum of a walk's tap offsets exact (see layer_k)?  They are
+// k, that is 2^23 less the shift's bytes plus the slot's, then k + x ES, + y
+// ROW_B and + z PLANE_B, each of which puts its part of the shift back in, up
+// to the box and, along z, a ring, a layer and a window of planes: less than
+// 2^20 in all.  Along z that allows shifts of -896 to 2048 planes (uint16) or
+// -1792 to 4096 (uint8).
+template <typename T>
+__device__ __forceinline__ bool shift_fits(const Plan &P)
+{
+    constexpr int64_t ES = sizeof(T), ROW_B = kBoxW * ES;
+    const int64_t c[3] = {-shift_rings<T>(P.a), P.DY * ROW_B, P.DX * ES};
+    int64_t up = 1 << 20, down = 0;
+    for (int i = 0; i < 3; ++i) {
+        up += max(c[i], (int64_t)0);
+        down += max(-c[i], (int64_t)0);
+    }
+    return up <= (1 << 23) && down <= (1 << 24);
+}
+
 // Plans walk w (one warp): the hull of the DF over the walk's node support
 // gives the staged box and the plane window.  staged = 0 when they do not
 // fit.  Every lane returns the same plan.
@@ -850,7 +879,6 @@ __device__ Plan plan_walk(const RJob &J, const Walk &w)
     }
     // staged walks index the node grid with 32 bits
     if (J.gsz[0] * J.gsz[1] * J.gsz[2] >= ((int64_t)1 << 31)) return P;
-    P.staged = 1;
     P.a = a;
     P.b = b;
     P.rx0 = (int)rx0;
@@ -858,6 +886,8 @@ __device__ Plan plan_walk(const RJob &J, const Walk &w)
     P.rows = rows;
     P.DX = (int)(w.Ox - J.src_o[0] - rx0);
     P.DY = -fy0;
+    if (!shift_fits<T>(P)) return P;
+    P.staged = 1;
     P.nplanes = (int)(w.z1 - w.z0) + b - a;
     P.j = w.j;
     P.ox = (int)w.Ox;
@@ -1130,13 +1160,18 @@ __device__ __forceinline__ void plane_positions(const RowLayer &L, float4 wz, fl
 // Offset of the floor tap of a staged sample at frame floors (x, y, z): byte
 // z PLANE_B + y ROW_B + x ES + k of the ring, taken modulo the ring's size (a
 // power of two: plane sequence s is slot s mod kRing).  The sum is formed in
-// floating point on both voxels at once, as kMagic + offset, whose bit
-// pattern's low bits are the offset (exact: every tap of a walk is within 2^22
-// bytes of its layer's frame).  Whatever the position -- NaN included -- the
-// masked offset is an element of the ring and its taps lie in shared memory
-// (the last plane's past it, in the mirror of slot 0 and the barriers after).
+// floating point on both voxels at once, as an integer of [2^23, 2^24) whose
+// bit pattern's low bits are the offset.  Whatever the position -- NaN included
+// -- the masked offset is an element of the ring and its taps lie in shared
+// memory (the last plane's past it, in the mirror of slot 0 and the barriers
+// after).
 //
-// layer_k: kMagic + k for the cell layer with frame origin Oz of a walk whose
+// z, y and x contain the walk's shift, so k takes it out again: z's in whole
+// rings (which leaves the offset as it is), y's and x's exactly.  The sums on
+// the way are integers, exact while below 2^24 in magnitude; plan_walk leaves a
+// walk with a larger shift to the gather kernel (shift_fits).
+//
+// layer_k: k for the cell layer with frame origin Oz of a walk whose
 // first plane (output plane z0 + a) has sequence seq0: the source plane Oz + z
 // has sequence seq0 + (Oz + z) - (z0 + a); DY, DX: row / column of frame (0, 0)
 // in the staged box.
@@ -1145,7 +1180,7 @@ __device__ __forceinline__ float layer_k(uint32_t seq0, int64_t Oz, int64_t z0, 
 {
     constexpr int ES = sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
     const uint32_t slot = (seq0 + (uint32_t)(Oz - z0) - (uint32_t)P.a) & (uint32_t)(kRing<T> - 1);
-    return kMagic + (float)((int)slot * PLANE_B + P.DY * ROW_B + P.DX * ES);
+    return (float)((1 << 23) + (int)slot * PLANE_B - (int)shift_rings<T>(P.a) + P.DY * ROW_B + P.DX * ES);
 }
 
 // A voxel pair of an interior walk from the staged planes, in three steps
@@ -1171,7 +1206,7 @@ __device__ __forceinline__ PairPrep prep_pair(uint32_t ring, float k, float2 px,
 {
     constexpr float ES = (float)sizeof(T), ROW_B = kBoxW * ES, PLANE_B = kHMax * ROW_B;
     constexpr uint32_t RING = kRing<T> * kHMax * kBoxW * (uint32_t)sizeof(T), MASK = RING - (uint32_t)sizeof(T);
-    static_assert((RING & (RING - 1)) == 0 && (kMagicBits & (RING - 1)) == 0, "the ring is a power of two of bytes");
+    static_assert((RING & (RING - 1)) == 0 && (0x4B000000u & (RING - 1)) == 0, "the ring is a power of two of bytes");
     const float2 MM = f2(kMagic, kMagic);
     if (NEAR) {
         const float2 half = f2(0.5f, 0.5f);
