@@ -239,6 +239,17 @@ __device__ __forceinline__ void bar_wait_free(const Ctl &C, Smem &S, unsigned lo
     if (n > 0) bar_wait(C, S, b, n - 1);
 }
 
+// The same for the fetching warp, before it copies into a buffer: false once the
+// CTA has given up.  The compute warps then no longer wait for what they read
+// and release, so a release says nothing about the buffer any more, and a second
+// copy counted on a "full" barrier whose phase is still open would let the CTA
+// end before its copies have landed.
+__device__ __forceinline__ bool claim_buf(const Ctl &C, Smem &S, unsigned long long *b, uint32_t n)
+{
+    bar_wait_free(C, S, b, n);
+    return *reinterpret_cast<volatile int *>(&S.abort) == 0;
+}
+
 // Waits (one thread) until *flag >= want; false once anyone has given up.
 __device__ bool flag_wait(const Ctl &C, Smem &S, const int *flag, int want)
 {
@@ -775,11 +786,11 @@ __device__ void chain_fetch(const Ctl &C, Smem &S)
     for (int k = 1; k < nblk; ++k) {
         const uint32_t n = (uint32_t)(k - 1);
         if (k >= 2 && !flag_wait(C, S, &C.pre_s[k - 1], 1)) return;
-        bar_wait_free(C, S, &S.empty[kBufX], n);
+        if (!claim_buf(C, S, &S.empty[kBufX], n)) return;
         fence_async();
         load_buf(S, kBufX, tile_ptr(C, k, k - 1), kTileB);
         if (k >= 2 && !flag_wait(C, S, &C.pre_d[k], 1)) return;
-        bar_wait_free(C, S, &S.empty[kBufD], n);
+        if (!claim_buf(C, S, &S.empty[kBufD], n)) return;
         fence_async();
         load_buf(S, kBufD, tile_ptr(C, k, k), kTileB);
     }
@@ -816,8 +827,7 @@ __device__ void chain_fetch(const Ctl &C, Smem &S)
 #pragma unroll
             for (int k = 0; k < kBufs; ++k)
                 if (k == b) u = used[k]++;
-            bar_wait_free(C, S, &S.empty[b], u);
-            if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+            if (!claim_buf(C, S, &S.empty[b], u)) return;
             load_buf(S, b, src, kTileB);
             ++q;
         }
@@ -1016,7 +1026,7 @@ __device__ void helper_fetch(const Ctl &C, Smem &S, const Task &T, uint32_t &sta
         for (int kb = nblk - 1; kb >= T.i + 4; --kb) {
             const int b = 2 * (int)(stage & 1u);
             if (kb == nblk - 1 && (!flag_wait(C, S, &C.F->pdone, nblk) || !flag_wait(C, S, &C.tdone[nblk], nblk))) return;
-            bar_wait_free(C, S, &S.empty[b], stage >> 1);
+            if (!claim_buf(C, S, &S.empty[b], stage >> 1)) return;
             fence_async();
             load_buf(S, b, tile_ptr(C, kb, T.i), kTileB);
             ++stage;
@@ -1031,8 +1041,7 @@ __device__ void helper_fetch(const Ctl &C, Smem &S, const Task &T, uint32_t &sta
             if (!flag_wait(C, S, &C.tdone[T.j], k + 1) || !flag_wait(C, S, &C.tdone[T.kind == 2 ? nblk : T.i], k + 1)) return;
             ready = min(ld_acquire(&C.tdone[T.j]), ld_acquire(&C.tdone[T.kind == 2 ? nblk : T.i]));
         }
-        bar_wait_free(C, S, &S.empty[b], stage >> 1);
-        if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+        if (!claim_buf(C, S, &S.empty[b], stage >> 1)) return;
         fence_async();
         const bool two = T.kind == 2 || T.i != T.j;
         // both operands count on the first buffer's barrier
@@ -1044,8 +1053,7 @@ __device__ void helper_fetch(const Ctl &C, Smem &S, const Task &T, uint32_t &sta
     }
     if (T.kind == 2 || T.i > T.j + 1) {
         if (!flag_wait(C, S, &C.F->pdone, T.j + 1)) return;
-        bar_wait_free(C, S, &S.empty[kBufL], diags);
-        if (*reinterpret_cast<volatile int *>(&S.abort)) return;
+        if (!claim_buf(C, S, &S.empty[kBufL], diags)) return;
         fence_async();
         load_buf(S, kBufL, tile_ptr(C, T.j, T.j), kTileB);
         ++diags;
