@@ -2411,7 +2411,9 @@ cudaError_t launch_affine_staged_t(const RJob *jobs, int njobs, int64_t total, u
     const auto k = k_affine_staged<T>;
     const int stages = (int)min((uint32_t)kAStages, (uint32_t)kAffineSmem / stage_b);
     const int smem = (int)(stage_b * (uint32_t)stages) + 128;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // (the limit is the process's, not this launch's: always the same value, or a
+    // thread with a smaller box could lower it between this call and the launch)
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kAffineSmem + 128);
     if (e != cudaSuccess) return e;
     const int64_t grid = total < sms ? total : sms;
     k<<<(unsigned)grid, kAStagedThreads, smem, st>>>(jobs, njobs, total, stages, stage_b, err);
