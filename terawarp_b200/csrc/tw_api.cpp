@@ -357,6 +357,16 @@ unsigned long long tw_internal_set_solve_barrier_ns(tw_ctx *ctx, unsigned long l
     return ctx->solve_barrier_ns.exchange(ns ? ns : 30000000000ull);
 }
 
+// Test hook, not part of the public header: how a node grid's evaluation is
+// dealt to threads (see EvalForm) on a device of sm_count SMs.  Needs no GPU.
+void tw_internal_eval_form(const int64_t gsz[3], int n, int sm_count, int form[3])
+{
+    const EvalForm f = eval_form(gsz, n, sm_count);
+    form[0] = f.npt;
+    form[1] = f.split;
+    form[2] = f.axis;
+}
+
 // Test hook, not part of the public header: turns the shared-memory staging
 // of TPS resample units on (1) or off (0) for this context and returns the
 // previous setting; off, every unit gathers its taps from global memory.

@@ -10,7 +10,8 @@
 // warp-wide broadcasts; a thread evaluates 2 or 4 nodes of one (x, y) column, so
 // dx^2 + dy^2 is computed once per landmark for all of them.  Per landmark and
 // two nodes what is left is one add, one multiply-add, two square roots and
-// three multiply-adds, the node pairs in FP32x2 instructions.  What bounds it:
+// three multiply-adds, the node pairs in FP32x2 instructions.  (Grids a few
+// nodes deep: nodes of one row, see eval_form.)  What bounds it:
 // the square roots, 16 per SM and clock (1.15 M nodes x 2000 landmarks: 0.51
 // ms of them; the call takes 648 us, 826 when each node had its own dx and dy
 // and the landmarks' components were staged twice over: a broadcast of 16
@@ -50,13 +51,14 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float x)
     s = t;
 }
 
-// NPT: nodes per thread, consecutive in z.  SPLIT: groups of threads that
+// NPT: nodes per thread, consecutive along axis AX (z, or x).  SPLIT: groups of threads that
 // share the 32-landmark partial sums of the same nodes out among themselves,
 // turn by turn; the partials then meet in shared memory and are added in
 // landmark order, so the sums are the same whatever the split.
-template <int NPT, int SPLIT>
+template <int NPT, int SPLIT, int AX>
 __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
 {
+    static_assert(AX == 0 || AX == 2, "runs along x or z");
     constexpr int UNITS = kEvalThreads / SPLIT, P2 = NPT / 2;
     static_assert(kTile / kSub == 8 && 8 % SPLIT == 0 && UNITS % 32 == 0, "whole warps, whole turns");
     __shared__ float4 s_a[kTile];  // -cx, -cy, -cz, wx
@@ -64,15 +66,18 @@ __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
     __shared__ float s_part[SPLIT > 1 ? SPLIT : 1][3 * NPT][SPLIT > 1 ? UNITS : 1];
     const int unit = threadIdx.x % UNITS, grp = threadIdx.x / UNITS;
     const int64_t U = (int64_t)blockIdx.x * UNITS + unit;
-    // units: x fastest, then y, then runs of NPT planes (past the end: the
-    // last node again, not stored)
-    const int64_t ix = U % p.gsz[0], iy = U / p.gsz[0] % p.gsz[1], iz = U / (p.gsz[0] * p.gsz[1]) * NPT;
-    const float px = (float)(p.node_o[0] + ix * p.g), py = (float)(p.node_o[1] + iy * p.g);
-    float pz[NPT];
+    // units: x (or runs of NPT columns) fastest, then y, then z (or runs of NPT
+    // planes); past the end: some node again, not stored
+    const int64_t nx = AX == 0 ? (p.gsz[0] + NPT - 1) / NPT : p.gsz[0];
+    const int64_t ix = U % nx * (AX == 0 ? NPT : 1), iy = U / nx % p.gsz[1];
+    const int64_t iz = U / (nx * p.gsz[1]) * (AX == 2 ? NPT : 1);
+    const auto coord = [&](int a, int64_t i) { return (float)(p.node_o[a] + min(i, p.gsz[a] - 1) * p.g); };
+    const float px = coord(0, ix), py = coord(1, iy), pz = coord(2, iz);
+    float pr[NPT];  // along the run
     float s[3][NPT], c[3][NPT];
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
-        pz[j] = (float)(p.node_o[2] + (iz + j < p.gsz[2] ? iz + j : p.gsz[2] - 1) * p.g);
+        pr[j] = coord(AX, (AX == 0 ? ix : iz) + j);
 #pragma unroll
         for (int q = 0; q < 3; ++q) s[q][j] = c[q][j] = 0.f;
     }
@@ -103,14 +108,24 @@ __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
                 for (int l = sb * kSub; l < sb * kSub + kSub; ++l) {
                     const float4 A = s_a[l];
                     const float2 B = s_b[l];
-                    const float dx = __fadd_rn(px, A.x), dy = __fadd_rn(py, A.y);
-                    const float r0 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
-                    const float2 r02 = make_float2(r0, r0), ncz = make_float2(A.z, A.z);
+                    // dx^2 + dy^2 + dz^2, added in this order whatever the run
+                    const float dy = __fadd_rn(py, A.y);
+                    float2 r02, dy2, dz2;
+                    if (AX == 2) {
+                        const float dx = __fadd_rn(px, A.x), r0 = __fmaf_rn(dy, dy, __fmul_rn(dx, dx));
+                        r02 = make_float2(r0, r0);
+                    } else {
+                        const float dz = __fadd_rn(pz, A.z);
+                        dy2 = make_float2(dy, dy);
+                        dz2 = make_float2(dz, dz);
+                    }
+                    const float nc = AX == 0 ? A.x : A.z;
                     const float2 wx = make_float2(A.w, A.w), wy = make_float2(B.x, B.x), wz = make_float2(B.y, B.y);
 #pragma unroll
                     for (int k = 0; k < P2; ++k) {
-                        const float2 dz = __fadd2_rn(make_float2(pz[2 * k], pz[2 * k + 1]), ncz);
-                        const float2 r2 = __ffma2_rn(dz, dz, r02);
+                        const float2 dr = __fadd2_rn(make_float2(pr[2 * k], pr[2 * k + 1]), make_float2(nc, nc));
+                        const float2 r2 = AX == 2 ? __ffma2_rn(dr, dr, r02)
+                                                  : __ffma2_rn(dz2, dz2, __ffma2_rn(dy2, dy2, __fmul2_rn(dr, dr)));
                         const float2 r = make_float2(fast_sqrt(r2.x), fast_sqrt(r2.y));
                         a[0][k] = __ffma2_rn(r, wx, a[0][k]);
                         a[1][k] = __ffma2_rn(r, wy, a[1][k]);
@@ -164,10 +179,12 @@ __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
     }
 #pragma unroll
     for (int j = 0; j < NPT; ++j) {
-        if (iz + j >= p.gsz[2]) break;
-        float dfx = a0[0] + alin[0][0] * px + alin[1][0] * py + alin[2][0] * pz[j];
-        float dfy = a0[1] + alin[0][1] * px + alin[1][1] * py + alin[2][1] * pz[j];
-        float dfz = a0[2] + alin[0][2] * px + alin[1][2] * py + alin[2][2] * pz[j];
+        const int64_t i = AX == 0 ? ix + j : ix, k = AX == 2 ? iz + j : iz;
+        if (i >= p.gsz[0] || k >= p.gsz[2]) break;
+        const float x = AX == 0 ? pr[j] : px, z = AX == 2 ? pr[j] : pz;
+        float dfx = __fmaf_rn(alin[2][0], z, __fmaf_rn(alin[1][0], py, __fmaf_rn(alin[0][0], x, a0[0])));
+        float dfy = __fmaf_rn(alin[2][1], z, __fmaf_rn(alin[1][1], py, __fmaf_rn(alin[0][1], x, a0[1])));
+        float dfz = __fmaf_rn(alin[2][2], z, __fmaf_rn(alin[1][2], py, __fmaf_rn(alin[0][2], x, a0[2])));
         // the running compensation holds minus the lost low-order part
         if constexpr (SPLIT > 1) {
             dfx += s_part[0][j][unit];
@@ -178,34 +195,58 @@ __global__ void __launch_bounds__(kEvalThreads) k_tps_eval(EvalParams p)
             dfy += s[1][j] - c[1][j];
             dfz += s[2][j] - c[2][j];
         }
-        p.out[((iz + j) * p.gsz[1] + iy) * p.gsz[0] + ix] = make_float4(dfx, dfy, dfz, 0.f);
+        p.out[(k * p.gsz[1] + iy) * p.gsz[0] + i] = make_float4(dfx, dfy, dfz, 0.f);
     }
 }
 
-template <int NPT, int SPLIT>
-cudaError_t launch_eval(const EvalParams &p, cudaStream_t st)
+template <int NPT, int SPLIT, int AX>
+cudaError_t launch_eval_along(const EvalParams &p, cudaStream_t st)
 {
-    const int64_t units = p.gsz[0] * p.gsz[1] * ((p.gsz[2] + NPT - 1) / NPT);
-    const int64_t per = kEvalThreads / SPLIT, grid = (units + per - 1) / per;
+    int64_t n[3] = {p.gsz[0], p.gsz[1], p.gsz[2]};
+    n[AX] = (n[AX] + NPT - 1) / NPT;
+    const int64_t per = kEvalThreads / SPLIT, grid = (n[0] * n[1] * n[2] + per - 1) / per;
     if (grid > 0x7fffffff) return cudaErrorInvalidValue;
-    k_tps_eval<NPT, SPLIT><<<(unsigned)grid, kEvalThreads, 0, st>>>(p);
+    k_tps_eval<NPT, SPLIT, AX><<<(unsigned)grid, kEvalThreads, 0, st>>>(p);
     return cudaGetLastError();
+}
+
+template <int NPT, int SPLIT>
+cudaError_t launch_eval(const EvalParams &p, cudaStream_t st, int axis)
+{
+    return axis == 0 ? launch_eval_along<NPT, SPLIT, 0>(p, st) : launch_eval_along<NPT, SPLIT, 2>(p, st);
 }
 
 }  // namespace
 
-cudaError_t launch_tps_eval(const EvalParams &p, cudaStream_t st, int sm_count)
+EvalForm eval_form(const int64_t gsz[3], int n, int sm_count)
 {
-    const int64_t nnodes = p.gsz[0] * p.gsz[1] * p.gsz[2];
-    if (nnodes <= 0) return cudaSuccess;
+    const int64_t nnodes = gsz[0] * gsz[1] * gsz[2];
+    EvalForm f;
     // A grid that fills the chip runs one thread per four nodes.  Smaller ones
     // share the landmarks of 32-node units out over a block's eight warps, if
     // there are enough of them (calls with 2000 landmarks: 847 nodes 129 us
     // unsplit, 49 split, 23,000 129 and 58 with two nodes a thread, 61 with
-    // four; 157,000 201, 150 and 134; 1.15 M 649, 793 and 677).
-    if (nnodes >= (int64_t)sm_count * 2048) return launch_eval<4, 1>(p, st);
-    if (nnodes >= (int64_t)sm_count * 256) return p.n > 128 ? launch_eval<4, 8>(p, st) : launch_eval<4, 1>(p, st);
-    return launch_eval<2, 8>(p, st);
+    // four; 157,000 201, 150 and 134; 1.15 M 649, 793 and 677; 292,000 227, -
+    // and 211, but with 300 landmarks 55, - and 58).
+    if (nnodes >= (int64_t)sm_count * (n > 512 ? 2048 : 1792)) f = {4, 1, 2};
+    else if (nnodes >= (int64_t)sm_count * 256) f = {4, n > 128 ? 8 : 1, 2};
+    else f = {2, 8, 2};
+    // The nodes of a thread lie along z, unless rounding the grid's depth up to
+    // whole runs costs clearly more than rounding its width up (2000 landmarks,
+    // us along z and along x: 515 x 515 x 1 607 and 198, x 3 632 and 521, x 5
+    // 1151 and 766, 259 x 259 x 9 481 and 361; a run along x has two more
+    // instructions per pair: 131 x 131 x 67 634 and 716)
+    const auto rounded = [&](int a) { return (double)((gsz[a] + f.npt - 1) / f.npt * f.npt) / (double)gsz[a]; };
+    if (rounded(2) > 1.1 * rounded(0)) f.axis = 0;
+    return f;
+}
+
+cudaError_t launch_tps_eval(const EvalParams &p, cudaStream_t st, int sm_count)
+{
+    if (p.gsz[0] * p.gsz[1] * p.gsz[2] <= 0) return cudaSuccess;
+    const EvalForm f = eval_form(p.gsz, p.n, sm_count);
+    if (f.npt == 2) return launch_eval<2, 8>(p, st, f.axis);
+    return f.split == 8 ? launch_eval<4, 8>(p, st, f.axis) : launch_eval<4, 1>(p, st, f.axis);
 }
 
 }  // namespace tw

@@ -123,6 +123,12 @@ struct EvalParams {
     float4 *out;
 };
 cudaError_t launch_tps_eval(const EvalParams &p, cudaStream_t st, int sm_count);
+// How a grid's nodes are dealt to threads: nodes per thread, groups of threads
+// that share the landmarks out, and the axis a thread's nodes lie along (0 or 2).
+struct EvalForm {
+    int npt, split, axis;
+};
+EvalForm eval_form(const int64_t gsz[3], int n, int sm_count);
 
 // ------------------------------------------------------------------- solve
 
