@@ -367,6 +367,14 @@ void tw_internal_eval_form(const int64_t gsz[3], int n, int sm_count, int form[3
     form[2] = f.axis;
 }
 
+// Test hook, not part of the public header: output planes of a TPS work unit of
+// a launch over one volume on a device of sm_count SMs.  Needs no GPU.
+int tw_internal_tps_unit_planes(const int64_t out_sz[3], int g, int staged, int sm_count)
+{
+    const RJob j = tps_job(nullptr, out_sz, nullptr, out_sz, nullptr, g, TW_U8, 0);
+    return tps_unit_planes(&j, 1, staged != 0, sm_count);
+}
+
 // Test hook, not part of the public header: turns the shared-memory staging
 // of TPS resample units on (1) or off (0) for this context and returns the
 // previous setting; off, every unit gathers its taps from global memory.

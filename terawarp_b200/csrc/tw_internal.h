@@ -92,6 +92,8 @@ size_t tps_stage_ws_bytes(int64_t total_bricks);
 // Brick extents for a (kind, g) pair: x, y and the z extent a unit's frame
 // is anchored to (a control cell layer for TPS).
 void brick_dims(int kind, int g, int64_t out[3]);
+// Output planes of a TPS work unit for a launch of these jobs.
+int tps_unit_planes(const RJob *jobs, int njobs, bool staged, int sm_count);
 // Fills j.tmap / j.tma_ok for a TPS job (false when the source buffer's
 // address or pitches do not meet the TMA rules; the job then gathers).
 bool encode_source_map(RJob &j);

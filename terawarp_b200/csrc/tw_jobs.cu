@@ -176,6 +176,30 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
     return TW_OK;
 }
 
+// TPS units walk 64 output planes (several cell layers: the staged source
+// window is loaded once per walk); when a launch has too few units to
+// balance, they get shorter.  Staged ones down to 16 planes -- below that the
+// windows and the per-layer set-up cost more than an even last wave gives (256 x
+// 256 x 128 uint8: 109 us at 4 planes, 91 at 16; 512^3 uint16: 573 at 64, 513 at
+// 16; 1024 x 1024 x 256 uint8, spacing 4: 2114 at 64, 2011 at 32).  Gathered units
+// keep no window: they need fewer to balance, and a small launch is better off
+// with many short ones (64^3 uint8, call: 61 us at 16 planes, 53 at 1).
+int tps_unit_planes(const RJob *jobs, int njobs, bool staged, int sm_count)
+{
+    int64_t bd[3];
+    brick_dims(1, jobs[0].g, bd);
+    int zs = std::max(64, jobs[0].g);
+    for (; zs > (staged ? 16 : 1); zs /= 2) {
+        int64_t total = 0;
+        for (int i = 0; i < njobs; ++i) {
+            const int64_t *n = jobs[i].out_n;
+            total += (n[0] + bd[0] - 1) / bd[0] * ((n[1] + bd[1] - 1) / bd[1]) * ((n[2] + zs - 1) / zs);
+        }
+        if (total >= (staged ? 32 : 8) * (int64_t)sm_count) break;
+    }
+    return zs;
+}
+
 namespace {
 
 // One launch over jobs that share (dtype, kind, g, interp); affine_box: bytes
@@ -197,20 +221,8 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
             total += jobs[i].bricks[0] * jobs[i].bricks[1] * jobs[i].bricks[2];
         }
     };
-    // TPS units walk 64 output planes (several cell layers: the staged source
-    // window is loaded once per walk); when a launch has too few units to
-    // balance, they get shorter, down to 16 planes -- below that the windows
-    // and the per-layer set-up cost more than an even last wave gives (256 x 256
-    // x 128 uint8: 109 us at 4 planes, 91 at 16; 512^3 uint16: 573 at 64, 513 at
-    // 16; 1024 x 1024 x 256 uint8, spacing 4: 2114 at 64, 2011 at 32).  Gathered
-    // units keep no window and need fewer to balance.
-    int zs = jobs[0].kind == 1 ? std::max(64, jobs[0].g) : 8;
-    count(zs);
     const bool staged = jobs[0].kind == 1 && jobs[0].tma_ok != 0, ragged = staged && jobs[0].ragged;
-    while (jobs[0].kind == 1 && zs > 16 && total < (staged ? 32 : 8) * (int64_t)ctx->sm_count) {
-        zs /= 2;
-        count(zs);
-    }
+    count(jobs[0].kind == 1 ? tps_unit_planes(jobs, njobs, staged, ctx->sm_count) : 8);
     if (total == 0) return TW_OK;
     // the units' staging plans and the list of units left to the gather kernel
     StreamBlock fb{ctx, st};

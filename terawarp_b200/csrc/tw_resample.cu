@@ -2323,8 +2323,11 @@ __global__ void __launch_bounds__(kTpsThreads, 1) k_tps_gather(const RJob *__res
     float4 *rw = Rw + (tid >> 5) * Gm::NRW;
     // a few leftover walks are cut along z, so that they do not run on as many
     // CTAs alone (65 us for the leftovers of a 999 x 501 x 301 uint8 job, 26 us
-    // in parts)
-    const int parts = fb && n < 4 * (int64_t)gridDim.x ? kGatherParts : 1;
+    // in parts), and no finer than it takes to have work for every CTA (512 walks
+    // of a 256 x 256 x 128 job under a wide field, call: 235 us in eighths, 196 in
+    // quarters)
+    int parts = 1;
+    while (fb && parts < kGatherParts && n * parts < 4 * (int64_t)gridDim.x) parts *= 2;
     for (int64_t i = blockIdx.x; i < n * parts; i += gridDim.x) {
         const int64_t k = i / parts;
         rows_gather<T, G, INTERP>(jobs, njobs, fb ? fb[1 + k] : k, (int)(i % parts), parts, W, rw, wx);
