@@ -375,6 +375,16 @@ int tw_internal_tps_unit_planes(const int64_t out_sz[3], int g, int staged, int 
     return tps_unit_planes(&j, 1, staged != 0, sm_count);
 }
 
+// Test hook, not part of the public header: how a trilinear affine warp of one
+// volume samples it: 0 gathered, 1 from boxes copied by TMA, 2 by granules.
+// Needs no GPU.
+int tw_internal_affine_path(const double M[16], int dtype, const int64_t src_sz[3], const int64_t dst_sz[3])
+{
+    RJob j = affine_job(nullptr, src_sz, nullptr, dst_sz, M, dtype, 0);
+    plan_affine_box(j, true);
+    return j.tma_ok;
+}
+
 // Test hook, not part of the public header: turns the shared-memory staging
 // of TPS resample units on (1) or off (0) for this context and returns the
 // previous setting; off, every unit gathers its taps from global memory.

@@ -99,8 +99,11 @@ int tps_unit_planes(const RJob *jobs, int njobs, bool staged, int sm_count);
 bool encode_source_map(RJob &j);
 // The staged box of an affine job's tiles: its geometry, and the descriptor
 // where TMA can describe the source; returns its bytes (a multiple of 128), 0
-// when the job has to gather.
+// when the job gathers.
 uint32_t encode_affine_box(RJob &j);
+// The same without the descriptor, on the host alone; j.tma_ok says how the box
+// would be copied.
+uint32_t plan_affine_box(RJob &j, bool can_tma);
 // Device error word bits set by the resample kernels.
 constexpr int kKernErrTimeout = 1;
 // The TMA box of the staged TPS path: source elements per staged row and rows

@@ -324,6 +324,10 @@ bool encode_source_map(RJob &j)
 
 namespace {
 
+// floor of a position for the estimates below, |q| < 8192 (no call of floor: these
+// run on every call, and 600 of them took 2 us)
+int low_int(double q) { return (int)(q + 8192.0) - 8192; }
+
 // How a warp's tap loads of a staged affine tile meet the 32 banks: floors of
 // the positions of a few of its rows (two rows of 16 lanes, a voxel pair
 // each).
@@ -337,15 +341,15 @@ struct TapRows {
             for (int l = 0; l < 32; ++l) {
                 const double p[3] = {2.0 * (l & 15), at[r][0] + (l >> 4), at[r][1]};
                 for (int a = 0; a < 3; ++a)
-                    q[r][l][a] = (int)std::floor(M[a * 4] * p[0] + M[a * 4 + 1] * p[1] + M[a * 4 + 2] * p[2] + at[r][2 + a]);
+                    q[r][l][a] = low_int(M[a * 4] * p[0] + M[a * 4 + 1] * p[1] + M[a * 4 + 2] * p[2] + at[r][2 + a]);
             }
     }
     // shared-memory passes per load, summed over the rows: the most distinct
-    // words any bank is asked for
-    int passes(int pr, int pp, int es) const
+    // words any bank is asked for (at least `limit` once the sum reaches it)
+    int passes(int pr, int pp, int es, int limit) const
     {
         int sum = 0;
-        for (int r = 0; r < kRows; ++r) {
+        for (int r = 0; r < kRows && sum < limit; ++r) {
             int word[32], depth[32] = {0}, chain[32], head[32], worst = 1;
             for (int k = 0; k < 32; ++k) head[k] = -1;
             for (int l = 0; l < 32; ++l) {
@@ -364,9 +368,95 @@ struct TapRows {
     }
 };
 
+// The part of an affine job's output tiles that have a sample inside the subject
+// volume, from 6 x 6 x 6 of them.
+double inside_part(const RJob &j)
+{
+    constexpr int N = 6;
+    // per axis of the source: the part of a position each axis of the output
+    // gives, and the limits of a tile's centre
+    double part[3][3][N], lo[3], hi[3];
+    for (int r = 0; r < 3; ++r) {
+        const double *m = j.M + 4 * r;
+        double h = 0.0;
+        for (int a = 0; a < 3; ++a) {
+            h += 0.5 * std::fabs(m[a]) * (kAffineTile[a] - 1);
+            for (int i = 0; i < N; ++i)
+                part[r][a][i] = m[a] * ((double)j.out_o[a] + (i + 0.5) / N * (double)j.out_n[a]) + (a == 0 ? m[3] : 0.0);
+        }
+        lo[r] = -h;
+        hi[r] = (double)(j.glob[r] - 1) + h;
+    }
+    int n = 0;
+    for (int z = 0; z < N; ++z)
+        for (int y = 0; y < N; ++y) {
+            double yz[3];
+            for (int r = 0; r < 3; ++r) yz[r] = part[r][1][y] + part[r][2][z];
+            for (int x = 0; x < N; ++x) {
+                bool in = true;
+                for (int r = 0; r < 3; ++r) {
+                    const double q = yz[r] + part[r][0][x];
+                    in = in & (q >= lo[r]) & (q <= hi[r]);
+                }
+                n += in;
+            }
+        }
+    return (double)n / (N * N * N);
+}
+
+// Is an affine job faster staged than gathered?  Both are estimated in cycles per
+// 64 voxels and SM, fitted to 2,200 timings: scales of 0.3 to 4 along some or all
+// axes, rotations, both, uint8 and uint16, rows of whole 16 bytes or not, sources
+// of 4 M to 0.5 G elements, 5 to 100 % of the output inside.  Gathered, a sample
+// costs by the 32-byte sectors of a row's tap loads, more where rows run along
+// source planes, and by the source bytes it consumes; one outside the source
+// costs the same whatever the matrix.  Staged, a sample costs by the bytes of the
+// box, dearer by granules, and with two or more stages also by its bank passes.
+// us gathered and staged at 1021 x 1019 x 509, by granules: reduction by 2 of
+// uint16 399 and 939, by 2.25 of uint8 249 and 567, no rotation, uint16, 2255 and
+// 2682, 15 degrees about each axis, uint16, 4980 and 3643; at 1024 x 1024 x 512,
+// by TMA: 396 and 366, 246 and 303, 2217 and 1500, 4967 and 1544; 512 x 512 x 256
+// uint16, a quarter turn about y and a reduction by 2, an eighth of the output
+// inside: 626 and 1205.  The factors lean towards staging where the estimates
+// meet.  Over the timings the choice costs 0.4 % over the faster one (staged
+// always: 7 %, up to 2.5 times).
+bool staging_pays(const RJob &j, bool tma, bool one_stage, double bytes, double passes)
+{
+    const int es = j.dtype == TW_U8 ? 1 : 2;
+    const double *M = j.M;
+    const double at[3][3] = {{.3, .6, .1}, {.7, .1, .5}, {.5, .9, .95}};
+    int sectors = 0;  // of three rows' loads, where a lane's is not the one before its
+    for (const auto &o : at) {
+        int64_t last = INT64_MIN;
+        for (int l = 0; l < 32; ++l) {
+            const int64_t q[3] = {low_int(M[0] * 2 * l + o[0]), low_int(M[4] * 2 * l + o[1]), low_int(M[8] * 2 * l + o[2])};
+            const int64_t s = ((q[2] * j.src_pz + q[1] * j.src_py + q[0]) * es) >> 5;
+            sectors += s != last;
+            last = s;
+        }
+    }
+    const double S = sectors / 3.0;
+    const double det = std::fabs(M[0] * (M[5] * M[10] - M[6] * M[9]) - M[1] * (M[4] * M[10] - M[6] * M[8]) +
+                                 M[2] * (M[4] * M[9] - M[5] * M[8]));
+    const double yz = std::fabs(M[9]) / (std::fabs(M[5]) + std::fabs(M[9]) + 1e-9);
+    const double xz = std::fabs(M[8]) / (std::fabs(M[0]) + std::fabs(M[4]) + std::fabs(M[8]) + 1e-9);
+    // (a sector per lane: 150 to 1160 cycles)
+    const double inside = S > 28.0 ? 400.0
+                                   : 54 + 2.8 * std::min(S, 16.0) + 7 * std::max(S - 16, 0.0) + 26 * yz + 100 * xz +
+                                         .037 * 64 * es * det;
+    const double f = inside_part(j), gathered = f * inside + (1 - f) * 115;
+    if (!tma) {  // (granules from a source that stays in L2 cost less)
+        const bool in_l2 = (double)j.src_pz * (double)j.src_n[2] * es < 100e6;
+        return 50 + .122 * bytes * (.3 + .7 * f) <= (in_l2 ? 1.2 : 1.1) * gathered;
+    }
+    const double staged = one_stage ? (es == 1 ? 70 : 62) + .0345 * bytes * (.8 + .2 * f) + 15 * std::max(passes - 3, 0.0)
+                                    : 33 + 10.3 * passes + .009 * bytes;
+    return staged <= 1.05 * gathered;
+}
+
 }  // namespace
 
-uint32_t encode_affine_box(RJob &j)
+uint32_t plan_affine_box(RJob &j, bool can_tma)
 {
     j.tma_ok = 0;
     const int es = j.dtype == TW_U8 ? 1 : 2;
@@ -400,9 +490,8 @@ uint32_t encode_affine_box(RJob &j)
     // passes -- unpadded, some matrices put most lanes in a few banks (8.8
     // passes at 10 degrees about each axis with rows of 1034 bytes, 16 at a
     // quarter turn about z).
-    const EncodeTiled fn = encode_fn();
     const int A = 16 / es, w1 = (box[0] + A - 1 + A - 1) / A * A;  // starts on a 16-byte boundary
-    const bool tma = fn && (j.src_py * es) % 16 == 0 && (j.src_pz * es) % 16 == 0 && w1 + A <= std::min<int64_t>(256, j.src_n[0]) &&
+    const bool tma = can_tma && (j.src_py * es) % 16 == 0 && (j.src_pz * es) % 16 == 0 && w1 + A <= std::min<int64_t>(256, j.src_n[0]) &&
                      box[1] + 7 <= j.src_n[1] && box[2] <= j.src_n[2] && (uint64_t)j.src_pz * es < (1ull << 40);
     const int dy = (int)((j.src_py * es) & 15), dz = (int)((j.src_pz * es) & 15);
     const TapRows rows(j.M);
@@ -424,7 +513,7 @@ uint32_t encode_affine_box(RJob &j)
         const int64_t need = ((int64_t)pp * box[2] + 32 + 127) / 128 * 128;
         if (need > kAffineSmem) continue;
         if (bytes && 2 * bytes <= kAffineSmem && 2 * need > kAffineSmem) continue;  // two stages are worth more
-        const int p = rows.passes(pr, pp, es);
+        const int p = rows.passes(pr, pp, es, best);
         if (p >= best) continue;
         best = p;
         bytes = need;
@@ -437,8 +526,20 @@ uint32_t encode_affine_box(RJob &j)
     // the box fits, and tap offsets and their partial sums (floating point,
     // exact below 2^22) stay small
     if (!bytes || reach[2] * j.st_pp + reach[1] * j.st_pr + reach[0] * es > 2097152.0) return 0;
-    j.tma_ok = 2;
-    if (tma) {
+    const double copied = (double)(tma ? j.st_pp : (box[0] * es + 30) / 16 * 16 * box[1]) * box[2];
+    const double passes = (double)best / TapRows::kRows;
+    if (!staging_pays(j, tma, 2 * bytes > kAffineSmem, copied / (kAffineTile[0] * kAffineTile[1] * kAffineTile[2] / 64), passes))
+        return 0;
+    j.tma_ok = tma ? 1 : 2;
+    return (uint32_t)bytes;
+}
+
+uint32_t encode_affine_box(RJob &j)
+{
+    const EncodeTiled fn = encode_fn();
+    const uint32_t bytes = plan_affine_box(j, fn != nullptr);
+    if (j.tma_ok == 1) {
+        const int es = j.dtype == TW_U8 ? 1 : 2;
         const cuuint64_t dims[3] = {(cuuint64_t)j.src_n[0], (cuuint64_t)j.src_n[1], (cuuint64_t)j.src_n[2]};
         const cuuint64_t strides[2] = {(cuuint64_t)j.src_py * es, (cuuint64_t)j.src_pz * es};
         const cuuint32_t b[3] = {(cuuint32_t)j.st_w, (cuuint32_t)j.st_h, (cuuint32_t)j.st_d};
@@ -449,9 +550,8 @@ uint32_t encode_affine_box(RJob &j)
             j.tma_ok = 0;
             return 0;
         }
-        j.tma_ok = 1;
     }
-    return (uint32_t)bytes;
+    return bytes;
 }
 
 // ------------------------------------------------------------ sample hulls
