@@ -101,15 +101,13 @@ tw_status upload(tw_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStre
     return TW_OK;
 }
 
+// Waits for the context's stream, then looks at the error word (in host memory:
+// reading a device word back took 8 us of every call).
 tw_status check_kernel_errors(tw_ctx *ctx)
 {
-    if (!ctx->d_err) return TW_OK;
-    int h = 0;
-    TW_CUDA_TRY(cudaMemcpyAsync(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     TW_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (h == 0) return TW_OK;
-    TW_CUDA_TRY(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-    TW_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (!ctx->err_word || __atomic_load_n(ctx->err_word, __ATOMIC_ACQUIRE) == 0) return TW_OK;
+    __atomic_store_n(ctx->err_word, 0, __ATOMIC_RELEASE);
     return fail(ctx, TW_ERR_TIMEOUT, "a resample kernel gave up waiting for a staged source plane");
 }
 
@@ -289,8 +287,8 @@ tw_status tw_ctx_create(int device, size_t hbm_budget_bytes, tw_ctx **out)
             return destroy_partial(c.release());
     if (cudaMallocHost((void **)&c->stage_h, tw_ctx::kStageBytes * tw_ctx::kStageSlots) != cudaSuccess)
         return destroy_partial(c.release());
-    if (cudaMalloc((void **)&c->d_err, 256) != cudaSuccess || cudaMemset(c->d_err, 0, 256) != cudaSuccess)
-        return destroy_partial(c.release());
+    if (cudaHostAlloc((void **)&c->err_word, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return destroy_partial(c.release());
+    *c->err_word = 0;
     for (int s = 0; s < tw_ctx::kStageSlots; ++s)
         if (cudaEventCreateWithFlags(&c->stage_ev[s], cudaEventDisableTiming) != cudaSuccess)
             return destroy_partial(c.release());
@@ -316,7 +314,7 @@ tw_status tw_ctx_destroy(tw_ctx *ctx)
     for (int s = 0; s < tw_ctx::kStageSlots; ++s)
         if (ctx->stage_ev[s]) cudaEventDestroy(ctx->stage_ev[s]);
     if (ctx->stage_h) cudaFreeHost(ctx->stage_h);
-    if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->err_word) cudaFreeHost(ctx->err_word);
     delete ctx;
     return TW_OK;
 }
@@ -392,6 +390,16 @@ int tw_internal_set_resample_staging(tw_ctx *ctx, int on)
 {
     if (!ctx) return 0;
     return ctx->resample_staging.exchange(on ? 1 : 0);
+}
+
+// Test hook, not part of the public header: sets the context's error word from
+// a kernel on its stream, as a resample kernel whose wait ran out does.
+tw_status tw_internal_raise_kernel_error(tw_ctx *ctx)
+{
+    if (!ctx) return TW_ERR_ARG;
+    TW_CUDA_TRY(cudaSetDevice(ctx->device));
+    TW_CUDA_TRY(launch_raise_error(ctx->err_word, ctx->stream));
+    return TW_OK;
 }
 
 int64_t tw_grid_size(int64_t sz, int g) { return g > 0 && sz > 0 ? grid_size(sz, g) : -1; }

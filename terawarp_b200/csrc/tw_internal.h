@@ -71,7 +71,7 @@ struct alignas(128) RJob {
 // Launch one resample pass over `njobs` jobs that share (dtype, kind, g).
 // jobs_dev is device memory holding the RJob array; total_bricks is the sum
 // of all jobs' bricks.  Returns a cudaError_t from the launch.
-// err: device word the kernel ORs a failure code into (a bounded wait that
+// err: word the kernel ORs a failure code into (a bounded wait that
 // gave up); may be null.  stage_ws: for trilinear TPS, device memory of
 // tps_stage_ws_bytes(total_bricks) whose first 8 bytes are zero: the units
 // are planned, staged units run the TMA-staged kernel and the rest the
@@ -104,8 +104,9 @@ uint32_t encode_affine_box(RJob &j);
 // The same without the descriptor, on the host alone; j.tma_ok says how the box
 // would be copied.
 uint32_t plan_affine_box(RJob &j, bool can_tma);
-// Device error word bits set by the resample kernels.
+// Error word bits set by the resample kernels.
 constexpr int kKernErrTimeout = 1;
+cudaError_t launch_raise_error(int *err, cudaStream_t st);  // sets it (a test's)
 // The TMA box of the staged TPS path: source elements per staged row and rows
 // per staged plane (the staged box of a unit is at most this large).  A row
 // of 128 elements keeps the row pitch in shared memory a multiple of 32
@@ -209,7 +210,7 @@ struct tw_ctx {
     int stage_next = 0;
     std::atomic<uint64_t> launches{0};
     std::atomic<uint64_t> h2d_bytes{0}, d2h_bytes{0};  // streamed by the slab and tile paths
-    int *d_err = nullptr;               // device word: kernels OR failure bits into it (kKernErrTimeout)
+    int *err_word = nullptr;            // pinned host word: kernels OR failure bits into it (kKernErrTimeout)
     // how long a CTA of the cooperative solve waits at a grid barrier before
     // it gives up (TW_ERR_TIMEOUT); tests shorten it through
     // tw_internal_set_solve_barrier_ns
@@ -251,7 +252,7 @@ void dfree_on(tw_ctx *ctx, void *p, size_t bytes, cudaStream_t st);
 // copies larger than a staging slot fall back to a pageable copy.
 tw_status upload(tw_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st);
 inline void count_launch(tw_ctx *ctx, uint64_t k = 1) { if (ctx) ctx->launches += k; }
-// Reads and clears the context's device error word (call after the work that
+// Reads and clears the context's error word (call after the work that
 // may have set it has completed); TW_ERR_TIMEOUT when a kernel gave up on a
 // bounded wait.
 tw_status check_kernel_errors(tw_ctx *ctx);

@@ -235,9 +235,9 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
     // plan, walk lists, staged (interior walks), staged (other walks), gather
     const uint64_t launches = staged ? 5 : 1;
     const auto launch = [&](const RJob *d) {
-        return affine_box ? launch_affine_staged(d, njobs, total, jobs[0].dtype, affine_box, st, ctx->sm_count, ctx->d_err)
+        return affine_box ? launch_affine_staged(d, njobs, total, jobs[0].dtype, affine_box, st, ctx->sm_count, ctx->err_word)
                           : launch_resample(d, njobs, total, jobs[0].dtype, jobs[0].kind, jobs[0].g, jobs[0].interp, st,
-                                            ctx->sm_count, ctx->d_err, d_fb, ragged);
+                                            ctx->sm_count, ctx->err_word, d_fb, ragged);
     };
     const size_t bytes = sizeof(RJob) * (size_t)njobs;
     if (njobs <= tw_ctx::kJobsPerSlot && ctx->job_d) {

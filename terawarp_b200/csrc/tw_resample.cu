@@ -2475,6 +2475,16 @@ cudaError_t launch_repitch(const RJob &j, void *dst, int64_t row_bytes, cudaStre
     return cudaGetLastError();
 }
 
+namespace {
+__global__ void k_raise_error(int *err) { atomicOr(err, kKernErrTimeout); }
+}  // namespace
+
+cudaError_t launch_raise_error(int *err, cudaStream_t st)
+{
+    k_raise_error<<<1, 1, 0, st>>>(err);
+    return cudaGetLastError();
+}
+
 bool g_supported(int g) { return g == 4 || g == 8 || g == 16 || g == 32 || g == 64; }
 
 void brick_dims(int kind, int g, int64_t out[3])
