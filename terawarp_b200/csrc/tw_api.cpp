@@ -24,6 +24,20 @@ tw_status fail(const tw_ctx *ctx, tw_status code, const std::string &msg)
     return code;
 }
 
+static const char kAllocText[] = "device allocation";
+
+ErrorText::ErrorText(tw_ctx *c) : ctx(c)
+{
+    std::lock_guard<std::mutex> lk(ctx->err_mu);
+    was = ctx->last_error;
+}
+
+void ErrorText::put_back()
+{
+    std::lock_guard<std::mutex> lk(ctx->err_mu);
+    if (ctx->last_error.compare(0, sizeof(kAllocText) - 1, kAllocText) == 0) ctx->last_error = was;
+}
+
 tw_status dmalloc(tw_ctx *ctx, void **p, size_t bytes)
 {
     *p = nullptr;
@@ -31,7 +45,7 @@ tw_status dmalloc(tw_ctx *ctx, void **p, size_t bytes)
     size_t prev = ctx->used.fetch_add(bytes);
     if (prev + bytes > ctx->budget) {
         ctx->used.fetch_sub(bytes);
-        return fail(ctx, TW_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes exceeds the HBM budget");
+        return fail(ctx, TW_ERR_OOM, std::string(kAllocText) + " of " + std::to_string(bytes) + " bytes exceeds the HBM budget");
     }
     // stream-ordered allocation from the context's pool on its compute
     // stream, made visible to every stream of the context before returning
@@ -41,7 +55,7 @@ tw_status dmalloc(tw_ctx *ctx, void **p, size_t bytes)
         ctx->used.fetch_sub(bytes);
         *p = nullptr;
         cudaGetLastError();
-        return fail(ctx, TW_ERR_OOM, std::string("device allocation: ") + cudaGetErrorString(e));
+        return fail(ctx, TW_ERR_OOM, std::string(kAllocText) + ": " + cudaGetErrorString(e));
     }
     return TW_OK;
 }
@@ -64,14 +78,14 @@ tw_status dmalloc_on(tw_ctx *ctx, void **p, size_t bytes, cudaStream_t st)
     size_t prev = ctx->used.fetch_add(bytes);
     if (prev + bytes > ctx->budget) {
         ctx->used.fetch_sub(bytes);
-        return fail(ctx, TW_ERR_OOM, "device allocation of " + std::to_string(bytes) + " bytes exceeds the HBM budget");
+        return fail(ctx, TW_ERR_OOM, std::string(kAllocText) + " of " + std::to_string(bytes) + " bytes exceeds the HBM budget");
     }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
     if (e != cudaSuccess) {
         ctx->used.fetch_sub(bytes);
         *p = nullptr;
         cudaGetLastError();
-        return fail(ctx, TW_ERR_OOM, std::string("device allocation: ") + cudaGetErrorString(e));
+        return fail(ctx, TW_ERR_OOM, std::string(kAllocText) + ": " + cudaGetErrorString(e));
     }
     return TW_OK;
 }

@@ -251,6 +251,14 @@ void dfree_on(tw_ctx *ctx, void *p, size_t bytes, cudaStream_t st);
 // the host does not wait for earlier work on `st` (a pageable copy would);
 // copies larger than a staging slot fall back to a pageable copy.
 tw_status upload(tw_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st);
+// The context's error text as it was when this was made, to put back when an
+// allocation failed after that and the call went on without it.
+struct ErrorText {
+    tw_ctx *ctx;
+    std::string was;
+    explicit ErrorText(tw_ctx *c);
+    void put_back();
+};
 inline void count_launch(tw_ctx *ctx, uint64_t k = 1) { if (ctx) ctx->launches += k; }
 // Reads and clears the context's error word (call after the work that
 // may have set it has completed); TW_ERR_TIMEOUT when a kernel gave up on a

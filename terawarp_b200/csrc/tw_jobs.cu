@@ -109,7 +109,12 @@ RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaSt
         vox += out;
         return true;
     });
-    if (last == first || vox < kMinVoxels || dmalloc_on(ctx, &copy.p, bytes, st) != TW_OK) return first;
+    if (last == first || vox < kMinVoxels) return first;
+    ErrorText text(ctx);
+    if (dmalloc_on(ctx, &copy.p, bytes, st) != TW_OK) {
+        text.put_back();
+        return first;
+    }
     copy.bytes = bytes;
     unsigned char *to = static_cast<unsigned char *>(copy.p);
     for (RJob *j = first; j < last; ++j) {
@@ -149,8 +154,10 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
         RJob *const mid = std::stable_partition(jobs, end, [](RJob &j) { return encode_source_map(j); });
         const auto run_tps = [&](RJob *b, RJob *e, bool gathers) -> tw_status {
             if (e == b) return TW_OK;
+            ErrorText text(ctx);
             tw_status s = run_group(ctx, b, (int)(e - b), 0, st);
             if (s == TW_ERR_OOM && gathers) {  // no room for the plans: gathering needs none
+                text.put_back();
                 for (RJob *j = b; j < e; ++j) j->tma_ok = 0;
                 s = run_group(ctx, b, (int)(e - b), 0, st);
             }
@@ -787,9 +794,11 @@ tw_status stream_slabs(tw_ctx *ctx, const SlabIO &io,
     if (src_dev && dst_dev) {
         // nothing to stream: the whole volume in one launch; in slabs only
         // when its workspace does not fit the budget
+        ErrorText text(ctx);
         const tw_status s = compute(0, io.dst_planes, io.src, io.dst, ctx->stream);
         if (s == TW_OK) return check_kernel_errors(ctx);
         if (s != TW_ERR_OOM) return s;
+        text.put_back();
     }
     const bool src_pin = !src_dev && is_pinned_ptr(io.src), dst_pin = !dst_dev && is_pinned_ptr(io.dst);
     const size_t src_bytes = io.src_plane_bytes * (size_t)io.src_planes;
