@@ -61,6 +61,7 @@ struct alignas(128) RJob {
     int tma_ok;            // units may stage their source footprint in shared memory: 1 through tmap, 2
                            // (affine) by granules
     int ragged;            // TPS: src is a copy with padded rows of a source TMA cannot describe
+    int arriving;          // the source may still be arriving from the host past what the job reads
     int st_w, st_h, st_d;  // affine: staged box, elements (row by row) or the TMA box
     int st_pr, st_pp;      // affine: its row and plane pitch in shared memory, bytes
     int dtype;             // 1 u8, 2 u16

@@ -103,6 +103,7 @@ RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaSt
     const auto size = [&](const RJob &j) { return (row_bytes(j) * (size_t)(j.src_n[1] * j.src_n[2]) + 255) / 256 * 256; };
     RJob *const last = std::stable_partition(first, end, [&](const RJob &j) {
         const int64_t out = j.out_n[0] * j.out_n[1] * j.out_n[2];
+        if (j.arriving) return false;  // (the copy would read all of it)
         if (j.src_n[0] < kStageBoxW || j.src_n[1] < kStageBoxH || j.src_n[2] < 2 || bytes + size(j) > kMostBytes) return false;
         if (2 * out < j.src_n[0] * j.src_n[1] * j.src_n[2]) return false;  // (a slab: the copy takes the whole source)
         bytes += size(j);

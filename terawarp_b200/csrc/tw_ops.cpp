@@ -46,7 +46,8 @@ tw_status tps_warp_volume(tw_ctx *ctx, const float4 *nodes, int g, int dtype, in
 {
     const int64_t gsz[3] = {grid_size(dst_sz[0], g), grid_size(dst_sz[1], g), grid_size(dst_sz[2], g)};
     std::vector<float> zmin, zmax;
-    if (!is_device_ptr(src)) TW_TRY(tps_layer_zhull(ctx, nodes, gsz, g, ctx->stream, zmin, zmax));
+    const bool from_host = !is_device_ptr(src);
+    if (from_host) TW_TRY(tps_layer_zhull(ctx, nodes, gsz, g, ctx->stream, zmin, zmax));
     const size_t es = elem_size(dtype);
     SlabIO io;
     io.src = src;
@@ -67,6 +68,7 @@ tw_status tps_warp_volume(tw_ctx *ctx, const float4 *nodes, int g, int dtype, in
     };
     auto compute = [&](int64_t z0, int64_t z1, const void *d_src, void *d_dst, cudaStream_t st) -> tw_status {
         RJob j = tps_job(d_src, src_sz, d_dst, dst_sz, nodes, g, dtype, interp);
+        j.arriving = from_host;
         j.out_o[2] = z0;
         j.out_n[2] = z1 - z0;
         j.dst = static_cast<char *>(d_dst) + (size_t)z0 * io.dst_plane_bytes;
