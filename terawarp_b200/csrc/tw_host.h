@@ -25,9 +25,12 @@ RJob tps_job(const void *src, const int64_t src_sz[3], void *dst, const int64_t 
              int dtype, int interp);
 RJob affine_job(const void *src, const int64_t src_sz[3], void *dst, const int64_t dst_sz[3], const double M[16],
                 int dtype, int interp);
-// Launches the jobs (all sharing dtype, kind, g, interp) in one persistent
-// resample launch on `st`.  Fills brick counts and prefix sums.
-tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st);
+// Launches the jobs (all sharing dtype, kind, g, interp) on `st`, those that are
+// sampled the same way together; orders them so and fills brick counts and prefix
+// sums.  Sources are copied into padded rows up to copy_limit bytes; *copied: the
+// bytes that were.
+tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st, size_t copy_limit = SIZE_MAX,
+                   size_t *copied = nullptr);
 
 // Per output cell-layer z hull of the TPS sample positions: for layer cz
 // (output z in [cz*g, (cz+1)*g)), zmin/zmax of q_z.  Host vectors of size

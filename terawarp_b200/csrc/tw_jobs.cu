@@ -93,10 +93,10 @@ tw_status run_group(tw_ctx *ctx, RJob *jobs, int njobs, uint32_t affine_box, cud
 // 389 x 203 uint16: 367 us gathered, 370 copied and staged; 801 x 601 x 301:
 // 1091 and 850), and the copies are held to 256 MiB, which the context's pool
 // then keeps, and to what the budget has left.
-RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaStream_t st)
+RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaStream_t st, size_t most)
 {
     constexpr int64_t kMinVoxels = 48 << 20;
-    constexpr size_t kMostBytes = (size_t)256 << 20;
+    const size_t most_bytes = std::min((size_t)256 << 20, most);
     int64_t vox = 0;
     size_t bytes = 0;
     const auto row_bytes = [](const RJob &j) { return (size_t)((j.src_n[0] * (j.dtype == TW_U8 ? 1 : 2) + 15) / 16 * 16); };
@@ -104,7 +104,7 @@ RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaSt
     RJob *const last = std::stable_partition(first, end, [&](const RJob &j) {
         const int64_t out = j.out_n[0] * j.out_n[1] * j.out_n[2];
         if (j.arriving) return false;  // (the copy would read all of it)
-        if (j.src_n[0] < kStageBoxW || j.src_n[1] < kStageBoxH || j.src_n[2] < 2 || bytes + size(j) > kMostBytes) return false;
+        if (j.src_n[0] < kStageBoxW || j.src_n[1] < kStageBoxH || j.src_n[2] < 2 || bytes + size(j) > most_bytes) return false;
         if (2 * out < j.src_n[0] * j.src_n[1] * j.src_n[2]) return false;  // (a slab: the copy takes the whole source)
         bytes += size(j);
         vox += out;
@@ -137,8 +137,9 @@ RJob *pad_sources(tw_ctx *ctx, RJob *first, RJob *end, StreamBlock &copy, cudaSt
 
 }  // namespace
 
-tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
+tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st, size_t copy_limit, size_t *copied)
 {
+    if (copied) *copied = 0;
     if (njobs <= 0) return TW_OK;
     const bool staging = ctx->resample_staging.load() != 0;
     if (jobs[0].kind == 1) {
@@ -166,7 +167,8 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st)
         };
         TW_TRY(run_tps(jobs, mid, nearest));
         StreamBlock copy{ctx, st};
-        RJob *const last = jobs[0].interp == 0 ? pad_sources(ctx, mid, end, copy, st) : mid;
+        RJob *const last = jobs[0].interp == 0 ? pad_sources(ctx, mid, end, copy, st, copy_limit) : mid;
+        if (copied) *copied = copy.bytes;
         TW_TRY(run_tps(mid, last, true));
         if (end > last) TW_TRY(run_group(ctx, last, (int)(end - last), 0, st));
         return TW_OK;

@@ -230,7 +230,20 @@ tw_status batch_round(tw_server *s, std::vector<JobRec *> &ready)
             else
                 rj.push_back(affine_job(j->d_src, sp.src_sz, j->d_dst, sp.dst_sz, sp.M, sp.dtype, sp.interp));
         }
-        TW_TRY(run_jobs(ctx, rj.data(), (int)rj.size(), s->batch));
+        // padded copies of ragged sources fit in what the budget has left, and
+        // count against it until the group's first job is finished
+        size_t left = 0, copied = 0;
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            left = s->budget > s->used ? s->budget - s->used : 0;
+        }
+        const tw_status st = run_jobs(ctx, rj.data(), (int)rj.size(), s->batch, left, &copied);
+        if (copied) {
+            std::lock_guard<std::mutex> lk(s->mu);
+            s->used += copied;
+            kv.second.front()->reserve += copied;
+        }
+        TW_TRY(st);
         // each job's stream continues after its own resample-end event, so a
         // job's completion is never stamped before the end of its resample
         for (JobRec *j : kv.second) TW_CUDA_TRY(cudaEventRecord(j->ev[JobRec::kRs1], s->batch));
