@@ -1588,6 +1588,16 @@ __device__ void rows_gather(const RJob *__restrict__ jobs, int njobs, int64_t u,
 
 constexpr int kABY = 8, kABZ = 8;
 
+// Position along axis r of the origin O of a brick, FP64, in the order the
+// gathered and the staged path share (written out, so that both round alike
+// however the compiler would contract it).
+__device__ __forceinline__ double affine_origin(const RJob &J, int r, const int64_t (&O)[3])
+{
+    return __dadd_rn(__fma_rn(J.M[r * 4 + 2], (double)O[2],
+                              __fma_rn(J.M[r * 4 + 0], (double)O[0], __dmul_rn(J.M[r * 4 + 1], (double)O[1]))),
+                     J.M[r * 4 + 3]);
+}
+
 // Rows of an affine brick with the same lane-pair layout as the TPS path:
 // lane l owns voxels (x, x+1), x = 2l + 64k; q = fo + M_lin l in FP32.
 template <typename T, int INTERP, bool FAST>
@@ -1601,9 +1611,9 @@ __device__ __forceinline__ void affine_rows(const float (&m)[3][3], const float 
         if (z >= ze) break;
         const int y = ty;
         if (y >= ye) continue;
-        const float bx0 = fo[0] + m[0][1] * (float)y + m[0][2] * (float)z;
-        const float by0 = fo[1] + m[1][1] * (float)y + m[1][2] * (float)z;
-        const float bz0 = fo[2] + m[2][1] * (float)y + m[2][2] * (float)z;
+        const float bx0 = fmaf(m[0][2], (float)z, fmaf(m[0][1], (float)y, fo[0]));
+        const float by0 = fmaf(m[1][2], (float)z, fmaf(m[1][1], (float)y, fo[1]));
+        const float bz0 = fmaf(m[2][2], (float)z, fmaf(m[2][1], (float)y, fo[2]));
         T *drow = dbrick + (int64_t)z * dpz + (int64_t)y * dpy;
 #pragma unroll
         for (int k = 0; k < kBX / 64; ++k) {
@@ -1655,8 +1665,7 @@ __device__ void affine_brick(const RJob &J, int64_t bx, int64_t by, int64_t bz, 
     // q(O + l) = M (O + l) = qO + Mlin l  (FP64 at the origin, FP32 increments)
     double qO[3];
     for (int r = 0; r < 3; ++r)
-        qO[r] = J.M[r * 4 + 0] * (double)O[0] + J.M[r * 4 + 1] * (double)O[1] + J.M[r * 4 + 2] * (double)O[2] +
-                J.M[r * 4 + 3];
+        qO[r] = affine_origin(J, r, O);
     // hull over the brick corners, relative to floor(qO)
     int64_t qf[3];
     float fo[3];
@@ -1869,9 +1878,8 @@ __device__ __forceinline__ void affine_tile_setup(const RJob &J, int64_t lb, ATi
         float mn[3], mx[3];
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-            // the brick's origin and hull as affine_brick computes them
-            const double q = fma(J.M[r * 4 + 2], (double)O[2],
-                                 fma(J.M[r * 4 + 0], (double)O[0], __dmul_rn(J.M[r * 4 + 1], (double)O[1]))) + J.M[r * 4 + 3];
+            // the brick's origin and hull (which only says whether clamps apply)
+            const double q = affine_origin(J, r, O);
             const double f = floor(q);
             qf[r] = (int64_t)f;
             F.fo[r] = (float)(q - f);
