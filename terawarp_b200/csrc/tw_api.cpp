@@ -393,17 +393,19 @@ int tw_internal_tps_unit_planes(const int64_t out_sz[3], int g, int staged, int 
 int tw_internal_affine_path(const double M[16], int dtype, const int64_t src_sz[3], const int64_t dst_sz[3])
 {
     RJob j = affine_job(nullptr, src_sz, nullptr, dst_sz, M, dtype, 0);
-    plan_affine_box(j, true);
+    plan_affine_box(j, true, false);
     return j.tma_ok;
 }
 
-// Test hook, not part of the public header: turns the shared-memory staging
-// of TPS resample units on (1) or off (0) for this context and returns the
-// previous setting; off, every unit gathers its taps from global memory.
+// Test hook, not part of the public header: turns the shared-memory staging of
+// resample units on (1) or off (0) for this context and returns the previous
+// setting; off, every unit gathers its taps from global memory.  2: affine jobs
+// are staged whenever their box fits, also where gathering is estimated to be
+// faster.
 int tw_internal_set_resample_staging(tw_ctx *ctx, int on)
 {
     if (!ctx) return 0;
-    return ctx->resample_staging.exchange(on ? 1 : 0);
+    return ctx->resample_staging.exchange(on == 2 ? 2 : on ? 1 : 0);
 }
 
 // Test hook, not part of the public header: sets the context's error word from

@@ -100,11 +100,12 @@ int tps_unit_planes(const RJob *jobs, int njobs, bool staged, int sm_count);
 bool encode_source_map(RJob &j);
 // The staged box of an affine job's tiles: its geometry, and the descriptor
 // where TMA can describe the source; returns its bytes (a multiple of 128), 0
-// when the job gathers.
-uint32_t encode_affine_box(RJob &j);
+// when the job gathers: its box does not fit, or (unless `always`) gathering is
+// estimated to be faster.
+uint32_t encode_affine_box(RJob &j, bool always);
 // The same without the descriptor, on the host alone; j.tma_ok says how the box
 // would be copied.
-uint32_t plan_affine_box(RJob &j, bool can_tma);
+uint32_t plan_affine_box(RJob &j, bool can_tma, bool always);
 // Error word bits set by the resample kernels.
 constexpr int kKernErrTimeout = 1;
 cudaError_t launch_raise_error(int *err, cudaStream_t st);  // sets it (a test's)

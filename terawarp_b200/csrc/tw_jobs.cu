@@ -141,7 +141,7 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st, size_t c
 {
     if (copied) *copied = 0;
     if (njobs <= 0) return TW_OK;
-    const bool staging = ctx->resample_staging.load() != 0;
+    const int staging = ctx->resample_staging.load();
     if (jobs[0].kind == 1) {
         // TPS jobs: those whose source TMA can describe, trilinear ones that
         // are resampled from a padded copy, and the rest, which gather
@@ -176,7 +176,7 @@ tw_status run_jobs(tw_ctx *ctx, RJob *jobs, int njobs, cudaStream_t st, size_t c
     // affine jobs whose tiles can be staged first, the others gather
     uint32_t box = 0;
     RJob *const mid = std::stable_partition(jobs, jobs + njobs, [&](RJob &j) {
-        const uint32_t b = staging ? encode_affine_box(j) : 0u;
+        const uint32_t b = staging ? encode_affine_box(j, staging == 2) : 0u;
         box = std::max(box, b);
         return b != 0;
     });
@@ -466,7 +466,7 @@ bool staging_pays(const RJob &j, bool tma, bool one_stage, double bytes, double 
 
 }  // namespace
 
-uint32_t plan_affine_box(RJob &j, bool can_tma)
+uint32_t plan_affine_box(RJob &j, bool can_tma, bool always)
 {
     j.tma_ok = 0;
     const int es = j.dtype == TW_U8 ? 1 : 2;
@@ -538,16 +538,16 @@ uint32_t plan_affine_box(RJob &j, bool can_tma)
     if (!bytes || reach[2] * j.st_pp + reach[1] * j.st_pr + reach[0] * es > 2097152.0) return 0;
     const double copied = (double)(tma ? j.st_pp : (box[0] * es + 30) / 16 * 16 * box[1]) * box[2];
     const double passes = (double)best / TapRows::kRows;
-    if (!staging_pays(j, tma, 2 * bytes > kAffineSmem, copied / (kAffineTile[0] * kAffineTile[1] * kAffineTile[2] / 64), passes))
-        return 0;
+    const double voxels64 = kAffineTile[0] * kAffineTile[1] * kAffineTile[2] / 64;
+    if (!always && !staging_pays(j, tma, 2 * bytes > kAffineSmem, copied / voxels64, passes)) return 0;
     j.tma_ok = tma ? 1 : 2;
     return (uint32_t)bytes;
 }
 
-uint32_t encode_affine_box(RJob &j)
+uint32_t encode_affine_box(RJob &j, bool always)
 {
     const EncodeTiled fn = encode_fn();
-    const uint32_t bytes = plan_affine_box(j, fn != nullptr);
+    const uint32_t bytes = plan_affine_box(j, fn != nullptr, always);
     if (j.tma_ok == 1) {
         const int es = j.dtype == TW_U8 ? 1 : 2;
         const cuuint64_t dims[3] = {(cuuint64_t)j.src_n[0], (cuuint64_t)j.src_n[1], (cuuint64_t)j.src_n[2]};
