@@ -100,7 +100,7 @@ void dfree_on(tw_ctx *ctx, void *p, size_t bytes, cudaStream_t st)
 tw_status upload(tw_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t st)
 {
     if (bytes == 0) return TW_OK;
-    if (bytes > tw_ctx::kStageBytes || !ctx->stage_h) {
+    if (bytes > tw_ctx::kStageMost || !ctx->stage_h) {
         TW_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         return TW_OK;
     }
@@ -301,7 +301,7 @@ tw_status tw_ctx_create(int device, size_t hbm_budget_bytes, tw_ctx **out)
             return destroy_partial(c.release());
     if (cudaMallocHost((void **)&c->stage_h, tw_ctx::kStageBytes * tw_ctx::kStageSlots) != cudaSuccess)
         return destroy_partial(c.release());
-    if (cudaHostAlloc((void **)&c->err_word, sizeof(int), cudaHostAllocMapped) != cudaSuccess) return destroy_partial(c.release());
+    c->err_word = reinterpret_cast<int *>(c->stage_h + tw_ctx::kStageMost);
     *c->err_word = 0;
     for (int s = 0; s < tw_ctx::kStageSlots; ++s)
         if (cudaEventCreateWithFlags(&c->stage_ev[s], cudaEventDisableTiming) != cudaSuccess)
@@ -328,7 +328,6 @@ tw_status tw_ctx_destroy(tw_ctx *ctx)
     for (int s = 0; s < tw_ctx::kStageSlots; ++s)
         if (ctx->stage_ev[s]) cudaEventDestroy(ctx->stage_ev[s]);
     if (ctx->stage_h) cudaFreeHost(ctx->stage_h);
-    if (ctx->err_word) cudaFreeHost(ctx->err_word);
     delete ctx;
     return TW_OK;
 }
@@ -358,11 +357,11 @@ tw_status tw_ctx_synchronize(tw_ctx *ctx)
     return check_kernel_errors(ctx);
 }
 
-// Test hook, not part of the public header: sets how long the solve's CTAs
-// wait at a grid barrier on this context (0 restores the 30 s default) and
-// returns the previous value.  A test shortens it to make the bounded wait
-// give up and checks that the solve reports TW_ERR_TIMEOUT and the context
-// keeps working.
+// Test hook, not part of the public header: sets how long any one wait of the
+// solve's CTAs for a tile, a flag or a buffer may take on this context (0
+// restores the 30 s default) and returns the previous value.  Tests shorten it
+// to make waits give up and check that the solve reports TW_ERR_TIMEOUT and the
+// context keeps working.
 unsigned long long tw_internal_set_solve_barrier_ns(tw_ctx *ctx, unsigned long long ns)
 {
     if (!ctx) return 0;

@@ -24,9 +24,11 @@
 //
 // In each CTA 8 warps compute, one warp fetches tiles ahead of them (bulk
 // copies into a ring of shared-memory buffers, after the flag that publishes
-// each tile) and one warp stores results and publishes them, so neither a
-// flag's round trip nor a store's completion stands on the compute warps'
-// path.  What bounds it: latency up to about 3000 landmarks -- per 64 columns
+// each tile) and one warp stores results and publishes them.  In the chain
+// neither a flag's round trip nor a store's completion stands on the compute
+// warps' path.  A helper's warps all meet between tasks, after its tile is
+// published: there a store's completion, the claim of the next task and that
+// task's first fetch do.  What bounds it: latency up to about 3000 landmarks -- per 64 columns
 // the chain takes some 25,000 cycles (diagonal tile 14,000: 64 dependent
 // pivots, each a reciprocal square root, a product and a multiply-add, and
 // three hand-overs between panels; panel tile's solution 5,000; its product

@@ -206,16 +206,17 @@ struct tw_ctx {
     // pinned staging ring for small host -> device uploads (landmarks, ...)
     static constexpr int kStageSlots = 8;
     static constexpr size_t kStageBytes = (size_t)1 << 20;
+    static constexpr size_t kStageMost = kStageBytes - 64;  // of which an upload may use (the first slot's end holds err_word)
     std::mutex stage_mu;
     unsigned char *stage_h = nullptr;   // pinned, kStageSlots x kStageBytes
     cudaEvent_t stage_ev[kStageSlots] = {};
     int stage_next = 0;
     std::atomic<uint64_t> launches{0};
     std::atomic<uint64_t> h2d_bytes{0}, d2h_bytes{0};  // streamed by the slab and tile paths
-    int *err_word = nullptr;            // pinned host word: kernels OR failure bits into it (kKernErrTimeout)
-    // how long a CTA of the cooperative solve waits at a grid barrier before
-    // it gives up (TW_ERR_TIMEOUT); tests shorten it through
-    // tw_internal_set_solve_barrier_ns
+    int *err_word = nullptr;            // pinned host word (in stage_h: an allocation of its own takes 2 ms): kernels OR failure bits into it (kKernErrTimeout)
+    // how long any one wait of the cooperative solve's CTAs (for a tile, a flag
+    // or a buffer) may take before the CTA gives up (TW_ERR_TIMEOUT); tests
+    // shorten it through tw_internal_set_solve_barrier_ns
     std::atomic<unsigned long long> solve_barrier_ns{30000000000ull};
     // TPS resample units may stage their source footprint in shared memory
     // (TMA); tests turn it off through tw_internal_set_resample_staging to
