@@ -1728,9 +1728,9 @@ __device__ void affine_brick(const RJob &J, int64_t bx, int64_t by, int64_t bz, 
 // memory through L1 the taps hit in it, but a tap load of a rotated row
 // touches a different line every few lanes and takes 7.7 cycles: 124 cycles
 // per 64 voxels at 15 degrees, whatever shape of voxel patch a warp takes.
-// In shared memory the same load takes 2.8 cycles for uint16, 2.2 for uint8,
-// with the densest row pitch that copies allow; pitches that are multiples of
-// 128 bytes conflict more under rotation.)
+// In shared memory the same load takes 2.3 wavefronts for uint16, and 64 voxels
+// 53 cycles; pitches that are multiples of 128 bytes conflict more under
+// rotation.)
 //
 // One CTA per SM, 16 warps that sample (warp w the tile's plane w, two rows of
 // 32 voxels at a time) and four that copy tiles ahead, in up to four stages.
